@@ -1,12 +1,18 @@
-"""ctypes binding of libnvfp4_b200.so (the C ABI declared in include/nvfp4_b200.h).
+"""Bindings of libnvfp4_b200.so (the C ABI declared in include/nvfp4_b200.h).
 
-There is no CPU path: if the library is missing this module raises, it never
-falls back to another implementation.
+Two of them: `fast` holds the functions of the compiled module `_native` (csrc/host/native.cpp), which do the common
+case of an entry point in one call and return None for anything else; `lib()` is the ctypes binding the entry points use
+then, and for everything that is not called per token.  There is no CPU path: if either is missing `lib()` raises, it
+never falls back to another implementation.
 """
 from __future__ import annotations
 
 import ctypes
+import importlib
 import pathlib
+import types
+
+import torch
 
 _PKG = pathlib.Path(__file__).resolve().parent
 LIB_PATH = _PKG / "libnvfp4_b200.so"
@@ -26,6 +32,29 @@ EXPORTS = (
 _lib = None
 
 
+def _not_common(*_args):
+    """Stands for a function of `_native` until that is built: nothing is the common case."""
+    return None
+
+
+fast = types.SimpleNamespace(**{name: _not_common for name in (
+    "quant_impl", "quant_out", "quant_dynamic", "global_scale", "channel_square_norm", "scaled_mm", "scaled_mm_prepared",
+    "scaled_mm_grouped", "make_chain", "chain_call", "make_group", "group_call")})
+
+
+def _bind_native() -> None:
+    importlib.invalidate_caches()
+    native = importlib.import_module("._native", __package__)
+    for name in vars(fast):
+        setattr(fast, name, getattr(native, name))
+
+
+try:
+    _bind_native()
+except ImportError:     # not built yet: lib() says so when something is to be launched
+    pass
+
+
 class Nvfp4Error(RuntimeError):
     """A launch was rejected or failed; `.status` holds the C ABI status code."""
 
@@ -41,6 +70,12 @@ def lib() -> ctypes.CDLL:
             raise RuntimeError(
                 f"{LIB_PATH} is missing: build it with `python -m nvfp4quant_test_b200.build` "
                 "(needs nvcc; there is no CPU fallback)")
+        if fast.quant_impl is _not_common:
+            try:
+                _bind_native()
+            except ImportError as e:
+                raise RuntimeError(f"the compiled module _native does not load ({e}): build it with "
+                                   "`python -m nvfp4quant_test_b200.build`") from e
         L = ctypes.CDLL(str(LIB_PATH))
         i64, ci, vp, f32 = ctypes.c_int64, ctypes.c_int, ctypes.c_void_p, ctypes.c_float
         L.nvfp4_quant_launch.restype = ci
@@ -112,8 +147,6 @@ def check(status: int, what: str) -> None:
 
 
 def dtype_code(dtype) -> int:
-    import torch
-
     try:
         return {torch.bfloat16: DT_BF16, torch.float16: DT_F16, torch.float32: DT_F32}[dtype]
     except KeyError:
@@ -126,8 +159,6 @@ _raw_stream = None
 def current_stream_ptr(device) -> int:
     """cudaStream_t of torch's current stream on `device`, as an integer."""
     global _raw_stream
-    import torch
-
     if _raw_stream is None:
         # the accessor torch's own launchers use: ~0.2 us instead of ~2 us for building a Stream object
         _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", False)
@@ -150,8 +181,6 @@ _NO_GUARD = _NoGuard()
 
 def device_guard(device):
     """Context that makes `device` current for a launch; free when it already is (the usual case)."""
-    import torch
-
     if device.index is None or device.index == torch.cuda.current_device():
         return _NO_GUARD
     return torch.cuda.device(device)
@@ -187,8 +216,6 @@ class StreamScratch:
         self._captures, self._spare = {}, {}
 
     def _zeros(self, device):
-        import torch
-
         return torch.zeros(self.words, dtype=torch.int32, device=device)
 
     def get(self, device, stream: int):

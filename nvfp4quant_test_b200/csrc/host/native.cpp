@@ -1,0 +1,661 @@
+// Host half of the Python entry points: argument checks, output allocation, current stream and launch in one C call.
+//
+// What bounds a small call is the host, not the GPU: a decode-sized quantization runs 2-3 us on the device, while the
+// same checks, two torch.empty, a dtype view and a 15-argument ctypes call cost 13-15 us of interpreter time.  Every
+// function here does the whole common case and returns None for anything else (a wrong shape, a CPU tensor, a strided
+// or misaligned operand, a tensor subclass, a stream under capture where scratch words are needed, a failed launch); the
+// Python entry point then takes its own path, which holds the conversions and all error messages.  So there is one place
+// that decides what an error is, and this file never raises.
+//
+// The kernels are reached through the C ABI of include/nvfp4_b200.h, like from any other caller.
+#include <Python.h>
+
+#include <ATen/core/Tensor.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <ATen/ops/zeros.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <cuda_runtime_api.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <list>
+#include <unordered_map>
+#include <vector>
+
+#include "nvfp4_b200.h"
+
+namespace {
+
+using at::Tensor;
+
+PyTypeObject* g_parameter_type = nullptr;   // torch.nn.Parameter: the one subclass that behaves like a plain tensor
+
+inline int64_t round_up(int64_t x, int64_t y) { return (x + y - 1) / y * y; }
+
+// The tensor behind a plain torch.Tensor or Parameter, NULL for everything else.
+inline const Tensor* tensor_of(PyObject* o) {
+    if (Py_TYPE(o) != reinterpret_cast<PyTypeObject*>(THPVariableClass) && Py_TYPE(o) != g_parameter_type) return nullptr;
+    return &THPVariable_Unpack(o);
+}
+
+inline bool plain_cuda(const Tensor& t) { return t.is_cuda() && t.layout() == at::kStrided; }
+inline uintptr_t address(const Tensor& t) { return reinterpret_cast<uintptr_t>(t.const_data_ptr()); }
+inline bool aligned(const Tensor& t, uintptr_t to) { return (address(t) & (to - 1)) == 0; }
+
+inline int dtype_code(at::ScalarType t) {
+    switch (t) {
+        case at::kBFloat16: return NVFP4_DT_BF16;
+        case at::kHalf: return NVFP4_DT_F16;
+        case at::kFloat: return NVFP4_DT_F32;
+        default: return -1;
+    }
+}
+
+inline cudaStream_t current_stream(c10::DeviceIndex device) { return c10::cuda::getCurrentCUDAStream(device).stream(); }
+
+// Runs `launch` with the tensor's device current and without the interpreter lock (a full launch queue blocks the caller).
+template <class F>
+inline int launch_on(c10::DeviceIndex device, F&& launch) {
+    c10::cuda::OptionalCUDAGuard guard;
+    if (c10::cuda::current_device() != device) guard.set_index(device);
+    int st;
+    Py_BEGIN_ALLOW_THREADS
+    st = launch();
+    Py_END_ALLOW_THREADS
+    return st;
+}
+
+inline Tensor empty(at::IntArrayRef sizes, at::ScalarType dtype, c10::DeviceIndex device) {
+    return at::detail::empty_cuda(sizes, dtype, c10::Device(c10::kCUDA, device), std::nullopt);
+}
+
+// 0-dim view of element `index` of a contiguous float vector, without a trip through the dispatcher.
+inline Tensor scalar_view(const Tensor& v, int64_t index) {
+    Tensor t = at::detail::make_tensor<c10::TensorImpl>(c10::TensorImpl::VIEW, c10::Storage(v.storage()), v.key_set(), v.dtype());
+    t.unsafeGetTensorImpl()->set_storage_offset(v.storage_offset() + index);
+    t.unsafeGetTensorImpl()->set_sizes_contiguous({});
+    return t;
+}
+
+inline PyObject* none() { Py_RETURN_NONE; }
+inline PyObject* truth() { Py_RETURN_TRUE; }
+
+// None or an int; false when it is neither.
+inline bool int_or_none(PyObject* o, int64_t if_none, int64_t* out) {
+    if (o == Py_None) {
+        *out = if_none;
+        return true;
+    }
+    if (!PyLong_CheckExact(o)) return false;
+    *out = PyLong_AsLongLong(o);
+    if (*out == -1 && PyErr_Occurred()) {
+        PyErr_Clear();
+        return false;
+    }
+    return true;
+}
+inline bool as_float(PyObject* o, float* out) {
+    if (!PyFloat_CheckExact(o) && !PyLong_CheckExact(o)) return false;
+    const double d = PyFloat_AsDouble(o);
+    if (d == -1.0 && PyErr_Occurred()) {
+        PyErr_Clear();
+        return false;
+    }
+    *out = static_cast<float>(d);
+    return true;
+}
+inline int small_int(PyObject* o) { return static_cast<int>(PyLong_AsLong(o)); }
+
+PyObject* pack(std::initializer_list<Tensor> ts) {
+    PyObject* t = PyTuple_New(static_cast<Py_ssize_t>(ts.size()));
+    if (!t) return nullptr;
+    Py_ssize_t i = 0;
+    for (const Tensor& x : ts) {
+        PyObject* o = THPVariable_Wrap(x);
+        if (!o) {
+            Py_DECREF(t);
+            return nullptr;
+        }
+        PyTuple_SET_ITEM(t, i++, o);
+    }
+    return t;
+}
+
+// Any C++ exception (a torch check, an allocation failure) becomes "not the common case": the Python path repeats the
+// call and reports it in its own words.
+template <class F>
+inline PyObject* guarded(F&& f) {
+    try {
+        return f();
+    } catch (...) {
+        PyErr_Clear();
+        return none();
+    }
+}
+
+// ---- scratch words of the global-scale kernel -----------------------------------------------------------------------
+// Two zeroed words per (device, stream), left zeroed by every launch; at most 32 streams, least recently used dropped (the
+// block goes back to torch's allocator, which hands it out again in stream order).  Under capture the caller takes the
+// Python path, which keeps a scratch per capture.  Guarded by the interpreter lock, which every caller holds.
+struct ScratchKey {
+    c10::DeviceIndex device;
+    cudaStream_t stream;
+    bool operator==(const ScratchKey& o) const { return device == o.device && stream == o.stream; }
+};
+struct ScratchHash {
+    size_t operator()(const ScratchKey& k) const { return reinterpret_cast<size_t>(k.stream) * 31 + static_cast<size_t>(k.device); }
+};
+constexpr size_t kScratchStreams = 32;
+std::list<std::pair<ScratchKey, Tensor>>& scratch_list() {
+    static auto* l = new std::list<std::pair<ScratchKey, Tensor>>();   // never destroyed: the CUDA context may be gone by then
+    return *l;
+}
+std::unordered_map<ScratchKey, std::list<std::pair<ScratchKey, Tensor>>::iterator, ScratchHash>& scratch_map() {
+    static auto* m = new std::unordered_map<ScratchKey, std::list<std::pair<ScratchKey, Tensor>>::iterator, ScratchHash>();
+    return *m;
+}
+
+uint32_t* scratch_words(c10::DeviceIndex device, cudaStream_t stream) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) {
+        cudaGetLastError();   // e.g. the legacy stream while another stream captures: the Python path decides
+        return nullptr;
+    }
+    if (status != cudaStreamCaptureStatusNone) return nullptr;
+    auto& l = scratch_list();
+    auto& m = scratch_map();
+    const ScratchKey key{device, stream};
+    auto it = m.find(key);
+    if (it != m.end()) {
+        if (it->second != l.begin()) l.splice(l.begin(), l, it->second);
+    } else {
+        Tensor words = at::zeros({2}, at::TensorOptions().dtype(at::kInt).device(c10::Device(c10::kCUDA, device)));
+        l.emplace_front(key, words);
+        m[key] = l.begin();
+        if (l.size() > kScratchStreams) {
+            m.erase(l.back().first);
+            l.pop_back();
+        }
+    }
+    return static_cast<uint32_t*>(l.front().second.mutable_data_ptr());
+}
+
+// ---- quantizers -----------------------------------------------------------------------------------------------------
+
+struct QuantIn {
+    const Tensor* x;
+    const float* importance;
+    int64_t m, n;
+    int dtype;
+    c10::DeviceIndex device;
+};
+
+// The input (and, for the weighted variant, the importance row) as every quantizer entry takes it.
+bool quant_input(PyObject* input, PyObject* importance, QuantIn* q) {
+    const Tensor* x = tensor_of(input);
+    if (!x || !plain_cuda(*x) || x->dim() != 2 || !x->is_contiguous()) return false;
+    q->x = x;
+    q->m = x->size(0);
+    q->n = x->size(1);
+    q->dtype = dtype_code(x->scalar_type());
+    q->device = x->device().index();
+    q->importance = nullptr;
+    if (q->dtype < 0 || q->m <= 0 || q->n <= 0 || q->n % 16 || !aligned(*x, 16)) return false;
+    if (importance != Py_None) {
+        const Tensor* w = tensor_of(importance);
+        if (!w || !plain_cuda(*w) || w->device() != x->device() || w->scalar_type() != at::kFloat || w->dim() != 2 ||
+            w->size(0) != 1 || w->size(1) != q->n || !w->is_contiguous() || !aligned(*w, 16))
+            return false;
+        q->importance = static_cast<const float*>(w->const_data_ptr());
+    }
+    return true;
+}
+
+bool scalar_input(PyObject* o, c10::DeviceIndex device, const float** out) {
+    const Tensor* s = tensor_of(o);
+    if (!s || !plain_cuda(*s) || s->device().index() != device || s->scalar_type() != at::kFloat || s->numel() < 1) return false;
+    *out = static_cast<const float*>(s->const_data_ptr());
+    return true;
+}
+
+// Shapes of vllm's create_fp4_output_tensors, the scale buffer typed float8_e4m3fn as the entry points return it.
+inline Tensor empty_scales(int64_t m, int64_t padded_n, bool tiled, c10::DeviceIndex device) {
+    if (tiled) return empty({round_up(m, 128), round_up(padded_n / 16, 4)}, at::kFloat8_e4m3fn, device);
+    return empty({m, padded_n / 16}, at::kFloat8_e4m3fn, device);
+}
+
+// quant_impl(variant, input, importance | None, input_scale, tiled, padded_n | None, lower, upper) -> (codes, scales)
+PyObject* quant_impl(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+    return guarded([&]() -> PyObject* {
+        if (nargs != 8) return none();
+        QuantIn q;
+        const float* gs_inv;
+        int64_t padded_n;
+        if (!quant_input(a[1], a[2], &q) || !scalar_input(a[3], q.device, &gs_inv) || !PyBool_Check(a[4]) ||
+            !int_or_none(a[5], q.n, &padded_n) || padded_n < q.n || padded_n % 16 || !PyLong_CheckExact(a[6]) || !PyLong_CheckExact(a[7]))
+            return none();
+        const int variant = small_int(a[0]), lower = small_int(a[6]), upper = small_int(a[7]);
+        const bool tiled = a[4] == Py_True;
+        Tensor codes = empty({q.m, padded_n / 2}, at::kByte, q.device);
+        Tensor scales = empty_scales(q.m, padded_n, tiled, q.device);
+        const cudaStream_t s = current_stream(q.device);
+        const int st = launch_on(q.device, [&] {
+            return nvfp4_quant_launch(variant, q.x->const_data_ptr(), q.dtype, q.importance, gs_inv,
+                                      static_cast<uint8_t*>(codes.mutable_data_ptr()), static_cast<uint8_t*>(scales.mutable_data_ptr()),
+                                      q.m, q.n, padded_n, lower, upper, tiled ? 1 : 0, s);
+        });
+        return st == NVFP4_OK ? pack({codes, scales}) : none();
+    });
+}
+
+// quant_out(variant, input, importance | None, input_scale, tiled, output, output_scale, lower, upper) -> True
+PyObject* quant_out(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+    return guarded([&]() -> PyObject* {
+        if (nargs != 9) return none();
+        QuantIn q;
+        const float* gs_inv;
+        if (!quant_input(a[1], a[2], &q) || !scalar_input(a[3], q.device, &gs_inv) || !PyBool_Check(a[4]) || !PyLong_CheckExact(a[7]) ||
+            !PyLong_CheckExact(a[8]))
+            return none();
+        const Tensor *codes = tensor_of(a[5]), *scales = tensor_of(a[6]);
+        if (!codes || !scales || !plain_cuda(*codes) || !plain_cuda(*scales) || codes->device() != q.x->device() ||
+            scales->device() != q.x->device() || codes->scalar_type() != at::kByte || codes->dim() != 2 || codes->size(0) != q.m ||
+            !codes->is_contiguous() || !scales->is_contiguous())
+            return none();
+        const int64_t padded_n = codes->size(1) * 2;
+        if (padded_n % 16 || padded_n < q.n) return none();
+        const bool tiled = a[4] == Py_True;
+        const int64_t need = tiled ? round_up(q.m, 128) * round_up(padded_n / 16, 4) : q.m * (padded_n / 16);
+        if (static_cast<int64_t>(scales->nbytes()) < need) return none();
+        const int variant = small_int(a[0]), lower = small_int(a[7]), upper = small_int(a[8]);
+        const cudaStream_t s = current_stream(q.device);
+        const int st = launch_on(q.device, [&] {
+            return nvfp4_quant_launch(variant, q.x->const_data_ptr(), q.dtype, q.importance, gs_inv,
+                                      static_cast<uint8_t*>(codes->mutable_data_ptr()), static_cast<uint8_t*>(scales->mutable_data_ptr()),
+                                      q.m, q.n, padded_n, lower, upper, tiled ? 1 : 0, s);
+        });
+        return st == NVFP4_OK ? truth() : none();
+    });
+}
+
+// global_scale(x, fp8_max, out | None) -> (global_scale, 1 / global_scale), 0-dim views of one pair
+PyObject* global_scale(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+    return guarded([&]() -> PyObject* {
+        if (nargs != 3) return none();
+        const Tensor* x = tensor_of(a[0]);
+        float fp8_max;
+        if (!x || !plain_cuda(*x) || !x->is_contiguous() || x->numel() == 0 || !aligned(*x, 16) || !as_float(a[1], &fp8_max)) return none();
+        const int dt = dtype_code(x->scalar_type());
+        if (dt < 0) return none();
+        const c10::DeviceIndex dev = x->device().index();
+        Tensor out;
+        if (a[2] == Py_None) {
+            out = empty({2}, at::kFloat, dev);
+        } else {
+            const Tensor* o = tensor_of(a[2]);
+            if (!o || o->device() != x->device() || o->scalar_type() != at::kFloat || o->dim() != 1 || o->size(0) != 2 || !o->is_contiguous())
+                return none();
+            out = *o;
+        }
+        const cudaStream_t s = current_stream(dev);
+        uint32_t* scratch = scratch_words(dev, s);
+        if (!scratch) return none();
+        const int st = launch_on(dev, [&] {
+            return nvfp4_global_scale_launch(x->const_data_ptr(), dt, x->numel(), fp8_max, static_cast<float*>(out.mutable_data_ptr()), scratch, s);
+        });
+        return st == NVFP4_OK ? pack({scalar_view(out, 0), scalar_view(out, 1)}) : none();
+    });
+}
+
+// quant_dynamic(variant, input, importance | None, fp8_max, tiled, padded_n | None, lower, upper)
+//   -> (codes, scales, global_scale, 1 / global_scale): the global scale and the quantizer that reads it, two dependent
+// launches from one call
+PyObject* quant_dynamic(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+    return guarded([&]() -> PyObject* {
+        if (nargs != 8) return none();
+        QuantIn q;
+        float fp8_max;
+        int64_t padded_n;
+        if (!quant_input(a[1], a[2], &q) || !as_float(a[3], &fp8_max) || !PyBool_Check(a[4]) || !int_or_none(a[5], q.n, &padded_n) ||
+            padded_n < q.n || padded_n % 16 || !PyLong_CheckExact(a[6]) || !PyLong_CheckExact(a[7]))
+            return none();
+        const int variant = small_int(a[0]), lower = small_int(a[6]), upper = small_int(a[7]);
+        const bool tiled = a[4] == Py_True;
+        const cudaStream_t s = current_stream(q.device);
+        uint32_t* scratch = scratch_words(q.device, s);
+        if (!scratch) return none();
+        Tensor codes = empty({q.m, padded_n / 2}, at::kByte, q.device);
+        Tensor scales = empty_scales(q.m, padded_n, tiled, q.device);
+        Tensor gs = empty({2}, at::kFloat, q.device);
+        const int st = launch_on(q.device, [&] {
+            return nvfp4_quant_chain_launch(variant, q.x->const_data_ptr(), q.dtype, q.importance, fp8_max,
+                                            static_cast<float*>(gs.mutable_data_ptr()), scratch, static_cast<uint8_t*>(codes.mutable_data_ptr()),
+                                            static_cast<uint8_t*>(scales.mutable_data_ptr()), q.m, q.n, padded_n, lower, upper, tiled ? 1 : 0, s);
+        });
+        return st == NVFP4_OK ? pack({codes, scales, scalar_view(gs, 0), scalar_view(gs, 1)}) : none();
+    });
+}
+
+// channel_square_norm(x, out | None) -> float32 [1, dim]
+PyObject* channel_square_norm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+    return guarded([&]() -> PyObject* {
+        if (nargs != 2) return none();
+        const Tensor* x = tensor_of(a[0]);
+        if (!x || !plain_cuda(*x) || x->dim() != 2 || x->size(1) % 4 || x->size(1) == 0 || !aligned(*x, 16)) return none();
+        const int dt = dtype_code(x->scalar_type());
+        const int64_t m = x->size(0), n = x->size(1);
+        // a column slice of a wider batch is read in place through its row pitch
+        const int64_t ld = m > 1 ? x->stride(0) : n;
+        if (dt < 0 || (m > 1 && (x->stride(1) != 1 || ld < n || ld % 4))) return none();
+        const c10::DeviceIndex dev = x->device().index();
+        Tensor out;
+        if (a[1] == Py_None) {
+            out = empty({1, n}, at::kFloat, dev);
+        } else {
+            const Tensor* o = tensor_of(a[1]);
+            if (!o || o->device() != x->device() || o->scalar_type() != at::kFloat || o->dim() != 2 || o->size(0) != 1 || o->size(1) != n ||
+                !o->is_contiguous())
+                return none();
+            out = *o;
+        }
+        const cudaStream_t s = current_stream(dev);
+        const int st = launch_on(dev, [&] {
+            return nvfp4_channel_sqnorm_launch_strided(x->const_data_ptr(), dt, m, n, ld, static_cast<float*>(out.mutable_data_ptr()), s);
+        });
+        if (st != NVFP4_OK) return none();
+        if (a[1] != Py_None) {
+            Py_INCREF(a[1]);
+            return a[1];
+        }
+        return THPVariable_Wrap(out);
+    });
+}
+
+// ---- GEMM -----------------------------------------------------------------------------------------------------------
+
+inline int64_t scale_bytes(int64_t rows, int64_t k) { return round_up(rows, 128) * round_up(k / 16, 4); }
+
+// Codes uint8 [rows, k/2] and their tiled scales, both contiguous.
+bool quantized_operand(PyObject* codes, PyObject* scales, const Tensor** c, const Tensor** s) {
+    *c = tensor_of(codes);
+    *s = tensor_of(scales);
+    if (!*c || !*s || !plain_cuda(**c) || !plain_cuda(**s) || (*c)->dim() != 2 || (*c)->scalar_type() != at::kByte || !(*c)->is_contiguous() ||
+        !(*s)->is_contiguous() || (*s)->device() != (*c)->device())
+        return false;
+    return static_cast<int64_t>((*s)->nbytes()) >= scale_bytes((*c)->size(0), (*c)->size(1) * 2);
+}
+
+// The caller's output or a fresh one; false when the caller's does not fit.
+bool output_matrix(PyObject* o, int64_t m, int64_t n, c10::DeviceIndex dev, Tensor* out) {
+    if (o == Py_None) {
+        *out = empty({m, n}, at::kBFloat16, dev);
+        return true;
+    }
+    const Tensor* t = tensor_of(o);
+    if (!t || !plain_cuda(*t) || t->device().index() != dev || t->scalar_type() != at::kBFloat16 || t->dim() != 2 || t->size(0) != m ||
+        t->size(1) != n || !t->is_contiguous())
+        return false;
+    *out = *t;
+    return true;
+}
+
+PyObject* output_object(PyObject* given, const Tensor& out) {
+    if (given != Py_None) {
+        Py_INCREF(given);
+        return given;
+    }
+    return THPVariable_Wrap(out);
+}
+
+// scaled_mm(a, b, block_scale_a, block_scale_b, alpha, out | None) -> bf16 [m, n]
+PyObject* scaled_mm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+    return guarded([&]() -> PyObject* {
+        if (nargs != 6) return none();
+        const Tensor *qa, *qb, *sa, *sb;
+        const float* alpha;
+        if (!quantized_operand(a[0], a[2], &qa, &sa) || !quantized_operand(a[1], a[3], &qb, &sb) || qa->device() != qb->device()) return none();
+        const c10::DeviceIndex dev = qa->device().index();
+        const int64_t m = qa->size(0), n = qb->size(0), k = qa->size(1) * 2;
+        Tensor out;
+        if (qb->size(1) * 2 != k || k % 64 || m == 0 || n == 0 || !scalar_input(a[4], dev, &alpha) || !output_matrix(a[5], m, n, dev, &out))
+            return none();
+        const cudaStream_t s = current_stream(dev);
+        const int st = launch_on(dev, [&] {
+            return nvfp4_gemm_launch(static_cast<const uint8_t*>(qa->const_data_ptr()), static_cast<const uint8_t*>(qb->const_data_ptr()),
+                                     static_cast<const uint8_t*>(sa->const_data_ptr()), static_cast<const uint8_t*>(sb->const_data_ptr()), alpha,
+                                     out.mutable_data_ptr(), m, n, k, nullptr, 0, s);
+        });
+        return st == NVFP4_OK ? output_object(a[5], out) : none();
+    });
+}
+
+// A prepared weight as the Python object keeps it for these calls: (handle, n, k, device index).
+struct Weight {
+    void* handle;
+    int64_t n, k;
+    c10::DeviceIndex device;
+};
+bool weight_of(PyObject* t, Weight* w) {
+    if (!PyTuple_CheckExact(t) || PyTuple_GET_SIZE(t) != 4) return false;
+    w->handle = PyLong_AsVoidPtr(PyTuple_GET_ITEM(t, 0));
+    w->n = PyLong_AsLongLong(PyTuple_GET_ITEM(t, 1));
+    w->k = PyLong_AsLongLong(PyTuple_GET_ITEM(t, 2));
+    w->device = static_cast<c10::DeviceIndex>(PyLong_AsLong(PyTuple_GET_ITEM(t, 3)));
+    return w->handle != nullptr && !PyErr_Occurred();
+}
+
+// scaled_mm_prepared(a, block_scale_a, alpha, weight, out | None) -> bf16 [m, n]
+PyObject* scaled_mm_prepared(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+    return guarded([&]() -> PyObject* {
+        if (nargs != 5) return none();
+        const Tensor *qa, *sa;
+        const float* alpha;
+        Weight w;
+        if (!weight_of(a[3], &w) || !quantized_operand(a[0], a[1], &qa, &sa)) {
+            PyErr_Clear();
+            return none();
+        }
+        const c10::DeviceIndex dev = qa->device().index();
+        const int64_t m = qa->size(0);
+        Tensor out;
+        if (w.device != dev || qa->size(1) * 2 != w.k || m == 0 || !scalar_input(a[2], dev, &alpha) || !output_matrix(a[4], m, w.n, dev, &out))
+            return none();
+        const cudaStream_t s = current_stream(dev);
+        const int st = launch_on(dev, [&] {
+            return nvfp4_gemm_launch_prepared(w.handle, static_cast<const uint8_t*>(qa->const_data_ptr()),
+                                              static_cast<const uint8_t*>(sa->const_data_ptr()), alpha, out.mutable_data_ptr(), m, nullptr, 0, s);
+        });
+        return st == NVFP4_OK ? output_object(a[4], out) : none();
+    });
+}
+
+// scaled_mm_grouped(a, block_scale_a, alpha_a | None, [weight], [alpha_w], [out] | None) -> [bf16 [m, n_i]]
+PyObject* scaled_mm_grouped(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+    return guarded([&]() -> PyObject* {
+        if (nargs != 6 || !PyList_CheckExact(a[3]) || !PyList_CheckExact(a[4]) || (a[5] != Py_None && !PyList_CheckExact(a[5]))) return none();
+        const Py_ssize_t count = PyList_GET_SIZE(a[3]);
+        if (count < 1 || count > 64 || PyList_GET_SIZE(a[4]) != count || (a[5] != Py_None && PyList_GET_SIZE(a[5]) != count)) return none();
+        const Tensor *qa, *sa;
+        if (!quantized_operand(a[0], a[1], &qa, &sa)) return none();
+        const c10::DeviceIndex dev = qa->device().index();
+        const int64_t m = qa->size(0), k = qa->size(1) * 2;
+        const float* alpha_a = nullptr;
+        if (m == 0 || (a[2] != Py_None && !scalar_input(a[2], dev, &alpha_a))) return none();
+        void *handles[64], *outs[64];
+        const float* alphas[64];
+        std::vector<Tensor> out(static_cast<size_t>(count));
+        for (Py_ssize_t i = 0; i < count; ++i) {
+            Weight w;
+            if (!weight_of(PyList_GET_ITEM(a[3], i), &w) || w.device != dev || w.k != k ||
+                !scalar_input(PyList_GET_ITEM(a[4], i), dev, &alphas[i]) ||
+                !output_matrix(a[5] == Py_None ? Py_None : PyList_GET_ITEM(a[5], i), m, w.n, dev, &out[i])) {
+                PyErr_Clear();
+                return none();
+            }
+            handles[i] = w.handle;
+            outs[i] = out[i].mutable_data_ptr();
+        }
+        const cudaStream_t s = current_stream(dev);
+        const int st = launch_on(dev, [&] {
+            return nvfp4_gemm_launch_grouped(handles, static_cast<int>(count), static_cast<const uint8_t*>(qa->const_data_ptr()),
+                                             static_cast<const uint8_t*>(sa->const_data_ptr()), alpha_a, alphas, outs, m, s);
+        });
+        if (st != NVFP4_OK) return none();
+        if (a[5] != Py_None) {
+            Py_INCREF(a[5]);
+            return a[5];
+        }
+        PyObject* l = PyList_New(count);
+        for (Py_ssize_t i = 0; l && i < count; ++i) {
+            PyObject* o = THPVariable_Wrap(out[i]);
+            if (!o) {
+                Py_DECREF(l);
+                return nullptr;
+            }
+            PyList_SET_ITEM(l, i, o);
+        }
+        return l;
+    });
+}
+
+// ---- preallocated decode blocks -------------------------------------------------------------------------------------
+// What kernels/linear.py checks and builds once: addresses and sizes of buffers that the Python object owns and keeps.
+
+struct Chain {   // global scale -> quantizer of an activation [m, n]
+    int dtype, variant, lower, upper;
+    c10::DeviceIndex device;
+    float fp8_max;
+    float* gs;
+    uint32_t* scratch;
+    uint8_t *codes, *scales;
+    int64_t m, n;
+};
+struct Group {   // one activation against several prepared weights
+    c10::DeviceIndex device;
+    int64_t m, k;
+    std::vector<void*> handles, outs;
+    std::vector<const float*> alphas;
+};
+constexpr const char* kChainName = "nvfp4.chain";
+constexpr const char* kGroupName = "nvfp4.group";
+
+void free_chain(PyObject* c) { delete static_cast<Chain*>(PyCapsule_GetPointer(c, kChainName)); }
+void free_group(PyObject* c) { delete static_cast<Group*>(PyCapsule_GetPointer(c, kGroupName)); }
+
+// make_chain(dtype code, variant, device index, fp8_max, gs ptr, scratch ptr, codes ptr, scales ptr, m, n, lower, upper)
+PyObject* make_chain(PyObject*, PyObject* args) {
+    Chain c;
+    int dev;
+    Py_ssize_t gs, scratch, codes, scales, m, n;
+    if (!PyArg_ParseTuple(args, "iiifnnnnnnii", &c.dtype, &c.variant, &dev, &c.fp8_max, &gs, &scratch, &codes, &scales, &m, &n, &c.lower, &c.upper))
+        return nullptr;
+    c.device = static_cast<c10::DeviceIndex>(dev);
+    c.gs = reinterpret_cast<float*>(gs);
+    c.scratch = reinterpret_cast<uint32_t*>(scratch);
+    c.codes = reinterpret_cast<uint8_t*>(codes);
+    c.scales = reinterpret_cast<uint8_t*>(scales);
+    c.m = m;
+    c.n = n;
+    return PyCapsule_New(new Chain(c), kChainName, free_chain);
+}
+
+// make_group(device index, m, k, (handle, ...), (alpha ptr, ...), (out ptr, ...))
+PyObject* make_group(PyObject*, PyObject* args) {
+    int dev;
+    Py_ssize_t m, k;
+    PyObject *handles, *alphas, *outs;
+    if (!PyArg_ParseTuple(args, "innO!O!O!", &dev, &m, &k, &PyTuple_Type, &handles, &PyTuple_Type, &alphas, &PyTuple_Type, &outs)) return nullptr;
+    const Py_ssize_t n = PyTuple_GET_SIZE(handles);
+    if (PyTuple_GET_SIZE(alphas) != n || PyTuple_GET_SIZE(outs) != n) {
+        PyErr_SetString(PyExc_ValueError, "handles, alphas and outs must have the same length");
+        return nullptr;
+    }
+    Group* g = new Group();
+    g->device = static_cast<c10::DeviceIndex>(dev);
+    g->m = m;
+    g->k = k;
+    for (Py_ssize_t i = 0; i < n; ++i) {
+        g->handles.push_back(PyLong_AsVoidPtr(PyTuple_GET_ITEM(handles, i)));
+        g->alphas.push_back(static_cast<const float*>(PyLong_AsVoidPtr(PyTuple_GET_ITEM(alphas, i))));
+        g->outs.push_back(PyLong_AsVoidPtr(PyTuple_GET_ITEM(outs, i)));
+    }
+    if (PyErr_Occurred()) {
+        delete g;
+        return nullptr;
+    }
+    return PyCapsule_New(g, kGroupName, free_group);
+}
+
+// chain_call(chain, x) -> True
+PyObject* chain_call(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+    return guarded([&]() -> PyObject* {
+        if (nargs != 2) return none();
+        const Chain* c = static_cast<const Chain*>(PyCapsule_GetPointer(a[0], kChainName));
+        const Tensor* x = tensor_of(a[1]);
+        if (!c || !x || !plain_cuda(*x) || x->device().index() != c->device || dtype_code(x->scalar_type()) != c->dtype || x->dim() != 2 ||
+            x->size(0) != c->m || x->size(1) != c->n || !x->is_contiguous() || !aligned(*x, 16)) {
+            PyErr_Clear();
+            return none();
+        }
+        const cudaStream_t s = current_stream(c->device);
+        const int st = launch_on(c->device, [&] {
+            return nvfp4_quant_chain_launch(c->variant, x->const_data_ptr(), c->dtype, nullptr, c->fp8_max, c->gs, c->scratch, c->codes,
+                                            c->scales, c->m, c->n, c->n, c->lower, c->upper, 1, s);
+        });
+        return st == NVFP4_OK ? truth() : none();
+    });
+}
+
+// group_call(group, codes, scales, alpha_a | None) -> True
+PyObject* group_call(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+    return guarded([&]() -> PyObject* {
+        if (nargs != 4) return none();
+        const Group* g = static_cast<const Group*>(PyCapsule_GetPointer(a[0], kGroupName));
+        const Tensor *qa, *sa;
+        const float* alpha_a = nullptr;
+        if (!g || !quantized_operand(a[1], a[2], &qa, &sa) || qa->device().index() != g->device || qa->size(0) != g->m ||
+            qa->size(1) * 2 != g->k || (a[3] != Py_None && !scalar_input(a[3], g->device, &alpha_a))) {
+            PyErr_Clear();
+            return none();
+        }
+        const cudaStream_t s = current_stream(g->device);
+        const int st = launch_on(g->device, [&] {
+            return nvfp4_gemm_launch_grouped(g->handles.data(), static_cast<int>(g->handles.size()), static_cast<const uint8_t*>(qa->const_data_ptr()),
+                                             static_cast<const uint8_t*>(sa->const_data_ptr()), alpha_a, g->alphas.data(), g->outs.data(), g->m, s);
+        });
+        return st == NVFP4_OK ? truth() : none();
+    });
+}
+
+#define FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(name)), METH_FASTCALL, nullptr}
+PyMethodDef kMethods[] = {
+    FAST(quant_impl),
+    FAST(quant_out),
+    FAST(quant_dynamic),
+    FAST(global_scale),
+    FAST(channel_square_norm),
+    FAST(scaled_mm),
+    FAST(scaled_mm_prepared),
+    FAST(scaled_mm_grouped),
+    FAST(chain_call),
+    FAST(group_call),
+    {"make_chain", make_chain, METH_VARARGS, nullptr},
+    {"make_group", make_group, METH_VARARGS, nullptr},
+    {nullptr, nullptr, 0, nullptr},
+};
+#undef FAST
+
+PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_native", "Host half of the entry points (None = not the common case).", -1, kMethods,
+                       nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__native(void) {
+    PyObject* nn = PyImport_ImportModule("torch.nn");
+    if (!nn) return nullptr;
+    PyObject* parameter = PyObject_GetAttrString(nn, "Parameter");
+    Py_DECREF(nn);
+    if (!parameter) return nullptr;
+    g_parameter_type = reinterpret_cast<PyTypeObject*>(parameter);   // kept for the life of the process
+    return PyModule_Create(&kModule);
+}

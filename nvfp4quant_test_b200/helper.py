@@ -20,6 +20,9 @@ _scratch = _lib.StreamScratch(2)
 def get_nvfp4_global_scale(x: torch.Tensor, FP8_MAX: float = FP8_E4M3_MAX_NVFP4, out: torch.Tensor | None = None):
     """(global_scale, global_scale_inv) as 0-dim float32 CUDA tensors; amax(|x|)/(6*FP8_MAX) and its reciprocal.
     `out` (optional): a contiguous float32 [2] CUDA tensor to write them into instead of a fresh one."""
+    got = _lib.fast.global_scale(x, FP8_MAX, out)
+    if got is not None:
+        return got
     if not x.is_cuda:
         raise ValueError("x must be a CUDA tensor")
     if out is not None and (out.dtype != torch.float32 or out.device != x.device or out.shape != (2,)
@@ -47,6 +50,9 @@ def channel_square_norm(x: torch.Tensor, out: torch.Tensor | None = None) -> tor
     """fp32 [1, dim]: squared L2 norm of every input channel (column) of the 2-D batch x - the importance
     vector for the operand x is multiplied with (README.md:11 of the reference).  `out` (optional): a contiguous
     float32 [1, dim] CUDA tensor to write into."""
+    got = _lib.fast.channel_square_norm(x, out)
+    if got is not None:
+        return got
     if x.ndim != 2 or not x.is_cuda:
         raise ValueError("x must be a 2D CUDA tensor")
     if out is not None and (out.dtype != torch.float32 or out.device != x.device or out.shape != (1, x.shape[1])

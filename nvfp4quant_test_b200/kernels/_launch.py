@@ -80,6 +80,9 @@ def quant_out(variant: int, input: torch.Tensor, importance: torch.Tensor | None
               is_sf_swizzled_layout: bool, output: torch.Tensor, output_scale: torch.Tensor,
               lower: int, upper: int, impl: int = 0) -> None:
     """Validate, then launch on the current stream of input.device.  Writes output / output_scale in place."""
+    if impl == 0 and _lib.fast.quant_out(variant, input, importance, input_scale, is_sf_swizzled_layout, output,
+                                         output_scale, lower, upper):
+        return
     _check_common(input, input_scale)
     if not input.is_contiguous():
         input = input.contiguous()

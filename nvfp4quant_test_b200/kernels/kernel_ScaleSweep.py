@@ -43,6 +43,11 @@ def scalesweep_weighted_mse_nvfp4_quant_impl(
     lower_bound: int = LOWER_BOUND,
     upper_bound: int = UPPER_BOUND,
 ) -> tuple[torch.Tensor, torch.Tensor]:
+    if importance is not None:      # None would be the unweighted call of the compiled module
+        got = _lib.fast.quant_impl(_lib.VARIANT_WEIGHTED, input, importance, input_scale, is_sf_swizzled_layout, padded_n,
+                                   lower_bound, upper_bound)
+        if got is not None:
+            return got
     check_importance(input, importance)
     m, n = input.shape
     output, output_scale = create_fp4_output_tensors(m, n, input.device, is_sf_swizzled_layout, padded_n=padded_n)

@@ -44,6 +44,10 @@ def scalesweep_mse_nvfp4_quant_impl(
     padded_n: int | None = None,
 ) -> tuple[torch.Tensor, torch.Tensor]:
     """Returns (codes uint8 [m, P/2], scales float8_e4m3fn) with P = padded_n or n."""
+    got = _lib.fast.quant_impl(_lib.VARIANT_MSE, input, None, input_scale, is_sf_swizzled_layout, padded_n, LOWER_BOUND,
+                               UPPER_BOUND)
+    if got is not None:
+        return got
     if input.ndim != 2:
         raise ValueError(f"input must be 2D [num_row, dim], got {tuple(input.shape)}")
     m, n = input.shape

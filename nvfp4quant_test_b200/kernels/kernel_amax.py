@@ -19,6 +19,9 @@ def amax_nvfp4_quant_out(input, input_scale, is_sf_swizzled_layout: bool = True,
 
 def amax_nvfp4_quant_impl(input: torch.Tensor, input_scale: torch.Tensor, is_sf_swizzled_layout: bool = True,
                           padded_n: int | None = None) -> tuple[torch.Tensor, torch.Tensor]:
+    got = _lib.fast.quant_impl(_lib.VARIANT_AMAX, input, None, input_scale, is_sf_swizzled_layout, padded_n, 0, 0)
+    if got is not None:
+        return got
     if input.ndim != 2:
         raise ValueError(f"input must be 2D [num_row, dim], got {tuple(input.shape)}")
     m, n = input.shape

@@ -2,9 +2,9 @@
 
 The reference computes the tensor-wide scale first (`get_nvfp4_global_scale`, helper.py:96-100 of
 efsotr/nvfp4quant_test) and hands its reciprocal to the quantizer (bench.py:57-67): two passes over the tensor
-and two launches.  For tensors that fit the GPU's resident grid (about 3 M elements on a B200: activations of up
-to a few hundred tokens) both happen in one launch here, with the tensor read once; larger tensors take the two
-launches.  Bytes and scales are identical either way.
+and two launches.  Here it is one host call that issues two dependent launches.  While a stream is being captured into a
+graph, tensors that fit the GPU's resident grid (about 3 M elements on a B200) become one cooperative launch instead, one
+node that reads the tensor once.  Bytes and scales are identical either way.
 """
 from __future__ import annotations
 
@@ -31,6 +31,16 @@ def scalesweep_nvfp4_quant_with_global_scale(
     """(codes, scales, global_scale, global_scale_inv).  Without `importance` this is ScaleSweep_MSE (window
     -3..+7), with it the importance-weighted ScaleSweep (window -8..+7 unless given); the two scale tensors are
     0-dim float32 views, as `get_nvfp4_global_scale` returns them."""
+    if importance is None:
+        got = _lib.fast.quant_dynamic(_lib.VARIANT_MSE, input, None, fp8_max, is_sf_swizzled_layout, padded_n,
+                                      _mse.LOWER_BOUND if lower_bound is None else lower_bound,
+                                      _mse.UPPER_BOUND if upper_bound is None else upper_bound)
+    else:
+        got = _lib.fast.quant_dynamic(_lib.VARIANT_WEIGHTED, input, importance, fp8_max, is_sf_swizzled_layout, padded_n,
+                                      _weighted.LOWER_BOUND if lower_bound is None else lower_bound,
+                                      _weighted.UPPER_BOUND if upper_bound is None else upper_bound)
+    if got is not None:
+        return got
     if input.ndim != 2:
         raise ValueError(f"input must be 2D [num_row, dim], got {tuple(input.shape)}")
     if importance is None:

@@ -20,6 +20,10 @@ def _scale_bytes(rows: int, k: int) -> int:
 def nvfp4_scaled_mm(a: torch.Tensor, b: torch.Tensor, block_scale_a: torch.Tensor, block_scale_b: torch.Tensor,
                     alpha: torch.Tensor, out_dtype: torch.dtype = torch.bfloat16,
                     out: torch.Tensor | None = None) -> torch.Tensor:
+    if out_dtype is torch.bfloat16:
+        got = _lib.fast.scaled_mm(a, b, block_scale_a, block_scale_b, alpha, out)
+        if got is not None:
+            return got
     if a.ndim != 2 or b.ndim != 2:
         raise ValueError("a and b must be 2D [rows, K/2] uint8 tensors")
     if a.dtype != torch.uint8 or b.dtype != torch.uint8:
@@ -93,11 +97,12 @@ class PreparedWeight:
         with _lib.device_guard(b.device):
             st = _lib.lib().nvfp4_gemm_prepare(b.data_ptr(), block_scale_b.data_ptr(), self.n, self.k, ctypes.byref(self._handle))
         _lib.check(st, "nvfp4_gemm_prepare")
+        self._fast = (self._handle.value, self.n, self.k, b.device.index)   # the form the compiled calls take
 
     def close(self) -> None:
         if getattr(self, "_handle", None):
             _lib.lib().nvfp4_gemm_release(self._handle)
-            self._handle = None
+            self._handle = self._fast = None
 
     def __del__(self):
         try:
@@ -109,6 +114,9 @@ class PreparedWeight:
 def nvfp4_scaled_mm_prepared(a: torch.Tensor, block_scale_a: torch.Tensor, alpha: torch.Tensor, weight: PreparedWeight,
                              out: torch.Tensor | None = None) -> torch.Tensor:
     """out[M, N] (bf16) = alpha * dq(a) @ dq(weight).T; same bits as nvfp4_scaled_mm(a, weight.b, ...)."""
+    got = _lib.fast.scaled_mm_prepared(a, block_scale_a, alpha, weight._fast, out)
+    if got is not None:
+        return got
     if a.ndim != 2 or a.dtype != torch.uint8 or a.device != weight.device:
         raise ValueError("a must be a uint8 [M, K/2] tensor on the weight's device")
     if a.shape[1] * 2 != weight.k:
@@ -152,6 +160,9 @@ def nvfp4_scaled_mm_grouped(a: torch.Tensor, block_scale_a: torch.Tensor, alpha_
     the kernel.  At decode-sized M the whole group is one launch (nvfp4_gemm_launch_grouped)."""
     import ctypes
 
+    got = _lib.fast.scaled_mm_grouped(a, block_scale_a, alpha_a, [w._fast for w in weights], alpha_w, outs)
+    if got is not None:
+        return got
     n = len(weights)
     if n == 0:
         return []

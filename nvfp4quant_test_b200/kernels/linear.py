@@ -39,9 +39,17 @@ class ActivationQuantizer:
         self._args = (self.global_scale.data_ptr(), self._scratch.data_ptr(), self.codes.data_ptr(), scales.data_ptr(),
                       tokens, k, k, _mse.LOWER_BOUND, _mse.UPPER_BOUND, 1)
         self._scales_storage = scales
+        self._result = (self.codes, self.scales, self.global_scale[0:1])
+        self._chain = None
+        if self.device.type == "cuda":
+            self._chain = _lib.fast.make_chain(
+                self._dtype_code, _lib.VARIANT_MSE, self.device.index, self.fp8_max, self.global_scale.data_ptr(),
+                self._scratch.data_ptr(), self.codes.data_ptr(), scales.data_ptr(), tokens, k, _mse.LOWER_BOUND, _mse.UPPER_BOUND)
 
     def __call__(self, x: torch.Tensor):
         """Returns (codes, scales, global_scale[0:1]); the three tensors are this object's buffers."""
+        if _lib.fast.chain_call(self._chain, x):
+            return self._result
         if x.shape != (self.tokens, self.k) or x.dtype != self.dtype or x.device != self.device or not x.is_contiguous():
             raise ValueError(f"x must be a contiguous {self.dtype} [{self.tokens}, {self.k}] tensor on {self.device}")
         if x.data_ptr() & 15:
@@ -50,7 +58,7 @@ class ActivationQuantizer:
             st = _lib.lib().nvfp4_quant_chain_launch(_lib.VARIANT_MSE, x.data_ptr(), self._dtype_code, None, self.fp8_max,
                                                      *self._args, _lib.current_stream_ptr(self.device))
         _lib.check(st, "nvfp4_quant_chain_launch")
-        return self.codes, self.scales, self.global_scale[0:1]
+        return self._result
 
 
 class LinearGroup:
@@ -74,10 +82,16 @@ class LinearGroup:
         self._outs = (ctypes.c_void_p * n)(*[o.data_ptr() for o in self.outs])
         self._n = n
         self._min_scale_bytes = _scale_bytes(tokens, self.k)
+        self._group = None
+        if self.device.type == "cuda":
+            self._group = _lib.fast.make_group(self.device.index, tokens, self.k, tuple(w._handle.value for w in weights),
+                                               tuple(s.data_ptr() for s in weight_scales), tuple(o.data_ptr() for o in self.outs))
 
     def __call__(self, codes: torch.Tensor, scales: torch.Tensor, alpha_a: torch.Tensor | None):
         """codes / scales: the quantized activation [tokens, K/2] and its tiled scales; alpha_a: its global scale (one
         float32 on the device) or None.  Returns this object's output tensors."""
+        if _lib.fast.group_call(self._group, codes, scales, alpha_a):
+            return self.outs
         if (codes.shape != (self.tokens, self.k // 2) or codes.dtype != torch.uint8 or codes.device != self.device
                 or not codes.is_contiguous()):
             raise ValueError(f"codes must be a contiguous uint8 [{self.tokens}, {self.k // 2}] tensor on {self.device}")

@@ -1,0 +1,122 @@
+"""GPU: the compiled half of the entry points gives what the Python path gives, and hands over what it does not cover."""
+import types
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def python_path(cuda_lib, monkeypatch):
+    """Switches the compiled functions off for the calls made inside `with`."""
+    import contextlib
+
+    from nvfp4quant_test_b200 import _lib
+
+    @contextlib.contextmanager
+    def off():
+        with monkeypatch.context() as mp:
+            mp.setattr(_lib, "fast", types.SimpleNamespace(**{k: _lib._not_common for k in vars(_lib.fast)}))
+            yield
+
+    return off
+
+
+def _flat(v):
+    return [t for x in v for t in _flat(x)] if isinstance(v, (tuple, list)) else [v]
+
+
+def _same(got, want):
+    got, want = _flat(got), _flat(want)
+    assert len(got) == len(want)
+    for g, w in zip(got, want):
+        assert g.shape == w.shape and g.dtype == w.dtype and g.device == w.device and g.is_contiguous() == w.is_contiguous()
+        assert torch.equal(g.contiguous().reshape(-1).view(torch.uint8), w.contiguous().reshape(-1).view(torch.uint8))
+
+
+def _calls(m, n, dtype, tiled, padded_n):
+    import nvfp4quant_test_b200.kernels as K
+    from nvfp4quant_test_b200 import helper as H
+
+    g = torch.Generator(device="cuda").manual_seed(m * 31 + n)
+    x = torch.randn((m, n), generator=g, device="cuda").to(dtype)
+    imp = torch.rand((1, n), generator=g, device="cuda")
+    gs_inv = H.get_nvfp4_global_scale(x, 256.0)[1]
+    wide = torch.randn((m, n + 16), generator=g, device="cuda").to(dtype)
+    yield lambda: H.get_nvfp4_global_scale(x, 448.0)
+    yield lambda: H.channel_square_norm(x)
+    yield lambda: H.channel_square_norm(wide[:, 16:])
+    yield lambda: K.scalesweep_mse_nvfp4_quant_impl(x, gs_inv, tiled, padded_n)
+    yield lambda: K.scalesweep_weighted_mse_nvfp4_quant_impl(x, imp, gs_inv, tiled, padded_n)
+    yield lambda: K.scalesweep_weighted_mse_nvfp4_quant_impl(x, imp.half(), gs_inv, tiled, padded_n)      # converted in Python
+    yield lambda: K.amax_nvfp4_quant_impl(x, gs_inv, tiled, padded_n)
+    yield lambda: K.scalesweep_nvfp4_quant_with_global_scale(x, 256.0, None, tiled, padded_n)
+    yield lambda: K.scalesweep_nvfp4_quant_with_global_scale(x, 256.0, imp, tiled, padded_n, lower_bound=-2, upper_bound=3)
+    yield lambda: K.scalesweep_mse_nvfp4_quant_impl(wide[:, :n], gs_inv, tiled, padded_n)                 # strided
+    yield lambda: K.scalesweep_mse_nvfp4_quant_impl(torch.nn.Parameter(x), gs_inv, tiled, padded_n)
+
+
+@pytest.mark.parametrize("m,n,dtype,tiled,padded_n", [
+    (1, 16, torch.bfloat16, True, None), (3, 8192, torch.bfloat16, True, None), (129, 208, torch.float16, True, 256),
+    (5, 48, torch.float32, False, None), (77, 4096, torch.bfloat16, False, 4160)])
+def test_compiled_calls_equal_the_python_path(python_path, m, n, dtype, tiled, padded_n):
+    for call in _calls(m, n, dtype, tiled, padded_n):
+        got = call()
+        with python_path():
+            want = call()
+        _same(got, want)
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 128, 64), (16, 72, 320), (130, 257, 512)])
+def test_compiled_gemm_calls_equal_the_python_path(python_path, m, n, k):
+    import nvfp4quant_test_b200.kernels as K
+    from nvfp4quant_test_b200 import helper as H
+
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    x = torch.randn((m, k), generator=g, device="cuda").bfloat16()
+    w = torch.randn((n, k), generator=g, device="cuda").bfloat16()
+    (gx, ix), (gw, iw) = H.get_nvfp4_global_scale(x), H.get_nvfp4_global_scale(w)
+    qx, sx = K.scalesweep_mse_nvfp4_quant_impl(x, ix)
+    qw, sw = K.scalesweep_mse_nvfp4_quant_impl(w, iw)
+    pw, alpha = K.PreparedWeight(qw, sw), (gx * gw).reshape(1)
+    out = torch.empty((m, n), dtype=torch.bfloat16, device="cuda")
+    calls = [lambda: K.nvfp4_scaled_mm(qx, qw, sx, sw, alpha, torch.bfloat16),
+             lambda: K.nvfp4_scaled_mm(qx, qw, sx, sw, alpha, torch.bfloat16, out),
+             lambda: K.nvfp4_scaled_mm_prepared(qx, sx, alpha, pw),
+             lambda: K.nvfp4_scaled_mm_grouped(qx, sx, gx.reshape(1), [pw, pw], [gw.reshape(1), gw.reshape(1)]),
+             lambda: K.LinearGroup([pw], [gw.reshape(1)], m)(qx, sx, gx.reshape(1)),
+             lambda: K.ActivationQuantizer(m, k, "cuda")(x)]
+    for call in calls:
+        got = [t.clone() for t in _flat(call())]
+        with python_path():
+            want = call()
+        _same(got, want)
+    assert K.nvfp4_scaled_mm(qx, qw, sx, sw, alpha, torch.bfloat16, out) is out
+    pw.close()
+    with pytest.raises(ValueError, match="closed"):
+        K.nvfp4_scaled_mm_prepared(qx, sx, alpha, pw)
+    with pytest.raises(ValueError, match="disagree on K"):
+        K.nvfp4_scaled_mm(qx[:, : k // 2 - 32].contiguous(), qw, sx, sw, alpha, torch.bfloat16)
+
+
+def test_compiled_calls_use_the_current_stream_and_record_into_a_graph(cuda_lib):
+    import nvfp4quant_test_b200.kernels as K
+    from nvfp4quant_test_b200 import helper as H
+
+    x = torch.randn((64, 4096), device="cuda").bfloat16()
+    want = K.scalesweep_nvfp4_quant_with_global_scale(x, 256.0)
+    streams = [torch.cuda.Stream() for _ in range(40)]      # more than scratch words are kept for
+    for s in streams:
+        s.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(s):
+            got = K.scalesweep_nvfp4_quant_with_global_scale(x, 256.0)
+        s.synchronize()
+        _same(got, want)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        gs, gs_inv = H.get_nvfp4_global_scale(x, 256.0)
+        q = K.scalesweep_mse_nvfp4_quant_impl(x, gs_inv)
+    graph.replay()
+    torch.cuda.synchronize()
+    _same(q, want[:2])
