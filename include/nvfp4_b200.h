@@ -259,6 +259,17 @@ int nvfp4_gemm_last_status(void* stream, uint32_t* status_host);
 int nvfp4_gemm_set_wait_limit_ns(uint64_t ns);
 int nvfp4_quant_fused_set_wait_limit_ns(uint64_t ns);
 
+/* out[m, n] (fp32) = (code * block scale) * *gs: the inverse of the quantizers, scales row-major [m, n/16] (n % 16 == 0).
+ * scales == NULL: the bare E2M1 values (gs unused, n % 8 == 0).  codes 4-byte, out 32-byte aligned.
+ * replaces helper.py:103-147 (unpack_fp4_e2m1, dequantize_base). */
+int nvfp4_dequant_launch(const uint8_t* codes, const uint8_t* scales, const float* gs, float* out, int64_t m, int64_t n,
+                         void* stream);
+
+/* Scale bytes of an [m, 16 k] tensor from row-major [m, k] to the tiled layout (to_tiled != 0; padding is written as zero)
+ * or back.  The tiled buffer is 16-byte aligned, the row-major one 4-byte aligned where k % 4 == 0.
+ * replaces kernels/kernel_vllm.py:29-70 (swizzle_vllm_fp4_scale, unswizzle_vllm_fp4_scale). */
+int nvfp4_scale_layout_launch(const uint8_t* src, uint8_t* dst, int64_t m, int64_t k, int to_tiled, void* stream);
+
 /* *id_host = 0 while `stream` is not being captured into a CUDA graph, else the id of the capture.  Host bookkeeping: the
  * scratch words of nvfp4_global_scale_launch / nvfp4_quant_fused_launch may be shared by launches that are ordered on one
  * stream, but graphs captured one after the other on the same stream can be replayed at the same time on different

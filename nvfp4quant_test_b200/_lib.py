@@ -26,7 +26,8 @@ EXPORTS = (
     "nvfp4_global_scale_launch", "nvfp4_global_scale_launch_static", "nvfp4_global_scale_static_max_bytes",
     "nvfp4_channel_sqnorm_launch", "nvfp4_channel_sqnorm_launch_strided", "nvfp4_gemm_peak_probe", "nvfp4_gemm_set_wait_limit_ns", "nvfp4_quant_fused_set_wait_limit_ns",
     "nvfp4_gemm_launch", "nvfp4_gemm_workspace_bytes", "nvfp4_gemm_prepare", "nvfp4_gemm_launch_prepared", "nvfp4_gemm_launch_grouped", "nvfp4_gemm_release", "nvfp4_gemm_last_status", "nvfp4_gemm_force_path", "nvfp4_gemm_tune", "nvfp4_gemm_tune_raster", "nvfp4_gemm_tune_pdl", "nvfp4_gemm_plan",
-    "nvfp4_status_string", "nvfp4_abi_version", "nvfp4_stream_capture_id",
+    "nvfp4_status_string", "nvfp4_abi_version", "nvfp4_stream_capture_id", "nvfp4_dequant_launch",
+    "nvfp4_scale_layout_launch",
 )
 
 _lib = None
@@ -39,14 +40,16 @@ def _not_common(*_args):
 
 fast = types.SimpleNamespace(**{name: _not_common for name in (
     "quant_impl", "quant_out", "quant_dynamic", "global_scale", "channel_square_norm", "scaled_mm", "scaled_mm_prepared",
-    "scaled_mm_grouped", "make_chain", "chain_call", "make_group", "group_call")})
+    "scaled_mm_grouped", "dequant", "scale_layout", "make_chain", "chain_call", "make_group", "group_call")})
 
 
 def _bind_native() -> None:
     importlib.invalidate_caches()
     native = importlib.import_module("._native", __package__)
-    for name in vars(fast):
-        setattr(fast, name, getattr(native, name))
+    missing = [name for name in vars(fast) if not hasattr(native, name)]
+    if missing:
+        raise ImportError(f"_native is older than the package (no {', '.join(missing)})")
+    vars(fast).update({name: getattr(native, name) for name in vars(fast)})
 
 
 try:
@@ -110,6 +113,10 @@ def lib() -> ctypes.CDLL:
         L.nvfp4_gemm_prepare.argtypes = [vp, vp, i64, i64, vp]
         L.nvfp4_gemm_launch_prepared.restype = ci
         L.nvfp4_gemm_launch_prepared.argtypes = [vp, vp, vp, vp, vp, i64, vp, ctypes.c_size_t, vp]
+        L.nvfp4_dequant_launch.restype = ci
+        L.nvfp4_dequant_launch.argtypes = [vp, vp, vp, vp, i64, i64, vp]
+        L.nvfp4_scale_layout_launch.restype = ci
+        L.nvfp4_scale_layout_launch.argtypes = [vp, vp, i64, i64, ci, vp]
         L.nvfp4_stream_capture_id.restype = ci
         L.nvfp4_stream_capture_id.argtypes = [vp, vp]
         L.nvfp4_gemm_launch_grouped.restype = ci

@@ -18,7 +18,7 @@ LIB = PKG / "libnvfp4_b200.so"
 NATIVE_SRC = CSRC / "host" / "native.cpp"
 NATIVE = PKG / ("_native" + sysconfig.get_config_var("EXT_SUFFIX"))
 
-SOURCES = ["quant.cu", "global_scale.cu", "global_scale_static.cu", "importance.cu", "gemm.cu", "status.cu"]
+SOURCES = ["quant.cu", "global_scale.cu", "global_scale_static.cu", "importance.cu", "dequant.cu", "gemm.cu", "status.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-fmad=false",  # every fused multiply-add in the kernels is written explicitly

@@ -371,6 +371,56 @@ PyObject* channel_square_norm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     });
 }
 
+// dequant(codes, block scales | None, global scale | None) -> float32 [m, n]
+PyObject* dequant(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+    return guarded([&]() -> PyObject* {
+        if (nargs != 3) return none();
+        const Tensor* q = tensor_of(a[0]);
+        if (!q || !plain_cuda(*q) || q->dim() != 2 || q->scalar_type() != at::kByte || !q->is_contiguous() || !aligned(*q, 4)) return none();
+        const int64_t m = q->size(0), n = q->size(1) * 2;
+        const c10::DeviceIndex dev = q->device().index();
+        const uint8_t* scales = nullptr;
+        const float* gs = nullptr;
+        if (m == 0 || n == 0) return none();
+        if (a[1] == Py_None) {
+            if (n % 8) return none();
+        } else {
+            const Tensor *s = tensor_of(a[1]), *g = tensor_of(a[2]);
+            if (!s || !g || s->device() != q->device() || s->scalar_type() != at::kFloat8_e4m3fn || s->dim() != 2 || s->size(0) != m ||
+                s->size(1) * 16 != n || !s->is_contiguous() || g->numel() != 1 || g->dim() > 2 || !scalar_input(a[2], dev, &gs))
+                return none();
+            scales = static_cast<const uint8_t*>(s->const_data_ptr());
+        }
+        Tensor out = empty({m, n}, at::kFloat, dev);
+        const cudaStream_t st = current_stream(dev);
+        const int rc = launch_on(dev, [&] {
+            return nvfp4_dequant_launch(static_cast<const uint8_t*>(q->const_data_ptr()), scales, gs, static_cast<float*>(out.mutable_data_ptr()),
+                                        m, n, st);
+        });
+        return rc == NVFP4_OK ? THPVariable_Wrap(out) : none();
+    });
+}
+
+// scale_layout(scales, m, k, to_tiled): row-major [m, k] -> flat tiled buffer, or a tiled buffer of any shape -> [m, k]
+PyObject* scale_layout(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+    return guarded([&]() -> PyObject* {
+        int64_t m, k;
+        if (nargs != 4 || !int_or_none(a[1], 0, &m) || !int_or_none(a[2], 0, &k) || m <= 0 || k <= 0) return none();
+        const bool to_tiled = a[3] == Py_True;
+        const Tensor* s = tensor_of(a[0]);
+        const int64_t padded = round_up(m, 128) * round_up(k, 4);
+        if (!s || !plain_cuda(*s) || s->element_size() != 1 || !s->is_contiguous() || s->numel() != (to_tiled ? m * k : padded)) return none();
+        const c10::DeviceIndex dev = s->device().index();
+        Tensor out = to_tiled ? empty({padded}, s->scalar_type(), dev) : empty({m, k}, s->scalar_type(), dev);
+        const cudaStream_t st = current_stream(dev);
+        const int rc = launch_on(dev, [&] {
+            return nvfp4_scale_layout_launch(static_cast<const uint8_t*>(s->const_data_ptr()), static_cast<uint8_t*>(out.mutable_data_ptr()), m, k,
+                                             to_tiled ? 1 : 0, st);
+        });
+        return rc == NVFP4_OK ? THPVariable_Wrap(out) : none();
+    });
+}
+
 // ---- GEMM -----------------------------------------------------------------------------------------------------------
 
 inline int64_t scale_bytes(int64_t rows, int64_t k) { return round_up(rows, 128) * round_up(k / 16, 4); }
@@ -634,6 +684,8 @@ PyMethodDef kMethods[] = {
     FAST(quant_dynamic),
     FAST(global_scale),
     FAST(channel_square_norm),
+    FAST(dequant),
+    FAST(scale_layout),
     FAST(scaled_mm),
     FAST(scaled_mm_prepared),
     FAST(scaled_mm_grouped),

@@ -1,8 +1,8 @@
 """Bench / evaluation helpers with the names of the reference's helper.py.
 
 `get_nvfp4_global_scale` (helper.py:96-100 of efsotr/nvfp4quant_test) runs as a CUDA
-reduction kernel here; the dequantizer and error metrics (helper.py:103-147) are
-plain torch and work on any device.
+reduction kernel here, the dequantizer (helper.py:103-147) as a CUDA kernel on CUDA
+tensors and as plain torch elsewhere; the error metrics are plain torch.
 """
 from __future__ import annotations
 
@@ -92,6 +92,9 @@ _E2M1 = (0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0)
 def unpack_fp4_e2m1(packed: torch.Tensor) -> torch.Tensor:
     """uint8 [m, k/2] -> float32 [m, k]; low nibble first."""
     assert packed.dtype == torch.uint8
+    got = _lib.fast.dequant(packed, None, None)
+    if got is not None:
+        return got
     lut = torch.tensor(_E2M1 + tuple(-v for v in _E2M1), dtype=torch.float32, device=packed.device)
     both = torch.stack((packed & 0x0F, packed >> 4), dim=-1).long()
     return lut[both].reshape(packed.shape[0], packed.shape[1] * 2)
@@ -99,6 +102,9 @@ def unpack_fp4_e2m1(packed: torch.Tensor) -> torch.Tensor:
 
 def dequantize_base(q, scale_fp8, global_scale):
     """q uint8 [m, k/2], scale_fp8 float8_e4m3fn [m, k/16] (row-major, i.e. already unswizzled)."""
+    got = None if scale_fp8 is None else _lib.fast.dequant(q, scale_fp8, global_scale)
+    if got is not None:
+        return got
     scales = scale_fp8.to(torch.float32).repeat_interleave(16, dim=1)
     return unpack_fp4_e2m1(q) * scales * global_scale.float()
 

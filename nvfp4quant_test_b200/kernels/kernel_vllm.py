@@ -9,11 +9,14 @@ Layout: scales of a [m, n] tensor form a [round_up(m,128), round_up(n/16,4)] byt
 matrix stored as 128-row x 4-column tiles of 512 contiguous bytes; inside a tile the
 byte of (row, col) sits at (row % 32) * 16 + (row % 128) // 32 * 4 + col % 4.  That is
 the operand layout tcgen05 block-scaled MMA reads, so the GEMM consumes it unchanged.
-These helpers are pure torch (gather/scatter by a computed index) and work on any device.
+Byte-sized scales on a GPU are converted by a CUDA kernel; anything else by a gather / scatter with a computed index in
+torch, on any device.
 """
 from __future__ import annotations
 
 import torch
+
+from .. import _lib
 
 
 def round_up(x, y):
@@ -32,6 +35,9 @@ def swizzle_vllm_fp4_scale(scale: torch.Tensor, m: int, n: int, block_size: int 
     assert n % block_size == 0
     k = n // block_size
     assert tuple(scale.shape) == (m, k)
+    got = _lib.fast.scale_layout(scale, m, k, True)
+    if got is not None:
+        return got
     m_pad, k_pad = round_up(m, 128), round_up(k, 4)
     raw = scale.view(torch.uint8) if scale.element_size() == 1 else scale
     flat = torch.zeros(m_pad * k_pad, dtype=raw.dtype, device=raw.device)
@@ -44,6 +50,9 @@ def unswizzle_vllm_fp4_scale(scale_swizzled: torch.Tensor, m: int, n: int, block
     """Flat (or [m_pad, k_pad]-shaped) tiled buffer -> [m, n/block_size] row-major scales."""
     assert n % block_size == 0
     k = n // block_size
+    got = _lib.fast.scale_layout(scale_swizzled, m, k, False)
+    if got is not None:
+        return got
     m_pad, k_pad = round_up(m, 128), round_up(k, 4)
     one_byte = scale_swizzled.element_size() == 1
     raw = scale_swizzled.view(torch.uint8) if one_byte else scale_swizzled

@@ -120,3 +120,30 @@ def test_compiled_calls_use_the_current_stream_and_record_into_a_graph(cuda_lib)
     graph.replay()
     torch.cuda.synchronize()
     _same(q, want[:2])
+
+
+@pytest.mark.parametrize("m,n", [(1, 16), (31, 208), (128, 64), (129, 4096), (300, 80)])
+@pytest.mark.parametrize("dtype", [torch.uint8, torch.float8_e4m3fn])
+def test_scale_layouts_and_dequantization_equal_torch(cuda_lib, m, n, dtype):
+    """Every code, scale byte (NaN included) and edge of a tile, against the same functions on CPU tensors (plain torch)."""
+    import nvfp4quant_test_b200.kernels as K
+    from nvfp4quant_test_b200 import _lib
+    from nvfp4quant_test_b200 import helper as H
+
+    g = torch.Generator().manual_seed(m * 7 + n)
+    codes = torch.randint(0, 256, (m, n // 2), dtype=torch.uint8, generator=g)
+    linear = torch.randint(0, 256, (m, n // 16), dtype=torch.uint8, generator=g)
+    gs = torch.tensor(0.0123)
+    tiled = K.swizzle_vllm_fp4_scale(linear.view(dtype), m, n)
+    got = K.swizzle_vllm_fp4_scale(linear.view(dtype).cuda(), m, n)
+    assert got.dtype == tiled.dtype and torch.equal(got.view(torch.uint8).cpu(), tiled.view(torch.uint8))
+    back = K.unswizzle_vllm_fp4_scale(got, m, n)
+    assert back.shape == (m, n // 16) and torch.equal(back.view(torch.uint8).cpu(), linear)
+    assert torch.equal(H.unpack_fp4_e2m1(codes.cuda()).cpu().view(torch.int32), H.unpack_fp4_e2m1(codes).view(torch.int32))
+    fp8 = linear.view(torch.float8_e4m3fn)
+    want = H.dequantize("base", codes, fp8, gs)
+    for g1 in (gs.cuda(), gs.reshape(1).cuda()):
+        have = H.dequantize("base", codes.cuda(), fp8.cuda(), g1).cpu()
+        assert have.shape == want.shape and torch.equal(have.isnan(), want.isnan())
+        assert torch.equal(have[~want.isnan()].view(torch.int32), want[~want.isnan()].view(torch.int32))
+    assert _lib.fast.dequant(codes.cuda(), fp8.cuda(), gs.cuda()) is not None and _lib.fast.scale_layout(got, m, n // 16, False) is not None
