@@ -199,6 +199,23 @@ int nvfp4_gemm_prepare(const uint8_t* b, const uint8_t* sfb, int64_t N, int64_t 
 int nvfp4_gemm_launch_prepared(void* handle, const uint8_t* a, const uint8_t* sfa, const float* alpha, void* out_bf16,
                                int64_t M, void* workspace, size_t workspace_bytes, void* stream);
 int nvfp4_gemm_release(void* handle);
+
+/*
+ * Several products of equal M in one call, each with its own activation, prepared weight (any K), scales and output:
+ *   out_bf16[M, N] = alpha_w[0] * alpha_a[0] * dq(a) dq(weight)^T      (alpha_a may be NULL: factor 1)
+ * for the matrices of a layer whose inputs are all at hand.  Up to 8 of them become one launch of a tile kernel; at
+ * decode-sized M those that share an activation become one grouped launch (below).  n_items <= 64.  Each output has the
+ * bits of nvfp4_gemm_launch_prepared, up to the order of the fp32 sums at decode-sized M.  No counterpart in the reference.
+ */
+typedef struct {
+    void* weight;            /* handle of nvfp4_gemm_prepare */
+    const uint8_t* a;
+    const uint8_t* sfa;
+    const float* alpha_a;
+    const float* alpha_w;
+    void* out_bf16;
+} nvfp4_gemm_item;
+int nvfp4_gemm_launch_multi(const nvfp4_gemm_item* items_host, int n_items, int64_t M, void* stream);
 /*
  * One activation against several prepared weights of equal K in one call (a layer's q / k / v projections, or gate /
  * up: what serving stacks fuse into one wider linear layer; no counterpart in the reference, whose weights are

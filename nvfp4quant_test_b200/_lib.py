@@ -25,7 +25,7 @@ EXPORTS = (
     "nvfp4_quant_launch", "nvfp4_quant_launch_impl", "nvfp4_quant_fused_launch", "nvfp4_quant_chain_launch", "nvfp4_quant_fused_last_status",
     "nvfp4_global_scale_launch", "nvfp4_global_scale_launch_static", "nvfp4_global_scale_static_max_bytes",
     "nvfp4_channel_sqnorm_launch", "nvfp4_channel_sqnorm_launch_strided", "nvfp4_gemm_peak_probe", "nvfp4_gemm_set_wait_limit_ns", "nvfp4_quant_fused_set_wait_limit_ns",
-    "nvfp4_gemm_launch", "nvfp4_gemm_workspace_bytes", "nvfp4_gemm_prepare", "nvfp4_gemm_launch_prepared", "nvfp4_gemm_launch_grouped", "nvfp4_gemm_release", "nvfp4_gemm_last_status", "nvfp4_gemm_force_path", "nvfp4_gemm_tune", "nvfp4_gemm_tune_raster", "nvfp4_gemm_tune_pdl", "nvfp4_gemm_plan",
+    "nvfp4_gemm_launch", "nvfp4_gemm_workspace_bytes", "nvfp4_gemm_prepare", "nvfp4_gemm_launch_prepared", "nvfp4_gemm_launch_grouped", "nvfp4_gemm_launch_multi", "nvfp4_gemm_release", "nvfp4_gemm_last_status", "nvfp4_gemm_force_path", "nvfp4_gemm_tune", "nvfp4_gemm_tune_raster", "nvfp4_gemm_tune_pdl", "nvfp4_gemm_plan",
     "nvfp4_status_string", "nvfp4_abi_version", "nvfp4_stream_capture_id", "nvfp4_dequant_launch",
     "nvfp4_scale_layout_launch",
 )
@@ -40,7 +40,7 @@ def _not_common(*_args):
 
 fast = types.SimpleNamespace(**{name: _not_common for name in (
     "quant_impl", "quant_out", "quant_dynamic", "global_scale", "channel_square_norm", "scaled_mm", "scaled_mm_prepared",
-    "scaled_mm_grouped", "dequant", "scale_layout", "make_chain", "chain_call", "make_group", "group_call")})
+    "scaled_mm_grouped", "scaled_mm_multi", "dequant", "scale_layout", "make_chain", "chain_call", "make_group", "group_call")})
 
 
 def _bind_native() -> None:
@@ -121,6 +121,8 @@ def lib() -> ctypes.CDLL:
         L.nvfp4_stream_capture_id.argtypes = [vp, vp]
         L.nvfp4_gemm_launch_grouped.restype = ci
         L.nvfp4_gemm_launch_grouped.argtypes = [vp, ci, vp, vp, vp, vp, vp, i64, vp]
+        L.nvfp4_gemm_launch_multi.restype = ci
+        L.nvfp4_gemm_launch_multi.argtypes = [vp, ci, i64, vp]
         L.nvfp4_gemm_release.restype = ci
         L.nvfp4_gemm_release.argtypes = [vp]
         L.nvfp4_gemm_workspace_bytes.restype = ctypes.c_size_t

@@ -25,6 +25,7 @@
 // all on the PTX wrappers of tc_ptx.cuh.  One translation unit, so that there is one status word.
 #include <cstdint>
 #include <new>
+#include <utility>
 
 #include "gemm_tile.cuh"
 #include "gemm_pair.cuh"
@@ -193,13 +194,10 @@ extern "C" int nvfp4_gemm_plan(int64_t M, int64_t N, int64_t K, int sms, int* pa
     return NVFP4_OK;
 }
 
-static int gemm_launch_impl(const uint8_t* a, const uint8_t* b, const uint8_t* sfa, const uint8_t* sfb,
-                            const float* alpha, void* out_bf16, int64_t M, int64_t N, int64_t K, void* workspace,
-                            size_t workspace_bytes, void* stream, const nvfp4::gemm::WeightHandle* wh,
-                            const float* alpha2 = nullptr) {
+// Fills one product's parameters; an NVFP4_ERR_* where an argument is wrong.  M, N > 0 are checked by the caller.
+static int gemm_params(nvfp4::gemm::GemmParams& p, const uint8_t* a, const uint8_t* b, const uint8_t* sfa, const uint8_t* sfb,
+                       const float* alpha, const float* alpha2, void* out_bf16, int64_t M, int64_t N, int64_t K) {
     using namespace nvfp4;
-    if (M < 0 || N < 0 || K < 0 || (K % 64) != 0) return NVFP4_ERR_BAD_SHAPE;
-    if (M == 0 || N == 0) return NVFP4_OK;
     if (M > 0x7fffff00LL || N > 0x7fffff00LL || K > 0x7fffff00LL) return NVFP4_ERR_TOO_LARGE;
     if (!a || !b || !sfa || !sfb || !alpha || !out_bf16) return NVFP4_ERR_NULL_POINTER;
     if (K == 0) return NVFP4_ERR_BAD_SHAPE;
@@ -208,12 +206,12 @@ static int gemm_launch_impl(const uint8_t* a, const uint8_t* b, const uint8_t* s
         (reinterpret_cast<uintptr_t>(out_bf16) & 15) || (reinterpret_cast<uintptr_t>(alpha) & 3) ||
         (reinterpret_cast<uintptr_t>(alpha2) & 3))
         return NVFP4_ERR_MISALIGNED;
-    gemm::GemmParams p;
+    p.a = a;
+    p.b = b;
     p.sfa = sfa;
     p.sfb = sfb;
     p.alpha = alpha;
     p.alpha2 = alpha2;
-    p.weights_ready = wh ? 1 : 0;
     p.out = static_cast<__nv_bfloat16*>(out_bf16);
     p.M = static_cast<int>(M);
     p.N = static_cast<int>(N);
@@ -226,9 +224,23 @@ static int gemm_launch_impl(const uint8_t* a, const uint8_t* b, const uint8_t* s
     p.k_tiles_per_split = (k_tiles_total + p.k_splits - 1) / p.k_splits;
     p.k_splits = (k_tiles_total + p.k_tiles_per_split - 1) / p.k_tiles_per_split;   // no empty range
     p.k_rotate = g_gemm_force_rotate > 0 ? 1 : 0;
-    p.partial = static_cast<float*>(workspace);
+    p.partial = nullptr;
     // default: one band over all m-tiles (band sizes 1..16 measured within noise of it on B200)
     p.raster_group = g_gemm_raster_group > 0 ? g_gemm_raster_group : (1 << 20);
+    return NVFP4_OK;
+}
+
+static int gemm_launch_impl(const uint8_t* a, const uint8_t* b, const uint8_t* sfa, const uint8_t* sfb,
+                            const float* alpha, void* out_bf16, int64_t M, int64_t N, int64_t K, void* workspace,
+                            size_t workspace_bytes, void* stream, const nvfp4::gemm::WeightHandle* wh,
+                            const float* alpha2 = nullptr) {
+    using namespace nvfp4;
+    if (M < 0 || N < 0 || K < 0 || (K % 64) != 0) return NVFP4_ERR_BAD_SHAPE;
+    if (M == 0 || N == 0) return NVFP4_OK;
+    gemm::GemmParams p;
+    const int bad = gemm_params(p, a, b, sfa, sfb, alpha, alpha2, out_bf16, M, N, K);
+    if (bad != NVFP4_OK) return bad;
+    p.partial = static_cast<float*>(workspace);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int sms = gemm::device_info().sms;
     int path = 0, ranges = 1;
@@ -245,12 +257,65 @@ static int gemm_launch_impl(const uint8_t* a, const uint8_t* b, const uint8_t* s
         if (!workspace || workspace_bytes < need) return NVFP4_ERR_WORKSPACE;
         if (reinterpret_cast<uintptr_t>(workspace) & 15) return NVFP4_ERR_MISALIGNED;
     }
-    if (path == 3) return gemm::pair::launch_pair<256>(a, b, p, s, wh);
-    if (path == 4) return gemm::pair::launch_pair<192>(a, b, p, s, wh);
-    if (path == 7) return gemm::pair::launch_pair<128>(a, b, p, s, wh);
-    if (path == 2) return gemm::launch<256>(a, b, p, s, wh);
-    if (path == 6) return gemm::launch<64>(a, b, p, s, wh);
-    return gemm::launch<128>(a, b, p, s, wh);
+    if (path == 3) return gemm::pair::launch_pair<256>(p, s, wh);
+    if (path == 4) return gemm::pair::launch_pair<192>(p, s, wh);
+    if (path == 7) return gemm::pair::launch_pair<128>(p, s, wh);
+    if (path == 2) return gemm::launch<256>(p, s, wh);
+    if (path == 6) return gemm::launch<64>(p, s, wh);
+    return gemm::launch<128>(p, s, wh);
+}
+
+// Kernel of a launch over several products (sorted by K): the same relative tile costs as plan_gemm, per K stage, times the
+// longest worker's stages.  0 = launch them one by one (a kernel is forced that has no form for lists).
+static int plan_list(const nvfp4::gemm::GemmParams* list, int n, int sms) {
+    using namespace nvfp4::gemm;
+    if (g_gemm_force_splits != 0) return 0;
+    if (g_gemm_force_path != 0)
+        return g_gemm_force_path == 1 || g_gemm_force_path == 3 || g_gemm_force_path == 4 || g_gemm_force_path == 7 ? g_gemm_force_path : 0;
+    struct { int path, rows, cols, pair; double cost; } const kinds[] = {
+        {1, 128, 128, 0, 0.70}, {7, 256, 128, 1, 0.60}, {4, 256, 192, 1, 0.68}, {3, 256, 256, 1, 0.96}};
+    double best = 0.0;
+    int path = 0;
+    for (const auto& kind : kinds) {
+        GroupTable<kMaxItems> g;
+        const int used = fill_group_table<kMaxItems>(g, list, n, (list[0].M + kind.rows - 1) / kind.rows, kind.cols, kind.pair ? sms / 2 : sms);
+        if (used == 0) continue;
+        const double t = kind.cost * list_makespan(g, list);
+        if (path == 0 || t < best) {
+            best = t;
+            path = kind.path;
+        }
+    }
+    return path;
+}
+
+// Several products of equal M in as few launches as the tile kernels allow.
+static int gemm_launch_list(nvfp4::gemm::GemmParams* list, const nvfp4::gemm::WeightHandle** wh, int n, void* stream) {
+    using namespace nvfp4::gemm;
+    // longest K first (insertion sort, stable): equal K end up next to one another
+    for (int i = 1; i < n; ++i)
+        for (int j = i; j > 0 && list[j].K > list[j - 1].K; --j) {
+            std::swap(list[j], list[j - 1]);
+            std::swap(wh[j], wh[j - 1]);
+        }
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    for (int first = 0; first < n; first += kMaxItems) {
+        const int m = n - first < kMaxItems ? n - first : kMaxItems;
+        const GemmParams* l = list + first;
+        const WeightHandle* const* w = wh + first;
+        const int path = m > 1 ? plan_list(l, m, device_info().sms) : 0;
+        int st = NVFP4_OK;
+        if (path == 1) st = launch_list<128, kMaxItems>(l, w, m, s);
+        else if (path == 7) st = pair::launch_pair_list<128, kMaxItems>(l, w, m, s);
+        else if (path == 4) st = pair::launch_pair_list<192, kMaxItems>(l, w, m, s);
+        else if (path == 3) st = pair::launch_pair_list<256, kMaxItems>(l, w, m, s);
+        else
+            for (int i = 0; i < m && st == NVFP4_OK; ++i)
+                st = gemm_launch_impl(l[i].a, l[i].b, l[i].sfa, l[i].sfb, l[i].alpha, l[i].out, l[i].M, l[i].N, l[i].K, nullptr, 0, stream,
+                                      w[i], l[i].alpha2);
+        if (st != NVFP4_OK) return st;
+    }
+    return NVFP4_OK;
 }
 
 extern "C" int nvfp4_gemm_launch(const uint8_t* a, const uint8_t* b, const uint8_t* sfa, const uint8_t* sfb,
@@ -313,8 +378,8 @@ extern "C" int nvfp4_gemm_launch_prepared(void* handle, const uint8_t* a, const 
 
 // One activation against several prepared weights of equal K, e.g. a layer's q / k / v projections:
 //   outs[i][M, N_i] = alpha_w[i][0] * alpha_a[0] * dq(a) dq(weight_i)^T      (alpha_a may be NULL: factor 1)
-// Decode-sized batches on shapes the decode-sized kernel is chosen for go out as ONE launch per 8 weights; everything
-// else as one launch per weight.  Each output has the bits nvfp4_gemm_launch_prepared gives for the same weight with
+// One launch per 8 weights: of the decode-sized kernel at batches and shapes it is chosen for, of a tile or pair kernel
+// over the list of products otherwise.  Each output has the bits nvfp4_gemm_launch_prepared gives for the same weight with
 // alpha = alpha_w[i][0] * alpha_a[0] whenever the K ranges per tile agree (they are chosen from the group's total tile count).
 extern "C" int nvfp4_gemm_launch_grouped(void* const* handles, int n_weights, const uint8_t* a, const uint8_t* sfa,
                                          const float* alpha_a, const float* const* alpha_w, void* const* outs_bf16,
@@ -376,10 +441,55 @@ extern "C" int nvfp4_gemm_launch_grouped(void* const* handles, int n_weights, co
         }
         return NVFP4_OK;
     }
+    gemm::GemmParams list[64];
+    const gemm::WeightHandle* wh[64];
     for (int i = 0; i < n_weights; ++i) {
-        auto* h = static_cast<const gemm::WeightHandle*>(handles[i]);
-        const int st = gemm_launch_impl(a, h->b, sfa, h->sfb, alpha_w[i], outs_bf16[i], M, h->N, h->K, nullptr, 0, stream, h,
-                                        alpha_a);
+        wh[i] = static_cast<const gemm::WeightHandle*>(handles[i]);
+        const int st = gemm_params(list[i], a, wh[i]->b, sfa, wh[i]->sfb, alpha_w[i], alpha_a, outs_bf16[i], M, wh[i]->N, K);
+        if (st != NVFP4_OK) return st;
+    }
+    return gemm_launch_list(list, wh, n_weights, stream);
+}
+
+// Several products of equal M, each with its own activation: the matrices of a layer whose inputs are all at hand.
+extern "C" int nvfp4_gemm_launch_multi(const nvfp4_gemm_item* items, int n_items, int64_t M, void* stream) {
+    using namespace nvfp4;
+    if (n_items < 0 || n_items > 64) return NVFP4_ERR_BAD_RANGE;
+    if (n_items == 0) return NVFP4_OK;
+    if (!items) return NVFP4_ERR_NULL_POINTER;
+    if (M < 0) return NVFP4_ERR_BAD_SHAPE;
+    const int device = gemm::device_info().device;
+    gemm::GemmParams list[64];
+    const gemm::WeightHandle* wh[64];
+    for (int i = 0; i < n_items; ++i) {
+        const nvfp4_gemm_item& it = items[i];
+        wh[i] = static_cast<const gemm::WeightHandle*>(it.weight);
+        if (!wh[i]) return NVFP4_ERR_NULL_POINTER;
+        if (wh[i]->magic != gemm::kWeightMagic) return NVFP4_ERR_BAD_ENUM;
+        if (wh[i]->device != device) return NVFP4_ERR_UNSUPPORTED;
+        if (M == 0) continue;
+        const int st = gemm_params(list[i], it.a, wh[i]->b, it.sfa, wh[i]->sfb, it.alpha_w, it.alpha_a, it.out_bf16, M, wh[i]->N, wh[i]->K);
+        if (st != NVFP4_OK) return st;
+    }
+    if (M == 0) return NVFP4_OK;
+    if (M > 64) return gemm_launch_list(list, wh, n_items, stream);
+    // decode-sized: items that share activation and scale go out as one grouped launch of the decode-sized kernel
+    bool done[64] = {false};
+    for (int i = 0; i < n_items; ++i) {
+        if (done[i]) continue;
+        void *handles[64], *outs[64];
+        const float* alphas[64];
+        int n = 0;
+        for (int j = i; j < n_items; ++j) {
+            if (done[j] || items[j].a != items[i].a || items[j].sfa != items[i].sfa || items[j].alpha_a != items[i].alpha_a ||
+                wh[j]->K != wh[i]->K)
+                continue;
+            done[j] = true;
+            handles[n] = items[j].weight;
+            outs[n] = items[j].out_bf16;
+            alphas[n++] = items[j].alpha_w;
+        }
+        const int st = nvfp4_gemm_launch_grouped(handles, n, items[i].a, items[i].sfa, items[i].alpha_a, alphas, outs, M, stream);
         if (st != NVFP4_OK) return st;
     }
     return NVFP4_OK;

@@ -81,11 +81,19 @@ __device__ __forceinline__ void tc_mma_pair(uint32_t d_tmem, uint32_t a_lo, uint
         : "memory");
 }
 
-template <int BN>
+// Operand maps and the work list of one launch over G products (G = 1: an ordinary GEMM).
+template <int G>
+struct PairParams {
+    CUtensorMap a[G], b[G], sfa[G], sfb[G];
+    GroupTable<G> g;
+    int M;
+    int raster_group;
+    int weights_ready;   // see TileParams
+};
+
+template <int BN, int G>
 __global__ void __launch_bounds__(kThreads, 1)
-gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                 const __grid_constant__ CUtensorMap tmap_sfa, const __grid_constant__ CUtensorMap tmap_sfb,
-                 const GemmParams p) {
+gemm_pair_kernel(const __grid_constant__ PairParams<G> p) {
     using C = PairCfg<BN>;
     extern __shared__ uint8_t smem_raw[];
     // The kernel queued behind this one may be scheduled at once: ahead of its own wait it reads nothing but a
@@ -107,7 +115,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     const int lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();           // 0 = leader (issues the MMAs)
     const int pair_id = blockIdx.x >> 1;
-    const int num_pairs = gridDim.x >> 1;
     if (threadIdx.x == 0) trace_mark(1, 0);
 
     if (threadIdx.x == 0) {
@@ -140,19 +147,26 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     if (warp >= 2) griddep_wait();    // the epilogue reads alpha and writes the output: only after the previous kernel
 
     const int m_tiles = (p.M + 255) / 256;
-    const int n_tiles = (p.N + BN - 1) / BN;
-    const int total_tiles = m_tiles * n_tiles;
-    const int k_tiles = (p.K + kBK - 1) / kBK;
+    TileCursor<G> cur;
+    cur.init(p.g, pair_id);
+    // tile -> its item (cur.item), m tile and n tile
+    auto locate = [&](int tile, int& mt, int& nt) {
+        cur.seek(p.g, tile);
+        const int n_tiles = (p.g.item[cur.item].N + BN - 1) / BN;
+        tile_to_mn(tile - cur.first_tile, m_tiles, n_tiles, p.raster_group, mt, nt);
+    };
 
     if (warp == 0) {
         // ------------------------------------------------------------------ producer (both CTAs)
         {
             const bool issuer = elect_one();
+            int mt, nt;
+            if (cur.local < cur.total) locate(cur.local, mt, nt);
             if (issuer) {
-            asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_a) : "memory");
-            asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_b) : "memory");
-            asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_sfa) : "memory");
-            asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_sfb) : "memory");
+                asm volatile("prefetch.tensormap [%0];" ::"l"(&p.a[cur.item]) : "memory");
+                asm volatile("prefetch.tensormap [%0];" ::"l"(&p.b[cur.item]) : "memory");
+                asm volatile("prefetch.tensormap [%0];" ::"l"(&p.sfa[cur.item]) : "memory");
+                asm volatile("prefetch.tensormap [%0];" ::"l"(&p.sfb[cur.item]) : "memory");
             }
             int stage = 0;
             uint32_t phase = 0;
@@ -164,30 +178,28 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                 const uint32_t sbase = base + st * C::kStageBytes;
                 if (weights) {
                     if (rank == 0) mbar_expect_tx(full_bar(st), 2u * C::kStageBytes);
-                    tma_load_2d_pair(sbase + C::kABytes, &tmap_b, kt * kBKBytes, nt * BN + static_cast<int>(rank) * (BN / 2), lead_full);
+                    tma_load_2d_pair(sbase + C::kABytes, &p.b[cur.item], kt * kBKBytes, nt * BN + static_cast<int>(rank) * (BN / 2), lead_full);
                     // scale tiles: x counts 8-byte elements (2048 B per K tile), y = 128-row group
-                    tma_load_2d_pair(sbase + C::kABytes + C::kBBytes + C::kSfaBytes, &tmap_sfb, kt * 256, (nt * BN) / 128, lead_full);
-                    tma_load_2d_pair(sbase + C::kABytes + C::kBBytes + C::kSfaBytes + 2048, &tmap_sfb, kt * 256, (nt * BN) / 128 + 1, lead_full);
+                    tma_load_2d_pair(sbase + C::kABytes + C::kBBytes + C::kSfaBytes, &p.sfb[cur.item], kt * 256, (nt * BN) / 128, lead_full);
+                    tma_load_2d_pair(sbase + C::kABytes + C::kBBytes + C::kSfaBytes + 2048, &p.sfb[cur.item], kt * 256, (nt * BN) / 128 + 1, lead_full);
                 }
                 if (tokens) {
-                    tma_load_2d_pair(sbase, &tmap_a, kt * kBKBytes, mt * 256 + static_cast<int>(rank) * 128, lead_full);
-                    tma_load_2d_pair(sbase + C::kABytes + C::kBBytes, &tmap_sfa, kt * 256, mt * 2 + static_cast<int>(rank), lead_full);
+                    tma_load_2d_pair(sbase, &p.a[cur.item], kt * kBKBytes, mt * 256 + static_cast<int>(rank) * 128, lead_full);
+                    tma_load_2d_pair(sbase + C::kABytes + C::kBBytes, &p.sfa[cur.item], kt * 256, mt * 2 + static_cast<int>(rank), lead_full);
                 }
             };
             int early = 0;
             if (!p.weights_ready) griddep_wait();
-            if (pair_id < total_tiles) {
-                int mt, nt;
-                tile_to_mn(pair_id, m_tiles, n_tiles, p.raster_group, mt, nt);
-                early = min(k_tiles, C::kStages);
+            if (cur.local < cur.total) {
+                early = min((p.g.item[cur.item].K + kBK - 1) / kBK, C::kStages);
                 if (issuer)
                     for (int i = 0; i < early; ++i) issue(i, mt, nt, i, true, false);
                 __syncwarp();
             }
             griddep_wait();
-            for (int tile = pair_id; ok && tile < total_tiles; tile += num_pairs) {
-                int mt, nt;
-                tile_to_mn(tile, m_tiles, n_tiles, p.raster_group, mt, nt);
+            for (int tile = cur.local; ok && tile < cur.total; tile += cur.workers) {
+                locate(tile, mt, nt);
+                const int k_tiles = (p.g.item[cur.item].K + kBK - 1) / kBK;
                 for (int kt = 0; kt < k_tiles; ++kt) {
                     if (!(ok = mbar_wait_warp(empty_bar(stage), phase ^ 1u, abort_flag, (1u << 24) | kt))) break;
                     if (issuer) issue(stage, mt, nt, kt, early == 0, true);
@@ -210,18 +222,20 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             uint32_t phase = 0, acc_phase = 0;
             int acc = 0;
             bool ok = true;
-            for (int tile = pair_id; ok && tile < total_tiles; tile += num_pairs) {
+            for (int tile = cur.local; ok && tile < cur.total; tile += cur.workers) {
                 if (!(ok = mbar_wait_warp(tempty_bar(acc), acc_phase ^ 1u, abort_flag, (2u << 24) | 0xffff))) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * BN;
                 // a 192-wide tile starts 0 or 64 rows into its first scale group: 64 rows = 2 TMEM columns
                 int mt_unused, nt_of_tile;
-                tile_to_mn(tile, m_tiles, n_tiles, p.raster_group, mt_unused, nt_of_tile);
+                locate(tile, mt_unused, nt_of_tile);
+                const int K = p.g.item[cur.item].K;
+                const int k_tiles = (K + kBK - 1) / kBK;
                 const uint32_t sfb_shift = (nt_of_tile * BN % 128) / 32;
                 for (int kt = 0; kt < k_tiles; ++kt) {
                     if (!(ok = mbar_wait_warp(full_bar(stage), phase, abort_flag, (2u << 24) | kt))) break;
                     tc_fence_after();
-                    const int kb_count = min(4, (p.K - kt * kBK + 63) / 64);
+                    const int kb_count = min(4, (K - kt * kBK + 63) / 64);
                     const uint32_t sbase = base + stage * C::kStageBytes;
                     const uint32_t a_lo = ((sbase & 0x3ffffu) >> 4) | (1u << 16);
                     const uint32_t b_lo = a_lo + (C::kABytes >> 4);
@@ -273,28 +287,35 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     } else {
         // ------------------------------------------------------------------ epilogue (both CTAs)
         const int sp = warp & 3;
-        const float alpha = load_alpha(p.alpha, p.alpha2);
+        int alpha_item = -1;
+        float alpha = 0.0f;
         uint32_t acc_phase = 0;
         int acc = 0;
         bool ok = true;
-        const bool vec_ok = (p.N % 8) == 0;
-        for (int tile = pair_id; ok && tile < total_tiles; tile += num_pairs) {
+        for (int tile = cur.local; ok && tile < cur.total; tile += cur.workers) {
             int mt, nt;
-            tile_to_mn(tile, m_tiles, n_tiles, p.raster_group, mt, nt);
+            locate(tile, mt, nt);
+            const GemmItem& it = p.g.item[cur.item];
+            const int N = it.N;
+            const bool vec_ok = (N % 8) == 0;
+            if (cur.item != alpha_item) {
+                alpha_item = cur.item;
+                alpha = load_alpha(it.alpha, it.alpha2);
+            }
             ok = mbar_wait(tfull_bar(acc), acc_phase, abort_flag, (3u << 24) | (tile & 0xffff));
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
             if (!ok) break;
             tc_fence_after();
             const int row = mt * 256 + static_cast<int>(rank) * 128 + sp * 32 + lane;
-            __nv_bfloat16* orow = p.out + static_cast<int64_t>(row) * p.N;
+            __nv_bfloat16* orow = it.out + static_cast<int64_t>(row) * N;
 #pragma unroll 1
             for (int c = 0; c < BN / 32; ++c) {
                 uint32_t v[32];
                 tc_ld_32x32b_x32(tmem_base + (static_cast<uint32_t>(sp * 32) << 16) + acc * BN + c * 32, v);
                 tc_ld_wait();
                 const int col0 = nt * BN + c * 32;
-                if (row < p.M && col0 < p.N) {
-                    if (vec_ok && col0 + 32 <= p.N) {
+                if (row < p.M && col0 < N) {
+                    if (vec_ok && col0 + 32 <= N) {
 #pragma unroll
                         for (int q = 0; q < 4; ++q) {
                             uint32_t w[4];
@@ -309,7 +330,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                         }
                     } else {
                         for (int e = 0; e < 32; ++e)
-                            if (col0 + e < p.N) orow[col0 + e] = __float2bfloat16_rn(__fmul_rn(__uint_as_float(v[e]), alpha));
+                            if (col0 + e < N) orow[col0 + e] = __float2bfloat16_rn(__fmul_rn(__uint_as_float(v[e]), alpha));
                     }
                 }
             }
@@ -361,25 +382,35 @@ static int make_scale_map(CUtensorMap* map, const void* ptr, int64_t groups, int
     return r == CUDA_SUCCESS ? NVFP4_OK : NVFP4_ERR_UNSUPPORTED;
 }
 
-template <int BN>
-static int launch_pair(const uint8_t* a, const uint8_t* b, const GemmParams& p, cudaStream_t stream, const WeightHandle* wh) {
+// One launch over the `n` products of `list` (1 <= n <= G), items of equal K next to one another, longest K first.
+template <int BN, int G>
+static int launch_pair_list(const GemmParams* list, const WeightHandle* const* wh, int n, cudaStream_t stream) {
     using C = PairCfg<BN>;
-    CUtensorMap ma, msa, mb_local, msb_local;
-    int st = make_operand_map(&ma, a, p.M, p.K / 2, 128);
-    if (st == NVFP4_OK) st = make_scale_map(&msa, p.sfa, p.sfa_groups, p.sf_group_stride);
-    if (st == NVFP4_OK && !wh) st = make_operand_map(&mb_local, b, p.N, p.K / 2, BN / 2);
-    if (st == NVFP4_OK && !wh) st = make_scale_map(&msb_local, p.sfb, p.sfb_groups, p.sf_group_stride);
-    if (st != NVFP4_OK) return st;
-    const CUtensorMap& mb = wh ? *wh->by_rows(BN / 2) : mb_local;
-    const CUtensorMap& msb = wh ? wh->scales : msb_local;
     static_assert(C::kSmemBytes <= kGemmDynSmemBytes, "ring does not fit");
+    PairParams<G> q;
+    q.M = list[0].M;
+    q.raster_group = list[0].raster_group;
+    q.weights_ready = 1;
+    const int m_tiles = (q.M + 255) / 256;
+    for (int i = 0; i < n; ++i) {
+        const GemmParams& p = list[i];
+        int st = make_operand_map(&q.a[i], p.a, p.M, p.K / 2, 128);
+        if (st == NVFP4_OK) st = make_scale_map(&q.sfa[i], p.sfa, p.sfa_groups, p.sf_group_stride);
+        if (wh[i]) {
+            q.b[i] = *wh[i]->by_rows(BN / 2);
+            q.sfb[i] = wh[i]->scales;
+        } else {
+            q.weights_ready = 0;
+            if (st == NVFP4_OK) st = make_operand_map(&q.b[i], p.b, p.N, p.K / 2, BN / 2);
+            if (st == NVFP4_OK) st = make_scale_map(&q.sfb[i], p.sfb, p.sfb_groups, p.sf_group_stride);
+        }
+        if (st != NVFP4_OK) return st;
+    }
     const DeviceInfo di = device_info();
+    const int pairs = fill_group_table<G>(q.g, list, n, m_tiles, BN, di.sms / 2);
     static bool attr_done[64] = {false};
-    cudaError_t e = allow_full_smem(gemm_pair_kernel<BN>, attr_done, di.device);
+    cudaError_t e = allow_full_smem(gemm_pair_kernel<BN, G>, attr_done, di.device);
     if (e != cudaSuccess) return static_cast<int>(e);
-    const int sms = di.sms;
-    const int tiles = ((p.M + 255) / 256) * ((p.N + BN - 1) / BN);
-    const int pairs = tiles < sms / 2 ? tiles : sms / 2;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * pairs, 1, 1);
     cfg.blockDim = dim3(kThreads, 1, 1);
@@ -394,8 +425,13 @@ static int launch_pair(const uint8_t* a, const uint8_t* b, const GemmParams& p, 
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = g_dependent_launch ? 2 : 1;
-    e = cudaLaunchKernelEx(&cfg, gemm_pair_kernel<BN>, ma, mb, msa, msb, p);
+    e = cudaLaunchKernelEx(&cfg, gemm_pair_kernel<BN, G>, q);
     return static_cast<int>(e);
+}
+
+template <int BN>
+static int launch_pair(const GemmParams& p, cudaStream_t stream, const WeightHandle* wh) {
+    return launch_pair_list<BN, 1>(&p, &wh, 1, stream);
 }
 
 }  // namespace pair

@@ -27,7 +27,10 @@ struct Cfg {
     static_assert(kSfaCol + 2 * kSfSetCols <= kTmemCols, "TMEM budget");
 };
 
+// One product, as the entry points see it.
 struct GemmParams {
+    const uint8_t* a;
+    const uint8_t* b;
     const uint8_t* sfa;
     const uint8_t* sfb;
     const float* alpha;
@@ -42,9 +45,57 @@ struct GemmParams {
     int k_rotate;             // != 0: each tile starts its K loop at a different stage (spreads requests for shared A rows)
     float* partial;
     int raster_group;         // m-tiles per band of the tile numbering (see tile_to_mn)
-    // != 0: the weight operand is a prepared weight, constant while launches with it are in flight, and may be read
-    // before griddep_wait(); 0 (raw pointers): it may be the output of the kernel just before this one, like the tokens
-    int weights_ready;
+};
+
+// One launch over several products (a layer's matrices at prefill): up to kMaxItems weights, each with its own activation,
+// K, output scale and output, all with the same M.  Tiles are numbered through the items; items of equal K form a class,
+// and every class has its own workers (CTAs or CTA pairs), because a tile's time is its K: with the workers dealt out by
+// the host so that the longest class is as short as possible, a K = 14336 product runs beside K = 4096 ones without leaving
+// SMs idle at the end (256 tokens, the seven matrices of a Llama-3-8B layer: one launch instead of seven on four streams).
+constexpr int kMaxItems = 8;
+
+struct GemmItem {
+    const uint8_t* sfa;       // single-CTA kernel: scales are fetched by address
+    const uint8_t* sfb;
+    const float* alpha;
+    const float* alpha2;
+    __nv_bfloat16* out;
+    int64_t sf_group_stride;
+    int N, K;
+    int sfb_groups;
+    int tile_end;             // tiles of this and the earlier items of its class
+};
+
+template <int G>
+struct GroupTable {
+    GemmItem item[G];
+    int n_classes;
+    int worker_end[G];        // workers of this and all earlier classes
+    int item_end[G];          // items of this and all earlier classes
+};
+
+// Where a worker of a grouped launch stands: its class, and the item that its current tile belongs to.  Every role of a
+// CTA walks the same tiles in the same order with a cursor of its own.
+template <int G>
+struct TileCursor {
+    int local, workers, total, item, first_tile;
+    __device__ __forceinline__ void init(const GroupTable<G>& g, int worker) {
+        int c = 0;
+        while (c + 1 < g.n_classes && worker >= g.worker_end[c]) ++c;
+        const int begin = c > 0 ? g.worker_end[c - 1] : 0;
+        local = worker - begin;
+        workers = g.worker_end[c] - begin;
+        item = c > 0 ? g.item_end[c - 1] : 0;
+        total = g.item[g.item_end[c] - 1].tile_end;
+        first_tile = 0;
+    }
+    // `tile` never decreases from call to call
+    __device__ __forceinline__ void seek(const GroupTable<G>& g, int tile) {
+        if constexpr (G > 1) while (tile >= g.item[item].tile_end) {
+            first_tile = g.item[item].tile_end;
+            ++item;
+        }
+    }
 };
 
 // Output scale of a launch: alpha[0], or alpha[0] * alpha2[0] rounded once (what a separate fp32 multiplication of the
@@ -67,9 +118,23 @@ __device__ __forceinline__ void tile_to_mn(int tile, int m_tiles, int n_tiles, i
     mt = first_m + in_band - nt * rows;
 }
 
-template <int BN>
+// Operand maps and the work list of one launch over G products (G = 1: an ordinary GEMM, whose K may be cut into ranges).
+template <int G>
+struct TileParams {
+    CUtensorMap a[G], b[G];
+    GroupTable<G> g;
+    int M;
+    int k_splits, k_tiles_per_split, k_rotate;   // G = 1 only, see GemmParams
+    float* partial;
+    int raster_group;
+    // != 0: every weight is a prepared weight, constant while launches with it are in flight, and may be read before
+    // griddep_wait(); 0 (raw pointers): one may be the output of the kernel just before this one, like the tokens
+    int weights_ready;
+};
+
+template <int BN, int G>
 __global__ void __launch_bounds__(kThreads, 1)
-gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const GemmParams p) {
+gemm_kernel(const __grid_constant__ TileParams<G> p) {
     using C = Cfg<BN>;
     extern __shared__ uint8_t smem_raw[];
     // The kernel queued behind this one may be scheduled at once: ahead of its own wait it reads nothing but a
@@ -129,18 +194,35 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     if (warp >= 2) griddep_wait();    // alpha, and the output buffer, belong to whatever ran before: epilogue only after it
 
     const int m_tiles = (p.M + kBM - 1) / kBM;
-    const int n_tiles = (p.N + BN - 1) / BN;
-    const int mn_tiles = m_tiles * n_tiles;
-    const int total_tiles = mn_tiles * p.k_splits;   // work items: (K range, n tile, m tile)
-    const int k_tiles = (p.K + kBK - 1) / kBK;
+    TileCursor<G> cur;
+    cur.init(p.g, blockIdx.x);
+    const int splits = G == 1 ? p.k_splits : 1;
+    const int total_tiles = cur.total * splits;   // work items: (K range, n tile, m tile)
+    // work item -> its product (cur.item), K range, m tile and n tile
+    auto locate = [&](int tile, int& ks, int& mt, int& nt) {
+        ks = splits > 1 ? tile / cur.total : 0;
+        const int t2 = tile - ks * cur.total;
+        cur.seek(p.g, t2);
+        const int n_tiles = (p.g.item[cur.item].N + BN - 1) / BN;
+        tile_to_mn(t2 - cur.first_tile, m_tiles, n_tiles, p.raster_group, mt, nt);
+    };
+    // stages of the current product's K range: first, count, and where the loop starts (see GemmParams::k_rotate)
+    auto k_range = [&](int ks, int tile, int& kt_begin, int& kcount, int& rot) {
+        const int k_tiles = (p.g.item[cur.item].K + kBK - 1) / kBK;
+        kt_begin = splits > 1 ? ks * p.k_tiles_per_split : 0;
+        kcount = (splits > 1 ? min(k_tiles, kt_begin + p.k_tiles_per_split) : k_tiles) - kt_begin;
+        rot = G == 1 && p.k_rotate ? ((tile - ks * cur.total) * 5) % kcount : 0;
+    };
 
     if (warp == 0) {
         // ------------------------------------------------------------------ producer
         {
             const bool issuer = elect_one();
+            int ks, mt, nt, kt_begin, kcount, rot;
+            if (cur.local < total_tiles) locate(cur.local, ks, mt, nt);
             if (issuer) {
-                asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_a) : "memory");
-                asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_b) : "memory");
+                asm volatile("prefetch.tensormap [%0];" ::"l"(&p.a[cur.item]) : "memory");
+                asm volatile("prefetch.tensormap [%0];" ::"l"(&p.b[cur.item]) : "memory");
             }
             int stage = 0;
             uint32_t phase = 0;
@@ -150,52 +232,45 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
             // weight halves of the first ring-full go out before griddep_wait(), so that with a programmatic dependent
             // launch the weight stream starts while the previous kernel is still finishing; `early` counts them.
             auto issue = [&](int st, int mt, int nt, int kt, bool weights, bool tokens) {
-                const int kb_count = min(4, (p.K - kt * kBK + 63) / 64);  // 64-element K blocks in this stage
+                const GemmItem& it = p.g.item[cur.item];
+                const int kb_count = min(4, (it.K - kt * kBK + 63) / 64);  // 64-element K blocks in this stage
                 const uint32_t sf_bytes = 512u * kb_count;
                 int sfb_present = 0;
                 const int grp0 = BN == 64 ? (nt >> 1) : nt * C::kNG;   // first 128-row scale group of this B tile
-                for (int g = 0; g < C::kNG; ++g) sfb_present += (grp0 + g < p.sfb_groups) ? 1 : 0;
+                for (int g = 0; g < C::kNG; ++g) sfb_present += (grp0 + g < it.sfb_groups) ? 1 : 0;
                 const uint32_t sbase = base + st * C::kStageBytes;
                 if (weights) {
                     mbar_expect_tx(full_bar(st), C::kABytes + C::kBBytes + sf_bytes * (1 + sfb_present));
-                    tma_load_2d(sbase + C::kABytes, &tmap_b, kt * kBKBytes, nt * BN, full_bar(st));
+                    tma_load_2d(sbase + C::kABytes, &p.b[cur.item], kt * kBKBytes, nt * BN, full_bar(st));
                     for (int g = 0; g < C::kNG; ++g) {
                         const int grp = grp0 + g;
-                        if (grp < p.sfb_groups)
+                        if (grp < it.sfb_groups)
                             bulk_load_1d(sbase + C::kABytes + C::kBBytes + C::kSfaBytes + g * 2048,
-                                         p.sfb + static_cast<int64_t>(grp) * p.sf_group_stride +
+                                         it.sfb + static_cast<int64_t>(grp) * it.sf_group_stride +
                                              static_cast<int64_t>(kt) * 2048,
                                          sf_bytes, full_bar(st));
                     }
                 }
                 if (tokens) {
-                    tma_load_2d(sbase, &tmap_a, kt * kBKBytes, mt * kBM, full_bar(st));
+                    tma_load_2d(sbase, &p.a[cur.item], kt * kBKBytes, mt * kBM, full_bar(st));
                     bulk_load_1d(sbase + C::kABytes + C::kBBytes,
-                                 p.sfa + static_cast<int64_t>(mt) * p.sf_group_stride + static_cast<int64_t>(kt) * 2048,
+                                 it.sfa + static_cast<int64_t>(mt) * it.sf_group_stride + static_cast<int64_t>(kt) * 2048,
                                  sf_bytes, full_bar(st));
                 }
             };
             int early = 0;
             if (!p.weights_ready) griddep_wait();
-            if (static_cast<int>(blockIdx.x) < total_tiles && !p.k_rotate) {
-                const int ks = blockIdx.x / mn_tiles, t2 = blockIdx.x - ks * mn_tiles;
-                int mt, nt;
-                tile_to_mn(t2, m_tiles, n_tiles, p.raster_group, mt, nt);
-                const int kt_begin = ks * p.k_tiles_per_split;
-                const int kcount = min(k_tiles, kt_begin + p.k_tiles_per_split) - kt_begin;
+            if (cur.local < total_tiles && !(G == 1 && p.k_rotate)) {
+                k_range(ks, cur.local, kt_begin, kcount, rot);
                 early = min(kcount, C::kStages);
                 if (issuer)
                     for (int i = 0; i < early; ++i) issue(i, mt, nt, kt_begin + i, true, false);
                 __syncwarp();
             }
             griddep_wait();
-            for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
-                const int ks = tile / mn_tiles, t2 = tile - ks * mn_tiles;
-                int mt, nt;
-                tile_to_mn(t2, m_tiles, n_tiles, p.raster_group, mt, nt);
-                const int kt_begin = ks * p.k_tiles_per_split;
-                const int kcount = min(k_tiles, kt_begin + p.k_tiles_per_split) - kt_begin;
-                const int rot = p.k_rotate ? (t2 * 5) % kcount : 0;
+            for (int tile = cur.local; ok && tile < total_tiles; tile += cur.workers) {
+                locate(tile, ks, mt, nt);
+                k_range(ks, tile, kt_begin, kcount, rot);
                 for (int i = 0; i < kcount; ++i) {
                     const int kt = kt_begin + (i + rot) % kcount;
                     if (!(ok = mbar_wait_warp(empty_bar(stage), phase ^ 1u, abort_flag, (1u << 24) | kt))) break;
@@ -219,26 +294,21 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
             int acc = 0;
             uint32_t acc_phase = 0;
             bool ok = true;
-            for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
+            for (int tile = cur.local; ok && tile < total_tiles; tile += cur.workers) {
                 if (!(ok = mbar_wait_warp(tempty_bar(acc), acc_phase ^ 1u, abort_flag, (2u << 24) | 0xffff))) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * BN;
-                const int ks = tile / mn_tiles, t2 = tile - ks * mn_tiles;
+                int ks, mt, nt, kt_begin, kcount, rot;
+                locate(tile, ks, mt, nt);
+                k_range(ks, tile, kt_begin, kcount, rot);
+                const int K = p.g.item[cur.item].K;
                 // a 64-row B tile is one half of a 128-row scale group: rows 64..127 sit two TMEM columns further on
-                uint32_t sfb_half = 0;
-                if (BN == 64) {
-                    int mt, nt;
-                    tile_to_mn(t2, m_tiles, n_tiles, p.raster_group, mt, nt);
-                    sfb_half = 2u * (nt & 1);
-                }
-                const int kt_begin = ks * p.k_tiles_per_split;
-                const int kcount = min(k_tiles, kt_begin + p.k_tiles_per_split) - kt_begin;
-                const int rot = p.k_rotate ? (t2 * 5) % kcount : 0;
+                const uint32_t sfb_half = BN == 64 ? 2u * (nt & 1) : 0u;
                 for (int i = 0; i < kcount; ++i) {
                     const int kt = kt_begin + (i + rot) % kcount;
                     if (!(ok = mbar_wait_warp(full_bar(stage), phase, abort_flag, (2u << 24) | kt))) break;
                     tc_fence_after();
-                    const int kb_count = min(4, (p.K - kt * kBK + 63) / 64);
+                    const int kb_count = min(4, (K - kt * kBK + 63) / 64);
                     const uint32_t sbase = base + stage * C::kStageBytes;
                     const uint32_t a_lo = ((sbase & 0x3ffffu) >> 4) | (1u << 16);
                     const uint32_t b_lo = a_lo + (C::kABytes >> 4);
@@ -292,42 +362,48 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     } else {
         // ------------------------------------------------------------------ epilogue (warps 2..5)
         const int sp = warp & 3;  // TMEM sub-partition this warp may read: lanes 32*sp .. 32*sp+31
-        const float alpha = load_alpha(p.alpha, p.alpha2);
+        int alpha_item = -1;
+        float alpha = 0.0f;
         int acc = 0;
         uint32_t acc_phase = 0;
         bool ok = true;
-        const bool vec_ok = (p.N % 8) == 0;
-        for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
-            const int ks = tile / mn_tiles, t2 = tile - ks * mn_tiles;
-            int mt, nt;
-            tile_to_mn(t2, m_tiles, n_tiles, p.raster_group, mt, nt);
+        for (int tile = cur.local; ok && tile < total_tiles; tile += cur.workers) {
+            int ks, mt, nt;
+            locate(tile, ks, mt, nt);
+            const GemmItem& it = p.g.item[cur.item];
+            const int N = it.N;
+            const bool vec_ok = (N % 8) == 0;
+            if (cur.item != alpha_item) {
+                alpha_item = cur.item;
+                alpha = load_alpha(it.alpha, it.alpha2);
+            }
             ok = mbar_wait(tfull_bar(acc), acc_phase, abort_flag, (3u << 24) | (tile & 0xffff));
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
             if (!ok) break;
             tc_fence_after();
             const int row = mt * kBM + sp * 32 + lane;
-            __nv_bfloat16* orow = p.out + static_cast<int64_t>(row) * p.N;
+            __nv_bfloat16* orow = it.out + static_cast<int64_t>(row) * N;
 #pragma unroll 1
             for (int c = 0; c < BN / 32; ++c) {
                 uint32_t v[32];
                 tc_ld_32x32b_x32(tmem_base + (static_cast<uint32_t>(sp * 32) << 16) + acc * BN + c * 32, v);
                 tc_ld_wait();
                 const int col0 = nt * BN + c * 32;
-                if (p.k_splits > 1) {
+                if (splits > 1) {
                     // fp32 partial of this K range; alpha and the bf16 rounding happen in the reduction kernel
-                    if (row < p.M && col0 < p.N) {
-                        float* prow = p.partial + (static_cast<int64_t>(ks) * p.M + row) * p.N + col0;
-                        if ((p.N % 4) == 0 && col0 + 32 <= p.N) {
+                    if (row < p.M && col0 < N) {
+                        float* prow = p.partial + (static_cast<int64_t>(ks) * p.M + row) * N + col0;
+                        if ((N % 4) == 0 && col0 + 32 <= N) {
 #pragma unroll
                             for (int q = 0; q < 8; ++q)
                                 *reinterpret_cast<uint4*>(prow + 4 * q) = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
                         } else {
                             for (int e = 0; e < 32; ++e)
-                                if (col0 + e < p.N) prow[e] = __uint_as_float(v[e]);
+                                if (col0 + e < N) prow[e] = __uint_as_float(v[e]);
                         }
                     }
-                } else if (row < p.M && col0 < p.N) {
-                    if (vec_ok && col0 + 32 <= p.N) {
+                } else if (row < p.M && col0 < N) {
+                    if (vec_ok && col0 + 32 <= N) {
 #pragma unroll
                         for (int q = 0; q < 4; ++q) {
                             uint32_t w[4];
@@ -342,7 +418,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
                         }
                     } else {
                         for (int e = 0; e < 32; ++e)
-                            if (col0 + e < p.N) orow[col0 + e] = __float2bfloat16_rn(__fmul_rn(__uint_as_float(v[e]), alpha));
+                            if (col0 + e < N) orow[col0 + e] = __float2bfloat16_rn(__fmul_rn(__uint_as_float(v[e]), alpha));
                     }
                 }
             }
@@ -460,45 +536,115 @@ struct WeightHandle {
 };
 constexpr uint32_t kWeightMagic = 0x4e56463u;
 
-template <int BN>
-static int launch(const uint8_t* a, const uint8_t* b, const GemmParams& p, cudaStream_t stream, const WeightHandle* wh) {
+// Fills the work list for `workers` CTAs (or CTA pairs) and returns how many are used (0: too few for the classes).
+// A class is a run of items of equal K.  With one class every worker takes tiles of it; with several the smallest makespan
+// T (in K stages) is searched for which the classes' workers, ceil(tiles / floor(T / k)) each, fit.
+template <int G>
+static int fill_group_table(GroupTable<G>& g, const GemmParams* list, int n, int m_tiles, int bn, int workers) {
+    int64_t tiles[G], k[G], stages = 0, longest = 0;
+    g.n_classes = 0;
+    for (int i = 0; i < n; ++i) {
+        const GemmParams& p = list[i];
+        GemmItem& it = g.item[i];
+        it.sfa = p.sfa;
+        it.sfb = p.sfb;
+        it.alpha = p.alpha;
+        it.alpha2 = p.alpha2;
+        it.out = p.out;
+        it.sf_group_stride = p.sf_group_stride;
+        it.N = p.N;
+        it.K = p.K;
+        it.sfb_groups = p.sfb_groups;
+        const bool same = i > 0 && list[i - 1].K == p.K;
+        if (!same) {
+            k[g.n_classes] = (p.K + kBK - 1) / kBK;
+            tiles[g.n_classes++] = 0;
+        }
+        const int c = g.n_classes - 1;
+        const int64_t mine = static_cast<int64_t>(m_tiles) * ((p.N + bn - 1) / bn);
+        tiles[c] += mine;
+        stages += mine * k[c];
+        if (k[c] > longest) longest = k[c];
+        it.tile_end = static_cast<int>(tiles[c]);
+        g.item_end[c] = i + 1;
+    }
+    if (g.n_classes == 1) {
+        const int64_t all = tiles[0] * (G == 1 ? list[0].k_splits : 1);
+        return g.worker_end[0] = static_cast<int>(all < workers ? all : workers);
+    }
+    if (workers < g.n_classes) return 0;
+    int64_t T = (stages + workers - 1) / workers;
+    if (T < longest) T = longest;
+    for (;;) {
+        int64_t used = 0, next = INT64_MAX;
+        for (int c = 0; c < g.n_classes; ++c) {
+            const int64_t per = T / k[c];
+            used += (tiles[c] + per - 1) / per;
+            g.worker_end[c] = static_cast<int>(used);
+            if ((per + 1) * k[c] < next) next = (per + 1) * k[c];
+        }
+        if (used <= workers) return static_cast<int>(used);
+        T = next;
+    }
+}
+
+// K stages of the busiest worker.
+template <int G>
+static double list_makespan(const GroupTable<G>& g, const GemmParams* list) {
+    int64_t longest = 0;
+    for (int c = 0; c < g.n_classes; ++c) {
+        const int64_t workers = g.worker_end[c] - (c > 0 ? g.worker_end[c - 1] : 0);
+        const int last = g.item_end[c] - 1;
+        const int64_t k = (list[last].K + kBK - 1) / kBK, tiles = g.item[last].tile_end;
+        const int64_t mine = (tiles + workers - 1) / workers * k;
+        if (mine > longest) longest = mine;
+    }
+    return static_cast<double>(longest);
+}
+
+// One launch over the `n` products of `list` (1 <= n <= G), items of equal K next to one another, longest K first.
+template <int BN, int G>
+static int launch_list(const GemmParams* list, const WeightHandle* const* wh, int n, cudaStream_t stream) {
     using C = Cfg<BN>;
-    CUtensorMap ma, mb_local;
-    int st = make_operand_map(&ma, a, p.M, p.K / 2, kBM);
-    if (st != NVFP4_OK) return st;
-    if (!wh) {
-        st = make_operand_map(&mb_local, b, p.N, p.K / 2, BN);
+    static_assert(C::kSmemBytes <= kGemmDynSmemBytes, "ring does not fit");
+    const GemmParams& p0 = list[0];
+    TileParams<G> q;
+    q.M = p0.M;
+    q.k_splits = p0.k_splits;
+    q.k_tiles_per_split = p0.k_tiles_per_split;
+    q.k_rotate = p0.k_rotate;
+    q.partial = p0.partial;
+    q.raster_group = p0.raster_group;
+    q.weights_ready = 1;
+    for (int i = 0; i < n; ++i) {
+        const GemmParams& p = list[i];
+        int st = make_operand_map(&q.a[i], p.a, p.M, p.K / 2, kBM);
+        if (wh[i]) {
+            q.b[i] = *wh[i]->by_rows(BN);
+        } else {
+            q.weights_ready = 0;
+            if (st == NVFP4_OK) st = make_operand_map(&q.b[i], p.b, p.N, p.K / 2, BN);
+        }
         if (st != NVFP4_OK) return st;
     }
-    const CUtensorMap& mb = wh ? *wh->by_rows(BN) : mb_local;
-    static_assert(C::kSmemBytes <= kGemmDynSmemBytes, "ring does not fit");
     const DeviceInfo di = device_info();
+    const int grid = fill_group_table<G>(q.g, list, n, (q.M + kBM - 1) / kBM, BN, di.sms);
     static bool attr_done[64] = {false};
-    cudaError_t e = allow_full_smem(gemm_kernel<BN>, attr_done, di.device);
+    cudaError_t e = allow_full_smem(gemm_kernel<BN, G>, attr_done, di.device);
     if (e != cudaSuccess) return static_cast<int>(e);
-    const int sms = di.sms;
-    const int tiles = ((p.M + kBM - 1) / kBM) * ((p.N + BN - 1) / BN) * p.k_splits;
-    const int grid = tiles < sms ? tiles : sms;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid, 1, 1);
-    cfg.blockDim = dim3(kThreads, 1, 1);
-    cfg.dynamicSmemBytes = kGemmDynSmemBytes;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // may start while its predecessor finishes
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = g_dependent_launch ? 1 : 0;
-    e = cudaLaunchKernelEx(&cfg, gemm_kernel<BN>, ma, mb, p);
-    if (e != cudaSuccess || p.k_splits == 1) return static_cast<int>(e);
-    const int64_t mn = static_cast<int64_t>(p.M) * p.N;
+    e = launch_dependent(gemm_kernel<BN, G>, dim3(grid), dim3(kThreads), kGemmDynSmemBytes, stream, q);
+    if (e != cudaSuccess || G > 1 || p0.k_splits == 1) return static_cast<int>(e);
+    const int64_t mn = static_cast<int64_t>(p0.M) * p0.N;
     int64_t rblocks = (mn + 255) / 256;
     if (rblocks > 148 * 8) rblocks = 148 * 8;
-    splitk_reduce_kernel<<<static_cast<unsigned>(rblocks), 256, 0, stream>>>(p.partial, p.alpha, p.alpha2, p.out, mn, p.k_splits);
+    splitk_reduce_kernel<<<static_cast<unsigned>(rblocks), 256, 0, stream>>>(p0.partial, p0.alpha, p0.alpha2, p0.out, mn, p0.k_splits);
     return static_cast<int>(cudaGetLastError());
 }
 
-
+template <int BN>
+static int launch(const GemmParams& p, cudaStream_t stream, const WeightHandle* wh) {
+    return launch_list<BN, 1>(&p, &wh, 1, stream);
+}
 
 }  // namespace gemm
 }  // namespace nvfp4

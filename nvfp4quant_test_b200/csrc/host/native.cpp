@@ -519,6 +519,19 @@ PyObject* scaled_mm_prepared(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     });
 }
 
+PyObject* tensor_list(const std::vector<Tensor>& ts) {
+    PyObject* l = PyList_New(static_cast<Py_ssize_t>(ts.size()));
+    for (size_t i = 0; l && i < ts.size(); ++i) {
+        PyObject* o = THPVariable_Wrap(ts[i]);
+        if (!o) {
+            Py_DECREF(l);
+            return nullptr;
+        }
+        PyList_SET_ITEM(l, static_cast<Py_ssize_t>(i), o);
+    }
+    return l;
+}
+
 // scaled_mm_grouped(a, block_scale_a, alpha_a | None, [weight], [alpha_w], [out] | None) -> [bf16 [m, n_i]]
 PyObject* scaled_mm_grouped(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     return guarded([&]() -> PyObject* {
@@ -555,16 +568,48 @@ PyObject* scaled_mm_grouped(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
             Py_INCREF(a[5]);
             return a[5];
         }
-        PyObject* l = PyList_New(count);
-        for (Py_ssize_t i = 0; l && i < count; ++i) {
-            PyObject* o = THPVariable_Wrap(out[i]);
-            if (!o) {
-                Py_DECREF(l);
-                return nullptr;
+        return tensor_list(out);
+    });
+}
+
+// scaled_mm_multi([a], [block_scale_a], [alpha_a | None], [weight], [alpha_w]) -> [bf16 [m, n_i]]
+PyObject* scaled_mm_multi(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+    return guarded([&]() -> PyObject* {
+        if (nargs != 5) return none();
+        for (int i = 0; i < 5; ++i)
+            if (!PyList_CheckExact(a[i]) || PyList_GET_SIZE(a[i]) != PyList_GET_SIZE(a[0])) return none();
+        const Py_ssize_t count = PyList_GET_SIZE(a[0]);
+        if (count < 1 || count > 64) return none();
+        nvfp4_gemm_item items[64];
+        std::vector<Tensor> out(static_cast<size_t>(count));
+        int64_t m = 0;
+        c10::DeviceIndex dev = 0;
+        for (Py_ssize_t i = 0; i < count; ++i) {
+            const Tensor *qa, *sa;
+            Weight w;
+            nvfp4_gemm_item& it = items[i];
+            it.alpha_a = nullptr;
+            if (!weight_of(PyList_GET_ITEM(a[3], i), &w) || !quantized_operand(PyList_GET_ITEM(a[0], i), PyList_GET_ITEM(a[1], i), &qa, &sa)) {
+                PyErr_Clear();
+                return none();
             }
-            PyList_SET_ITEM(l, i, o);
+            if (i == 0) {
+                m = qa->size(0);
+                dev = qa->device().index();
+            }
+            PyObject* alpha_a = PyList_GET_ITEM(a[2], i);
+            if (m == 0 || qa->size(0) != m || qa->device().index() != dev || w.device != dev || qa->size(1) * 2 != w.k ||
+                (alpha_a != Py_None && !scalar_input(alpha_a, dev, &it.alpha_a)) || !scalar_input(PyList_GET_ITEM(a[4], i), dev, &it.alpha_w))
+                return none();
+            out[i] = empty({m, w.n}, at::kBFloat16, dev);
+            it.weight = w.handle;
+            it.a = static_cast<const uint8_t*>(qa->const_data_ptr());
+            it.sfa = static_cast<const uint8_t*>(sa->const_data_ptr());
+            it.out_bf16 = out[i].mutable_data_ptr();
         }
-        return l;
+        const cudaStream_t s = current_stream(dev);
+        const int st = launch_on(dev, [&] { return nvfp4_gemm_launch_multi(items, static_cast<int>(count), m, s); });
+        return st == NVFP4_OK ? tensor_list(out) : none();
     });
 }
 
@@ -689,6 +734,7 @@ PyMethodDef kMethods[] = {
     FAST(scaled_mm),
     FAST(scaled_mm_prepared),
     FAST(scaled_mm_grouped),
+    FAST(scaled_mm_multi),
     FAST(chain_call),
     FAST(group_call),
     {"make_chain", make_chain, METH_VARARGS, nullptr},

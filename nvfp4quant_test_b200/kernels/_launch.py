@@ -96,38 +96,3 @@ def quant_out(variant: int, input: torch.Tensor, importance: torch.Tensor | None
     with _lib.device_guard(input.device):   # launch with the tensor's device current
         st = _lib.lib().nvfp4_quant_launch_impl(*args)
     _raise(st, "nvfp4_quant_launch")
-
-
-_fused_scratch = _lib.StreamScratch(4)
-
-
-def quant_fused_out(variant: int, input: torch.Tensor, importance: torch.Tensor | None, fp8_max: float,
-                    is_sf_swizzled_layout: bool, output: torch.Tensor, output_scale: torch.Tensor,
-                    lower: int, upper: int) -> torch.Tensor | None:
-    """Global scale and sweep in ONE launch (the tensor's blocks stay in registers across a grid-wide wait).
-    Returns a float32 [2] CUDA tensor (global_scale, 1 / global_scale), or None when the tensor does not fit the
-    resident grid of the device, in which case nothing was launched and the caller uses the two-launch path."""
-    if not isinstance(input, torch.Tensor) or input.ndim != 2:
-        raise ValueError(f"input must be 2D [num_row, dim], got {tuple(getattr(input, 'shape', ()))}")
-    if input.shape[-1] % BLOCK_SIZE != 0:
-        raise ValueError(f"input.shape[-1] must be divisible by {BLOCK_SIZE}")
-    if not input.is_cuda:
-        raise ValueError("input must be a CUDA tensor: these kernels have no CPU path")
-    if not input.is_contiguous():
-        input = input.contiguous()
-    m, n, physical_n = _check_outputs(input, is_sf_swizzled_layout, output, output_scale)
-    if m == 0 or n == 0:
-        raise ValueError("the global scale of an empty tensor is undefined")
-    imp_ptr, _keep = _importance_ptr(variant, importance)
-    stream = _lib.current_stream_ptr(input.device)
-    scratch = _fused_scratch.get(input.device, stream)
-    gs = torch.empty(2, dtype=torch.float32, device=input.device)
-    with _lib.device_guard(input.device):
-        st = _lib.lib().nvfp4_quant_fused_launch(
-            variant, input.data_ptr(), _lib.dtype_code(input.dtype), imp_ptr, float(fp8_max), gs.data_ptr(),
-            scratch.data_ptr(), output.data_ptr(), output_scale.data_ptr(), m, n, physical_n,
-            lower, upper, 1 if is_sf_swizzled_layout else 0, stream)
-    if st == _lib.ERR_TOO_LARGE:
-        return None
-    _raise(st, "nvfp4_quant_fused_launch")
-    return gs

@@ -207,6 +207,20 @@ def nvfp4_scaled_mm_grouped(a: torch.Tensor, block_scale_a: torch.Tensor, alpha_
     return outs
 
 
+def nvfp4_scaled_mm_multi(acts: list[torch.Tensor], block_scales: list[torch.Tensor], alpha_a: list[torch.Tensor | None],
+                          weights: list[PreparedWeight], alpha_w: list[torch.Tensor]) -> list[torch.Tensor]:
+    """[alpha_w[i] * alpha_a[i] * dq(acts[i]) @ dq(weights[i]).T for i]: products of equal M whose inputs are all at hand,
+    each with its own activation and K, in as few launches as the kernels allow (nvfp4_gemm_launch_multi: beyond decode
+    sizes one persistent launch for up to eight of them).  Bits as nvfp4_scaled_mm_grouped with one weight at a time."""
+    got = _lib.fast.scaled_mm_multi(acts, block_scales, alpha_a, [w._fast for w in weights], alpha_w)
+    if got is not None:
+        return got
+    if not len(acts) == len(block_scales) == len(alpha_a) == len(weights) == len(alpha_w):
+        raise ValueError("acts, block_scales, alpha_a, weights and alpha_w must have the same length")
+    return [nvfp4_scaled_mm_grouped(a, sa, aa, [w], [aw])[0]
+            for a, sa, aa, w, aw in zip(acts, block_scales, alpha_a, weights, alpha_w)]
+
+
 def cutlass_scaled_fp4_mm(a, b, block_scale_a, block_scale_b, alpha, out_dtype):
     """Drop-in name of the vllm op."""
     return nvfp4_scaled_mm(a, b, block_scale_a, block_scale_b, alpha, out_dtype)

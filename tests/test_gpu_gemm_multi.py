@@ -1,0 +1,70 @@
+"""GPU: one launch over several products gives the bits of the products launched one by one."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _operand(rows, k, seed):
+    import nvfp4quant_test_b200.kernels as K
+
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.randn((rows, k), generator=g, device="cuda").bfloat16()
+    codes, scales, gs, _ = K.scalesweep_nvfp4_quant_with_global_scale(x, 256.0)
+    return codes, scales, gs
+
+
+@pytest.mark.parametrize("path", [0, 1, 3, 4, 7])
+@pytest.mark.parametrize("m,shapes", [
+    (65, [(64, 64)] * 3),                                                        # tiles of one K stage, mostly padding
+    (129, [(257, 320), (1000, 1024), (128, 320), (72, 2560)]),                   # ragged N, three K classes
+    (300, [(4096, 4096), (1024, 4096), (1024, 4096), (4096, 4096), (2048, 4096), (4096, 14336)]),
+    (700, [(512, 256)] * 9 + [(4100, 1984), (256, 512)]),                        # more than one launch takes
+    (16, [(512, 1024), (256, 1024), (512, 320)]),                                # decode-sized: grouped by activation
+])
+def test_list_of_products_equals_one_by_one(cuda_lib, path, m, shapes):
+    import nvfp4quant_test_b200.kernels as K
+    from nvfp4quant_test_b200.kernels.kernel_gemm import gemm_last_status
+
+    if m <= 64 and path:
+        pytest.skip("the decode-sized kernel takes these")
+    acts = {k: _operand(m, k, m + k) for k in {k for _, k in shapes}}
+    weights = [_operand(n, k, 7 * i + n) for i, (n, k) in enumerate(shapes)]
+    prepared = [K.PreparedWeight(c, s) for c, s, _ in weights]
+    scale = [w[2].reshape(1) for w in weights]
+    use = [acts[k] for _, k in shapes]
+    want = [K.nvfp4_scaled_mm_grouped(a[0], a[1], a[2], [p], [s])[0] for a, p, s in zip(use, prepared, scale)]
+    try:
+        assert cuda_lib.nvfp4_gemm_force_path(path) == 0
+        got = K.nvfp4_scaled_mm_multi([a[0] for a in use], [a[1] for a in use], [a[2] for a in use], prepared, scale)
+        first = [i for i, (_, k) in enumerate(shapes) if k == shapes[0][1]]
+        grouped = K.nvfp4_scaled_mm_grouped(use[0][0], use[0][1], use[0][2], [prepared[i] for i in first], [scale[i] for i in first])
+        torch.cuda.synchronize()
+    finally:
+        cuda_lib.nvfp4_gemm_force_path(0)
+    assert gemm_last_status() == 0
+    if m > 64:      # K ranges per tile of the decode-sized kernel depend on the group
+        for g, w in zip(got, want):
+            assert torch.equal(g, w)
+        for g, i in zip(grouped, first):
+            assert torch.equal(g, want[i])
+    else:
+        for g, w in zip(got, want):
+            assert torch.allclose(g.float(), w.float(), rtol=2.0 ** -7, atol=float(w.abs().max()) * 2.0 ** -12)
+
+
+def test_list_arguments_are_checked(cuda_lib):
+    import nvfp4quant_test_b200.kernels as K
+
+    a, s, gs = _operand(80, 128, 1)
+    c, sw, gw = _operand(64, 128, 2)
+    w = K.PreparedWeight(c, sw)
+    with pytest.raises(ValueError, match="same length"):
+        K.nvfp4_scaled_mm_multi([a, a], [s], [gs], [w], [gw])
+    with pytest.raises(ValueError, match="disagree on K"):
+        K.nvfp4_scaled_mm_multi([a[:, :32].contiguous()], [s], [gs], [w], [gw])
+    assert cuda_lib.nvfp4_gemm_launch_multi(None, 1, 8, None) == -1
+    assert cuda_lib.nvfp4_gemm_launch_multi(None, 65, 8, None) == -5
+    w.close()
+    with pytest.raises(ValueError, match="closed"):
+        K.nvfp4_scaled_mm_multi([a], [s], [gs], [w], [gw])
