@@ -15,11 +15,15 @@
 // Mapping: one 16-element block per thread; a warp covers 32 consecutive blocks
 // of one row (1 KiB of bf16).  Three interchangeable loop bodies give identical
 // bytes: the scalar transcription (1), one candidate per trip with packed
-// multiplies and the mixed-precision subtract (2), and the default (3): two
+// multiplies and the mixed-precision subtract (2), and the default: two
 // candidates per trip whose FMA chains share one f32x2 instruction (each lane of
 // a packed instruction is an independent IEEE operation).
 //
-// Body 4 is body 3 with the tensor-wide global scale (helper.py:96-100: amax / (6 * fp8_max) and its reciprocal)
+// Bodies 3 and 7 to 9 are the default loop over different grids: 3 and 9 number the slots of the real rows through (9 in
+// small CTAs, for a few tokens), 7 and 8 have a two-dimensional grid for rows of whole chunks (8 for tensors without any
+// padding, without predicates).  (5 is another name of 3 and 6 of 7, for callers that ask for a body by number.)
+//
+// Body 4 is the default loop with the tensor-wide global scale (helper.py:96-100: amax / (6 * fp8_max) and its reciprocal)
 // computed inside the same launch: every thread keeps its block in registers, the CTAs combine their maxima
 // through a scratch word and wait for one another (cooperative launch: all CTAs are resident; the wait is bounded
 // by the global timer), then the sweep runs as usual.  x is read from HBM once and one launch replaces two; the
@@ -33,38 +37,32 @@ namespace nvfp4 {
 namespace {
 
 constexpr int kThreads = 256;
-// Resident CTAs per SM the register allocation aims for: the unweighted sweep fits 5 (48 registers) without
-// spilling; the weighted one keeps 16 importance weights live and needs 64 registers (4 CTAs).
-#ifndef NVFP4_QUANT_MIN_BLOCKS
-#define NVFP4_QUANT_MIN_BLOCKS 5
-#endif
-// The two-dimensional-grid body has less index arithmetic alive and takes one more CTA per SM (40 registers, a few
-// bytes of spill outside the loop): 121.1 -> 118.5 us at 8192 x 8192; the flat body gets slower with the same bound.
-// Weighted sweep, two-dimensional grid, at 8192 x 8192: 5 CTAs (48 registers, spills) 223 us, 4 CTAs (64) 192 us,
-// 3 CTAs (80) 199 us, 2 CTAs (90, importance pairs kept in registers) 205 us.
-#ifndef NVFP4_QUANT_MIN_BLOCKS_2D
-#define NVFP4_QUANT_MIN_BLOCKS_2D 6
-#endif
-#ifndef NVFP4_QUANT_MIN_BLOCKS_W2D
-#define NVFP4_QUANT_MIN_BLOCKS_W2D 4
-#endif
-// Body 9 (a few tokens): CTAs of 64 threads over the slots of the real rows only.  A 256-thread CTA puts two warps on
-// every scheduler of one SM, and a warp's sweep is ~750 instructions; 64-thread CTAs spread the same blocks over four
-// times as many SMs with at most one warp per scheduler.  The padding rows of the tiled scale layout (127 of 128 for
-// one token) get a few CTAs at the end of the grid that write their zero words.
+// The sweeps' bodies 3, 7 and 8 run in CTAs of 128 threads with up to 72 registers (7 CTAs, 28 warps per SM).  A large
+// sweep takes the same time with anything from 20 to 48 warps per SM (8192 x 8192, us, unweighted / weighted: 256 threads
+// at 40 registers 110.4 / 237, at 64 114.4 / 191; 128 threads at 96 registers 110.7 / 193, at 72 110.5 / 190.5): operand
+// reads from the register file bound it, not latency.  Below a few hundred tokens latency does, and there more registers
+// (independent work in flight per warp) and smaller CTAs (an even spread over the SMs) decide: 256 x 8192 7.2 -> 4.9 us
+// unweighted and 9.1 -> 7.9 weighted against 256 threads at 40 and 64 registers, 128 x 8192 5.4 -> 3.3 and 7.0 -> 5.1.
+constexpr int kSweepThreads = 128;
+constexpr int kSweepMinBlocks = 7;
+// Body 9 (few tokens): CTAs of 64 threads with up to 128 registers.  A warp's sweep is ~750 instructions; the smallest CTAs
+// spread the blocks over the most SMs.
 constexpr int kSmallThreads = 64;
-// Real 16-element blocks up to which body 9 is the default.  Measured in a chain of launches (us, body 9 against the
-// better of the other bodies): unweighted 1 x 4096 1.72 / 2.38, 1 x 14336 1.78 / 2.74, 32 x 8192 1.94 / 2.81, 64 x 8192
-// 2.50 / 2.84, 128 x 4096 2.55 / 2.54, 96 x 8192 3.57 / 3.37; weighted 1 x 8192 2.35 / 3.85, 48 x 8192 3.59 / 4.87,
-// 64 x 8192 3.61 / 4.07, 128 x 4096 3.59 / 3.40, 96 x 8192 6.39 / 5.28.
-constexpr int64_t kSmallBlocks = 32768;
-constexpr int64_t kSmallBlocksWeighted = 24576;
-__host__ __device__ constexpr int block_threads(int impl) { return impl == 9 ? kSmallThreads : kThreads; }
+// Real 16-element blocks up to which body 9 is the default, for rows of whole chunks (against body 7) and for others
+// (against body 3).  Measured in a chain of launches (us, body 9 / the other): whole chunks, unweighted 4 x 8192 1.92 / 2.03,
+// 32 x 8192 2.10 / 3.23, 96 x 4096 2.48 / 3.00, 40 x 8192 3.28 / 3.06, 128 x 8192 3.52 / 3.14; weighted 32 x 8192 2.90 / 5.23,
+// 40 x 8192 3.52 / 4.73, 48 x 8192 5.69 / 4.91, 128 x 8192 6.30 / 5.33.  Ragged rows, unweighted 77 x 5104 2.86 / 3.69, 300 x
+// 5104 4.85 / 5.05, 200 x 10000 5.52 / 5.09; weighted 150 x 5104 6.29 / 7.98, 500 x 10000 17.47 / 17.60.
+constexpr int64_t kSmallBlocks = 24576;
+constexpr int64_t kSmallBlocksRagged = 98304;
+constexpr int64_t kSmallBlocksRaggedWeighted = 327680;
+__host__ __device__ constexpr int block_threads(int variant, int impl) {
+    return impl == 9 ? kSmallThreads : (variant != NVFP4_VARIANT_AMAX && (impl == 3 || impl >= 7)) ? kSweepThreads : kThreads;
+}
 constexpr int min_blocks(int variant, int impl) {
     if (impl == 9) return 8;
-    return variant == NVFP4_VARIANT_WEIGHTED ? (impl >= 6 ? NVFP4_QUANT_MIN_BLOCKS_W2D : 4)
-           : (impl >= 6 && variant == NVFP4_VARIANT_MSE) ? NVFP4_QUANT_MIN_BLOCKS_2D
-                                                         : NVFP4_QUANT_MIN_BLOCKS;
+    if (block_threads(variant, impl) == kSweepThreads) return kSweepMinBlocks;
+    return variant == NVFP4_VARIANT_WEIGHTED ? 4 : 5;
 }
 
 struct QuantParams {
@@ -78,6 +76,7 @@ struct QuantParams {
     int64_t width, rows;    // slot grid: scale columns / rows that get written
     int64_t k_pad;          // padded scale columns (swizzled layout)
     int64_t total;          // rows * width
+    uint32_t div_mul, div_shift;  // division by width: see width_div
     int lower, ncand;
     int swizzled;
     // fused global-scale variant only
@@ -85,6 +84,18 @@ struct QuantParams {
     float* gs_out;          // [2]: global scale, its reciprocal
     uint32_t* fused_scratch;  // [4]: running maximum, arrivals, readers, unused; zero between calls
 };
+
+// n / width for n < 2^31, as (n * ceil(2^(32 + shift) / width)) >> (32 + shift) with 2^shift < width <= 2^(shift + 1): the
+// rounding of the multiplier adds less than n * width / 2^(32 + shift) < 1 / width to the quotient's fraction.
+inline void set_width_div(QuantParams& p) {
+    p.div_mul = p.div_shift = 0;
+    if (p.width <= 1 || p.width > 0x7fffffffLL) return;
+    while ((2ll << p.div_shift) < p.width) ++p.div_shift;
+    p.div_mul = static_cast<uint32_t>(((1ull << (32 + p.div_shift)) + p.width - 1) / p.width);
+}
+__device__ __forceinline__ uint32_t width_div(const QuantParams& p, uint32_t n) {
+    return p.width == 1 ? n : __umulhi(n, p.div_mul) >> p.div_shift;
+}
 
 __device__ uint32_t g_quant_status;   // 0 = ok; 1 = the grid-wide wait of the fused kernel gave up
 constexpr uint64_t kFusedWaitLimitNs = 2000000000ull;
@@ -353,9 +364,9 @@ __device__ __forceinline__ uint32_t sweep_single(const float v[16], const float 
 }
 
 template <int DT, int VARIANT, int IMPL>
-__global__ void __launch_bounds__(block_threads(IMPL), min_blocks(VARIANT, IMPL))
+__global__ void __launch_bounds__(block_threads(VARIANT, IMPL), min_blocks(VARIANT, IMPL))
 quant_kernel(const QuantParams p) {
-    constexpr int T = block_threads(IMPL);   // threads per CTA
+    constexpr int T = block_threads(VARIANT, IMPL);   // threads per CTA
     static_assert(kTabSize % T == 0, "every thread builds the same number of table entries");
     __shared__ float4 tab[kTabSize];
     constexpr bool FUSED = IMPL == 4;
@@ -371,22 +382,22 @@ quant_kernel(const QuantParams p) {
     const void* const x_in = after_wait(p.x);
     const float* const importance_in = after_wait(p.importance);
     float gs_inv = FUSED ? 0.0f : load_f32_after_wait(p.gs_inv);
-    // Body 6 = body 3 with a two-dimensional grid: blockIdx.x is the row, blockIdx.y the 256-block column chunk.
-    // The row is then uniform over the CTA, so the division below, the row part of the addresses and most of the
-    // tiled scale offset leave the per-thread instruction stream.  Used when the slot grid is a whole number of
-    // chunks wide (e.g. 512 blocks per row at 8192 columns); narrow or ragged widths keep the flat numbering.
-    constexpr bool GRID2D = IMPL == 6 || IMPL == 7 || IMPL == 8;   // 7 = 6 with the reference's candidate count compiled in
-    constexpr bool WHOLE = IMPL == 8;                              // 8 = 7 on tensors without any padding: no predicates
-    constexpr bool SMALL = IMPL == 9;   // threads for the slots of the real rows only (see the end of the kernel)
+    // Two-dimensional grid: blockIdx.x is the row, blockIdx.y the column chunk.  The row is then uniform over the CTA, so
+    // the division below, the row part of the addresses and most of the tiled scale offset leave the per-thread
+    // instruction stream (8192 x 8192 sweep: 126 us numbered through, 112 us with this grid).
+    constexpr bool GRID2D = IMPL == 7 || IMPL == 8;
+    constexpr bool WHOLE = IMPL == 8;
+    constexpr bool FLAT = IMPL == 3 || IMPL == 9;   // real rows' slots numbered through, then CTAs that fill the padding rows
     const int64_t id = GRID2D ? 0 : static_cast<int64_t>(blockIdx.x) * T + threadIdx.x;
-    const bool in_range = GRID2D ? true : id < (SMALL ? p.m * p.width : p.total);
+    const int64_t slots = FLAT ? p.m * p.width : p.total;
+    const bool in_range = GRID2D ? true : id < slots;
     int64_t row = 0, col = 0;
     if (GRID2D) {
         row = blockIdx.x;
-        col = static_cast<int64_t>(blockIdx.y) * kThreads + threadIdx.x;
+        col = static_cast<int64_t>(blockIdx.y) * T + threadIdx.x;
     } else if (in_range) {
-        if (p.total <= 0x7fffffffLL) {  // 32-bit division is several times cheaper than the 64-bit one
-            const uint32_t r32 = static_cast<uint32_t>(id) / static_cast<uint32_t>(p.width);
+        if (p.total <= 0x7fffffffLL) {
+            const uint32_t r32 = width_div(p, static_cast<uint32_t>(id));
             row = r32;
             col = static_cast<uint32_t>(id) - r32 * static_cast<uint32_t>(p.width);
         } else {
@@ -395,14 +406,18 @@ quant_kernel(const QuantParams p) {
         }
     }
     const bool valid = WHOLE ? true : (in_range && row < p.m && col < p.bout);
-    if (SMALL && static_cast<int64_t>(blockIdx.x) * T >= p.m * p.width) {
+    if (IMPL == 7 && row >= p.m) {   // a padding row of the tiled scale layout: zero words, nothing else
+        if ((threadIdx.x & 3) == 0) *reinterpret_cast<uint32_t*>(p.scales + swizzled_scale_offset(row, col, p.k_pad)) = 0u;
+        return;
+    }
+    if (FLAT && static_cast<int64_t>(blockIdx.x) * T >= slots) {
         // A CTA behind the real rows' slots.  The rows m .. rows-1 of the tiled scale layout (127 of 128 for one token)
         // hold no data; these CTAs write their zero scale bytes, four 32-bit words (of four columns each) per thread,
         // and leave before the candidate table is built.  (Rows beyond m exist only in the tiled layout, whose width is
         // a multiple of 4; the launcher sizes this part of the grid, and at most 127 rows are padding.)
         const uint32_t words_per_row = static_cast<uint32_t>(p.width >> 2);
         const uint32_t words = static_cast<uint32_t>(p.rows - p.m) * words_per_row;
-        const uint32_t real_ctas = static_cast<uint32_t>((p.m * p.width + T - 1) / T);
+        const uint32_t real_ctas = static_cast<uint32_t>((slots + T - 1) / T);
         const uint32_t fill_threads = (gridDim.x - real_ctas) * T;
         for (uint32_t wi = (blockIdx.x - real_ctas) * T + threadIdx.x; wi < words; wi += fill_threads) {
             const uint32_t r = wi / words_per_row;
@@ -495,11 +510,7 @@ quant_kernel(const QuantParams p) {
 
     uint32_t sbyte = 0;
     float inv = 0.0f;
-    // Body 5 = body 3 plus: a warp whose 32 slots are all padding (rows beyond m in the tiled scale layout: 127 of
-    // 128 rows for a single token) has nothing to sweep and only writes its zero scale bytes below.  A separate
-    // instantiation because the vote and branch cost the full-size kernel 6 % (8192 x 8192: 123.7 -> 131.8 us);
-    // the launcher picks it when at least a quarter of the slot grid is padding rows.
-    if ((IMPL == 5 || IMPL == 9) && !__any_sync(0xffffffffu, valid)) {
+    if (FLAT && !__any_sync(0xffffffffu, valid)) {   // only padding columns, or threads behind the last slot
         // nothing
     } else if (VARIANT == NVFP4_VARIANT_AMAX) {
         const float amax = max_abs16(v);
@@ -522,7 +533,8 @@ quant_kernel(const QuantParams p) {
         const int first_idx = min(max(base_raw + p.lower, -kTabPad), 127) + kTabPad;
         sbyte = (IMPL == 1)   ? sweep_scalar<W>(v, w, first_idx, p.ncand, tab)
                 : (IMPL == 2) ? sweep_single<W>(v, w, first_idx, p.ncand, tab)
-                : (IMPL == 7 || IMPL == 8 || (IMPL == 9 && p.ncand == (W ? 16 : 11)))
+                // the reference's own windows (11 candidates unweighted, 16 weighted) are compiled in, unrolled
+                : (WHOLE || ((IMPL == 7 || FLAT) && p.ncand == (W ? 16 : 11)))
                     ? sweep_paired<W, W ? 16 : 11>(v, w, first_idx, p.ncand, tab)
                     : sweep_paired<W>(v, w, first_idx, p.ncand, tab);
         // sbyte is 0 only when no candidate had a comparable (non-NaN, < inf) error: 1/0 as the reference computes it
@@ -558,54 +570,39 @@ quant_kernel(const QuantParams p) {
     }
 }
 
+// Grid of the bodies that number the real rows' slots through: CTAs for those, then CTAs that zero the padding rows' scale
+// words (4 words per thread).
+template <int DT, int VARIANT, int IMPL>
+cudaError_t launch_flat(const QuantParams& p, cudaStream_t stream) {
+    constexpr int T = block_threads(VARIANT, IMPL);
+    const int64_t pad_words = (p.rows - p.m) * (p.width >> 2);
+    if (pad_words > 0x7fffffffLL) return cudaErrorInvalidValue;   // at most 127 rows: a width beyond 2^26 columns
+    const int64_t grid = (p.m * p.width + T - 1) / T + (pad_words + 4 * T - 1) / (4 * T);
+    if (grid > 0x7fffffffLL) return cudaErrorInvalidValue;
+    return launch_dependent(quant_kernel<DT, VARIANT, IMPL>, static_cast<unsigned>(grid), dim3(T), 0, stream, p);
+}
 
 template <int DT, int VARIANT>
 cudaError_t launch_impl(int impl, const QuantParams& p, cudaStream_t stream) {
-    const int64_t grid = (p.total + kThreads - 1) / kThreads;
-    // body 8: tensors without padding whose rows are whole 256-block chunks (every slot of the scale layout is a
-    // real block): body 7 without its validity predicates
-    const bool whole = VARIANT != NVFP4_VARIANT_AMAX && p.rows == p.m && p.bin == p.bout && p.bout == p.width &&
-                       (p.width % kThreads) == 0 && p.width / kThreads <= 65535 && p.rows <= 0x7fffffffLL &&
-                       (VARIANT == NVFP4_VARIANT_MSE ? p.ncand == 11 : p.ncand == 16);
-    const bool small = VARIANT != NVFP4_VARIANT_AMAX &&
-                       p.m * p.bout <= (VARIANT == NVFP4_VARIANT_WEIGHTED ? kSmallBlocksWeighted : kSmallBlocks);
-    if constexpr (VARIANT != NVFP4_VARIANT_AMAX) {
-        if ((impl == 8 || (impl == 0 && !small)) && whole) {
-            const dim3 grid2(static_cast<unsigned>(p.rows), static_cast<unsigned>(p.width / kThreads));
-            return launch_dependent(quant_kernel<DT, VARIANT, 8>, grid2, dim3(kThreads), 0, stream, p);
-        }
+    constexpr bool kSweep = VARIANT != NVFP4_VARIANT_AMAX;
+    constexpr int T = block_threads(VARIANT, 7);
+    if (impl == 1 || impl == 2) {
+        const unsigned grid = static_cast<unsigned>((p.total + kThreads - 1) / kThreads);
+        return impl == 1 ? launch_dependent(quant_kernel<DT, VARIANT, 1>, grid, dim3(kThreads), 0, stream, p)
+                         : launch_dependent(quant_kernel<DT, VARIANT, 2>, grid, dim3(kThreads), 0, stream, p);
     }
-    // body 9: tensors of a few tokens (up to kSmallBlocks real blocks), where latency is all that matters
-    if (impl == 9 || (impl == 0 && small)) {
-        // CTAs for the slots of the real rows, then CTAs that zero the padding rows' scale words (4 words per thread)
-        const int64_t pad_words = (p.rows - p.m) * (p.width >> 2);
-        if (pad_words > 0x7fffffffLL) return cudaErrorInvalidValue;   // at most 127 rows: a width beyond 2^26 columns
-        const int64_t grid9 = (p.m * p.width + kSmallThreads - 1) / kSmallThreads +
-                              (pad_words + 4 * kSmallThreads - 1) / (4 * kSmallThreads);
-        if (grid9 > 0x7fffffffLL) return cudaErrorInvalidValue;
-        return launch_dependent(quant_kernel<DT, VARIANT, 9>, static_cast<unsigned>(grid9), dim3(kSmallThreads), 0, stream, p);
+    const bool chunks = (p.width % T) == 0 && p.width / T <= 65535 && p.rows <= 0x7fffffffLL;
+    const bool small = kSweep && p.m * p.bout <= (chunks ? kSmallBlocks : VARIANT == NVFP4_VARIANT_WEIGHTED ? kSmallBlocksRaggedWeighted : kSmallBlocksRagged);
+    if (impl == 9 || (impl == 0 && small)) return launch_flat<DT, VARIANT, 9>(p, stream);
+    if (chunks && impl != 3 && impl != 5) {
+        const dim3 grid2(static_cast<unsigned>(p.rows), static_cast<unsigned>(p.width / T));
+        // no padding anywhere: every slot of the scale layout is a real block
+        const bool whole = p.rows == p.m && p.bin == p.bout && p.bout == p.width && p.ncand == (VARIANT == NVFP4_VARIANT_MSE ? 11 : 16);
+        if constexpr (kSweep)
+            if (whole && (impl == 0 || impl == 8)) return launch_dependent(quant_kernel<DT, VARIANT, 8>, grid2, dim3(T), 0, stream, p);
+        return launch_dependent(quant_kernel<DT, VARIANT, 7>, grid2, dim3(T), 0, stream, p);
     }
-    if (impl >= 8) impl = 0;
-    cudaError_t e;
-    if (impl == 1)
-        e = launch_dependent(quant_kernel<DT, VARIANT, 1>, static_cast<unsigned>(grid), dim3(kThreads), 0, stream, p);
-    else if (impl == 2)
-        e = launch_dependent(quant_kernel<DT, VARIANT, 2>, static_cast<unsigned>(grid), dim3(kThreads), 0, stream, p);
-    else if (impl == 5 || (impl == 0 && (p.rows - p.m) * 4 >= p.rows))
-        e = launch_dependent(quant_kernel<DT, VARIANT, 5>, static_cast<unsigned>(grid), dim3(kThreads), 0, stream, p);
-    else if ((impl == 6 || impl == 7 || impl == 0) && (p.width % kThreads) == 0 && p.width / kThreads <= 65535 &&
-             p.rows <= 0x7fffffffLL) {
-        const dim3 grid2(static_cast<unsigned>(p.rows), static_cast<unsigned>(p.width / kThreads));
-        // the reference's own windows (11 candidates unweighted, 16 weighted) have an unrolled instantiation
-        const bool fixed = VARIANT == NVFP4_VARIANT_MSE ? p.ncand == 11 : VARIANT == NVFP4_VARIANT_WEIGHTED && p.ncand == 16;
-        if (fixed && (impl == 7 || (impl == 0 && VARIANT == NVFP4_VARIANT_MSE)))
-            e = launch_dependent(quant_kernel<DT, VARIANT, 7>, grid2, dim3(kThreads), 0, stream, p);
-        else
-            e = launch_dependent(quant_kernel<DT, VARIANT, 6>, grid2, dim3(kThreads), 0, stream, p);
-    }
-    else
-        e = launch_dependent(quant_kernel<DT, VARIANT, 3>, static_cast<unsigned>(grid), dim3(kThreads), 0, stream, p);
-    return e;
+    return launch_flat<DT, VARIANT, 3>(p, stream);
 }
 
 template <int DT>
@@ -639,6 +636,7 @@ extern "C" int nvfp4_quant_launch_impl(int impl, int variant, const void* x, int
     p.width = swizzled ? p.k_pad : p.bout;
     p.rows = swizzled ? round_up_i64(m, 128) : m;
     p.total = p.rows * p.width;
+    set_width_div(p);
     if (p.total == 0) return NVFP4_OK;
     if ((p.total + kThreads - 1) / kThreads > 0x7fffffffLL) return NVFP4_ERR_TOO_LARGE;
     if (!gs_inv || !codes || !scales || (!x && m * n > 0)) return NVFP4_ERR_NULL_POINTER;
@@ -726,6 +724,7 @@ extern "C" int nvfp4_quant_fused_launch(int variant, const void* x, int x_dtype,
     p.width = swizzled ? p.k_pad : p.bout;
     p.rows = swizzled ? round_up_i64(m, 128) : m;
     p.total = p.rows * p.width;
+    set_width_div(p);
     if (p.total == 0 || m * n == 0) return NVFP4_ERR_BAD_SHAPE;   // an empty tensor has no maximum
     if (!gs_out || !scratch || !codes || !scales || !x) return NVFP4_ERR_NULL_POINTER;
     if (variant == NVFP4_VARIANT_WEIGHTED && !importance) return NVFP4_ERR_NULL_POINTER;

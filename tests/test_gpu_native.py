@@ -147,3 +147,29 @@ def test_scale_layouts_and_dequantization_equal_torch(cuda_lib, m, n, dtype):
         assert have.shape == want.shape and torch.equal(have.isnan(), want.isnan())
         assert torch.equal(have[~want.isnan()].view(torch.int32), want[~want.isnan()].view(torch.int32))
     assert _lib.fast.dequant(codes.cuda(), fp8.cuda(), gs.cuda()) is not None and _lib.fast.scale_layout(got, m, n // 16, False) is not None
+
+
+@pytest.mark.parametrize("m,n,padded_n,tiled", [(129, 16, None, False), (300, 32, None, True), (77, 48, None, False), (3, 112, 176, True),
+                                                (127, 2048, None, True), (129, 2048, 4096, True), (1, 6144, None, True),
+                                                (200, 2064, None, True), (45, 6128, 6144, False)])
+def test_quantizer_grids_equal_the_scalar_body(cuda_lib, m, n, padded_n, tiled):
+    """Every grid (slots numbered through in two CTA sizes, rows of whole chunks with and without padding) against the scalar
+    transcription, at widths where the division by the row length and the padding can go wrong."""
+    from nvfp4quant_test_b200 import _lib
+
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    x = torch.randn((m, n), generator=g, device="cuda").bfloat16()
+    imp = torch.rand((1, n), generator=g, device="cuda")
+    gs_inv = torch.tensor([37.5], device="cuda")
+    p = padded_n or n
+    size = (m + 127) // 128 * 128 * ((p // 16 + 3) // 4 * 4) if tiled else m * p // 16
+    for variant, lower, upper in ((0, -3, 7), (0, -2, 5), (1, -8, 7), (1, -1, 1)):
+        want = None
+        for impl in (1, 0, 3, 7, 8, 9):
+            codes = torch.full((m, p // 2), 0xA5, dtype=torch.uint8, device="cuda")
+            scales = torch.full((size,), 0xA5, dtype=torch.uint8, device="cuda")
+            _lib.check(cuda_lib.nvfp4_quant_launch_impl(impl, variant, x.data_ptr(), 0, imp.data_ptr(), gs_inv.data_ptr(), codes.data_ptr(),
+                                                        scales.data_ptr(), m, n, p, lower, upper, int(tiled), None), "launch")
+            torch.cuda.synchronize()
+            want = want or (codes, scales)
+            assert torch.equal(codes, want[0]) and torch.equal(scales, want[1]), (impl, variant, lower)
