@@ -117,13 +117,26 @@ int nvfp4_quant_fused_launch(int variant, const void* x, int x_dtype, const floa
                              float* gs_out, uint32_t* scratch, uint8_t* codes, uint8_t* scales, int64_t m, int64_t n,
                              int64_t padded_n, int lower, int upper, int swizzled, void* stream);
 /*
- * The same two steps as two launches from ONE host call (global scale kernel, then the quantizer reading gs_out[1]):
- * for callers that pay per host call, e.g. an eager decode loop.  Any variant (amax included), any size; `scratch` = the
- * 2 zeroed uint32 of nvfp4_global_scale_launch.  Bytes and scales equal the two separate calls.
+ * The same two steps from ONE host call, for callers that pay per host call, e.g. an eager decode loop: global scale
+ * kernel, then the quantizer reading gs_out[1]; a tensor of a few tokens takes one launch.  Any variant (amax included), any
+ * size; `scratch` = the 2 zeroed uint32 of nvfp4_global_scale_launch.  Bytes and scales equal the two separate calls.
  */
 int nvfp4_quant_chain_launch(int variant, const void* x, int x_dtype, const float* importance, float fp8_max,
                              float* gs_out, uint32_t* scratch, uint8_t* codes, uint8_t* scales, int64_t m, int64_t n,
                              int64_t padded_n, int lower, int upper, int swizzled, void* stream);
+/* nvfp4_quant_chain_launch over several tensors of one dtype (a layer's activations), up to four per launch.  n_items <= 64.
+ * Each item has the arguments of the single form and its own scratch words. */
+typedef struct {
+    const void* x;
+    const float* importance;   /* WEIGHTED only, else NULL */
+    float* gs_out;
+    uint32_t* scratch;
+    uint8_t* codes;
+    uint8_t* scales;
+    int64_t m, n, padded_n;
+} nvfp4_chain_item;
+int nvfp4_quant_chain_multi_launch(int variant, int x_dtype, float fp8_max, const nvfp4_chain_item* items_host, int n_items,
+                                   int lower, int upper, int swizzled, void* stream);
 /* Synchronises `stream`; *status = 0, or 1 if a fused launch on this device gave up its grid-wide wait (its
  * outputs are then invalid and its scratch must be zeroed again).  Reading a non-zero status clears it. */
 int nvfp4_quant_fused_last_status(void* stream, uint32_t* status);

@@ -22,7 +22,8 @@ DT_BF16, DT_F16, DT_F32 = 0, 1, 2
 ERR_TOO_LARGE = -8
 
 EXPORTS = (
-    "nvfp4_quant_launch", "nvfp4_quant_launch_impl", "nvfp4_quant_fused_launch", "nvfp4_quant_chain_launch", "nvfp4_quant_fused_last_status",
+    "nvfp4_quant_launch", "nvfp4_quant_launch_impl", "nvfp4_quant_fused_launch", "nvfp4_quant_chain_launch", "nvfp4_quant_chain_multi_launch",
+    "nvfp4_quant_fused_last_status",
     "nvfp4_global_scale_launch", "nvfp4_global_scale_launch_static", "nvfp4_global_scale_static_max_bytes",
     "nvfp4_channel_sqnorm_launch", "nvfp4_channel_sqnorm_launch_strided", "nvfp4_gemm_peak_probe", "nvfp4_gemm_set_wait_limit_ns", "nvfp4_quant_fused_set_wait_limit_ns",
     "nvfp4_gemm_launch", "nvfp4_gemm_workspace_bytes", "nvfp4_gemm_prepare", "nvfp4_gemm_launch_prepared", "nvfp4_gemm_launch_grouped", "nvfp4_gemm_launch_multi", "nvfp4_gemm_release", "nvfp4_gemm_last_status", "nvfp4_gemm_force_path", "nvfp4_gemm_tune", "nvfp4_gemm_tune_raster", "nvfp4_gemm_tune_pdl", "nvfp4_gemm_plan",
@@ -39,8 +40,9 @@ def _not_common(*_args):
 
 
 fast = types.SimpleNamespace(**{name: _not_common for name in (
-    "quant_impl", "quant_out", "quant_dynamic", "global_scale", "channel_square_norm", "scaled_mm", "scaled_mm_prepared",
-    "scaled_mm_grouped", "scaled_mm_multi", "dequant", "scale_layout", "make_chain", "chain_call", "make_group", "group_call")})
+    "quant_impl", "quant_out", "quant_dynamic", "quant_dynamic_multi", "global_scale", "channel_square_norm", "scaled_mm", "scaled_mm_prepared",
+    "scaled_mm_grouped", "scaled_mm_multi", "dequant", "scale_layout", "make_chain", "chain_call", "make_group", "group_call", "make_program",
+    "program_call")})
 
 
 def _bind_native() -> None:
@@ -89,6 +91,8 @@ def lib() -> ctypes.CDLL:
         L.nvfp4_quant_fused_launch.argtypes = [ci, vp, ci, vp, f32, vp, vp, vp, vp, i64, i64, i64, ci, ci, ci, vp]
         L.nvfp4_quant_chain_launch.restype = ci
         L.nvfp4_quant_chain_launch.argtypes = [ci, vp, ci, vp, f32, vp, vp, vp, vp, i64, i64, i64, ci, ci, ci, vp]
+        L.nvfp4_quant_chain_multi_launch.restype = ci
+        L.nvfp4_quant_chain_multi_launch.argtypes = [ci, ci, f32, vp, ci, ci, ci, ci, vp]
         L.nvfp4_quant_fused_last_status.restype = ci
         L.nvfp4_quant_fused_last_status.argtypes = [vp, vp]
         L.nvfp4_global_scale_launch.restype = ci

@@ -140,6 +140,17 @@ inline cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 b
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
+// One tensor of a global-scale launch (global_scale.cu): out = (amax / (6 * fp8_max), its reciprocal), scratch = two zeroed words.
+struct GsItem {
+    const void* x;
+    int64_t numel;
+    float* out;
+    uint32_t* scratch;
+};
+int check_global_scale(const GsItem& item, int x_dtype);
+// 1 <= n <= 4 tensors of one dtype in one launch
+int launch_global_scales(const GsItem* items, int n, int x_dtype, float fp8_max, cudaStream_t stream);
+
 // Byte offset of block (row, col) in the 128x4-tiled scale layout.
 __host__ __device__ inline int64_t swizzled_scale_offset(int64_t row, int64_t col, int64_t k_pad) {
     return (row >> 7) * (k_pad * 128) + (col >> 2) * 512 + (row & 31) * 16 + ((row & 127) >> 5) * 4 + (col & 3);

@@ -247,10 +247,10 @@ static int gemm_launch_impl(const uint8_t* a, const uint8_t* b, const uint8_t* s
     plan_gemm(M, N, K, sms, p.k_splits, &path, &ranges);
     if (path == 5) {
         const int forced = g_gemm_force_path == 5 ? g_gemm_force_splits : 0;
-        if (M <= 16) return gemm::skinny::launch_skinny<16>(a, b, p, forced, s, wh);
-        if (M <= 32) return gemm::skinny::launch_skinny<32>(a, b, p, forced, s, wh);
-        if (M <= 64) return gemm::skinny::launch_skinny<64>(a, b, p, forced, s, wh);
-        return gemm::skinny::launch_skinny<128>(a, b, p, forced, s, wh);
+        if (M <= 16) return gemm::skinny::launch_skinny<16>(p, forced, s, wh);
+        if (M <= 32) return gemm::skinny::launch_skinny<32>(p, forced, s, wh);
+        if (M <= 64) return gemm::skinny::launch_skinny<64>(p, forced, s, wh);
+        return gemm::skinny::launch_skinny<128>(p, forced, s, wh);
     }
     if (p.k_splits > 1) {
         const size_t need = static_cast<size_t>(p.k_splits) * static_cast<size_t>(M) * static_cast<size_t>(N) * sizeof(float);
@@ -376,6 +376,21 @@ extern "C" int nvfp4_gemm_launch_prepared(void* handle, const uint8_t* a, const 
     return gemm_launch_impl(a, h->b, sfa, h->sfb, alpha, out_bf16, M, h->N, h->K, workspace, workspace_bytes, stream, h);
 }
 
+// Products of equal M in launches of the decode-sized kernel, kMaxGroup at a time.
+static int launch_skinny_items(int M, const nvfp4::gemm::skinny::SkinnyItem* items, int n, cudaStream_t s) {
+    using namespace nvfp4::gemm::skinny;
+    const int forced = g_gemm_force_path == 5 ? g_gemm_force_splits : 0;
+    for (int first = 0; first < n; first += kMaxGroup) {
+        const int c = n - first < kMaxGroup ? n - first : kMaxGroup;
+        const int st = M <= 16   ? launch_skinny_group<16>(M, items + first, c, forced, s)
+                       : M <= 32 ? launch_skinny_group<32>(M, items + first, c, forced, s)
+                       : M <= 64 ? launch_skinny_group<64>(M, items + first, c, forced, s)
+                                 : launch_skinny_group<128>(M, items + first, c, forced, s);
+        if (st != NVFP4_OK) return st;
+    }
+    return NVFP4_OK;
+}
+
 // One activation against several prepared weights of equal K, e.g. a layer's q / k / v projections:
 //   outs[i][M, N_i] = alpha_w[i][0] * alpha_a[0] * dq(a) dq(weight_i)^T      (alpha_a may be NULL: factor 1)
 // One launch per 8 weights: of the decode-sized kernel at batches and shapes it is chosen for, of a tile or pair kernel
@@ -417,29 +432,12 @@ extern "C" int nvfp4_gemm_launch_grouped(void* const* handles, int n_weights, co
         if (M <= 64 && g_gemm_force_path == 0 && g_gemm_force_splits == 0) path = 5;
     }
     if (path == 5) {
-        const int forced = g_gemm_force_path == 5 ? g_gemm_force_splits : 0;
-        const int64_t stride = round_up_i64(K / 16, 4) * 128;
-        for (int first = 0; first < n_weights; first += gemm::skinny::kMaxGroup) {
-            const int n = n_weights - first < gemm::skinny::kMaxGroup ? n_weights - first : gemm::skinny::kMaxGroup;
-            gemm::skinny::SkinnyItem items[gemm::skinny::kMaxGroup];
-            for (int i = 0; i < n; ++i) {
-                auto* h = static_cast<const gemm::WeightHandle*>(handles[first + i]);
-                items[i].w = h->b;
-                items[i].sfw = h->sfb;
-                items[i].alpha = alpha_w[first + i];
-                items[i].out = static_cast<__nv_bfloat16*>(outs_bf16[first + i]);
-                items[i].N = h->N;
-                items[i].wh = h;
-            }
-            const int m = static_cast<int>(M), k = static_cast<int>(K);
-            int st;
-            if (M <= 16) st = gemm::skinny::launch_skinny_group<16>(a, sfa, alpha_a, m, k, stride, items, n, forced, s);
-            else if (M <= 32) st = gemm::skinny::launch_skinny_group<32>(a, sfa, alpha_a, m, k, stride, items, n, forced, s);
-            else if (M <= 64) st = gemm::skinny::launch_skinny_group<64>(a, sfa, alpha_a, m, k, stride, items, n, forced, s);
-            else st = gemm::skinny::launch_skinny_group<128>(a, sfa, alpha_a, m, k, stride, items, n, forced, s);
-            if (st != NVFP4_OK) return st;
+        gemm::skinny::SkinnyItem items[64];
+        for (int i = 0; i < n_weights; ++i) {
+            auto* h = static_cast<const gemm::WeightHandle*>(handles[i]);
+            items[i] = {a, sfa, alpha_a, h->b, h->sfb, alpha_w[i], static_cast<__nv_bfloat16*>(outs_bf16[i]), h->N, K, h};
         }
-        return NVFP4_OK;
+        return launch_skinny_items(static_cast<int>(M), items, n_weights, s);
     }
     gemm::GemmParams list[64];
     const gemm::WeightHandle* wh[64];
@@ -472,27 +470,22 @@ extern "C" int nvfp4_gemm_launch_multi(const nvfp4_gemm_item* items, int n_items
         if (st != NVFP4_OK) return st;
     }
     if (M == 0) return NVFP4_OK;
-    if (M > 64) return gemm_launch_list(list, wh, n_items, stream);
-    // decode-sized: items that share activation and scale go out as one grouped launch of the decode-sized kernel
-    bool done[64] = {false};
+    // with different K, beyond 24 tokens one launch of a tile kernel over the list is faster than the decode-sized kernel (Llama-3-8B layer, all
+    // seven matrices, us, tile kernel / decode-sized kernel: 16 tokens 26.2 / 24.5, 24: 26.6 / 25.7, 32: 26.5 / 26.9, 48: 25.9 / 31.6)
+    bool mixed = false;
+    for (int i = 1; i < n_items; ++i) mixed = mixed || list[i].K != list[0].K;
+    if (M > (mixed ? 24 : 64) || n_items == 1 || (g_gemm_force_path != 0 && g_gemm_force_path != 5))
+        return gemm_launch_list(list, wh, n_items, stream);
+    // decode-sized: one launch of the decode-sized kernel per 8 products, longest K first
+    gemm::skinny::SkinnyItem s_items[64];
     for (int i = 0; i < n_items; ++i) {
-        if (done[i]) continue;
-        void *handles[64], *outs[64];
-        const float* alphas[64];
-        int n = 0;
-        for (int j = i; j < n_items; ++j) {
-            if (done[j] || items[j].a != items[i].a || items[j].sfa != items[i].sfa || items[j].alpha_a != items[i].alpha_a ||
-                wh[j]->K != wh[i]->K)
-                continue;
-            done[j] = true;
-            handles[n] = items[j].weight;
-            outs[n] = items[j].out_bf16;
-            alphas[n++] = items[j].alpha_w;
-        }
-        const int st = nvfp4_gemm_launch_grouped(handles, n, items[i].a, items[i].sfa, items[i].alpha_a, alphas, outs, M, stream);
-        if (st != NVFP4_OK) return st;
+        const gemm::GemmParams& p = list[i];
+        const gemm::skinny::SkinnyItem it = {p.a, p.sfa, p.alpha2, p.b, p.sfb, p.alpha, p.out, p.N, p.K, wh[i]};
+        int j = i;
+        for (; j > 0 && s_items[j - 1].K < it.K; --j) s_items[j] = s_items[j - 1];
+        s_items[j] = it;
     }
-    return NVFP4_OK;
+    return launch_skinny_items(static_cast<int>(M), s_items, n_items, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int nvfp4_gemm_last_status(void* stream, uint32_t* status_host) {

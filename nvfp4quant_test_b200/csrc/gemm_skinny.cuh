@@ -57,25 +57,25 @@ __device__ __forceinline__ void bulk_copy_to_cta(uint32_t dst_cluster, uint32_t 
                  : "memory");
 }
 
-// One launch may multiply the same token tile with several weight matrices of equal K (a layer's q / k / v, or gate /
-// up projections): the weight tiles of all of them are numbered through, and a CTA looks up whose tile it owns.  The
-// launch's fixed costs (prologue, ramp-up and drain of the weight stream) are then paid once per group.
+// One launch may hold several products of equal M (a layer's q / k / v, or gate / up projections, or all of its matrices):
+// the weight tiles of all of them are numbered through, and a CTA looks up whose tile it owns.  The launch's fixed costs
+// (prologue, ramp-up and drain of the weight stream) are then paid once per group.
 constexpr int kMaxGroup = 8;
 
 struct SkinnyWeight {
     const uint8_t* sfw;   // weight scales
+    const uint8_t* sfx;   // token scales (group 0 of the tiled layout)
+    const float* alpha_x; // optional second factor of the output scale
     const float* alpha;   // output scale of this weight (times alpha_x when that is given)
     __nv_bfloat16* out;   // [M, N]
-    int N;
+    int N, K;
+    int k_tiles_per_rank;
+    int64_t sf_group_stride;
     int tile_end;         // number of 128-row tiles of this and all earlier weights of the group
 };
 
 struct SkinnyParams {
-    const uint8_t* sfx;   // token scales (group 0 of the tiled layout)
-    const float* alpha_x; // optional common factor of every output scale
-    int M, K;
-    int64_t sf_group_stride;
-    int k_tiles_per_rank;
+    int M;
     int stages;
     int n_weights;
     int weights_ready;    // != 0: all weights are prepared weights (constant while in use): read them before griddep_wait()
@@ -84,11 +84,12 @@ struct SkinnyParams {
 
 struct SkinnyMaps {
     CUtensorMap m[kMaxGroup];   // one per weight: [N, K/2] bytes in boxes of 128 rows x 128 bytes
+    CUtensorMap x[kMaxGroup];   // its activation: [M, K/2] bytes in boxes of BT rows
 };
 
 template <int BT>
 __global__ void __launch_bounds__(kThreads)
-skinny_kernel(const __grid_constant__ SkinnyMaps maps, const __grid_constant__ CUtensorMap tmap_x, const SkinnyParams p) {
+skinny_kernel(const __grid_constant__ SkinnyMaps maps, const __grid_constant__ SkinnyParams p) {
     using C = SkinnyCfg<BT>;
     extern __shared__ uint8_t smem_raw[];
     // The kernel queued behind this one may be scheduled at once: ahead of its own wait it reads nothing but a
@@ -118,8 +119,10 @@ skinny_kernel(const __grid_constant__ SkinnyMaps maps, const __grid_constant__ C
     while (gi + 1 < p.n_weights && tile >= p.w[gi].tile_end) ++gi;
     const int nt = tile - (gi > 0 ? p.w[gi - 1].tile_end : 0);
     const CUtensorMap* tmap_w = &maps.m[gi];
-    const uint8_t* const sfw = p.w[gi].sfw;
-    const int N = p.w[gi].N;
+    const CUtensorMap* tmap_x = &maps.x[gi];
+    const uint8_t *const sfw = p.w[gi].sfw, *const sfx = p.w[gi].sfx;
+    const int N = p.w[gi].N, K = p.w[gi].K;
+    const int64_t sf_group_stride = p.w[gi].sf_group_stride;
     // reduce-scatter: token column c belongs to rank c / cols_per_rank
     const uint32_t m_cols = static_cast<uint32_t>(min(p.M, BT));
     const uint32_t cols_per_rank = (m_cols + ranks - 1) / ranks;
@@ -140,9 +143,9 @@ skinny_kernel(const __grid_constant__ SkinnyMaps maps, const __grid_constant__ C
         // the cluster barrier below the main loop)
         if (ranks > 1 && my_cols > 0) mbar_expect_tx(recv_bar, (ranks - 1) * my_cols * 512u);
     }
-    const int k_tiles = (p.K + kBK - 1) / kBK;
-    const int kt_begin = static_cast<int>(rank) * p.k_tiles_per_rank;
-    const int kcount = max(0, min(k_tiles, kt_begin + p.k_tiles_per_rank) - kt_begin);   // host: never 0
+    const int k_tiles = (K + kBK - 1) / kBK;
+    const int kt_begin = static_cast<int>(rank) * p.w[gi].k_tiles_per_rank;
+    const int kcount = max(0, min(k_tiles, kt_begin + p.w[gi].k_tiles_per_rank) - kt_begin);   // host: never 0
 
     // Producer state (warp 0).  The first ring-full of copies is issued BEFORE the CTA-wide barrier of the prologue:
     // the copies need the mbarriers (initialised by this warp's thread 0 just above) but neither TMEM nor the other
@@ -157,17 +160,17 @@ skinny_kernel(const __grid_constant__ SkinnyMaps maps, const __grid_constant__ C
             const int stage = p_stage;
             const uint32_t phase = p_phase;
             if (!(p_ok = mbar_wait_warp(empty_bar(stage), phase ^ 1u, abort_flag, (7u << 24) | kt))) break;
-            const int kb_count = min(4, (p.K - kt * kBK + 63) / 64);
+            const int kb_count = min(4, (K - kt * kBK + 63) / 64);
             const uint32_t sf_bytes = 512u * kb_count;
             const uint32_t sbase = base + stage * C::kStageBytes;
             if (issuer) {
                 mbar_expect_tx(full_bar(stage), C::kWBytes + C::kXBytes + 2 * sf_bytes);
                 tma_load_2d(sbase, tmap_w, kt * kBKBytes, nt * 128, full_bar(stage));
-                tma_load_2d(sbase + C::kWBytes, &tmap_x, kt * kBKBytes, 0, full_bar(stage));
+                tma_load_2d(sbase + C::kWBytes, tmap_x, kt * kBKBytes, 0, full_bar(stage));
                 bulk_load_1d(sbase + C::kWBytes + C::kXBytes,
-                             sfw + static_cast<int64_t>(nt) * p.sf_group_stride + static_cast<int64_t>(kt) * 2048, sf_bytes,
+                             sfw + static_cast<int64_t>(nt) * sf_group_stride + static_cast<int64_t>(kt) * 2048, sf_bytes,
                              full_bar(stage));
-                bulk_load_1d(sbase + C::kWBytes + C::kXBytes + C::kSfBytes, p.sfx + static_cast<int64_t>(kt) * 2048, sf_bytes,
+                bulk_load_1d(sbase + C::kWBytes + C::kXBytes + C::kSfBytes, sfx + static_cast<int64_t>(kt) * 2048, sf_bytes,
                              full_bar(stage));
             }
             __syncwarp();
@@ -181,7 +184,7 @@ skinny_kernel(const __grid_constant__ SkinnyMaps maps, const __grid_constant__ C
         __syncwarp();   // thread 0's barrier initialisation above, before any lane of this warp uses the barriers
         if (elect_one()) {
             asm volatile("prefetch.tensormap [%0];" ::"l"(tmap_w) : "memory");
-            asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_x) : "memory");
+            asm volatile("prefetch.tensormap [%0];" ::"l"(tmap_x) : "memory");
         }
         // First ring-full.  The weights do not depend on whatever ran before this kernel on the stream, the token tile
         // and its scales (the quantizer's output) do: with a programmatic dependent launch the weight copies go out
@@ -192,12 +195,12 @@ skinny_kernel(const __grid_constant__ SkinnyMaps maps, const __grid_constant__ C
         if (issuer) {
             for (int i = 0; i < first; ++i) {
                 const int kt = kt_begin + i;
-                const uint32_t sf_bytes = 512u * min(4, (p.K - kt * kBK + 63) / 64);
+                const uint32_t sf_bytes = 512u * min(4, (K - kt * kBK + 63) / 64);
                 const uint32_t sbase = base + i * C::kStageBytes;
                 mbar_expect_tx(full_bar(i), C::kWBytes + C::kXBytes + 2 * sf_bytes);
                 tma_load_2d(sbase, tmap_w, kt * kBKBytes, nt * 128, full_bar(i));
                 bulk_load_1d(sbase + C::kWBytes + C::kXBytes,
-                             sfw + static_cast<int64_t>(nt) * p.sf_group_stride + static_cast<int64_t>(kt) * 2048, sf_bytes,
+                             sfw + static_cast<int64_t>(nt) * sf_group_stride + static_cast<int64_t>(kt) * 2048, sf_bytes,
                              full_bar(i));
             }
         }
@@ -205,10 +208,10 @@ skinny_kernel(const __grid_constant__ SkinnyMaps maps, const __grid_constant__ C
         if (issuer) {
             for (int i = 0; i < first; ++i) {
                 const int kt = kt_begin + i;
-                const uint32_t sf_bytes = 512u * min(4, (p.K - kt * kBK + 63) / 64);
+                const uint32_t sf_bytes = 512u * min(4, (K - kt * kBK + 63) / 64);
                 const uint32_t sbase = base + i * C::kStageBytes;
-                tma_load_2d(sbase + C::kWBytes, &tmap_x, kt * kBKBytes, 0, full_bar(i));
-                bulk_load_1d(sbase + C::kWBytes + C::kXBytes + C::kSfBytes, p.sfx + static_cast<int64_t>(kt) * 2048, sf_bytes,
+                tma_load_2d(sbase + C::kWBytes, tmap_x, kt * kBKBytes, 0, full_bar(i));
+                bulk_load_1d(sbase + C::kWBytes + C::kXBytes + C::kSfBytes, sfx + static_cast<int64_t>(kt) * 2048, sf_bytes,
                              full_bar(i));
             }
         }
@@ -243,7 +246,7 @@ skinny_kernel(const __grid_constant__ SkinnyMaps maps, const __grid_constant__ C
         for (int i = 0; i < kcount; ++i) {
             if (!(ok = mbar_wait_warp(full_bar(stage), phase, abort_flag, (8u << 24) | i))) break;
             tc_fence_after();
-            const int kb_count = min(4, (p.K - (kt_begin + i) * kBK + 63) / 64);
+            const int kb_count = min(4, (K - (kt_begin + i) * kBK + 63) / 64);
             const uint32_t sbase = base + stage * C::kStageBytes;
             const uint32_t w_lo = ((sbase & 0x3ffffu) >> 4) | (1u << 16);
             const uint32_t x_lo = w_lo + (C::kWBytes >> 4);
@@ -286,7 +289,7 @@ skinny_kernel(const __grid_constant__ SkinnyMaps maps, const __grid_constant__ C
     const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(sp * 32) << 16);
     if (ranks == 1) {
         if (warp >= 2 && have) {
-            const float alpha = load_alpha(p.w[gi].alpha, p.alpha_x);
+            const float alpha = load_alpha(p.w[gi].alpha, p.w[gi].alpha_x);
             __nv_bfloat16* const out = p.w[gi].out;
 #pragma unroll 1
             for (int c = 0; c < BT / 16 && c * 16 < p.M; ++c) {
@@ -334,7 +337,7 @@ skinny_kernel(const __grid_constant__ SkinnyMaps maps, const __grid_constant__ C
             bool ok = mbar_wait(recv_bar, 0, abort_flag, (10u << 24) | nt);
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
             if (ok && n < N) {
-                const float alpha = load_alpha(p.w[gi].alpha, p.alpha_x);
+                const float alpha = load_alpha(p.w[gi].alpha, p.w[gi].alpha_x);
                 // this rank's own partial sits in `recv` terms at part[my_first ..]; eight columns at a time so that
                 // the shared-memory loads of one rank's partials are in flight together
                 const float* own = part + my_first * 128 + n_local;
@@ -396,23 +399,27 @@ static int choose_ranks(int n_tiles, int k_tiles, int sms, int forced, int bt) {
 
 // One weight of a grouped launch, as the host sees it.
 struct SkinnyItem {
+    const uint8_t* x;         // codes [M, K/2]
+    const uint8_t* sfx;       // tiled scales
+    const float* alpha_x;     // or NULL
     const uint8_t* w;         // codes [N, K/2]
     const uint8_t* sfw;       // tiled scales
     const float* alpha;
     __nv_bfloat16* out;       // [M, N]
-    int64_t N;
+    int64_t N, K;
     const WeightHandle* wh;   // prepared tensor maps, or NULL
 };
 
 // Ring depth: the deepest ring with which the whole grid is resident at once (as many CTAs per SM as that takes, at
 // most what the TMEM columns allow), since a CTA that has to wait for a free SM starts its weight stream late.
 template <int BT>
-static int choose_stages(int ctas, int sms) {
+static int choose_stages(int ctas, int sms, int max_per_sm) {
     using C = SkinnyCfg<BT>;
     constexpr int kMaxPerSm = kTmemCols / C::kTmemCols;
     int per_sm = (ctas + sms - 1) / sms;
     if (per_sm < 1) per_sm = 1;
     if (per_sm > kMaxPerSm) per_sm = kMaxPerSm;
+    if (per_sm > max_per_sm) per_sm = max_per_sm;
     // an SM has 233472 bytes of shared memory, of which 1 KiB per resident CTA is reserved; a CTA asks for its ring
     // plus 1 KiB of alignment slack plus 256 bytes of barriers
     int stages = (233472 / per_sm - 1024 - 1024 - 256) / C::kStageBytes;
@@ -424,49 +431,65 @@ static int choose_stages(int ctas, int sms) {
     return stages;
 }
 
+// Items are in order of descending K (the longest tiles start first).
 template <int BT>
-static int launch_skinny_group(const uint8_t* x, const uint8_t* sfx, const float* alpha_x, int M, int K,
-                               int64_t sf_group_stride, const SkinnyItem* items, int n_items, int forced_ranks,
-                               cudaStream_t stream) {
+static int launch_skinny_group(int M, const SkinnyItem* items, int n_items, int forced_ranks, cudaStream_t stream) {
     using C = SkinnyCfg<BT>;
     if (n_items < 1 || n_items > kMaxGroup) return NVFP4_ERR_BAD_RANGE;
     SkinnyMaps maps;
-    CUtensorMap mx;
-    int st = make_operand_map(&mx, x, M, K / 2, BT);
     SkinnyParams p;
-    int n_tiles = 0;
+    int n_tiles = 0, st = NVFP4_OK;
     p.weights_ready = 1;
     for (int i = 0; i < n_items && st == NVFP4_OK; ++i) {
         const SkinnyItem& it = items[i];
         if (!it.wh) p.weights_ready = 0;
         if (it.wh) maps.m[i] = it.wh->rows128;
-        else st = make_operand_map(&maps.m[i], it.w, it.N, K / 2, 128);
+        else st = make_operand_map(&maps.m[i], it.w, it.N, it.K / 2, 128);
+        if (i > 0 && it.x == items[i - 1].x && it.K == items[i - 1].K) maps.x[i] = maps.x[i - 1];
+        else if (st == NVFP4_OK) st = make_operand_map(&maps.x[i], it.x, M, it.K / 2, BT);
         n_tiles += static_cast<int>((it.N + 127) / 128);
         p.w[i].sfw = it.sfw;
+        p.w[i].sfx = it.sfx;
         p.w[i].alpha = it.alpha;
+        p.w[i].alpha_x = it.alpha_x;
         p.w[i].out = it.out;
         p.w[i].N = static_cast<int>(it.N);
+        p.w[i].K = static_cast<int>(it.K);
+        p.w[i].sf_group_stride = round_up_i64(it.K / 16, 4) * 128;
         p.w[i].tile_end = n_tiles;
     }
     if (st != NVFP4_OK) return st;
-    for (int i = n_items; i < kMaxGroup; ++i) {   // unused slots: defined values, never dereferenced
-        maps.m[i] = maps.m[0];
-        p.w[i] = p.w[n_items - 1];
-    }
     const DeviceInfo di = device_info();
     const int sms = di.sms;
-    const int k_tiles = (K + kBK - 1) / kBK;
-    int ranks = choose_ranks(n_tiles, k_tiles, sms, forced_ranks, BT);
-    p.sfx = sfx;
-    p.alpha_x = alpha_x;
+    const int longest = (p.w[0].K + kBK - 1) / kBK, shortest = (p.w[n_items - 1].K + kBK - 1) / kBK;
+    // Products of different K: enough ranges that the longest tile's are not much longer than what every SM has to stream
+    // (at two CTAs per SM), and three CTAs per SM.  The seven matrices of a Llama-3-8B layer at 1 token, K 4096 and 14336:
+    // 23.2 us with two ranges, 30.8 with one, 25.1 with three; 24.4 with two CTAs per SM, 27.1 with four (32.9 as four launches).
+    const bool mixed = longest != shortest;
+    int ranks = 1;
+    if (mixed && forced_ranks == 0) {
+        int64_t stages = 0;
+        for (int i = 0; i < n_items; ++i)
+            stages += static_cast<int64_t>((p.w[i].N + 127) / 128) * ((p.w[i].K + kBK - 1) / kBK);
+        while (ranks < 8 && ranks < shortest / 2 && static_cast<int64_t>(longest) * 8 * sms > stages * 5 * ranks) ranks *= 2;
+    } else {
+        ranks = choose_ranks(n_tiles, shortest, sms, forced_ranks, BT);
+    }
+    // no empty K range in any item: with every rank holding ceil(k / ranks) stages the last one must get some
+    auto fits = [&](int r) {
+        for (int i = 0; i < n_items; ++i) {
+            const int k = (p.w[i].K + kBK - 1) / kBK;
+            if ((r - 1) * ((k + r - 1) / r) >= k) return false;
+        }
+        return true;
+    };
+    while (ranks > 1 && !fits(ranks)) --ranks;
+    for (int i = 0; i < n_items; ++i) p.w[i].k_tiles_per_rank = ((p.w[i].K + kBK - 1) / kBK + ranks - 1) / ranks;
     p.M = M;
-    p.K = K;
-    p.sf_group_stride = sf_group_stride;
     p.n_weights = n_items;
-    p.k_tiles_per_rank = (k_tiles + ranks - 1) / ranks;
-    ranks = (k_tiles + p.k_tiles_per_rank - 1) / p.k_tiles_per_rank;   // no empty range
-    p.stages = choose_stages<BT>(n_tiles * ranks, sms);
-    if (p.stages > p.k_tiles_per_rank) p.stages = p.k_tiles_per_rank < 2 ? 2 : p.k_tiles_per_rank;
+    p.stages = choose_stages<BT>(n_tiles * ranks, sms, mixed ? 3 : kTmemCols);
+    const int per_rank = (longest + ranks - 1) / ranks;
+    if (p.stages > per_rank) p.stages = per_rank < 2 ? 2 : per_rank;
     // the ring doubles as the reduce-scatter buffers: the partial tile plus one slot per rank of the owned columns
     while (ranks > 1 && (2 * BT + 8) * 512 > p.stages * C::kStageBytes) ++p.stages;
     if (p.stages > C::kMaxStages) return NVFP4_ERR_UNSUPPORTED;
@@ -497,21 +520,15 @@ static int launch_skinny_group(const uint8_t* x, const uint8_t* sfx, const float
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = g_dependent_launch ? 2 : 1;
-    e = cudaLaunchKernelEx(&cfg, skinny_kernel<BT>, maps, mx, p);
+    e = cudaLaunchKernelEx(&cfg, skinny_kernel<BT>, maps, p);
     return static_cast<int>(e);
 }
 
 template <int BT>
-static int launch_skinny(const uint8_t* x, const uint8_t* w, const GemmParams& g, int forced_ranks, cudaStream_t stream,
+static int launch_skinny(const GemmParams& g, int forced_ranks, cudaStream_t stream,
                          const WeightHandle* wh) {
-    SkinnyItem it;
-    it.w = w;
-    it.sfw = g.sfb;
-    it.alpha = g.alpha;
-    it.out = g.out;
-    it.N = g.N;
-    it.wh = wh;
-    return launch_skinny_group<BT>(x, g.sfa, g.alpha2, g.M, g.K, g.sf_group_stride, &it, 1, forced_ranks, stream);
+    const SkinnyItem it = {g.a, g.sfa, g.alpha2, g.b, g.sfb, g.alpha, g.out, g.N, g.K, wh};
+    return launch_skinny_group<BT>(g.M, &it, 1, forced_ranks, stream);
 }
 
 }  // namespace skinny

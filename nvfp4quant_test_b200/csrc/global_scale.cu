@@ -20,19 +20,32 @@ constexpr int kGsThreads = 512;
 
 __device__ __forceinline__ uint32_t umax2x16(uint32_t a, uint32_t b) { return __vmaxu2(a, b); }
 
-template <int DT>
-__global__ void __launch_bounds__(kGsThreads) global_scale_kernel(const void* x, int64_t numel, float fp8_max,
-                                                                  float* out, uint32_t* scratch) {
+template <int G>
+struct GsParams {
+    GsItem item[G];
+    unsigned cta_end[G];   // CTAs of this and all earlier tensors
+    float fp8_max;
+};
+
+template <int DT, int G>
+__global__ void __launch_bounds__(kGsThreads) global_scale_kernel(const __grid_constant__ GsParams<G> p) {
     // launched as a programmatic dependent: x, the scratch words and `out` belong to the kernel before this one until
     // it has finished.  The kernel behind this one (the quantizer, which waits before it touches anything) may be
     // scheduled at once.
     griddep_launch();
     griddep_wait();
+    int gi = 0;
+    if (G > 1) while (blockIdx.x >= p.cta_end[gi]) ++gi;
+    const unsigned first = gi > 0 ? p.cta_end[gi - 1] : 0, bx = blockIdx.x - first, ctas = p.cta_end[gi] - first;
+    const void* x = p.item[gi].x;
+    const int64_t numel = p.item[gi].numel;
+    float* const out = p.item[gi].out;
+    uint32_t* const scratch = p.item[gi].scratch;
     constexpr int kPerVec = (DT == NVFP4_DT_F32) ? 4 : 8;
     const int64_t nvec = numel / kPerVec;
     x = after_wait(x);   // loads of x stay behind the wait
     const uint4* xv = static_cast<const uint4*>(x);
-    const int64_t stride = static_cast<int64_t>(gridDim.x) * kGsThreads;
+    const int64_t stride = static_cast<int64_t>(ctas) * kGsThreads;
     uint32_t acc = 0;
     auto fold = [&](const uint4& q) {
         if (DT == NVFP4_DT_F32) {
@@ -42,7 +55,7 @@ __global__ void __launch_bounds__(kGsThreads) global_scale_kernel(const void* x,
                                          umax2x16(q.z & 0x7fff7fffu, q.w & 0x7fff7fffu)));
         }
     };
-    int64_t i = static_cast<int64_t>(blockIdx.x) * kGsThreads + threadIdx.x;
+    int64_t i = static_cast<int64_t>(bx) * kGsThreads + threadIdx.x;
     // four independent 16-byte loads in flight per thread: with one, a resident grid holds too few bytes in
     // flight to cover the HBM latency
     for (; i + 3 * stride < nvec; i += 4 * stride) {
@@ -65,7 +78,7 @@ __global__ void __launch_bounds__(kGsThreads) global_scale_kernel(const void* x,
         fold(q2);
     }
     // ragged tail (numel not a multiple of the vector width): first threads of block 0
-    if (blockIdx.x == 0) {
+    if (bx == 0) {
         const int64_t t = nvec * kPerVec + threadIdx.x;
         if (t < numel) {
             if (DT == NVFP4_DT_F32) acc = max(acc, static_cast<const uint32_t*>(x)[t] & 0x7fffffffu);
@@ -90,13 +103,13 @@ __global__ void __launch_bounds__(kGsThreads) global_scale_kernel(const void* x,
         for (int i = 0; i < kGsThreads / 32; ++i) b = max(b, warp_max[i]);
         // a one-block grid (activations of a few tokens) has its maximum already: no trip through the scratch words,
         // whose three dependent atomics would cost more than the rest of the kernel
-        bool last = gridDim.x == 1;
+        bool last = ctas == 1;
         uint32_t mx = b;
         if (!last) {
             atomicMax(&scratch[0], b);
             __threadfence();
             const uint32_t ticket = atomicAdd(&scratch[1], 1u);
-            last = ticket == gridDim.x - 1;
+            last = ticket == ctas - 1;
             if (last) {
                 __threadfence();
                 mx = atomicExch(&scratch[0], 0u);
@@ -105,7 +118,7 @@ __global__ void __launch_bounds__(kGsThreads) global_scale_kernel(const void* x,
         }
         if (last) {
             const float amax = __uint_as_float(mx);
-            const float inv_den = __fdiv_rn(1.0f, __fmul_rn(6.0f, fp8_max));
+            const float inv_den = __fdiv_rn(1.0f, __fmul_rn(6.0f, p.fp8_max));
             const float gs = __fmul_rn(amax, inv_den);
             out[0] = gs;
             out[1] = __fdiv_rn(1.0f, gs);
@@ -113,38 +126,62 @@ __global__ void __launch_bounds__(kGsThreads) global_scale_kernel(const void* x,
     }
 }
 
+// CTAs for one tensor.  Up to four 16-byte loads per thread (all in flight at once) stay in one block, which needs no atomics.
+// A few resident blocks per SM are enough to keep HBM busy; more only adds atomics: measured at 8192 x 8192 bf16, 1 CTA per
+// SM 29.0 us, 2: 25.4, 3: 25.0, 4: 25.2-26.5, 8: 27.5, 16: 29.2.
+int64_t gs_ctas(int64_t numel, int x_dtype, int sms) {
+    const int64_t nvec = numel / (x_dtype == NVFP4_DT_F32 ? 4 : 8);
+    int64_t blocks = nvec <= 4 * kGsThreads ? 1 : (nvec + kGsThreads - 1) / kGsThreads;
+    const int64_t cap = static_cast<int64_t>(sms) * 3;
+    if (blocks > cap) blocks = cap;
+    return blocks < 1 ? 1 : blocks;
+}
+
+template <int G>
+cudaError_t launch_group(const GsItem* items, int n, int x_dtype, float fp8_max, int sms, cudaStream_t s) {
+    GsParams<G> p;
+    p.fp8_max = fp8_max;
+    unsigned end = 0;
+    for (int i = 0; i < n; ++i) {
+        p.item[i] = items[i];
+        p.cta_end[i] = end += static_cast<unsigned>(gs_ctas(items[i].numel, x_dtype, sms));
+    }
+    const dim3 grid(end), block(kGsThreads);
+    switch (x_dtype) {
+        case NVFP4_DT_BF16: return launch_dependent(global_scale_kernel<NVFP4_DT_BF16, G>, grid, block, 0, s, p);
+        case NVFP4_DT_F16: return launch_dependent(global_scale_kernel<NVFP4_DT_F16, G>, grid, block, 0, s, p);
+        default: return launch_dependent(global_scale_kernel<NVFP4_DT_F32, G>, grid, block, 0, s, p);
+    }
+}
+
 }  // namespace
+
+int check_global_scale(const GsItem& item, int x_dtype) {
+    if (x_dtype < NVFP4_DT_BF16 || x_dtype > NVFP4_DT_F32) return NVFP4_ERR_BAD_ENUM;
+    if (item.numel < 0) return NVFP4_ERR_BAD_SHAPE;
+    if (!item.out || !item.scratch || (!item.x && item.numel > 0)) return NVFP4_ERR_NULL_POINTER;
+    if ((reinterpret_cast<uintptr_t>(item.x) & 15) || (reinterpret_cast<uintptr_t>(item.out) & 3) ||
+        (reinterpret_cast<uintptr_t>(item.scratch) & 3))
+        return NVFP4_ERR_MISALIGNED;
+    return NVFP4_OK;
+}
+
+int launch_global_scales(const GsItem* items, int n, int x_dtype, float fp8_max, cudaStream_t stream) {
+    static int sm_count[64] = {0};
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64) {
+        if (sm_count[dev] == 0) cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev);
+        if (sm_count[dev] > 0) sms = sm_count[dev];
+    }
+    return static_cast<int>(n == 1 ? launch_group<1>(items, n, x_dtype, fp8_max, sms, stream)
+                                   : launch_group<4>(items, n, x_dtype, fp8_max, sms, stream));
+}
+
 }  // namespace nvfp4
 
 extern "C" int nvfp4_global_scale_launch(const void* x, int x_dtype, int64_t numel, float fp8_max, float* out,
                                          uint32_t* scratch, void* stream) {
-    using namespace nvfp4;
-    if (x_dtype < NVFP4_DT_BF16 || x_dtype > NVFP4_DT_F32) return NVFP4_ERR_BAD_ENUM;
-    if (numel < 0) return NVFP4_ERR_BAD_SHAPE;
-    if (!out || !scratch || (!x && numel > 0)) return NVFP4_ERR_NULL_POINTER;
-    if ((reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(out) & 3) ||
-        (reinterpret_cast<uintptr_t>(scratch) & 3))
-        return NVFP4_ERR_MISALIGNED;
-    const int per_vec = (x_dtype == NVFP4_DT_F32) ? 4 : 8;
-    const int64_t nvec = numel / per_vec;
-    // up to four 16-byte loads per thread (all in flight at once) stay in one block, which needs no atomics
-    int64_t blocks = nvec <= 4 * kGsThreads ? 1 : (nvec + kGsThreads - 1) / kGsThreads;
-    // a few resident blocks per SM is enough to keep HBM busy; more only adds atomics
-    // measured at 8192 x 8192 bf16: 1 CTA per SM 29.0 us, 2: 25.4, 3: 25.0, 4: 25.2-26.5, 8: 27.5, 16: 29.2
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int64_t cap = static_cast<int64_t>(sms) * 3;
-    if (blocks > cap) blocks = cap;
-    if (blocks < 1) blocks = 1;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const unsigned g = static_cast<unsigned>(blocks);
-    const dim3 grid(g), block(kGsThreads);
-    switch (x_dtype) {
-        case NVFP4_DT_BF16:
-            return static_cast<int>(launch_dependent(global_scale_kernel<NVFP4_DT_BF16>, grid, block, 0, s, x, numel, fp8_max, out, scratch));
-        case NVFP4_DT_F16:
-            return static_cast<int>(launch_dependent(global_scale_kernel<NVFP4_DT_F16>, grid, block, 0, s, x, numel, fp8_max, out, scratch));
-        default:
-            return static_cast<int>(launch_dependent(global_scale_kernel<NVFP4_DT_F32>, grid, block, 0, s, x, numel, fp8_max, out, scratch));
-    }
+    const nvfp4::GsItem item = {x, numel, out, scratch};
+    const int st = nvfp4::check_global_scale(item, x_dtype);
+    return st != NVFP4_OK ? st : nvfp4::launch_global_scales(&item, 1, x_dtype, fp8_max, static_cast<cudaStream_t>(stream));
 }

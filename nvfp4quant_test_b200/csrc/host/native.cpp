@@ -134,7 +134,7 @@ inline PyObject* guarded(F&& f) {
 }
 
 // ---- scratch words of the global-scale kernel -----------------------------------------------------------------------
-// Two zeroed words per (device, stream), left zeroed by every launch; at most 32 streams, least recently used dropped (the
+// Two zeroed words for each of up to 16 tensors per (device, stream), left zeroed by every launch; at most 32 streams, least recently used dropped (the
 // block goes back to torch's allocator, which hands it out again in stream order).  Under capture the caller takes the
 // Python path, which keeps a scratch per capture.  Guarded by the interpreter lock, which every caller holds.
 struct ScratchKey {
@@ -169,7 +169,7 @@ uint32_t* scratch_words(c10::DeviceIndex device, cudaStream_t stream) {
     if (it != m.end()) {
         if (it->second != l.begin()) l.splice(l.begin(), l, it->second);
     } else {
-        Tensor words = at::zeros({2}, at::TensorOptions().dtype(at::kInt).device(c10::Device(c10::kCUDA, device)));
+        Tensor words = at::zeros({32}, at::TensorOptions().dtype(at::kInt).device(c10::Device(c10::kCUDA, device)));
         l.emplace_front(key, words);
         m[key] = l.begin();
         if (l.size() > kScratchStreams) {
@@ -333,6 +333,48 @@ PyObject* quant_dynamic(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
                                             static_cast<uint8_t*>(scales.mutable_data_ptr()), q.m, q.n, padded_n, lower, upper, tiled ? 1 : 0, s);
         });
         return st == NVFP4_OK ? pack({codes, scales, scalar_view(gs, 0), scalar_view(gs, 1)}) : none();
+    });
+}
+
+// quant_dynamic_multi(variant, [input], fp8_max, lower, upper) -> [(codes, scales, global_scale, 1 / global_scale)], tiled scales,
+// no padding: quant_dynamic over several unweighted tensors, sharing their launches
+PyObject* quant_dynamic_multi(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+    return guarded([&]() -> PyObject* {
+        float fp8_max;
+        if (nargs != 5 || !PyList_CheckExact(a[1]) || !as_float(a[2], &fp8_max) || !PyLong_CheckExact(a[3]) || !PyLong_CheckExact(a[4])) return none();
+        const Py_ssize_t n = PyList_GET_SIZE(a[1]);
+        constexpr Py_ssize_t kMost = 16;
+        if (n < 1 || n > kMost) return none();
+        QuantIn q[kMost];
+        for (Py_ssize_t i = 0; i < n; ++i)
+            if (!quant_input(PyList_GET_ITEM(a[1], i), Py_None, &q[i]) || q[i].device != q[0].device || q[i].dtype != q[0].dtype) return none();
+        const c10::DeviceIndex dev = q[0].device;
+        const cudaStream_t s = current_stream(dev);
+        uint32_t* scratch = scratch_words(dev, s);
+        if (!scratch) return none();
+        nvfp4_chain_item items[kMost];
+        Tensor codes[kMost], scales[kMost], gs[kMost];
+        for (Py_ssize_t i = 0; i < n; ++i) {
+            codes[i] = empty({q[i].m, q[i].n / 2}, at::kByte, dev);
+            scales[i] = empty_scales(q[i].m, q[i].n, true, dev);
+            gs[i] = empty({2}, at::kFloat, dev);
+            items[i] = {q[i].x->const_data_ptr(), nullptr, static_cast<float*>(gs[i].mutable_data_ptr()), scratch + 2 * i,
+                        static_cast<uint8_t*>(codes[i].mutable_data_ptr()), static_cast<uint8_t*>(scales[i].mutable_data_ptr()), q[i].m, q[i].n, q[i].n};
+        }
+        const int st = launch_on(dev, [&] {
+            return nvfp4_quant_chain_multi_launch(small_int(a[0]), q[0].dtype, fp8_max, items, static_cast<int>(n), small_int(a[3]), small_int(a[4]), 1, s);
+        });
+        if (st != NVFP4_OK) return none();
+        PyObject* l = PyList_New(n);
+        for (Py_ssize_t i = 0; l && i < n; ++i) {
+            PyObject* t = pack({codes[i], scales[i], scalar_view(gs[i], 0), scalar_view(gs[i], 1)});
+            if (!t) {
+                Py_DECREF(l);
+                return nullptr;
+            }
+            PyList_SET_ITEM(l, i, t);
+        }
+        return l;
     });
 }
 
@@ -681,14 +723,18 @@ PyObject* make_group(PyObject*, PyObject* args) {
     return PyCapsule_New(g, kGroupName, free_group);
 }
 
+bool chain_input(const Chain& c, const Tensor& x) {
+    return plain_cuda(x) && x.device().index() == c.device && dtype_code(x.scalar_type()) == c.dtype && x.dim() == 2 && x.size(0) == c.m &&
+           x.size(1) == c.n && x.is_contiguous() && aligned(x, 16);
+}
+
 // chain_call(chain, x) -> True
 PyObject* chain_call(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     return guarded([&]() -> PyObject* {
         if (nargs != 2) return none();
         const Chain* c = static_cast<const Chain*>(PyCapsule_GetPointer(a[0], kChainName));
         const Tensor* x = tensor_of(a[1]);
-        if (!c || !x || !plain_cuda(*x) || x->device().index() != c->device || dtype_code(x->scalar_type()) != c->dtype || x->dim() != 2 ||
-            x->size(0) != c->m || x->size(1) != c->n || !x->is_contiguous() || !aligned(*x, 16)) {
+        if (!c || !x || !chain_input(*c, *x)) {
             PyErr_Clear();
             return none();
         }
@@ -722,11 +768,77 @@ PyObject* group_call(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     });
 }
 
+// A layer whose activations are all at hand: their chains and every product, two to three launches from one call.
+struct Program {
+    std::vector<const Chain*> chains;
+    std::vector<nvfp4_gemm_item> products;
+    int64_t m;
+};
+constexpr const char* kProgramName = "nvfp4.program";
+void free_program(PyObject* c) { delete static_cast<Program*>(PyCapsule_GetPointer(c, kProgramName)); }
+
+// make_program((chain, ...), (index of the activation, ...), (group, ...)): the chains and groups stay the caller's and outlive it
+PyObject* make_program(PyObject*, PyObject* args) {
+    PyObject *chains, *index, *groups;
+    if (!PyArg_ParseTuple(args, "O!O!O!", &PyTuple_Type, &chains, &PyTuple_Type, &index, &PyTuple_Type, &groups)) return nullptr;
+    Program* p = new Program();
+    bool ok = PyTuple_GET_SIZE(chains) > 0 && PyTuple_GET_SIZE(chains) <= 64 && PyTuple_GET_SIZE(index) == PyTuple_GET_SIZE(groups);
+    for (Py_ssize_t i = 0; ok && i < PyTuple_GET_SIZE(chains); ++i) {
+        const Chain* c = static_cast<const Chain*>(PyCapsule_GetPointer(PyTuple_GET_ITEM(chains, i), kChainName));
+        const Chain* f = i > 0 ? p->chains[0] : c;
+        ok = c && c->dtype == f->dtype && c->variant == f->variant && c->lower == f->lower && c->upper == f->upper && c->device == f->device &&
+             c->fp8_max == f->fp8_max && c->m == f->m;
+        p->chains.push_back(c);
+    }
+    for (Py_ssize_t i = 0; ok && i < PyTuple_GET_SIZE(groups); ++i) {
+        const Group* g = static_cast<const Group*>(PyCapsule_GetPointer(PyTuple_GET_ITEM(groups, i), kGroupName));
+        const Py_ssize_t at = PyLong_AsSsize_t(PyTuple_GET_ITEM(index, i));
+        ok = g && at >= 0 && at < static_cast<Py_ssize_t>(p->chains.size()) && g->m == p->chains[at]->m && g->k == p->chains[at]->n &&
+             g->device == p->chains[at]->device;
+        for (size_t j = 0; ok && j < g->handles.size(); ++j)
+            p->products.push_back({g->handles[j], p->chains[at]->codes, p->chains[at]->scales, p->chains[at]->gs, g->alphas[j], g->outs[j]});
+    }
+    if (!ok || p->products.empty() || p->products.size() > 64) {
+        PyErr_Clear();
+        delete p;
+        return none();
+    }
+    p->m = p->chains[0]->m;
+    return PyCapsule_New(p, kProgramName, free_program);
+}
+
+// program_call(program, x0, x1, ...) -> True
+PyObject* program_call(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+    return guarded([&]() -> PyObject* {
+        const Program* p = nargs > 0 ? static_cast<const Program*>(PyCapsule_GetPointer(a[0], kProgramName)) : nullptr;
+        if (!p || nargs != 1 + static_cast<Py_ssize_t>(p->chains.size())) {
+            PyErr_Clear();
+            return none();
+        }
+        nvfp4_chain_item items[64];
+        const int n = static_cast<int>(p->chains.size());
+        for (int i = 0; i < n; ++i) {
+            const Chain* c = p->chains[i];
+            const Tensor* x = tensor_of(a[1 + i]);
+            if (!x || !chain_input(*c, *x)) return none();
+            items[i] = {x->const_data_ptr(), nullptr, c->gs, c->scratch, c->codes, c->scales, c->m, c->n, c->n};
+        }
+        const Chain* c = p->chains[0];
+        const cudaStream_t s = current_stream(c->device);
+        const int st = launch_on(c->device, [&] {
+            const int q = nvfp4_quant_chain_multi_launch(c->variant, c->dtype, c->fp8_max, items, n, c->lower, c->upper, 1, s);
+            return q != NVFP4_OK ? q : nvfp4_gemm_launch_multi(p->products.data(), static_cast<int>(p->products.size()), p->m, s);
+        });
+        return st == NVFP4_OK ? truth() : none();
+    });
+}
+
 #define FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(name)), METH_FASTCALL, nullptr}
 PyMethodDef kMethods[] = {
     FAST(quant_impl),
     FAST(quant_out),
     FAST(quant_dynamic),
+    FAST(quant_dynamic_multi),
     FAST(global_scale),
     FAST(channel_square_norm),
     FAST(dequant),
@@ -737,8 +849,10 @@ PyMethodDef kMethods[] = {
     FAST(scaled_mm_multi),
     FAST(chain_call),
     FAST(group_call),
+    FAST(program_call),
     {"make_chain", make_chain, METH_VARARGS, nullptr},
     {"make_group", make_group, METH_VARARGS, nullptr},
+    {"make_program", make_program, METH_VARARGS, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };
 #undef FAST

@@ -57,13 +57,16 @@ constexpr int64_t kSmallBlocks = 24576;
 constexpr int64_t kSmallBlocksRagged = 98304;
 constexpr int64_t kSmallBlocksRaggedWeighted = 327680;
 __host__ __device__ constexpr int block_threads(int variant, int impl) {
-    return impl == 9 ? kSmallThreads : (variant != NVFP4_VARIANT_AMAX && (impl == 3 || impl >= 7)) ? kSweepThreads : kThreads;
+    return impl == 9 ? kSmallThreads : (variant != NVFP4_VARIANT_AMAX && (impl == 3 || impl == 7 || impl == 8 || impl == 10)) ? kSweepThreads : kThreads;
 }
 constexpr int min_blocks(int variant, int impl) {
     if (impl == 9) return 8;
+    if (impl == 10) return 4;
     if (block_threads(variant, impl) == kSweepThreads) return kSweepMinBlocks;
     return variant == NVFP4_VARIANT_WEIGHTED ? 4 : 5;
 }
+
+constexpr int kMaxChain = 4;   // tensors per launch of the chain
 
 struct QuantParams {
     const void* x;
@@ -363,13 +366,46 @@ __device__ __forceinline__ uint32_t sweep_single(const float v[16], const float 
     return best_raw;
 }
 
+// Largest magnitude of `nvec` 16-byte vectors as an fp32 bit pattern, by the whole CTA (what global_scale_kernel computes).
+template <int DT, int T>
+__device__ __forceinline__ uint32_t cta_amax_bits(const uint4* x, uint32_t nvec) {
+    constexpr int kBatch = 16;   // loads in flight per thread
+    uint32_t acc = 0;
+    for (uint32_t i = threadIdx.x; i < nvec; i += kBatch * T) {
+        uint4 q[kBatch];
+#pragma unroll
+        for (int b = 0; b < kBatch; ++b) q[b] = i + b * T < nvec ? __ldg(x + i + b * T) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int b = 0; b < kBatch; ++b) {
+            if (DT == NVFP4_DT_F32)
+                acc = max(acc, max(max(q[b].x & 0x7fffffffu, q[b].y & 0x7fffffffu), max(q[b].z & 0x7fffffffu, q[b].w & 0x7fffffffu)));
+            else
+                acc = __vmaxu2(acc, __vmaxu2(__vmaxu2(q[b].x & 0x7fff7fffu, q[b].y & 0x7fff7fffu),
+                                             __vmaxu2(q[b].z & 0x7fff7fffu, q[b].w & 0x7fff7fffu)));
+        }
+    }
+    uint32_t bits = acc;
+    if (DT != NVFP4_DT_F32) {
+        const uint32_t h = max(acc & 0xffffu, acc >> 16);
+        bits = DT == NVFP4_DT_BF16 ? h << 16 : __float_as_uint(__half2float(__ushort_as_half(static_cast<unsigned short>(h))));
+    }
+    bits = __reduce_max_sync(0xffffffffu, bits);
+    __shared__ uint32_t warp_max[T / 32];
+    if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = bits;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < T / 32; ++i) bits = max(bits, warp_max[i]);
+    return bits;
+}
+
+// One CTA's share of a quantization: CTA `bx` of `ctas` (blockIdx.x of gridDim.x where the launch holds one tensor).
 template <int DT, int VARIANT, int IMPL>
-__global__ void __launch_bounds__(block_threads(VARIANT, IMPL), min_blocks(VARIANT, IMPL))
-quant_kernel(const QuantParams p) {
+__device__ __forceinline__ void quant_body(const QuantParams& p, const uint32_t bx, const uint32_t ctas) {
     constexpr int T = block_threads(VARIANT, IMPL);   // threads per CTA
     static_assert(kTabSize % T == 0, "every thread builds the same number of table entries");
     __shared__ float4 tab[kTabSize];
     constexpr bool FUSED = IMPL == 4;
+    constexpr bool OWN_SCALE = IMPL == 10;   // every CTA takes the global scale of the whole (small) tensor itself
     static_assert(!FUSED || VARIANT != NVFP4_VARIANT_AMAX, "the fused variant covers the two sweeps");
     // Launched as a programmatic dependent: the input, the global scale and the output buffers may still be in use by
     // the kernel before this one on the stream, so everything waits.  The kernel BEHIND this one may be scheduled right
@@ -381,19 +417,19 @@ quant_kernel(const QuantParams p) {
     // everything the kernel before this one may have written is read through pointers taken behind the wait
     const void* const x_in = after_wait(p.x);
     const float* const importance_in = after_wait(p.importance);
-    float gs_inv = FUSED ? 0.0f : load_f32_after_wait(p.gs_inv);
+    float gs_inv = FUSED || OWN_SCALE ? 0.0f : load_f32_after_wait(p.gs_inv);
     // Two-dimensional grid: blockIdx.x is the row, blockIdx.y the column chunk.  The row is then uniform over the CTA, so
     // the division below, the row part of the addresses and most of the tiled scale offset leave the per-thread
     // instruction stream (8192 x 8192 sweep: 126 us numbered through, 112 us with this grid).
     constexpr bool GRID2D = IMPL == 7 || IMPL == 8;
     constexpr bool WHOLE = IMPL == 8;
-    constexpr bool FLAT = IMPL == 3 || IMPL == 9;   // real rows' slots numbered through, then CTAs that fill the padding rows
-    const int64_t id = GRID2D ? 0 : static_cast<int64_t>(blockIdx.x) * T + threadIdx.x;
+    constexpr bool FLAT = IMPL == 3 || IMPL == 9 || IMPL == 10;   // real rows' slots numbered through, then CTAs that fill the padding rows
+    const int64_t id = GRID2D ? 0 : static_cast<int64_t>(bx) * T + threadIdx.x;
     const int64_t slots = FLAT ? p.m * p.width : p.total;
     const bool in_range = GRID2D ? true : id < slots;
     int64_t row = 0, col = 0;
     if (GRID2D) {
-        row = blockIdx.x;
+        row = bx;
         col = static_cast<int64_t>(blockIdx.y) * T + threadIdx.x;
     } else if (in_range) {
         if (p.total <= 0x7fffffffLL) {
@@ -410,7 +446,7 @@ quant_kernel(const QuantParams p) {
         if ((threadIdx.x & 3) == 0) *reinterpret_cast<uint32_t*>(p.scales + swizzled_scale_offset(row, col, p.k_pad)) = 0u;
         return;
     }
-    if (FLAT && static_cast<int64_t>(blockIdx.x) * T >= slots) {
+    if (FLAT && static_cast<int64_t>(bx) * T >= slots) {
         // A CTA behind the real rows' slots.  The rows m .. rows-1 of the tiled scale layout (127 of 128 for one token)
         // hold no data; these CTAs write their zero scale bytes, four 32-bit words (of four columns each) per thread,
         // and leave before the candidate table is built.  (Rows beyond m exist only in the tiled layout, whose width is
@@ -418,8 +454,8 @@ quant_kernel(const QuantParams p) {
         const uint32_t words_per_row = static_cast<uint32_t>(p.width >> 2);
         const uint32_t words = static_cast<uint32_t>(p.rows - p.m) * words_per_row;
         const uint32_t real_ctas = static_cast<uint32_t>((slots + T - 1) / T);
-        const uint32_t fill_threads = (gridDim.x - real_ctas) * T;
-        for (uint32_t wi = (blockIdx.x - real_ctas) * T + threadIdx.x; wi < words; wi += fill_threads) {
+        const uint32_t fill_threads = (ctas - real_ctas) * T;
+        for (uint32_t wi = (bx - real_ctas) * T + threadIdx.x; wi < words; wi += fill_threads) {
             const uint32_t r = wi / words_per_row;
             const uint32_t c = (wi - r * words_per_row) * 4u;
             *reinterpret_cast<uint32_t*>(p.scales + swizzled_scale_offset(p.m + r, c, p.k_pad)) = 0u;
@@ -436,6 +472,17 @@ quant_kernel(const QuantParams p) {
     if (WHOLE || (valid && col < p.bin)) {
         load16<DT>(x_in, row * p.n + col * kBlock, v);
         if (VARIANT == NVFP4_VARIANT_WEIGHTED) load16<NVFP4_DT_F32>(importance_in, col * kBlock, w);
+    }
+
+    if constexpr (OWN_SCALE) {
+        const uint32_t nvec = static_cast<uint32_t>(p.m * p.n / (DT == NVFP4_DT_F32 ? 4 : 8));
+        const float amax_x = __uint_as_float(cta_amax_bits<DT, T>(static_cast<const uint4*>(x_in), nvec));
+        const float gs = __fmul_rn(amax_x, __fdiv_rn(1.0f, __fmul_rn(6.0f, p.fp8_max)));
+        gs_inv = __fdiv_rn(1.0f, gs);
+        if (bx == 0 && threadIdx.x == 0) {
+            p.gs_out[0] = gs;
+            p.gs_out[1] = gs_inv;
+        }
     }
 
     // The global scale and the block's elements were requested above; the candidate table is built while they are
@@ -570,14 +617,36 @@ quant_kernel(const QuantParams p) {
     }
 }
 
+template <int DT, int VARIANT, int IMPL>
+__global__ void __launch_bounds__(block_threads(VARIANT, IMPL), min_blocks(VARIANT, IMPL))
+quant_kernel(const QuantParams p) {
+    quant_body<DT, VARIANT, IMPL>(p, blockIdx.x, gridDim.x);
+}
+
+// Several tensors in one launch (a layer's activations): CTAs are numbered through the tensors.
+struct MultiParams {
+    QuantParams q[kMaxChain];
+    uint32_t cta_end[kMaxChain];
+};
+template <int DT, int VARIANT, int IMPL>
+__global__ void __launch_bounds__(block_threads(VARIANT, IMPL), min_blocks(VARIANT, IMPL))
+quant_multi_kernel(const __grid_constant__ MultiParams p) {
+    int i = 0;
+    while (blockIdx.x >= p.cta_end[i]) ++i;
+    const uint32_t begin = i > 0 ? p.cta_end[i - 1] : 0;
+    quant_body<DT, VARIANT, IMPL>(p.q[i], blockIdx.x - begin, p.cta_end[i] - begin);
+}
 // Grid of the bodies that number the real rows' slots through: CTAs for those, then CTAs that zero the padding rows' scale
 // words (4 words per thread).
+int64_t flat_ctas(const QuantParams& p, int T) {
+    const int64_t pad_words = (p.rows - p.m) * (p.width >> 2);
+    if (pad_words > 0x7fffffffLL) return INT64_MAX;   // at most 127 rows: a width beyond 2^26 columns
+    return (p.m * p.width + T - 1) / T + (pad_words + 4 * T - 1) / (4 * T);
+}
 template <int DT, int VARIANT, int IMPL>
 cudaError_t launch_flat(const QuantParams& p, cudaStream_t stream) {
     constexpr int T = block_threads(VARIANT, IMPL);
-    const int64_t pad_words = (p.rows - p.m) * (p.width >> 2);
-    if (pad_words > 0x7fffffffLL) return cudaErrorInvalidValue;   // at most 127 rows: a width beyond 2^26 columns
-    const int64_t grid = (p.m * p.width + T - 1) / T + (pad_words + 4 * T - 1) / (4 * T);
+    const int64_t grid = flat_ctas(p, T);
     if (grid > 0x7fffffffLL) return cudaErrorInvalidValue;
     return launch_dependent(quant_kernel<DT, VARIANT, IMPL>, static_cast<unsigned>(grid), dim3(T), 0, stream, p);
 }
@@ -617,16 +686,16 @@ cudaError_t launch_variant(int variant, int impl, const QuantParams& p, cudaStre
 }  // namespace
 }  // namespace nvfp4
 
-extern "C" int nvfp4_quant_launch_impl(int impl, int variant, const void* x, int x_dtype, const float* importance,
-                                       const float* gs_inv, uint8_t* codes, uint8_t* scales, int64_t m, int64_t n,
-                                       int64_t padded_n, int lower, int upper, int swizzled, void* stream) {
-    using namespace nvfp4;
+namespace nvfp4 {
+namespace {
+// Checks one tensor's arguments and fills its parameters.  NVFP4_OK with p.total == 0: nothing to do.  `gs_inv` is required
+// here; the chain passes the pair its first kernel writes.
+int fill_params(QuantParams& p, int variant, const void* x, int x_dtype, const float* importance, const float* gs_inv, uint8_t* codes,
+                uint8_t* scales, int64_t m, int64_t n, int64_t padded_n, int lower, int upper, int swizzled) {
     if (variant < NVFP4_VARIANT_MSE || variant > NVFP4_VARIANT_AMAX) return NVFP4_ERR_BAD_ENUM;
     if (x_dtype < NVFP4_DT_BF16 || x_dtype > NVFP4_DT_F32) return NVFP4_ERR_BAD_ENUM;
-    if (impl < 0 || impl > 9 || impl == 4) return NVFP4_ERR_BAD_ENUM;
     if (m < 0 || n < 0 || (n % kBlock) != 0 || (padded_n % kBlock) != 0 || padded_n < n) return NVFP4_ERR_BAD_SHAPE;
     if (variant != NVFP4_VARIANT_AMAX && (upper < lower || upper - lower + 1 > 64)) return NVFP4_ERR_BAD_RANGE;
-    QuantParams p;
     p.m = m;
     p.n = n;
     p.bin = n / kBlock;
@@ -654,6 +723,22 @@ extern "C" int nvfp4_quant_launch_impl(int impl, int variant, const void* x, int
     p.scales = scales;
     p.lower = lower;
     p.ncand = (variant == NVFP4_VARIANT_AMAX) ? 0 : upper - lower + 1;
+    p.fp8_max = 0.0f;
+    p.gs_out = nullptr;
+    p.fused_scratch = nullptr;
+    return NVFP4_OK;
+}
+}  // namespace
+}  // namespace nvfp4
+
+extern "C" int nvfp4_quant_launch_impl(int impl, int variant, const void* x, int x_dtype, const float* importance,
+                                       const float* gs_inv, uint8_t* codes, uint8_t* scales, int64_t m, int64_t n,
+                                       int64_t padded_n, int lower, int upper, int swizzled, void* stream) {
+    using namespace nvfp4;
+    if (impl < 0 || impl > 9 || impl == 4) return NVFP4_ERR_BAD_ENUM;
+    QuantParams p;
+    const int st = fill_params(p, variant, x, x_dtype, importance, gs_inv, codes, scales, m, n, padded_n, lower, upper, swizzled);
+    if (st != NVFP4_OK || p.total == 0) return st;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     cudaError_t err;
     switch (x_dtype) {
@@ -689,20 +774,110 @@ cudaError_t launch_fused_variant(int variant, const QuantParams& p, int sms, cud
 }  // namespace
 }  // namespace nvfp4
 
-// Global scale, then the quantizer with that scale, as two launches from one host call: what get_nvfp4_global_scale followed
-// by scalesweep_*_quant_out do (helper.py:96-100, bench.py:57-67 of the reference), for callers that pay per host call
-// (an eager decode loop).  gs_out[0] = amax|x| / (6 * fp8_max), gs_out[1] = 1 / gs_out[0]; `scratch` = the 2 zeroed words
-// of nvfp4_global_scale_launch.  Both kernels are programmatic dependent launches; bytes equal the two separate calls.
+namespace nvfp4 {
+namespace {
+// Tensors of up to this many bytes take their global scale inside the quantizer: every CTA reads the whole tensor (from L2,
+// 16 loads per thread in flight at once) instead of waiting for a kernel before it.  One launch instead of two: chain of
+// launches, 1 x 4096 bf16 3.2 -> 2.4 us, 4 x 8192 (64 KiB) 4.8 -> 3.5, 16 x 4096 (128 KiB) 5.0 -> 4.8, but 16 x 8192 5.4 -> 8.0.
+constexpr int64_t kOwnScaleBytes = 131072;
+// Several tensors with up to this many blocks in all share their launches, slots numbered through; beyond it the
+// two-dimensional grids of separate launches gain more than the launches cost.
+constexpr int64_t kMultiBlocks = 524288;
+constexpr int64_t kMultiSmallBlocks = 98304;   // as kSmallBlocksRagged
+
+template <int DT, int VARIANT, int IMPL>
+cudaError_t launch_multi(const QuantParams* q, int n, cudaStream_t stream) {
+    constexpr int T = block_threads(VARIANT, IMPL);
+    if (n == 1) return launch_flat<DT, VARIANT, IMPL>(q[0], stream);
+    MultiParams mp;
+    int64_t end = 0;
+    for (int i = 0; i < n; ++i) {
+        mp.q[i] = q[i];
+        end += flat_ctas(q[i], T);
+        mp.cta_end[i] = static_cast<uint32_t>(end);
+    }
+    return launch_dependent(quant_multi_kernel<DT, VARIANT, IMPL>, dim3(static_cast<unsigned>(end)), dim3(T), 0, stream, mp);
+}
+
+// The quantizer half of a chain over n tensors of one variant (n > 1, or own_scale).
+template <int DT>
+cudaError_t launch_chain(int variant, bool own_scale, bool small, const QuantParams* q, int n, cudaStream_t s) {
+    if (variant == NVFP4_VARIANT_MSE)
+        return own_scale ? launch_multi<DT, NVFP4_VARIANT_MSE, 10>(q, n, s)
+               : small   ? launch_multi<DT, NVFP4_VARIANT_MSE, 9>(q, n, s)
+                         : launch_multi<DT, NVFP4_VARIANT_MSE, 3>(q, n, s);
+    return own_scale ? launch_multi<DT, NVFP4_VARIANT_WEIGHTED, 10>(q, n, s)
+           : small   ? launch_multi<DT, NVFP4_VARIANT_WEIGHTED, 9>(q, n, s)
+                     : launch_multi<DT, NVFP4_VARIANT_WEIGHTED, 3>(q, n, s);
+}
+}  // namespace
+}  // namespace nvfp4
+
+// Global scale, then the quantizer with that scale, of up to kMaxChain tensors per launch: what get_nvfp4_global_scale
+// followed by scalesweep_*_quant_out do (helper.py:96-100, bench.py:57-67 of the reference), for callers that pay per
+// launch and per host call (an eager decode loop).  Bytes equal the separate calls.
+extern "C" int nvfp4_quant_chain_multi_launch(int variant, int x_dtype, float fp8_max, const nvfp4_chain_item* items, int n_items,
+                                              int lower, int upper, int swizzled, void* stream) {
+    using namespace nvfp4;
+    if (n_items < 0 || n_items > 64) return NVFP4_ERR_BAD_RANGE;
+    if (n_items == 0) return NVFP4_OK;
+    if (!items) return NVFP4_ERR_NULL_POINTER;
+    if (!(fp8_max > 0.0f)) return NVFP4_ERR_BAD_RANGE;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    for (int first = 0; first < n_items; first += kMaxChain) {
+        const int n = n_items - first < kMaxChain ? n_items - first : kMaxChain;
+        const nvfp4_chain_item* it = items + first;
+        QuantParams q[kMaxChain];
+        GsItem gs[kMaxChain];
+        bool own_scale = variant != NVFP4_VARIANT_AMAX;
+        int64_t blocks = 0;
+        for (int i = 0; i < n; ++i) {
+            if (it[i].m <= 0 || it[i].n <= 0) return NVFP4_ERR_BAD_SHAPE;   // an empty tensor has no maximum
+            if (!it[i].gs_out) return NVFP4_ERR_NULL_POINTER;
+            gs[i] = GsItem{it[i].x, it[i].m * it[i].n, it[i].gs_out, it[i].scratch};
+            int st = check_global_scale(gs[i], x_dtype);
+            if (st == NVFP4_OK)
+                st = fill_params(q[i], variant, it[i].x, x_dtype, it[i].importance, it[i].gs_out + 1, it[i].codes, it[i].scales, it[i].m,
+                                 it[i].n, it[i].padded_n, lower, upper, swizzled);
+            if (st != NVFP4_OK) return st;
+            q[i].fp8_max = fp8_max;
+            q[i].gs_out = it[i].gs_out;
+            blocks += q[i].m * q[i].width;
+            own_scale = own_scale && it[i].m * it[i].n * (x_dtype == NVFP4_DT_F32 ? 4 : 2) <= kOwnScaleBytes;
+        }
+        const bool together = own_scale || (n > 1 && variant != NVFP4_VARIANT_AMAX && blocks <= kMultiBlocks);
+        if (!own_scale) {
+            const int st = launch_global_scales(gs, together ? n : 1, x_dtype, fp8_max, s);
+            if (st != NVFP4_OK) return st;
+        }
+        if (together) {
+            const bool small = blocks <= kMultiSmallBlocks;
+            cudaError_t e;
+            switch (x_dtype) {
+                case NVFP4_DT_BF16: e = launch_chain<NVFP4_DT_BF16>(variant, own_scale, small, q, n, s); break;
+                case NVFP4_DT_F16: e = launch_chain<NVFP4_DT_F16>(variant, own_scale, small, q, n, s); break;
+                default: e = launch_chain<NVFP4_DT_F32>(variant, own_scale, small, q, n, s); break;
+            }
+            if (e != cudaSuccess) return static_cast<int>(e);
+            continue;
+        }
+        for (int i = 0; i < n; ++i) {
+            int st = i > 0 ? launch_global_scales(gs + i, 1, x_dtype, fp8_max, s) : NVFP4_OK;
+            if (st == NVFP4_OK)
+                st = nvfp4_quant_launch(variant, it[i].x, x_dtype, it[i].importance, it[i].gs_out + 1, it[i].codes, it[i].scales, it[i].m,
+                                        it[i].n, it[i].padded_n, lower, upper, swizzled, stream);
+            if (st != NVFP4_OK) return st;
+        }
+    }
+    return NVFP4_OK;
+}
+
 extern "C" int nvfp4_quant_chain_launch(int variant, const void* x, int x_dtype, const float* importance, float fp8_max,
                                         float* gs_out, uint32_t* scratch, uint8_t* codes, uint8_t* scales, int64_t m,
                                         int64_t n, int64_t padded_n, int lower, int upper, int swizzled, void* stream) {
-    if (m <= 0 || n <= 0) return NVFP4_ERR_BAD_SHAPE;   // an empty tensor has no maximum
-    if (!(fp8_max > 0.0f)) return NVFP4_ERR_BAD_RANGE;
-    if (!gs_out) return NVFP4_ERR_NULL_POINTER;
-    const int st = nvfp4_global_scale_launch(x, x_dtype, m * n, fp8_max, gs_out, scratch, stream);
-    if (st != NVFP4_OK) return st;
-    return nvfp4_quant_launch(variant, x, x_dtype, importance, gs_out + 1, codes, scales, m, n, padded_n, lower, upper,
-                              swizzled, stream);
+    const nvfp4_chain_item item = {x, importance, gs_out, scratch, codes, scales, m, n, padded_n};
+    if (m <= 0 || n <= 0) return NVFP4_ERR_BAD_SHAPE;
+    return nvfp4_quant_chain_multi_launch(variant, x_dtype, fp8_max, &item, 1, lower, upper, swizzled, stream);
 }
 
 extern "C" int nvfp4_quant_fused_launch(int variant, const void* x, int x_dtype, const float* importance, float fp8_max,
@@ -710,37 +885,13 @@ extern "C" int nvfp4_quant_fused_launch(int variant, const void* x, int x_dtype,
                                         int64_t n, int64_t padded_n, int lower, int upper, int swizzled, void* stream) {
     using namespace nvfp4;
     if (variant != NVFP4_VARIANT_MSE && variant != NVFP4_VARIANT_WEIGHTED) return NVFP4_ERR_BAD_ENUM;
-    if (x_dtype < NVFP4_DT_BF16 || x_dtype > NVFP4_DT_F32) return NVFP4_ERR_BAD_ENUM;
-    if (m < 0 || n < 0 || (n % kBlock) != 0 || (padded_n % kBlock) != 0 || padded_n < n) return NVFP4_ERR_BAD_SHAPE;
-    if (upper < lower || upper - lower + 1 > 64) return NVFP4_ERR_BAD_RANGE;
     if (!(fp8_max > 0.0f)) return NVFP4_ERR_BAD_RANGE;
     QuantParams p;
-    p.m = m;
-    p.n = n;
-    p.bin = n / kBlock;
-    p.bout = padded_n / kBlock;
-    p.k_pad = round_up_i64(p.bout, 4);
-    p.swizzled = swizzled ? 1 : 0;
-    p.width = swizzled ? p.k_pad : p.bout;
-    p.rows = swizzled ? round_up_i64(m, 128) : m;
-    p.total = p.rows * p.width;
-    set_width_div(p);
+    const int st = fill_params(p, variant, x, x_dtype, importance, gs_out, codes, scales, m, n, padded_n, lower, upper, swizzled);
+    if (st != NVFP4_OK) return st;
     if (p.total == 0 || m * n == 0) return NVFP4_ERR_BAD_SHAPE;   // an empty tensor has no maximum
-    if (!gs_out || !scratch || !codes || !scales || !x) return NVFP4_ERR_NULL_POINTER;
-    if (variant == NVFP4_VARIANT_WEIGHTED && !importance) return NVFP4_ERR_NULL_POINTER;
-    if ((reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(codes) & 7) ||
-        (reinterpret_cast<uintptr_t>(gs_out) & 3) || (reinterpret_cast<uintptr_t>(scratch) & 3))
-        return NVFP4_ERR_MISALIGNED;
-    if (swizzled && (reinterpret_cast<uintptr_t>(scales) & 3)) return NVFP4_ERR_MISALIGNED;
-    if (!swizzled && (p.width & 3) == 0 && (reinterpret_cast<uintptr_t>(scales) & 3)) return NVFP4_ERR_MISALIGNED;
-    if (variant == NVFP4_VARIANT_WEIGHTED && (reinterpret_cast<uintptr_t>(importance) & 15)) return NVFP4_ERR_MISALIGNED;
-    p.x = x;
-    p.importance = importance;
-    p.gs_inv = nullptr;
-    p.codes = codes;
-    p.scales = scales;
-    p.lower = lower;
-    p.ncand = upper - lower + 1;
+    if (!scratch) return NVFP4_ERR_NULL_POINTER;
+    if (reinterpret_cast<uintptr_t>(scratch) & 3) return NVFP4_ERR_MISALIGNED;
     p.fp8_max = fp8_max;
     p.gs_out = gs_out;
     p.fused_scratch = scratch;

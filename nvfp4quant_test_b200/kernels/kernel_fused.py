@@ -62,3 +62,11 @@ def scalesweep_nvfp4_quant_with_global_scale(
     g, g_inv = _helper.get_nvfp4_global_scale(input, fp8_max)
     quant_out(variant, input, importance, g_inv, is_sf_swizzled_layout, output, output_scale, lower, upper)
     return output, output_scale.view(torch.float8_e4m3fn), g, g_inv
+
+
+def scalesweep_nvfp4_quant_with_global_scales(inputs: list[torch.Tensor], fp8_max: float = _helper.FP8_E4M3_MAX_4OVER6):
+    """[scalesweep_nvfp4_quant_with_global_scale(x, fp8_max) for x in inputs], sharing launches: a layer's activations."""
+    got = _lib.fast.quant_dynamic_multi(_lib.VARIANT_MSE, inputs, fp8_max, _mse.LOWER_BOUND, _mse.UPPER_BOUND)
+    if got is not None:
+        return got
+    return [scalesweep_nvfp4_quant_with_global_scale(x, fp8_max) for x in inputs]

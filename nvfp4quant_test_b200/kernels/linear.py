@@ -103,3 +103,32 @@ class LinearGroup:
                                                       self._outs, self.tokens, _lib.current_stream_ptr(self.device))
         _lib.check(st, "nvfp4_gemm_launch_grouped")
         return self.outs
+
+
+class DecodeStep:
+    """Everything a layer computes from activations that are all at hand, in one host call: the quantization of each
+    activation (ActivationQuantizer) and the products that read it (LinearGroup).  One or two launches quantize the
+    activations together, one multiplies (nvfp4_quant_chain_multi_launch, nvfp4_gemm_launch_multi).  Outputs are the
+    groups' own; bits equal calling quantizers and groups one by one, up to the order of the fp32 sums."""
+
+    def __init__(self, quantizers: list[ActivationQuantizer], groups: list[tuple[int, LinearGroup]]):
+        """groups: (index of the quantizer whose output it reads, group)."""
+        for i, group in groups:
+            q = quantizers[i]
+            if q.k != group.k or q.tokens != group.tokens or q.device != group.device:
+                raise ValueError("a group and the quantizer it reads must agree on device, tokens and K")
+        self.quantizers, self.groups = list(quantizers), list(groups)
+        self._program = None
+        if all(q._chain is not None for q in quantizers) and all(g._group is not None for _, g in groups):
+            self._program = _lib.fast.make_program(tuple(q._chain for q in quantizers), tuple(i for i, _ in groups),
+                                                   tuple(g._group for _, g in groups))
+
+    def __call__(self, *acts: torch.Tensor) -> list[list[torch.Tensor]]:
+        """One activation per quantizer; returns each group's outputs."""
+        if not _lib.fast.program_call(self._program, *acts):
+            if len(acts) != len(self.quantizers):
+                raise ValueError(f"{len(self.quantizers)} activations are needed, got {len(acts)}")
+            quantized = [q(x) for q, x in zip(self.quantizers, acts)]
+            for i, group in self.groups:
+                group(*quantized[i])
+        return [group.outs for _, group in self.groups]

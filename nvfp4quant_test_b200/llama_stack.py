@@ -127,9 +127,9 @@ def layer_gemms_grouped(qlayer: dict, acts: dict[int, torch.Tensor], weight_scal
 
 class DecodeLayer:
     """layer_gemms_grouped with everything that does not depend on the activations done once: buffers allocated,
-    arguments checked, argument arrays built (kernels.ActivationQuantizer / kernels.LinearGroup).  A call is two
-    quantizer calls and four grouped GEMM calls into the C ABI, which is what lets a decode step be launched eagerly at
-    about the speed of a CUDA-graph replay.  Outputs are overwritten by the next call."""
+    arguments checked, argument arrays built (kernels.ActivationQuantizer / LinearGroup / DecodeStep).  The activations of
+    a call are all given, so it is one host call that quantizes them and multiplies with every matrix, two launches at a
+    few tokens.  Outputs are overwritten by the next call."""
 
     def __init__(self, qlayer: dict, weight_scales: dict, prepared: dict, tokens: int, device):
         self.quantizers = {}
@@ -141,19 +141,23 @@ class DecodeLayer:
             vec, slots = weight_scales[k]
             self.groups.append((group, k, K.LinearGroup([prepared[n] for n in group],
                                                         [vec[slots[n]:slots[n] + 1] for n in group], tokens)))
+        self._keys = list(self.quantizers)
+        self._step = K.DecodeStep(list(self.quantizers.values()), [(self._keys.index(k), g) for _, k, g in self.groups])
+        self._out = {name: out for group, _, linear in self.groups for name, out in zip(group, linear.outs)}
 
     def __call__(self, acts: dict[int, torch.Tensor]) -> dict[str, torch.Tensor]:
-        quantized = {k: q(acts[k]) for k, q in self.quantizers.items()}
-        out = {}
-        for group, k, linear in self.groups:
-            codes, scales, gs = quantized[k]
-            out.update(zip(group, linear(codes, scales, gs)))
-        return out
+        self._step(*[acts[k] for k in self._keys])
+        return dict(self._out)
 
 
 def _layer_gemms_prepared(qlayer: dict, acts: dict[int, torch.Tensor], act_importance: dict[str, torch.Tensor],
                           weight_scales: dict, prepared: dict) -> dict[str, torch.Tensor]:
     qact: dict[int, tuple] = {}
+    if not act_importance:      # the layer's activations are quantized together
+        used = list(dict.fromkeys(prepared[name].k for name in qlayer))
+        for k, (qa, sa, gs, _) in zip(used, K.scalesweep_nvfp4_quant_with_global_scales([acts[k] for k in used])):
+            vec, slots = weight_scales[k]
+            qact[k] = (qa, sa, gs, vec.unbind(0), slots)
     columns: tuple[list, ...] = ([], [], [], [], [])
     for name in qlayer:
         weight = prepared[name]

@@ -173,3 +173,49 @@ def test_quantizer_grids_equal_the_scalar_body(cuda_lib, m, n, padded_n, tiled):
             torch.cuda.synchronize()
             want = want or (codes, scales)
             assert torch.equal(codes, want[0]) and torch.equal(scales, want[1]), (impl, variant, lower)
+
+
+@pytest.mark.parametrize("shapes", [[(1, 64)], [(1, 4096), (1, 14336)], [(3, 4096), (3, 16384), (200, 320)],
+                                    [(64, 4096), (64, 14336)], [(256, 4096), (256, 14336)], [(1100, 8192), (9, 48)],
+                                    [(2, 128)] * 6])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_chains_over_several_tensors_equal_single_calls(cuda_lib, shapes, dtype):
+    """Global scale inside the quantizer, two launches shared by the tensors, or launches of their own: same bytes."""
+    import nvfp4quant_test_b200.kernels as K
+    from nvfp4quant_test_b200 import helper as H
+
+    xs = [torch.randn(s, device="cuda").to(dtype) * (i + 1) for i, s in enumerate(shapes)]
+    for _ in range(2):      # scratch words come back zeroed
+        got = K.scalesweep_nvfp4_quant_with_global_scales(xs, 256.0)
+        for x, g in zip(xs, got):
+            gs, gs_inv = H.get_nvfp4_global_scale(x, 256.0)
+            _same(g, [*K.scalesweep_mse_nvfp4_quant_impl(x, gs_inv), gs, gs_inv])
+            imp = torch.rand((1, x.shape[1]), device="cuda")
+            _same(K.scalesweep_nvfp4_quant_with_global_scale(x, 256.0, imp),
+                  [*K.scalesweep_weighted_mse_nvfp4_quant_impl(x, imp, gs_inv), gs, gs_inv])
+
+
+@pytest.mark.parametrize("tokens", [1, 16, 33, 64])
+def test_decode_step_equals_quantizers_and_groups_one_by_one(python_path, tokens):
+    import nvfp4quant_test_b200.kernels as K
+    from nvfp4quant_test_b200.kernels.kernel_gemm import gemm_last_status
+
+    def weight(n, k):
+        c, s, gs, _ = K.scalesweep_nvfp4_quant_with_global_scale(torch.randn((n, k), device="cuda").bfloat16(), 256.0)
+        return K.PreparedWeight(c, s), gs.reshape(1)
+
+    sets = [[weight(512, 1024), weight(200, 1024)], [weight(512, 1024)], [weight(1024, 2752)]]
+    quantizers = [K.ActivationQuantizer(tokens, 1024, "cuda"), K.ActivationQuantizer(tokens, 2752, "cuda")]
+    groups = [(i, K.LinearGroup([w for w, _ in ws], [s for _, s in ws], tokens)) for i, ws in zip((0, 0, 1), sets)]
+    step = K.DecodeStep(quantizers, groups)
+    acts = [torch.randn((tokens, k), device="cuda").bfloat16() for k in (1024, 2752)]
+    got = [o.clone() for o in _flat(step(*acts))]
+    assert gemm_last_status() == 0
+    with python_path():
+        want = _flat(step(*acts))
+    for g, w in zip(got, want):
+        assert torch.allclose(g.float(), w.float(), rtol=2.0 ** -7, atol=float(w.abs().max()) * 2.0 ** -12)
+    with pytest.raises(ValueError, match="activations are needed"):
+        step(acts[0])
+    with pytest.raises(ValueError, match="agree"):
+        K.DecodeStep(quantizers, [(1, groups[0][1])])
