@@ -29,8 +29,12 @@ struct PairCfg {
     static constexpr int kSfaBytes = 2048;                  // scales of this CTA's A rows
     static constexpr int kSfbBytes = 4096;                  // two 128-row scale groups cover the B tile
     static constexpr int kStageBytes = kABytes + kBBytes + kSfaBytes + kSfbBytes;
+    // ring stages against staged output pieces per epilogue warp: as deep a ring as leaves one piece (256 x 192 tiles with 5
+    // stages and two pieces: 5 % faster at K = 1024, 4 % slower at K = 8192)
     static constexpr int kStages = (BN == 128) ? 7 : (BN == 192) ? 6 : 5;
-    static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256;
+    static constexpr int kOutBufs = (BN == 256) ? 2 : 1;
+    static constexpr int kEpilogueBytes = 4 * kOutBufs * kPieceBytes;
+    static constexpr int kSmemBytes = kStages * kStageBytes + kEpilogueBytes + 256;
     static constexpr int kSfaCol = kAcc * BN;               // scale set 0; set 1 follows 48 columns later
     static constexpr int kSfbCol = kSfaCol + 16;
     static constexpr int kSfSetCols = 48;
@@ -84,7 +88,7 @@ __device__ __forceinline__ void tc_mma_pair(uint32_t d_tmem, uint32_t a_lo, uint
 // Operand maps and the work list of one launch over G products (G = 1: an ordinary GEMM).
 template <int G>
 struct PairParams {
-    CUtensorMap a[G], b[G], sfa[G], sfb[G];
+    CUtensorMap a[G], b[G], sfa[G], sfb[G], out[G];
     GroupTable<G> g;
     int M;
     int raster_group;
@@ -95,14 +99,13 @@ template <int BN, int G>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_pair_kernel(const __grid_constant__ PairParams<G> p) {
     using C = PairCfg<BN>;
-    extern __shared__ uint8_t smem_raw[];
+    extern __shared__ __align__(1024) uint8_t smem[];   // the 128-byte swizzle repeats every 1024 bytes
     // The kernel queued behind this one may be scheduled at once: ahead of its own wait it reads nothing but a
     // prepared (constant) weight, and that wait covers this kernel's completion.
     griddep_launch();
-    const uint32_t raw_addr = smem_u32(smem_raw);
-    const uint32_t base = (raw_addr + 1023u) & ~1023u;
-    uint8_t* aligned = smem_raw + (base - raw_addr);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(aligned + C::kStages * C::kStageBytes);
+    uint8_t* const aligned = smem;
+    const uint32_t base = smem_u32(aligned);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(aligned + C::kStages * C::kStageBytes + C::kEpilogueBytes);
     const uint32_t bar_base = smem_u32(bars);
     auto full_bar = [&](int s) { return bar_base + 8u * s; };
     auto empty_bar = [&](int s) { return bar_base + 8u * (C::kStages + s); };
@@ -287,6 +290,9 @@ gemm_pair_kernel(const __grid_constant__ PairParams<G> p) {
     } else {
         // ------------------------------------------------------------------ epilogue (both CTAs)
         const int sp = warp & 3;
+        // staged output, behind the ring
+        uint8_t* epilogue_stage = aligned + C::kStages * C::kStageBytes + sp * (C::kEpilogueBytes / 4);
+        int out_turn = 0;
         int alpha_item = -1;
         float alpha = 0.0f;
         uint32_t acc_phase = 0;
@@ -297,7 +303,6 @@ gemm_pair_kernel(const __grid_constant__ PairParams<G> p) {
             locate(tile, mt, nt);
             const GemmItem& it = p.g.item[cur.item];
             const int N = it.N;
-            const bool vec_ok = (N % 8) == 0;
             if (cur.item != alpha_item) {
                 alpha_item = cur.item;
                 alpha = load_alpha(it.alpha, it.alpha2);
@@ -306,37 +311,12 @@ gemm_pair_kernel(const __grid_constant__ PairParams<G> p) {
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
             if (!ok) break;
             tc_fence_after();
-            const int row = mt * 256 + static_cast<int>(rank) * 128 + sp * 32 + lane;
-            __nv_bfloat16* orow = it.out + static_cast<int64_t>(row) * N;
-#pragma unroll 1
-            for (int c = 0; c < BN / 32; ++c) {
-                uint32_t v[32];
-                tc_ld_32x32b_x32(tmem_base + (static_cast<uint32_t>(sp * 32) << 16) + acc * BN + c * 32, v);
-                tc_ld_wait();
-                const int col0 = nt * BN + c * 32;
-                if (row < p.M && col0 < N) {
-                    if (vec_ok && col0 + 32 <= N) {
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            uint32_t w[4];
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                const float lo = __fmul_rn(__uint_as_float(v[q * 8 + 2 * e]), alpha);
-                                const float hi = __fmul_rn(__uint_as_float(v[q * 8 + 2 * e + 1]), alpha);
-                                __nv_bfloat162 b2 = __floats2bfloat162_rn(lo, hi);
-                                w[e] = *reinterpret_cast<uint32_t*>(&b2);
-                            }
-                            *reinterpret_cast<uint4*>(orow + col0 + q * 8) = make_uint4(w[0], w[1], w[2], w[3]);
-                        }
-                    } else {
-                        for (int e = 0; e < 32; ++e)
-                            if (col0 + e < N) orow[col0 + e] = __float2bfloat16_rn(__fmul_rn(__uint_as_float(v[e]), alpha));
-                    }
-                }
-            }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(map_to_cta(tempty_bar(acc), 0));
+            store_accumulator<BN, C::kOutBufs>(tmem_base + (static_cast<uint32_t>(sp * 32) << 16) + acc * BN, it.out, &p.out[cur.item], p.M, N,
+                                  mt * 256 + static_cast<int>(rank) * 128 + sp * 32, nt * BN, alpha, epilogue_stage, out_turn, [&] {
+                                      tc_fence_before();
+                                      __syncwarp();
+                                      if (lane == 0) mbar_arrive_cluster(map_to_cta(tempty_bar(acc), 0));
+                                  });
             if (++acc == C::kAcc) {
                 acc = 0;
                 acc_phase ^= 1u;
@@ -344,6 +324,7 @@ gemm_pair_kernel(const __grid_constant__ PairParams<G> p) {
         }
     }
 
+    if (warp >= 2 && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     if (lane == 0) trace_mark(1, warp == 0 ? 3 : warp == 1 ? 4 : 5);
     // ---------------------------------------------------------------------- teardown
     if (*abort_flag) {
@@ -396,6 +377,7 @@ static int launch_pair_list(const GemmParams* list, const WeightHandle* const* w
         const GemmParams& p = list[i];
         int st = make_operand_map(&q.a[i], p.a, p.M, p.K / 2, 128);
         if (st == NVFP4_OK) st = make_scale_map(&q.sfa[i], p.sfa, p.sfa_groups, p.sf_group_stride);
+        if (st == NVFP4_OK) st = make_output_map(&q.out[i], p.out, p.M, p.N);
         if (wh[i]) {
             q.b[i] = *wh[i]->by_rows(BN / 2);
             q.sfb[i] = wh[i]->scales;

@@ -6,6 +6,12 @@
 namespace nvfp4 {
 namespace gemm {
 
+// Epilogue staging, per epilogue warp: a piece of 32 rows x 64 columns of bf16 for a TMA store, or half of one (with a word
+// of padding per row) that is turned for rows TMA cannot write.
+constexpr int kPieceBytes = 4096;
+constexpr int kTurnPitch = 17;   // 32-bit words per row: conflict-free both ways
+constexpr int kTurnBytes = 32 * kTurnPitch * 4;
+
 template <int BN>
 struct Cfg {
     static constexpr int kNG = (BN + 127) / 128;            // 128-row scale groups a B tile touches (a 64-row tile: half of one)
@@ -17,8 +23,13 @@ struct Cfg {
     static constexpr int kStageBytes = kABytes + kBBytes + kSfaBytes + kSfbBytes;
     // ring depth: as many stages as fit in shared memory (the bytes in flight per SM are what keeps HBM busy when
     // few CTAs stream a long K)
-    static constexpr int kStages = (BN == 64) ? 8 : (BN == 128) ? 6 : 4;
-    static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*align*/ + 256 /*barriers*/;
+    static constexpr int kStages = (BN == 64) ? 7 : (BN == 128) ? 6 : 4;
+    // staged output pieces per epilogue warp; 0: the ring is worth more than they are (with 5 stages and two pieces 128 x 128
+    // tiles gain 7 % at K = 1088 and lose 5 % at K = 2880), so rows go out of the registers
+    static constexpr int kOutBufs = 0;
+    static constexpr int kEpilogueBytes = 4 * (kOutBufs > 0 ? kOutBufs * kPieceBytes : kTurnBytes);
+    static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*align*/ + 256 /*barriers*/ + kEpilogueBytes;
+
     // scale factors sit behind the accumulators, in two sets used by alternate K tiles so that the
     // copies for the next K tile do not have to wait for the MMAs still reading the current set
     static constexpr int kSfSetCols = 16 + 16 * kNG;
@@ -65,6 +76,118 @@ struct GemmItem {
     int sfb_groups;
     int tile_end;             // tiles of this and the earlier items of its class
 };
+
+// ---- epilogue -----------------------------------------------------------------------------------------------------
+// A warp holds 32 rows of an accumulator, lane = row, and writes them as bf16(alpha * v).
+//
+// Written 16 bytes per lane straight from the registers, a store instruction touches 32 rows, half a sector of each: that
+// bound every product whose K is short, and 2 bytes per lane where rows are no multiple of 16 bytes bound those at any K.
+// Now, rows of a multiple of 16 bytes go out as TMA stores of 32 x 64 pieces (asynchronous, whole lines; pieces of 32 columns
+// are 10 % slower; ragged edges clipped by the tensor map) or, where the ring leaves no room, 32 bytes per lane; other rows
+// are turned through shared memory so that an instruction covers neighbours of one or two rows.  Measured (us): 4585 x 12864 x
+// 2880 104 -> 82, 5644 x 16832 x 1088 140 -> 80, 8192^3 210 -> 198, 517 x 738 x 2240 22.7 -> 7.0, 2092 x 17604 x 6784 442 -> 115.
+
+__device__ __forceinline__ uint32_t scaled_pair(uint32_t lo, uint32_t hi, float alpha) {
+    const __nv_bfloat162 b2 = __floats2bfloat162_rn(__fmul_rn(__uint_as_float(lo), alpha), __fmul_rn(__uint_as_float(hi), alpha));
+    return *reinterpret_cast<const uint32_t*>(&b2);
+}
+
+// 32 columns (16-byte chunks first .. first + 3 of a row) of a piece laid out for a TMA store with 128-byte swizzle.
+__device__ __forceinline__ void stage_half(uint32_t piece, int first, float alpha, const uint32_t v[32]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(piece + lane * 128 + (((first + q) ^ (lane & 7)) << 4)),
+                     "r"(scaled_pair(v[8 * q], v[8 * q + 1], alpha)), "r"(scaled_pair(v[8 * q + 2], v[8 * q + 3], alpha)),
+                     "r"(scaled_pair(v[8 * q + 4], v[8 * q + 5], alpha)), "r"(scaled_pair(v[8 * q + 6], v[8 * q + 7], alpha))
+                     : "memory");
+}
+
+// 32 columns from the registers, by way of `turn` where they do not start on 16-byte boundaries.
+__device__ __forceinline__ void store_half(__nv_bfloat16* out, int M, int N, int row0, int col0, float alpha, const uint32_t v[32],
+                                           uint32_t* turn) {
+    const int lane = threadIdx.x & 31;
+    uint32_t w[16];
+#pragma unroll
+    for (int e = 0; e < 16; ++e) w[e] = scaled_pair(v[2 * e], v[2 * e + 1], alpha);
+    if ((N & 7) == 0 && col0 + 32 <= N) {
+        if (row0 + lane >= M) return;
+        __nv_bfloat16* dst = out + static_cast<int64_t>(row0 + lane) * N + col0;
+        if ((N & 15) == 0 && (reinterpret_cast<uintptr_t>(out) & 31) == 0) {
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+                asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst + 16 * q), "r"(w[8 * q]),
+                             "r"(w[8 * q + 1]), "r"(w[8 * q + 2]), "r"(w[8 * q + 3]), "r"(w[8 * q + 4]), "r"(w[8 * q + 5]),
+                             "r"(w[8 * q + 6]), "r"(w[8 * q + 7])
+                             : "memory");
+        } else {
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                *reinterpret_cast<uint4*>(dst + 8 * q) = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+        }
+        return;
+    }
+    __syncwarp();   // what was turned before has been read
+#pragma unroll
+    for (int e = 0; e < 16; ++e) turn[lane * kTurnPitch + e] = w[e];
+    __syncwarp();
+    const int cols = min(32, N - col0), rows = min(32, M - row0);
+    if ((N & 1) == 0) {   // rows start on 4-byte boundaries (col0 is even): two rows per store
+        const int c = lane & 15;
+        if (2 * c < cols)
+            for (int r = lane >> 4; r < rows; r += 2)
+                *reinterpret_cast<uint32_t*>(out + static_cast<int64_t>(row0 + r) * N + col0 + 2 * c) = turn[r * kTurnPitch + c];
+    } else if (lane < cols) {
+        const uint16_t* half = reinterpret_cast<const uint16_t*>(turn) + lane;
+        for (int r = 0; r < rows; ++r)
+            reinterpret_cast<uint16_t*>(out)[static_cast<int64_t>(row0 + r) * N + col0 + lane] = half[r * kTurnPitch * 2];
+    }
+}
+
+// One warp's 32 rows of an accumulator of BN columns.  The next 32 columns are on their way from TMEM while the current ones
+// are rounded and stored, and `release` (the accumulator may be overwritten) runs as soon as the last ones have arrived.
+// `turn` says which of the BUFS staged pieces is next; the caller waits for the last TMA stores before it returns.
+template <int BN, int BUFS, class Release>
+__device__ __forceinline__ void store_accumulator(uint32_t taddr, __nv_bfloat16* out, const CUtensorMap* map, int M, int N, int row0, int col0,
+                                                  float alpha, uint8_t* stage, int& turn, Release release) {
+    static_assert(BN % 64 == 0, "pieces of 64 columns");
+    const bool tma = BUFS > 0 && (N & 7) == 0;
+    const bool first_lane = (threadIdx.x & 31) == 0;
+    uint32_t a[32], b[32];
+    tc_ld_32x32b_x32(taddr, a);
+#pragma unroll 1
+    for (int c = 0; c < BN; c += 64) {
+        const bool inside = row0 < M && col0 + c < N;
+        const uint32_t piece = smem_u32(stage) + (BUFS > 1 ? turn : 0) * kPieceBytes;
+        if (BUFS > 1 && ++turn == BUFS) turn = 0;
+        tc_ld_wait();
+        tc_ld_32x32b_x32(taddr + c + 32, b);
+        if (tma) {
+            if (first_lane) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(BUFS > 0 ? BUFS - 1 : 0) : "memory");
+            __syncwarp();   // what was staged here before has been read
+            stage_half(piece, 0, alpha, a);
+        } else if (inside) {
+            store_half(out, M, N, row0, col0 + c, alpha, a, reinterpret_cast<uint32_t*>(stage));
+        }
+        tc_ld_wait();
+        if (c + 64 < BN) tc_ld_32x32b_x32(taddr + c + 64, a);
+        else release();
+        if (tma) {
+            stage_half(piece, 4, alpha, b);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (first_lane) {
+                if (inside)
+                    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(map), "r"(piece),
+                                 "r"(col0 + c), "r"(row0)
+                                 : "memory");
+                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            }
+        } else if (inside && col0 + c + 32 < N) {
+            store_half(out, M, N, row0, col0 + c + 32, alpha, b, reinterpret_cast<uint32_t*>(stage));
+        }
+    }
+}
 
 template <int G>
 struct GroupTable {
@@ -121,7 +244,7 @@ __device__ __forceinline__ void tile_to_mn(int tile, int m_tiles, int n_tiles, i
 // Operand maps and the work list of one launch over G products (G = 1: an ordinary GEMM, whose K may be cut into ranges).
 template <int G>
 struct TileParams {
-    CUtensorMap a[G], b[G];
+    CUtensorMap a[G], b[G], out[G];
     GroupTable<G> g;
     int M;
     int k_splits, k_tiles_per_split, k_rotate;   // G = 1 only, see GemmParams
@@ -144,7 +267,7 @@ gemm_kernel(const __grid_constant__ TileParams<G> p) {
     const uint32_t base = (raw_addr + 1023u) & ~1023u;
     uint8_t* aligned = smem_raw + (base - raw_addr);
     // ring: [stage][A | B | SFA | SFB]; then barriers
-    uint64_t* bars = reinterpret_cast<uint64_t*>(aligned + C::kStages * C::kStageBytes);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(aligned + C::kStages * C::kStageBytes + C::kEpilogueBytes);
     const uint32_t bar_base = smem_u32(bars);
     auto full_bar = [&](int s) { return bar_base + 8u * s; };
     auto empty_bar = [&](int s) { return bar_base + 8u * (C::kStages + s); };
@@ -362,6 +485,9 @@ gemm_kernel(const __grid_constant__ TileParams<G> p) {
     } else {
         // ------------------------------------------------------------------ epilogue (warps 2..5)
         const int sp = warp & 3;  // TMEM sub-partition this warp may read: lanes 32*sp .. 32*sp+31
+        // staged output, behind the ring
+        uint8_t* epilogue_stage = aligned + C::kStages * C::kStageBytes + sp * (C::kEpilogueBytes / 4);
+        int out_turn = 0;
         int alpha_item = -1;
         float alpha = 0.0f;
         int acc = 0;
@@ -372,7 +498,6 @@ gemm_kernel(const __grid_constant__ TileParams<G> p) {
             locate(tile, ks, mt, nt);
             const GemmItem& it = p.g.item[cur.item];
             const int N = it.N;
-            const bool vec_ok = (N % 8) == 0;
             if (cur.item != alpha_item) {
                 alpha_item = cur.item;
                 alpha = load_alpha(it.alpha, it.alpha2);
@@ -381,50 +506,36 @@ gemm_kernel(const __grid_constant__ TileParams<G> p) {
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
             if (!ok) break;
             tc_fence_after();
-            const int row = mt * kBM + sp * 32 + lane;
-            __nv_bfloat16* orow = it.out + static_cast<int64_t>(row) * N;
+            const int row0 = mt * kBM + sp * 32;
+            const uint32_t taddr = tmem_base + (static_cast<uint32_t>(sp * 32) << 16) + acc * BN;
+            auto release = [&] {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(tempty_bar(acc));
+            };
+            if (splits == 1) {
+                store_accumulator<BN, C::kOutBufs>(taddr, it.out, &p.out[cur.item], p.M, N, row0, nt * BN, alpha, epilogue_stage, out_turn, release);
+            } else {
+                // fp32 partials of this K range; alpha and the bf16 rounding happen in the reduction kernel
 #pragma unroll 1
-            for (int c = 0; c < BN / 32; ++c) {
-                uint32_t v[32];
-                tc_ld_32x32b_x32(tmem_base + (static_cast<uint32_t>(sp * 32) << 16) + acc * BN + c * 32, v);
-                tc_ld_wait();
-                const int col0 = nt * BN + c * 32;
-                if (splits > 1) {
-                    // fp32 partial of this K range; alpha and the bf16 rounding happen in the reduction kernel
-                    if (row < p.M && col0 < N) {
-                        float* prow = p.partial + (static_cast<int64_t>(ks) * p.M + row) * N + col0;
-                        if ((N % 4) == 0 && col0 + 32 <= N) {
+                for (int c = 0; c < BN / 32; ++c) {
+                    uint32_t v[32];
+                    tc_ld_32x32b_x32(taddr + c * 32, v);
+                    tc_ld_wait();
+                    const int col0 = nt * BN + c * 32;
+                    if (row0 + lane >= p.M || col0 >= N) continue;
+                    float* prow = p.partial + (static_cast<int64_t>(ks) * p.M + row0 + lane) * N + col0;
+                    if ((N % 4) == 0 && col0 + 32 <= N) {
 #pragma unroll
-                            for (int q = 0; q < 8; ++q)
-                                *reinterpret_cast<uint4*>(prow + 4 * q) = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-                        } else {
-                            for (int e = 0; e < 32; ++e)
-                                if (col0 + e < N) prow[e] = __uint_as_float(v[e]);
-                        }
-                    }
-                } else if (row < p.M && col0 < N) {
-                    if (vec_ok && col0 + 32 <= N) {
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            uint32_t w[4];
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                const float lo = __fmul_rn(__uint_as_float(v[q * 8 + 2 * e]), alpha);
-                                const float hi = __fmul_rn(__uint_as_float(v[q * 8 + 2 * e + 1]), alpha);
-                                __nv_bfloat162 b2 = __floats2bfloat162_rn(lo, hi);
-                                w[e] = *reinterpret_cast<uint32_t*>(&b2);
-                            }
-                            *reinterpret_cast<uint4*>(orow + col0 + q * 8) = make_uint4(w[0], w[1], w[2], w[3]);
-                        }
+                        for (int q = 0; q < 8; ++q)
+                            *reinterpret_cast<uint4*>(prow + 4 * q) = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
                     } else {
                         for (int e = 0; e < 32; ++e)
-                            if (col0 + e < N) orow[col0 + e] = __float2bfloat16_rn(__fmul_rn(__uint_as_float(v[e]), alpha));
+                            if (col0 + e < N) prow[e] = __uint_as_float(v[e]);
                     }
                 }
+                release();
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(tempty_bar(acc));
             if (++acc == C::kAcc) {
                 acc = 0;
                 acc_phase ^= 1u;
@@ -432,6 +543,7 @@ gemm_kernel(const __grid_constant__ TileParams<G> p) {
         }
     }
 
+    if (warp >= 2 && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     if (lane == 0) trace_mark(0, warp == 0 ? 3 : warp == 1 ? 4 : 5);
     // ---------------------------------------------------------------------- teardown
     if (*abort_flag) {
@@ -492,6 +604,20 @@ static int make_operand_map(CUtensorMap* map, const void* ptr, int64_t rows, int
     CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(ptr), dims, strides, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? NVFP4_OK : NVFP4_ERR_UNSUPPORTED;
+}
+
+// The output [M, N] bf16 in pieces of 32 rows x 64 columns; only for rows of a multiple of 16 bytes (else left undefined).
+static int make_output_map(CUtensorMap* map, void* ptr, int64_t M, int64_t N) {
+    if (N % 8) return NVFP4_OK;
+    EncodeTiledFn enc = encode_tiled_fn();
+    if (!enc) return NVFP4_ERR_UNSUPPORTED;
+    cuuint64_t dims[2] = {static_cast<cuuint64_t>(N), static_cast<cuuint64_t>(M)};
+    cuuint64_t strides[1] = {static_cast<cuuint64_t>(N * 2)};
+    cuuint32_t box[2] = {64, 32};
+    cuuint32_t estr[2] = {1, 1};
+    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                     CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? NVFP4_OK : NVFP4_ERR_UNSUPPORTED;
 }
 
@@ -619,6 +745,7 @@ static int launch_list(const GemmParams* list, const WeightHandle* const* wh, in
     for (int i = 0; i < n; ++i) {
         const GemmParams& p = list[i];
         int st = make_operand_map(&q.a[i], p.a, p.M, p.K / 2, kBM);
+        if (st == NVFP4_OK) st = make_output_map(&q.out[i], p.out, p.M, p.N);
         if (wh[i]) {
             q.b[i] = *wh[i]->by_rows(BN);
         } else {

@@ -68,3 +68,30 @@ def test_list_arguments_are_checked(cuda_lib):
     w.close()
     with pytest.raises(ValueError, match="closed"):
         K.nvfp4_scaled_mm_multi([a], [s], [gs], [w], [gw])
+
+
+@pytest.mark.parametrize("path", [1, 2, 3, 4, 6, 7])
+@pytest.mark.parametrize("m,n", [(33, 8), (129, 63), (130, 66), (257, 100), (300, 191), (128, 193), (100, 255), (257, 260), (65, 768)])
+def test_every_row_alignment_and_edge_of_the_epilogue(cuda_lib, path, m, n):
+    """Rows of whole 16 bytes, of 4 bytes and of 2, pieces cut by both edges of the matrix, nothing written beside it."""
+    import nvfp4quant_test_b200.kernels as K
+    from nvfp4quant_test_b200 import helper as H
+
+    k = 320
+    a, sa, ga = _operand(m, k, m)
+    b, sb, gb = _operand(n, k, n)
+    alpha = (ga * gb).reshape(1)
+    guard = torch.full((m * n + 256,), 7.0, dtype=torch.bfloat16, device="cuda")
+    out = guard[128:128 + m * n].view(m, n)
+    try:
+        assert cuda_lib.nvfp4_gemm_force_path(path) == 0
+        K.nvfp4_scaled_mm(a, b, sa, sb, alpha, torch.bfloat16, out)
+        torch.cuda.synchronize()
+    finally:
+        cuda_lib.nvfp4_gemm_force_path(0)
+    one = torch.ones((), device="cuda")
+    da = H.dequantize("base", a, K.unswizzle_vllm_fp4_scale(sa, m, k), one).double()
+    db = H.dequantize("base", b, K.unswizzle_vllm_fp4_scale(sb, n, k), one).double()
+    want = (da @ db.T) * alpha.double()
+    assert ((out.double() - want).abs() <= want.abs() * 2.0 ** -7 + want.abs().max() * 2.0 ** -16).all()
+    assert (guard[:128] == 7.0).all() and (guard[128 + m * n:] == 7.0).all()
