@@ -23,6 +23,8 @@
 // This file holds the C entry points and the kernel choice; the kernels live in gemm_tile.cuh (one CTA per tile),
 // gemm_pair.cuh (CTA pairs, cta_group::2) and gemm_skinny.cuh (decode-sized batches, K ranges across a cluster),
 // all on the PTX wrappers of tc_ptx.cuh.  One translation unit, so that there is one status word.
+#include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <new>
 #include <utility>
@@ -105,26 +107,69 @@ static int table_path(int64_t M, int64_t N, int64_t K) {
     return path;
 }
 
+// Microseconds of one launch, by kernel.  A tile (or a pair's tile) takes the longer of its K stages and its share of the
+// weights, tokens and output at the rate the kernel streams them; tiles go over the SMs in waves, of which the first hides
+// no epilogue and is otherwise the same.  The constants are a fit to 930 random shapes (17 .. 8192 tokens, N 512 .. 28672, K
+// 1024 .. 14336), a third of them with the weights coming from HBM every time: rms error 8-12 %, and the kernel chosen by it
+// is on average 0.5 % slower than the fastest one from 65 tokens on (the cost model before it: 3-5 %, up to 55 % at 65-128).
+struct TileCost {
+    int path, rows, cols, pair;
+    double launch, first_stage, stage, epilogue, rate, out_weight;   // us, us per K stage, us, KB per us
+};
+static const TileCost kTileCosts[] = {
+    {1, 128, 128, 0, 3.49, 0.294, 0.304, 0.60, 5437.0, 2.06}, {2, 128, 256, 0, 4.09, 0.380, 0.464, 1.52, 5371.0, 1.49},
+    {3, 256, 256, 1, 5.16, 0.299, 0.371, 1.37, 5863.0, 2.14}, {4, 256, 192, 1, 5.07, 0.230, 0.300, 0.81, 5397.0, 1.42},
+    {6, 128, 64, 0, 3.28, 0.285, 0.282, 0.52, 3663.0, 0.39},  {7, 256, 128, 1, 4.72, 0.191, 0.235, 0.89, 4850.0, 1.36}};
+
+static double tile_time(const TileCost& c, int64_t M, int64_t N, int64_t K, int sms) {
+    const double workers = c.pair ? (sms > 1 ? sms / 2 : 1) : sms;
+    const double tiles = static_cast<double>((M + c.rows - 1) / c.rows) * static_cast<double>((N + c.cols - 1) / c.cols);
+    const double k = static_cast<double>((K + 255) / 256);
+    const double kbytes = (static_cast<double>(M + N) * static_cast<double>(K) * 9.0 / 16.0 + c.out_weight * 2.0 * M * N) / 1000.0;
+    const double share = kbytes / tiles / c.rate, steady = k * c.stage + c.epilogue;
+    const double full = std::floor(tiles / workers), rest = tiles - full * workers;
+    double t = c.launch + std::max(k * c.first_stage, share * std::min(tiles, workers));
+    if (full > 1.0) t += (full - 1.0) * std::max(steady, share * workers);
+    if (full > 0.0 && rest > 0.0) t += std::max(steady, share * rest);
+    return t;
+}
+
+// The decode-sized kernel, 33 to 128 tokens: it streams the weights whatever its K ranges, and its epilogue grows with the
+// token tile.
+static double skinny_time(int64_t M, int64_t N, int64_t K) {
+    return 4.1 + static_cast<double>(M + N) * static_cast<double>(K) * (9.0 / 16.0) / 5.4e6 + 0.03 * static_cast<double>(M);
+}
+
 // Kernel choice for one shape: host arithmetic only.  *path: 1 = 128x128 tiles, 2 = 128x256, 3 = pair 256x256,
 // 4 = pair 256x192, 5 = skinny, 6 = 128x64, 7 = pair 256x128; *k_ranges: cluster size of the skinny kernel (1 for the others).
 static void plan_gemm(int64_t M, int64_t N, int64_t K, int sms, int k_splits, int* path_out, int* ranges_out) {
     const int k_tiles_total = static_cast<int>((K + 255) / 256);
     const int n_tiles = static_cast<int>((N + 127) / 128);
     *ranges_out = 1;
-    // Decode-sized batches: weight rows on the MMA's 128 rows, tokens on its N dimension, K ranges across a cluster.
-    // Measured on B200 with the weights streaming from HBM: faster than every other kernel up to 32 tokens; from 33
-    // to 128 tokens only where few weight tiles meet a long K (at least 4 K ranges of at least 12 stages each, e.g.
-    // 64 x 4096 x 14336: 13.2 us against 19.4 us), because its epilogue grows with the token tile.
+    int best = 0;
+    double best_time = 0.0;
+    for (const TileCost& c : kTileCosts) {
+        if (c.pair && N <= 128) continue;
+        double t = tile_time(c, M, N, K, sms);
+        // Two corrections the fit does not see: with a long K the pair that shares its weight rows is ahead of what the model
+        // says when those come from HBM (256 x 8192 x 8192, weights cold: 18.0 us against 21.1 with 128x128 or 256x192 tiles),
+        // and 256x192 tiles, whose two accumulators overlap, lose less than 256x256 ones to the power cap over long launches
+        // (8192 x 16384 x 4096 211 against 225 us, 20000 x 8192 x 8192 603 against 623).
+        if (c.path == 7 && M > 128 && k_tiles_total >= 28) t *= 0.9;
+        if (c.path == 4 && M > 128) t *= 0.95;
+        if (best == 0 || t < best_time) {
+            best = c.path;
+            best_time = t;
+        }
+    }
+    // Decode-sized batches: weight rows on the MMA's 128 rows, tokens on its N dimension, K ranges across a cluster.  Up to 32
+    // tokens always; up to 48 where more than 64 weight tiles make it a plain stream, which the tile kernels sustain less well
+    // than the model says (45 x 27520 x 4352: 15.0 us against 17.3); up to 128 where the model puts it clearly ahead.
     bool skinny = false;
     if (g_gemm_force_path == 5) {
         skinny = M <= kSkinnyMaxM;
     } else if (g_gemm_force_path == 0 && g_gemm_force_splits == 0 && M <= kSkinnyMaxM) {
-        const int ranks = nvfp4::gemm::skinny::choose_ranks(n_tiles, k_tiles_total, sms, 0, M <= 64 ? 64 : 128);
-        // measured with the weights streaming from HBM (microseconds, decode-sized kernel against the best tile / pair
-        // kernel): 48 x 4096 x 4096 6.5 / 7.3, 48 x 6144 x 4096 7.6 / 8.8, 48 x 8192 x 8192 11.7 / 12.1, but 48 x 28672 x
-        // 8192 33.9 / 27.4; 64 x 1024 x 4096 5.0 / 6.3, 64 x 6144 x 4096 8.1 / 7.7
-        skinny = M <= kSkinnyAutoM || (M <= 48 && n_tiles <= 64) || (M <= 64 && n_tiles <= 8) ||
-                 (ranks >= 4 && k_tiles_total / ranks >= 12);
+        skinny = M <= kSkinnyAutoM || (M <= 48 && n_tiles > 64) || skinny_time(M, N, K) < 0.95 * best_time;
     }
     if (skinny) {
         const int forced = g_gemm_force_path == 5 ? g_gemm_force_splits : 0;
@@ -136,51 +181,10 @@ static void plan_gemm(int64_t M, int64_t N, int64_t K, int sms, int k_splits, in
         *ranges_out = ranks;
         return;
     }
-    // Kernel choice by a small cost model fitted to measurements on B200: time ~ waves x cost of one tile, where a
-    // wave is one single-CTA tile per SM or one CTA-pair tile per two SMs (148 / 74 on a B200).  Relative tile costs: 128x64 -> 0.45, 128x128 -> 0.7, 128x256 -> 1.0,
-    // pair 256x192 -> 0.68 (0.75 of the MMA work per SM, and its epilogue overlaps the next tile), pair 256x256 -> 0.96,
-    // pair 256x128 -> 0.6.
     int path = g_gemm_force_path == 5 ? 0 : g_gemm_force_path;   // 0 = choose by shape
     // shapes of the measured table (on the GPU it was measured on) take the kernel that was fastest there
     if (path == 0 && k_splits == 1 && sms == 148) path = table_path(M, N, K);
-    if (path == 0) {
-        const int64_t mt = (M + 127) / 128;
-        const int64_t wave1 = sms, wave2 = sms / 2 > 0 ? sms / 2 : 1;   // tiles per wave: single CTAs, CTA pairs
-        const double c1 = static_cast<double>((mt * ((N + 127) / 128) + wave1 - 1) / wave1) * 0.7;
-        const double c2 = static_cast<double>((mt * ((N + 255) / 256) + wave1 - 1) / wave1) * 1.0;
-        const double c4 = static_cast<double>((((M + 255) / 256) * ((N + 191) / 192) + wave2 - 1) / wave2) * 0.68;
-        path = (c1 <= c2) ? 1 : 2;
-        double best = c1 <= c2 ? c1 : c2;
-        // the pair kernels need a clear margin: at equal wave counts the single-CTA kernels put more CTAs on the
-        // weight stream (512 x 4096 x 4096: 128x128 tiles 9.8 us, pair 256x192 10.5 us)
-        // ... while per K stage the pair is cheaper, so from ~26 stages on it wins again (512 x 4096 x 14336: 19.8 / 21.7 us)
-        const double margin = k_tiles_total >= 26 ? 0.0 : 0.03;
-        if (M > 128 && N > 128 && k_splits == 1 && c4 < best - margin) {
-            path = 4;
-            best = c4;
-        }
-        // pair 256x256: 0.96 per wave of 74 pairs; wins where it needs fewer waves than the others (1024 x 4096 x
-        // 14336: 25.4 us against 28.1 us with 128x256 tiles)
-        const double c3 = static_cast<double>((((M + 255) / 256) * ((N + 255) / 256) + wave2 - 1) / wave2) * 0.96;
-        if (M > 128 && N > 128 && k_splits == 1 && c3 < best) {
-            path = 3;
-            best = c3;
-        }
-        // pair 256x128: 0.6 per wave; the kernel for a few hundred tokens (256 x 8192 x 8192: 13.4 us against 14.8 us
-        // with 128x128 tiles): as many CTAs as those, each loading only half of its tile's weight rows
-        const double c7 = static_cast<double>((((M + 255) / 256) * ((N + 127) / 128) + wave2 - 1) / wave2) * 0.6;
-        // (with one token tile the second CTA of a pair has no rows, yet from ~20 K stages on sharing the weight
-        // rows still wins: 64 x 8192 x 8192 12.6 us against 13.3 us with 128x64 tiles)
-        if ((M > 128 || k_tiles_total >= 20) && N > 128 && k_splits == 1 && c7 < best) {
-            path = 7;
-            best = c7;
-        }
-        // few tiles (one or two token tiles): 64 weight rows per CTA put twice as many SMs on the weight stream; every
-        // CTA re-reads the token tile, which costs per K stage, so from ~20 stages on it is rated 1.4x
-        // (256 x 4096 x 14336: 20.0 us against 16.6 us with pair 256x128)
-        const double c6 = static_cast<double>((mt * ((N + 63) / 64) + wave1 - 1) / wave1) * 0.45 * (k_tiles_total >= 20 ? 1.4 : 1.0);
-        if (mt <= 2 && c6 < best) path = 6;
-    }
+    if (path == 0) path = best;
     if (k_splits > 1 && path != 1 && path != 2 && path != 6) path = 1;
     *path_out = path;
 }
@@ -265,25 +269,28 @@ static int gemm_launch_impl(const uint8_t* a, const uint8_t* b, const uint8_t* s
     return gemm::launch<128>(p, s, wh);
 }
 
-// Kernel of a launch over several products (sorted by K): the same relative tile costs as plan_gemm, per K stage, times the
-// longest worker's stages.  0 = launch them one by one (a kernel is forced that has no form for lists).
+// Kernel of a launch over several products (sorted by K): the tile costs of plan_gemm over the busiest worker's tiles.  0 = launch them one by one (a kernel is forced that has no form for lists).
 static int plan_list(const nvfp4::gemm::GemmParams* list, int n, int sms) {
     using namespace nvfp4::gemm;
     if (g_gemm_force_splits != 0) return 0;
     if (g_gemm_force_path != 0)
         return g_gemm_force_path == 1 || g_gemm_force_path == 3 || g_gemm_force_path == 4 || g_gemm_force_path == 7 ? g_gemm_force_path : 0;
-    struct { int path, rows, cols, pair; double cost; } const kinds[] = {
-        {1, 128, 128, 0, 0.70}, {7, 256, 128, 1, 0.60}, {4, 256, 192, 1, 0.68}, {3, 256, 256, 1, 0.96}};
-    double best = 0.0;
+    double best = 0.0, kbytes = 0.0;
+    for (int i = 0; i < n; ++i) kbytes += static_cast<double>(list[i].M + list[i].N) * list[i].K * 9.0 / 16000.0 + 2.0 * list[i].M * list[i].N / 1000.0;
     int path = 0;
-    for (const auto& kind : kinds) {
+    for (const TileCost& c : kTileCosts) {
+        if (c.path == 2 || c.path == 6) continue;   // no form for lists
+        // one token tile: the second CTA of a pair has no rows (Llama-3-8B layer, 128 tokens: 24.8 us with 128x128 tiles, 29.0
+        // with 256x192, 30.1 with 256x256)
+        if (c.pair && list[0].M <= 128) continue;
         GroupTable<kMaxItems> g;
-        const int used = fill_group_table<kMaxItems>(g, list, n, (list[0].M + kind.rows - 1) / kind.rows, kind.cols, kind.pair ? sms / 2 : sms);
+        const int used = fill_group_table<kMaxItems>(g, list, n, (list[0].M + c.rows - 1) / c.rows, c.cols, c.pair ? sms / 2 : sms);
         if (used == 0) continue;
-        const double t = kind.cost * list_makespan(g, list);
+        double t = c.launch + std::max(list_makespan(g, list, c.stage, c.epilogue), kbytes / c.rate);
+        if (c.path == 4) t *= 0.95;   // as in plan_gemm
         if (path == 0 || t < best) {
             best = t;
-            path = kind.path;
+            path = c.path;
         }
     }
     return path;

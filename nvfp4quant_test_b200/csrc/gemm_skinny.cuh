@@ -378,6 +378,16 @@ skinny_kernel(const __grid_constant__ SkinnyMaps maps, const __grid_constant__ S
     }
 }
 
+// Clusters of `ranks` CTAs that are resident at once with `per_sm` CTAs on an SM (cudaOccupancyMaxActiveClusters on a B200; a
+// cluster lives in one GPC, so large ones leave SMs over: 15 clusters of eight at one CTA per SM, not 18).
+static int resident_clusters(int ranks, int per_sm, int sms) {
+    static const int kOn148[4][8] = {{148, 74, 45, 33, 26, 22, 15, 15},
+                                     {296, 148, 93, 71, 56, 45, 37, 33},
+                                     {444, 222, 142, 104, 82, 71, 56, 48},
+                                     {592, 296, 187, 142, 112, 93, 78, 71}};
+    return kOn148[per_sm - 1][ranks - 1] * sms / 148;
+}
+
 // K ranges per weight tile: the largest power of two that keeps every CTA of the grid resident at once (one per
 // SM), with at least two K stages each and at most 8 (the portable cluster size).  With small token tiles two
 // CTAs fit on an SM, and where the K range is already cut, cutting it once more measured faster (16 x 8192 x 8192:
@@ -389,7 +399,9 @@ static int choose_ranks(int n_tiles, int k_tiles, int sms, int forced, int bt) {
     if (forced > 0) {
         r = forced;
     } else {
-        while (r < 8 && n_tiles * (2 * r) <= sms) r *= 2;
+        // 128 tokens need a ring that leaves room for one CTA per SM: there the GPCs' room for clusters counts (119 x 2164 x 8448,
+        // 17 tiles: 18.8 us with eight ranges, whose 16th cluster waits for the first to finish, 10.6 with four)
+        while (r < 8 && n_tiles * (2 * r) <= sms && (bt <= 64 || n_tiles <= resident_clusters(2 * r, 1, sms))) r *= 2;
         if (bt <= 32 && r >= 2 && r < 8 && n_tiles * (2 * r) <= 2 * sms - 40 && k_tiles / (2 * r) >= 4) r *= 2;
     }
     if (r > 8) r = 8;
@@ -413,13 +425,11 @@ struct SkinnyItem {
 // Ring depth: the deepest ring with which the whole grid is resident at once (as many CTAs per SM as that takes, at
 // most what the TMEM columns allow), since a CTA that has to wait for a free SM starts its weight stream late.
 template <int BT>
-static int choose_stages(int ctas, int sms, int max_per_sm) {
+static int choose_stages(int clusters, int ranks, int sms, int max_per_sm) {
     using C = SkinnyCfg<BT>;
     constexpr int kMaxPerSm = kTmemCols / C::kTmemCols;
-    int per_sm = (ctas + sms - 1) / sms;
-    if (per_sm < 1) per_sm = 1;
-    if (per_sm > kMaxPerSm) per_sm = kMaxPerSm;
-    if (per_sm > max_per_sm) per_sm = max_per_sm;
+    int per_sm = 1;
+    while (per_sm < kMaxPerSm && per_sm < max_per_sm && clusters > resident_clusters(ranks, per_sm, sms)) ++per_sm;
     // an SM has 233472 bytes of shared memory, of which 1 KiB per resident CTA is reserved; a CTA asks for its ring
     // plus 1 KiB of alignment slack plus 256 bytes of barriers
     int stages = (233472 / per_sm - 1024 - 1024 - 256) / C::kStageBytes;
@@ -487,7 +497,7 @@ static int launch_skinny_group(int M, const SkinnyItem* items, int n_items, int 
     for (int i = 0; i < n_items; ++i) p.w[i].k_tiles_per_rank = ((p.w[i].K + kBK - 1) / kBK + ranks - 1) / ranks;
     p.M = M;
     p.n_weights = n_items;
-    p.stages = choose_stages<BT>(n_tiles * ranks, sms, mixed ? 3 : kTmemCols);
+    p.stages = choose_stages<BT>(n_tiles, ranks, sms, mixed ? 3 : kTmemCols);
     const int per_rank = (longest + ranks - 1) / ranks;
     if (p.stages > per_rank) p.stages = per_rank < 2 ? 2 : per_rank;
     // the ring doubles as the reduce-scatter buffers: the partial tile plus one slot per rank of the owned columns

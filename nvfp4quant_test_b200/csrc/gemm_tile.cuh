@@ -714,18 +714,18 @@ static int fill_group_table(GroupTable<G>& g, const GemmParams* list, int n, int
     }
 }
 
-// K stages of the busiest worker.
+// Time of the busiest worker, at `stage` per K stage and `epilogue` per tile.
 template <int G>
-static double list_makespan(const GroupTable<G>& g, const GemmParams* list) {
-    int64_t longest = 0;
+static double list_makespan(const GroupTable<G>& g, const GemmParams* list, double stage, double epilogue) {
+    double longest = 0.0;
     for (int c = 0; c < g.n_classes; ++c) {
-        const int64_t workers = g.worker_end[c] - (c > 0 ? g.worker_end[c - 1] : 0);
+        const int workers = g.worker_end[c] - (c > 0 ? g.worker_end[c - 1] : 0);
         const int last = g.item_end[c] - 1;
-        const int64_t k = (list[last].K + kBK - 1) / kBK, tiles = g.item[last].tile_end;
-        const int64_t mine = (tiles + workers - 1) / workers * k;
+        const int tiles = (g.item[last].tile_end + workers - 1) / workers;
+        const double mine = tiles * ((list[last].K + kBK - 1) / kBK * stage + epilogue);
         if (mine > longest) longest = mine;
     }
-    return static_cast<double>(longest);
+    return longest;
 }
 
 // One launch over the `n` products of `list` (1 <= n <= G), items of equal K next to one another, longest K first.
