@@ -74,22 +74,25 @@ struct SkinnyWeight {
     int tile_end;         // number of 128-row tiles of this and all earlier weights of the group
 };
 
+// G: products the launch has room for; 1 for the usual case, whose parameters then stay small.
+template <int G>
 struct SkinnyParams {
     int M;
     int stages;
     int n_weights;
     int weights_ready;    // != 0: all weights are prepared weights (constant while in use): read them before griddep_wait()
-    SkinnyWeight w[kMaxGroup];
+    SkinnyWeight w[G];
 };
 
+template <int G>
 struct SkinnyMaps {
-    CUtensorMap m[kMaxGroup];   // one per weight: [N, K/2] bytes in boxes of 128 rows x 128 bytes
-    CUtensorMap x[kMaxGroup];   // its activation: [M, K/2] bytes in boxes of BT rows
+    CUtensorMap m[G];   // one per weight: [N, K/2] bytes in boxes of 128 rows x 128 bytes
+    CUtensorMap x[G];   // its activation: [M, K/2] bytes in boxes of BT rows
 };
 
-template <int BT>
+template <int BT, int G>
 __global__ void __launch_bounds__(kThreads)
-skinny_kernel(const __grid_constant__ SkinnyMaps maps, const __grid_constant__ SkinnyParams p) {
+skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant__ SkinnyParams<G> p) {
     using C = SkinnyCfg<BT>;
     extern __shared__ uint8_t smem_raw[];
     // The kernel queued behind this one may be scheduled at once: ahead of its own wait it reads nothing but a
@@ -116,7 +119,8 @@ skinny_kernel(const __grid_constant__ SkinnyMaps maps, const __grid_constant__ S
     // clusters run along x: cluster index = 128-row weight tile, numbered through the weights of the group
     const int tile = blockIdx.x / ranks;
     int gi = 0;
-    while (gi + 1 < p.n_weights && tile >= p.w[gi].tile_end) ++gi;
+    if (G > 1)
+        while (gi + 1 < p.n_weights && tile >= p.w[gi].tile_end) ++gi;
     const int nt = tile - (gi > 0 ? p.w[gi - 1].tile_end : 0);
     const CUtensorMap* tmap_w = &maps.m[gi];
     const CUtensorMap* tmap_x = &maps.x[gi];
@@ -442,12 +446,11 @@ static int choose_stages(int clusters, int ranks, int sms, int max_per_sm) {
 }
 
 // Items are in order of descending K (the longest tiles start first).
-template <int BT>
-static int launch_skinny_group(int M, const SkinnyItem* items, int n_items, int forced_ranks, cudaStream_t stream) {
+template <int BT, int G>
+static int launch_skinny_list(int M, const SkinnyItem* items, int n_items, int forced_ranks, cudaStream_t stream) {
     using C = SkinnyCfg<BT>;
-    if (n_items < 1 || n_items > kMaxGroup) return NVFP4_ERR_BAD_RANGE;
-    SkinnyMaps maps;
-    SkinnyParams p;
+    SkinnyMaps<G> maps;
+    SkinnyParams<G> p;
     int n_tiles = 0, st = NVFP4_OK;
     p.weights_ready = 1;
     for (int i = 0; i < n_items && st == NVFP4_OK; ++i) {
@@ -512,7 +515,7 @@ static int launch_skinny_group(int M, const SkinnyItem* items, int n_items, int 
     if (smem < kMinSmem) smem = kMinSmem;
     static_assert(C::kMaxStages * C::kStageBytes + 1024 + 256 <= kGemmDynSmemBytes, "ring does not fit");
     static bool attr_done[64] = {false};
-    cudaError_t e = allow_full_smem(skinny_kernel<BT>, attr_done, di.device);
+    cudaError_t e = allow_full_smem(skinny_kernel<BT, G>, attr_done, di.device);
     if (e != cudaSuccess) return static_cast<int>(e);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(n_tiles * ranks, 1, 1);
@@ -530,8 +533,15 @@ static int launch_skinny_group(int M, const SkinnyItem* items, int n_items, int 
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = g_dependent_launch ? 2 : 1;
-    e = cudaLaunchKernelEx(&cfg, skinny_kernel<BT>, maps, p);
+    e = cudaLaunchKernelEx(&cfg, skinny_kernel<BT, G>, maps, p);
     return static_cast<int>(e);
+}
+
+template <int BT>
+static int launch_skinny_group(int M, const SkinnyItem* items, int n_items, int forced_ranks, cudaStream_t stream) {
+    if (n_items < 1 || n_items > kMaxGroup) return NVFP4_ERR_BAD_RANGE;
+    return n_items == 1 ? launch_skinny_list<BT, 1>(M, items, 1, forced_ranks, stream)
+                        : launch_skinny_list<BT, kMaxGroup>(M, items, n_items, forced_ranks, stream);
 }
 
 template <int BT>
