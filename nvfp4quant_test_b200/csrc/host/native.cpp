@@ -11,6 +11,7 @@
 #include <Python.h>
 
 #include <ATen/core/Tensor.h>
+#include <ATen/core/CachingHostAllocator.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/ops/zeros.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -19,6 +20,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <list>
+#include <memory>
 #include <unordered_map>
 #include <vector>
 
@@ -833,6 +835,157 @@ PyObject* program_call(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     });
 }
 
+// ---- pinned host memory in and out ----------------------------------------------------------------------------------
+// What host_pipeline.HostQuantizer lays out once: row chunks, staging buffers and streams (the Python object's), and the
+// events that order them (this object's).
+struct HostPipe {
+    c10::DeviceIndex device;
+    int dtype, variant, lower, upper;
+    int64_t rows, dim;
+    std::vector<std::pair<int64_t, int64_t>> plan;
+    std::vector<void*> in, codes, scales;      // `depth` staging slots
+    cudaStream_t up, run, down;
+    std::vector<cudaEvent_t> ev_up, ev_run, ev_down;
+    std::vector<bool> used;                    // slot j's events have been recorded, by this call or an earlier one
+    cudaEvent_t begin = nullptr, end_run = nullptr, end_down = nullptr;
+    ~HostPipe() {
+        for (auto* v : {&ev_up, &ev_run, &ev_down})
+            for (cudaEvent_t e : *v) cudaEventDestroy(e);
+        for (cudaEvent_t e : {begin, end_run, end_down})
+            if (e) cudaEventDestroy(e);
+    }
+};
+constexpr const char* kHostPipeName = "nvfp4.host_pipe";
+void free_host_pipe(PyObject* c) { delete static_cast<HostPipe*>(PyCapsule_GetPointer(c, kHostPipeName)); }
+
+bool pointers(PyObject* t, std::vector<void*>* out) {
+    for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(t); ++i) out->push_back(PyLong_AsVoidPtr(PyTuple_GET_ITEM(t, i)));
+    return !PyErr_Occurred();
+}
+
+// make_host_pipe(device, dtype code, variant, lower, upper, rows, dim, (start, stop, start, stop, ...), (in ptr, ...),
+//                (codes ptr, ...), (scales ptr, ...), up, run, down)
+PyObject* make_host_pipe(PyObject*, PyObject* args) {
+    int dev;
+    Py_ssize_t rows, dim, up, run, down;
+    PyObject *plan, *in, *codes, *scales;
+    auto p = std::make_unique<HostPipe>();
+    if (!PyArg_ParseTuple(args, "iiiiinnO!O!O!O!nnn", &dev, &p->dtype, &p->variant, &p->lower, &p->upper, &rows, &dim, &PyTuple_Type, &plan,
+                          &PyTuple_Type, &in, &PyTuple_Type, &codes, &PyTuple_Type, &scales, &up, &run, &down))
+        return nullptr;
+    p->device = static_cast<c10::DeviceIndex>(dev);
+    p->rows = rows;
+    p->dim = dim;
+    for (Py_ssize_t i = 0; i + 1 < PyTuple_GET_SIZE(plan); i += 2)
+        p->plan.emplace_back(PyLong_AsLongLong(PyTuple_GET_ITEM(plan, i)), PyLong_AsLongLong(PyTuple_GET_ITEM(plan, i + 1)));
+    if (!pointers(in, &p->in) || !pointers(codes, &p->codes) || !pointers(scales, &p->scales)) return nullptr;
+    p->up = reinterpret_cast<cudaStream_t>(up);
+    p->run = reinterpret_cast<cudaStream_t>(run);
+    p->down = reinterpret_cast<cudaStream_t>(down);
+    p->used.assign(p->in.size(), false);
+    c10::cuda::CUDAGuard guard(p->device);
+    auto event = [](cudaEvent_t* e) { return cudaEventCreateWithFlags(e, cudaEventDisableTiming) == cudaSuccess; };
+    bool ok = event(&p->begin) && event(&p->end_run) && event(&p->end_down);
+    for (auto* v : {&p->ev_up, &p->ev_run, &p->ev_down})
+        for (size_t i = 0; ok && i < p->in.size(); ++i) {
+            cudaEvent_t e = nullptr;
+            ok = event(&e);
+            if (ok) v->push_back(e);
+        }
+    if (!ok) {
+        PyErr_SetString(PyExc_RuntimeError, "cudaEventCreate failed");
+        return nullptr;
+    }
+    return PyCapsule_New(p.release(), kHostPipeName, free_host_pipe);
+}
+
+// Keeps a pinned block of torch's host allocator from being handed out again before `stream` is done with it.
+inline void keep_pinned(const Tensor& t, cudaStream_t stream, c10::DeviceIndex device) {
+    if (t.is_cuda() || !t.is_pinned()) return;
+    at::getHostAllocator(at::kCUDA)->record_event(const_cast<void*>(t.const_data_ptr()), t.storage().data_ptr().get_context(),
+                                                  c10::cuda::getStreamFromExternal(stream, device).unwrap());
+}
+
+cudaError_t host_pipe_run(HostPipe& p, const char* x, const float* gs_inv, const float* importance, char* codes, char* scales, cudaStream_t cur,
+                          int* status) {
+    const int64_t row_in = p.dim * (p.dtype == NVFP4_DT_F32 ? 4 : 2), row_codes = p.dim / 2, scale_row = round_up(p.dim / 16, 4);
+    const size_t depth = p.in.size();
+    cudaError_t e = cudaSuccess;
+    auto ok = [&](cudaError_t r) {
+        if (e == cudaSuccess) e = r;
+        return e == cudaSuccess;
+    };
+    // One chunk has nothing to overlap: everything in order on the caller's stream, without the round trips between streams.
+    const bool one = p.plan.size() == 1;
+    const cudaStream_t up = one ? cur : p.up, run = one ? cur : p.run, down = one ? cur : p.down;
+    if (!one && ok(cudaEventRecord(p.begin, cur)))
+        for (cudaStream_t s : {up, run, down}) ok(cudaStreamWaitEvent(s, p.begin, 0));
+    for (size_t i = 0; e == cudaSuccess && *status == NVFP4_OK && i < p.plan.size(); ++i) {
+        const size_t j = i % depth;
+        const int64_t a = p.plan[i].first, n = p.plan[i].second - a;
+        if (p.used[j]) ok(cudaStreamWaitEvent(up, p.ev_run[j], 0));          // staging input free once its kernel ran
+        ok(cudaMemcpyAsync(p.in[j], x + a * row_in, static_cast<size_t>(n * row_in), cudaMemcpyDefault, up));
+        if (!one && ok(cudaEventRecord(p.ev_up[j], up))) ok(cudaStreamWaitEvent(run, p.ev_up[j], 0));
+        if (p.used[j]) ok(cudaStreamWaitEvent(run, p.ev_down[j], 0));        // staging outputs free once downloaded
+        if (e != cudaSuccess) break;
+        *status = nvfp4_quant_launch(p.variant, p.in[j], p.dtype, importance, gs_inv, static_cast<uint8_t*>(p.codes[j]),
+                                     static_cast<uint8_t*>(p.scales[j]), n, p.dim, p.dim, p.lower, p.upper, 1, run);
+        if (*status != NVFP4_OK) break;
+        if (ok(cudaEventRecord(p.ev_run[j], run)) && !one) ok(cudaStreamWaitEvent(down, p.ev_run[j], 0));
+        ok(cudaMemcpyAsync(codes + a * row_codes, p.codes[j], static_cast<size_t>(n * row_codes), cudaMemcpyDefault, down));
+        ok(cudaMemcpyAsync(scales + a * scale_row, p.scales[j], static_cast<size_t>(round_up(n, 128) * scale_row), cudaMemcpyDefault, down));
+        ok(cudaEventRecord(p.ev_down[j], down));
+        p.used[j] = true;
+    }
+    if (!one) {
+        if (ok(cudaEventRecord(p.end_run, run))) ok(cudaStreamWaitEvent(cur, p.end_run, 0));
+        if (ok(cudaEventRecord(p.end_down, down))) ok(cudaStreamWaitEvent(cur, p.end_down, 0));
+    }
+    return e;
+}
+
+// host_pipe_call(pipe, x, gs_inv, codes, scales, importance | None) -> True; the operands are checked by the caller except
+// for what their addresses need
+PyObject* host_pipe_call(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+    return guarded([&]() -> PyObject* {
+        HostPipe* p = nargs == 6 ? static_cast<HostPipe*>(PyCapsule_GetPointer(a[0], kHostPipeName)) : nullptr;
+        const Tensor *x = tensor_of(a[1]), *codes = tensor_of(a[3]), *scales = tensor_of(a[4]);
+        const float *gs_inv = nullptr, *importance = nullptr;
+        if (!p || !x || !codes || !scales || !scalar_input(a[2], p->device, &gs_inv)) {
+            PyErr_Clear();
+            return none();
+        }
+        if (x->dim() != 2 || x->size(0) != p->rows || x->size(1) != p->dim || dtype_code(x->scalar_type()) != p->dtype || !x->is_contiguous() ||
+            codes->scalar_type() != at::kByte || codes->numel() != p->rows * (p->dim / 2) || !codes->is_contiguous() || !scales->is_contiguous() ||
+            static_cast<int64_t>(scales->nbytes()) < round_up(p->rows, 128) * round_up(p->dim / 16, 4))
+            return none();
+        if (a[5] != Py_None) {
+            const Tensor* w = tensor_of(a[5]);
+            if (!w || !plain_cuda(*w) || w->device().index() != p->device || w->scalar_type() != at::kFloat || w->numel() != p->dim ||
+                !w->is_contiguous() || !aligned(*w, 16))
+                return none();
+            importance = static_cast<const float*>(w->const_data_ptr());
+        } else if (p->variant == NVFP4_VARIANT_WEIGHTED) {
+            return none();
+        }
+        const cudaStream_t cur = current_stream(p->device);
+        const bool one = p->plan.size() == 1;
+        int status = NVFP4_OK;
+        const int e = launch_on(p->device, [&] {
+            return static_cast<int>(host_pipe_run(*p, static_cast<const char*>(x->const_data_ptr()), gs_inv, importance,
+                                                  static_cast<char*>(codes->mutable_data_ptr()), static_cast<char*>(scales->mutable_data_ptr()), cur, &status));
+        });
+        keep_pinned(*x, one ? cur : p->up, p->device);
+        keep_pinned(*codes, one ? cur : p->down, p->device);
+        keep_pinned(*scales, one ? cur : p->down, p->device);
+        if (e != cudaSuccess || status != NVFP4_OK) {
+            PyErr_Format(PyExc_RuntimeError, "host pipeline: %s", e != cudaSuccess ? cudaGetErrorString(static_cast<cudaError_t>(e)) : nvfp4_status_string(status));
+            return nullptr;
+        }
+        return truth();
+    });
+}
+
 #define FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(name)), METH_FASTCALL, nullptr}
 PyMethodDef kMethods[] = {
     FAST(quant_impl),
@@ -850,9 +1003,11 @@ PyMethodDef kMethods[] = {
     FAST(chain_call),
     FAST(group_call),
     FAST(program_call),
+    FAST(host_pipe_call),
     {"make_chain", make_chain, METH_VARARGS, nullptr},
     {"make_group", make_group, METH_VARARGS, nullptr},
     {"make_program", make_program, METH_VARARGS, nullptr},
+    {"make_host_pipe", make_host_pipe, METH_VARARGS, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };
 #undef FAST

@@ -219,3 +219,37 @@ def test_decode_step_equals_quantizers_and_groups_one_by_one(python_path, tokens
         step(acts[0])
     with pytest.raises(ValueError, match="agree"):
         K.DecodeStep(quantizers, [(1, groups[0][1])])
+
+
+@pytest.mark.parametrize("rows,dim,dtype,chunk", [(1, 16, torch.bfloat16, 128), (300, 48, torch.float16, 128), (1000, 4096, torch.float32, 256),
+                                                  (700, 8192, torch.bfloat16, 1024)])
+def test_host_pipeline_forms(cuda_lib, rows, dim, dtype, chunk):
+    """One chunk and many, weighted, pageable and strided operands, calls back to back from two streams."""
+    import nvfp4quant_test_b200.kernels as K
+    from nvfp4quant_test_b200 import _lib
+    from nvfp4quant_test_b200.host_pipeline import HostQuantizer
+
+    g = torch.Generator().manual_seed(rows)
+    x = torch.randn((rows, dim), generator=g).to(dtype)
+    imp = torch.rand((1, dim), generator=g).cuda()
+    gs_inv = torch.tensor([41.0], device="cuda")
+    codes, scales = (t.cpu() for t in K.scalesweep_weighted_mse_nvfp4_quant_impl(x.cuda(), imp, gs_inv))
+    scales = scales.view(torch.uint8).reshape(-1)
+    hq = HostQuantizer(rows, dim, dtype, "cuda", chunk_rows=chunk, variant=_lib.VARIANT_WEIGHTED, lower=-8, upper=7)
+    wide = torch.zeros((rows, dim), dtype=torch.uint8)
+    for xs, out in ((x.pin_memory(), torch.zeros_like(codes).pin_memory()), (x, torch.zeros_like(codes)),
+                    (x.t().contiguous().t(), wide[:, : dim // 2])):
+        sc = torch.zeros_like(scales).pin_memory()
+        for s in (torch.cuda.current_stream(), torch.cuda.Stream()):
+            out.zero_()
+            with torch.cuda.stream(s):
+                hq(xs, gs_inv, out, sc, imp)
+                hq(xs, gs_inv, out, sc, imp)
+            torch.cuda.synchronize()
+            assert torch.equal(out, codes) and torch.equal(sc, scales)
+    with pytest.raises(ValueError, match="importance"):
+        hq(x, gs_inv, torch.zeros_like(codes), scales)
+    with pytest.raises(ValueError, match="scales_host"):
+        hq(x, gs_inv, torch.zeros_like(codes), scales[:-1], imp)
+    with pytest.raises(ValueError, match="does not match"):
+        hq(x[:, :0], gs_inv, codes, scales, imp)

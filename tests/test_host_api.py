@@ -235,3 +235,17 @@ def test_capture_id_is_zero_without_a_capture():
     from nvfp4quant_test_b200 import _lib
 
     assert _lib.capture_id(0) == 0          # no GPU, or the default stream outside a capture
+
+
+def test_tapered_plan_covers_the_rows_once():
+    from nvfp4quant_test_b200.host_pipeline import tapered_plan
+
+    assert tapered_plan(256, 2048, 1024) == [(0, 256)]                      # small: one chunk
+    for rows, row_bytes, chunk in ((4096, 16384, 1024), (5000, 8192, 4096), (130, 1 << 20, 128), (1, 16, 1024), (0, 32, 128), (20000, 64, 256)):
+        plan = tapered_plan(rows, row_bytes, chunk)
+        assert [a for a, _ in plan] == ([0] + [b for _, b in plan])[: len(plan)] and (not plan or plan[-1][1] == rows)
+        assert all(a % 128 == 0 and 0 <= b - a <= chunk for a, b in plan)
+    sizes = [b - a for a, b in tapered_plan(4096, 16384, 1024)]
+    assert sizes == sorted(sizes, reverse=True) and sizes[-1] == 128
+    with pytest.raises(ValueError):
+        tapered_plan(1024, 64, 100)
