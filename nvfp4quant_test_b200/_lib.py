@@ -41,7 +41,7 @@ def _not_common(*_args):
 
 fast = types.SimpleNamespace(**{name: _not_common for name in (
     "quant_impl", "quant_out", "quant_dynamic", "quant_dynamic_multi", "global_scale", "channel_square_norm", "scaled_mm", "scaled_mm_prepared",
-    "scaled_mm_grouped", "scaled_mm_multi", "dequant", "scale_layout", "make_chain", "chain_call", "make_group", "group_call", "make_program",
+    "scaled_mm_grouped", "scaled_mm_multi", "linear_multi", "dequant", "scale_layout", "make_chain", "chain_call", "make_group", "group_call", "make_program",
     "program_call", "make_host_pipe", "host_pipe_call")})
 
 

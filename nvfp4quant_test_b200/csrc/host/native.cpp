@@ -363,8 +363,9 @@ PyObject* quant_dynamic_multi(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
             items[i] = {q[i].x->const_data_ptr(), nullptr, static_cast<float*>(gs[i].mutable_data_ptr()), scratch + 2 * i,
                         static_cast<uint8_t*>(codes[i].mutable_data_ptr()), static_cast<uint8_t*>(scales[i].mutable_data_ptr()), q[i].m, q[i].n, q[i].n};
         }
+        const int variant = small_int(a[0]), lower = small_int(a[3]), upper = small_int(a[4]);
         const int st = launch_on(dev, [&] {
-            return nvfp4_quant_chain_multi_launch(small_int(a[0]), q[0].dtype, fp8_max, items, static_cast<int>(n), small_int(a[3]), small_int(a[4]), 1, s);
+            return nvfp4_quant_chain_multi_launch(variant, q[0].dtype, fp8_max, items, static_cast<int>(n), lower, upper, 1, s);
         });
         if (st != NVFP4_OK) return none();
         PyObject* l = PyList_New(n);
@@ -653,6 +654,63 @@ PyObject* scaled_mm_multi(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         }
         const cudaStream_t s = current_stream(dev);
         const int st = launch_on(dev, [&] { return nvfp4_gemm_launch_multi(items, static_cast<int>(count), m, s); });
+        return st == NVFP4_OK ? tensor_list(out) : none();
+    });
+}
+
+// linear_multi(variant, [x], fp8_max, lower, upper, [index of x], [weight], [vector of weight scales], [slot in it])
+//   -> [bf16 [m, n_i]]: every activation quantized with its own global scale, then every product with it; codes, scales and
+// global scales stay inside, in one workspace
+PyObject* linear_multi(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+    return guarded([&]() -> PyObject* {
+        constexpr Py_ssize_t kMostActs = 16, kMost = 64;
+        float fp8_max;
+        if (nargs != 9 || !PyList_CheckExact(a[1]) || !as_float(a[2], &fp8_max) || !PyLong_CheckExact(a[3]) || !PyLong_CheckExact(a[4])) return none();
+        for (int i = 5; i < 9; ++i)
+            if (!PyList_CheckExact(a[i]) || PyList_GET_SIZE(a[i]) != PyList_GET_SIZE(a[5])) return none();
+        const Py_ssize_t acts = PyList_GET_SIZE(a[1]), count = PyList_GET_SIZE(a[5]);
+        if (acts < 1 || acts > kMostActs || count < 1 || count > kMost) return none();
+        QuantIn q[kMostActs];
+        int64_t at[kMostActs][2], bytes = 0;
+        for (Py_ssize_t i = 0; i < acts; ++i) {
+            if (!quant_input(PyList_GET_ITEM(a[1], i), Py_None, &q[i]) || q[i].device != q[0].device || q[i].dtype != q[0].dtype || q[i].m != q[0].m)
+                return none();
+            at[i][0] = bytes;
+            at[i][1] = bytes += round_up(q[i].m * q[i].n / 2, 256);
+            bytes += round_up(scale_bytes(q[i].m, q[i].n), 256);
+        }
+        const int64_t gs_at = bytes;
+        const c10::DeviceIndex dev = q[0].device;
+        const cudaStream_t s = current_stream(dev);
+        uint32_t* scratch = scratch_words(dev, s);
+        if (!scratch) return none();
+        nvfp4_gemm_item items[kMost];
+        std::vector<Tensor> out(static_cast<size_t>(count));
+        Tensor work = empty({gs_at + 256}, at::kByte, dev);
+        uint8_t* base = static_cast<uint8_t*>(work.mutable_data_ptr());
+        float* gs = reinterpret_cast<float*>(base + gs_at);
+        for (Py_ssize_t i = 0; i < count; ++i) {
+            int64_t x, slot;
+            Weight w;
+            const Tensor* vec = tensor_of(PyList_GET_ITEM(a[7], i));
+            if (!int_or_none(PyList_GET_ITEM(a[5], i), -1, &x) || !int_or_none(PyList_GET_ITEM(a[8], i), -1, &slot) || x < 0 || x >= acts ||
+                !weight_of(PyList_GET_ITEM(a[6], i), &w) || w.device != dev || w.k != q[x].n || w.k % 64 || !vec || !plain_cuda(*vec) ||
+                vec->device().index() != dev || vec->scalar_type() != at::kFloat || !vec->is_contiguous() || slot < 0 || slot >= vec->numel()) {
+                PyErr_Clear();
+                return none();
+            }
+            out[i] = empty({q[0].m, w.n}, at::kBFloat16, dev);
+            items[i] = {w.handle, base + at[x][0], base + at[x][1], gs + 2 * x, static_cast<const float*>(vec->const_data_ptr()) + slot,
+                        out[i].mutable_data_ptr()};
+        }
+        nvfp4_chain_item chain[kMostActs];
+        for (Py_ssize_t i = 0; i < acts; ++i)
+            chain[i] = {q[i].x->const_data_ptr(), nullptr, gs + 2 * i, scratch + 2 * i, base + at[i][0], base + at[i][1], q[i].m, q[i].n, q[i].n};
+        const int variant = small_int(a[0]), lower = small_int(a[3]), upper = small_int(a[4]);
+        const int st = launch_on(dev, [&] {
+            const int c = nvfp4_quant_chain_multi_launch(variant, q[0].dtype, fp8_max, chain, static_cast<int>(acts), lower, upper, 1, s);
+            return c != NVFP4_OK ? c : nvfp4_gemm_launch_multi(items, static_cast<int>(count), q[0].m, s);
+        });
         return st == NVFP4_OK ? tensor_list(out) : none();
     });
 }
@@ -1000,6 +1058,7 @@ PyMethodDef kMethods[] = {
     FAST(scaled_mm_prepared),
     FAST(scaled_mm_grouped),
     FAST(scaled_mm_multi),
+    FAST(linear_multi),
     FAST(chain_call),
     FAST(group_call),
     FAST(program_call),

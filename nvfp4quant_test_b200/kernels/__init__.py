@@ -19,4 +19,4 @@ from .kernel_vllm import (  # noqa: F401
     swizzle_vllm_fp4_scale,
     unswizzle_vllm_fp4_scale,
 )
-from .linear import ActivationQuantizer, DecodeStep, LinearGroup  # noqa: F401
+from .linear import ActivationQuantizer, DecodeStep, LinearGroup, nvfp4_linear_multi  # noqa: F401

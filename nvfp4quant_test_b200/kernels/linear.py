@@ -15,7 +15,8 @@ import torch
 from .. import _lib
 from .. import helper as _helper
 from . import kernel_ScaleSweep_MSE as _mse
-from .kernel_gemm import PreparedWeight, _scale_bytes
+from .kernel_fused import scalesweep_nvfp4_quant_with_global_scales
+from .kernel_gemm import PreparedWeight, _scale_bytes, nvfp4_scaled_mm_multi
 from .kernel_vllm import create_fp4_output_tensors
 
 
@@ -132,3 +133,19 @@ class DecodeStep:
             for i, group in self.groups:
                 group(*quantized[i])
         return [group.outs for _, group in self.groups]
+
+
+def nvfp4_linear_multi(acts: list[torch.Tensor], index: list[int], weights: list[PreparedWeight], scale_vecs: list[torch.Tensor],
+                       slots: list[int], fp8_max: float = _helper.FP8_E4M3_MAX_4OVER6) -> list[torch.Tensor]:
+    """[acts[index[i]] @ weights[i].T for i], in bf16: every activation [M, K] is quantized with its own global scale
+    (ScaleSweep_MSE), the weights' global scales are scale_vecs[i][slots[i]].  One host call and three to four launches for
+    a layer's matrices; the quantized activations are not returned.  Bits as scalesweep_nvfp4_quant_with_global_scale and
+    nvfp4_scaled_mm_multi."""
+    got = _lib.fast.linear_multi(_lib.VARIANT_MSE, acts, fp8_max, _mse.LOWER_BOUND, _mse.UPPER_BOUND, index,
+                                 [w._fast for w in weights], scale_vecs, slots)
+    if got is not None:
+        return got
+    quantized = scalesweep_nvfp4_quant_with_global_scales(acts, fp8_max)
+    return nvfp4_scaled_mm_multi([quantized[i][0] for i in index], [quantized[i][1] for i in index],
+                                 [quantized[i][2] for i in index], weights,
+                                 [vec[s:s + 1] for vec, s in zip(scale_vecs, slots)])

@@ -152,12 +152,19 @@ class DecodeLayer:
 
 def _layer_gemms_prepared(qlayer: dict, acts: dict[int, torch.Tensor], act_importance: dict[str, torch.Tensor],
                           weight_scales: dict, prepared: dict) -> dict[str, torch.Tensor]:
-    qact: dict[int, tuple] = {}
     if not act_importance:      # the layer's activations are quantized together
-        used = list(dict.fromkeys(prepared[name].k for name in qlayer))
-        for k, (qa, sa, gs, _) in zip(used, K.scalesweep_nvfp4_quant_with_global_scales([acts[k] for k in used])):
+        used: dict[int, int] = {}
+        index, weights, vecs, where = [], [], [], []
+        for name in qlayer:
+            weight = prepared[name]
+            k = weight.k
             vec, slots = weight_scales[k]
-            qact[k] = (qa, sa, gs, vec.unbind(0), slots)
+            index.append(used.setdefault(k, len(used)))
+            weights.append(weight)
+            vecs.append(vec)
+            where.append(slots[name])
+        return dict(zip(qlayer, K.nvfp4_linear_multi([acts[k] for k in used], index, weights, vecs, where)))
+    qact: dict[int, tuple] = {}
     columns: tuple[list, ...] = ([], [], [], [], [])
     for name in qlayer:
         weight = prepared[name]

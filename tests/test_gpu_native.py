@@ -253,3 +253,29 @@ def test_host_pipeline_forms(cuda_lib, rows, dim, dtype, chunk):
         hq(x, gs_inv, torch.zeros_like(codes), scales[:-1], imp)
     with pytest.raises(ValueError, match="does not match"):
         hq(x[:, :0], gs_inv, codes, scales, imp)
+
+
+@pytest.mark.parametrize("m", [3, 65, 300])
+def test_linear_multi_equals_its_steps(python_path, m):
+    import nvfp4quant_test_b200.kernels as K
+    from nvfp4quant_test_b200.kernels.kernel_gemm import gemm_last_status
+
+    def weight(n, k):
+        c, s, gs, _ = K.scalesweep_nvfp4_quant_with_global_scale(torch.randn((n, k), device="cuda").bfloat16(), 256.0)
+        return K.PreparedWeight(c, s), gs
+
+    ks = (512, 1024, 512, 512)
+    made = [weight(n, k) for n, k in zip((256, 1000, 72, 512), ks)]
+    acts = [torch.randn((m, k), device="cuda").bfloat16() * (k / 100) for k in (512, 1024)]
+    vecs = {512: torch.stack([made[i][1] for i in (0, 2, 3)]), 1024: made[1][1].reshape(1)}
+    args = (acts, [0, 1, 0, 0], [w for w, _ in made], [vecs[k] for k in ks], [0, 0, 1, 2])
+    got = K.nvfp4_linear_multi(*args)
+    assert gemm_last_status() == 0
+    with python_path():
+        want = K.nvfp4_linear_multi(*args)
+    if m > 64:
+        _same(got, want)
+    for g, w in zip(got, want):
+        assert torch.allclose(g.float(), w.float(), rtol=2.0 ** -7, atol=float(w.abs().max()) * 2.0 ** -12)
+    with pytest.raises(ValueError, match="disagree on K"):
+        K.nvfp4_linear_multi(acts, [1, 1, 0, 0], *args[2:])
