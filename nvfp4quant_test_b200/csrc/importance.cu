@@ -41,6 +41,11 @@ __device__ __forceinline__ void load4(const void* x, int64_t elem, float v[4]) {
 template <int DT>
 __global__ void __launch_bounds__(kSqThreads) channel_sqnorm_kernel(const void* x, int64_t m, int64_t n, int64_t ld,
                                                                     float* out) {
+    // A programmatic dependent launch like the library's others: everything waits, the kernel behind this one (the weight's
+    // global scale) may be scheduled at once.
+    griddep_launch();
+    griddep_wait();
+    x = after_wait(x);
     const int lane = threadIdx.x % kSqLanes, rg = threadIdx.x / kSqLanes;
     const int64_t col = static_cast<int64_t>(blockIdx.x) * kSqCols + lane * 4;
     float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -99,11 +104,10 @@ extern "C" int nvfp4_channel_sqnorm_launch_strided(const void* x, int x_dtype, i
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const unsigned g = static_cast<unsigned>(blocks);
     switch (x_dtype) {
-        case NVFP4_DT_BF16: channel_sqnorm_kernel<NVFP4_DT_BF16><<<g, kSqThreads, 0, s>>>(x, m, n, ld, out); break;
-        case NVFP4_DT_F16: channel_sqnorm_kernel<NVFP4_DT_F16><<<g, kSqThreads, 0, s>>>(x, m, n, ld, out); break;
-        default: channel_sqnorm_kernel<NVFP4_DT_F32><<<g, kSqThreads, 0, s>>>(x, m, n, ld, out); break;
+        case NVFP4_DT_BF16: return static_cast<int>(launch_dependent(channel_sqnorm_kernel<NVFP4_DT_BF16>, g, kSqThreads, 0, s, x, m, n, ld, out));
+        case NVFP4_DT_F16: return static_cast<int>(launch_dependent(channel_sqnorm_kernel<NVFP4_DT_F16>, g, kSqThreads, 0, s, x, m, n, ld, out));
+        default: return static_cast<int>(launch_dependent(channel_sqnorm_kernel<NVFP4_DT_F32>, g, kSqThreads, 0, s, x, m, n, ld, out));
     }
-    return static_cast<int>(cudaGetLastError());
 }
 
 extern "C" int nvfp4_channel_sqnorm_launch(const void* x, int x_dtype, int64_t m, int64_t n, float* out, void* stream) {
