@@ -70,8 +70,9 @@ struct SkinnyWeight {
     __nv_bfloat16* out;   // [M, N]
     int N, K;
     int k_tiles_per_rank;
+    int ranks;            // K ranges of a tile: a power of two of the cluster's CTAs, or all of them
     int64_t sf_group_stride;
-    int tile_end;         // number of 128-row tiles of this and all earlier weights of the group
+    int cluster_end;      // clusters of this and all earlier weights of the group
 };
 
 // G: products the launch has room for; 1 for the usual case, whose parameters then stay small.
@@ -113,15 +114,19 @@ skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant_
 
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
     const int lane = threadIdx.x & 31;
-    const uint32_t rank = cluster_ctarank();
-    uint32_t ranks;
-    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(ranks));
-    // clusters run along x: cluster index = 128-row weight tile, numbered through the weights of the group
-    const int tile = blockIdx.x / ranks;
+    // Clusters run along x and are numbered through the weights of the group.  A cluster holds cluster / ranks weight tiles of
+    // one weight, a tile's K ranges side by side.
+    uint32_t cluster;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(cluster));
+    const uint32_t crank = cluster_ctarank();
+    const int cluster_id = blockIdx.x / cluster;
     int gi = 0;
     if (G > 1)
-        while (gi + 1 < p.n_weights && tile >= p.w[gi].tile_end) ++gi;
-    const int nt = tile - (gi > 0 ? p.w[gi - 1].tile_end : 0);
+        while (gi + 1 < p.n_weights && cluster_id >= p.w[gi].cluster_end) ++gi;
+    const uint32_t ranks = G > 1 ? static_cast<uint32_t>(p.w[gi].ranks) : cluster;
+    const uint32_t sub = G > 1 ? crank / ranks : 0u;             // this tile among the cluster's
+    const uint32_t rank = crank - sub * ranks, first_peer = sub * ranks;
+    const int nt = (cluster_id - (gi > 0 ? p.w[gi - 1].cluster_end : 0)) * static_cast<int>(cluster / ranks) + static_cast<int>(sub);
     const CUtensorMap* tmap_w = &maps.m[gi];
     const CUtensorMap* tmap_x = &maps.x[gi];
     const uint8_t *const sfw = p.w[gi].sfw, *const sfx = p.w[gi].sfx;
@@ -149,7 +154,9 @@ skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant_
     }
     const int k_tiles = (K + kBK - 1) / kBK;
     const int kt_begin = static_cast<int>(rank) * p.w[gi].k_tiles_per_rank;
-    const int kcount = max(0, min(k_tiles, kt_begin + p.w[gi].k_tiles_per_rank) - kt_begin);   // host: never 0
+    // never 0, but for a CTA of a weight's last cluster behind its last tile: that one streams nothing, takes part in the
+    // barriers and stores nothing (its rows lie beyond N)
+    const int kcount = nt * 128 < N ? max(0, min(k_tiles, kt_begin + p.w[gi].k_tiles_per_rank) - kt_begin) : 0;
 
     // Producer state (warp 0).  The first ring-full of copies is issued BEFORE the CTA-wide barrier of the prologue:
     // the copies need the mbarriers (initialised by this warp's thread 0 just above) but neither TMEM nor the other
@@ -333,8 +340,8 @@ skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant_
                 const uint32_t first = o * cols_per_rank;
                 if (o == rank || first >= m_cols) continue;
                 const uint32_t cols = min(cols_per_rank, m_cols - first);
-                bulk_copy_to_cta(map_to_cta(smem_u32(recv + (rank * cols_per_rank) * 128), o), smem_u32(part + first * 128),
-                                 cols * 512u, map_to_cta(recv_bar, o));
+                bulk_copy_to_cta(map_to_cta(smem_u32(recv + (rank * cols_per_rank) * 128), first_peer + o),
+                                 smem_u32(part + first * 128), cols * 512u, map_to_cta(recv_bar, first_peer + o));
             }
         }
         if (warp >= 2 && have && my_cols > 0) {
@@ -393,11 +400,13 @@ static int resident_clusters(int ranks, int per_sm, int sms) {
 }
 
 // K ranges per weight tile: the largest power of two that keeps every CTA of the grid resident at once (one per
-// SM), with at least two K stages each and at most 8 (the portable cluster size).  With small token tiles two
-// CTAs fit on an SM, and where the K range is already cut, cutting it once more measured faster (16 x 8192 x 8192:
-// 12.2 -> 11.4 us); going from one range to two when the tiles already cover most SMs did not (16 x 14336 x 4096:
-// 10.5 -> 11.1 us).  Cluster sizes that are not a power of two measured slower (6144 x 4096: 3 ranges 11.9 us,
-// 2 ranges 8.0 us).
+// SM), with at least two K stages each and at most 8 (the portable cluster size); measured (us):
+// - a K of few stages is not cut where the tiles are many already (4 x 8512 x 1536, 67 tiles of 6 stages: one range 4.9, two 5.5);
+// - with small token tiles two CTAs fit on an SM, and where the K range is already cut, cutting it once more is faster
+//   (16 x 8192 x 8192: 12.2 -> 11.4), as it is for up to 1.4 tiles per SM (one at 17 to 32 tokens) with a long K, where one range
+//   leaves the last tiles alone on their SMs (24 x 10048 x 11008 17.4 -> 14.7, 2 x 10624 x 6720 12.3 -> 10.6, 4 x 26496 x 12928 34.3 ->
+//   32.7; but 16 x 28672 x 8192 23.4 -> 24.5, 31 x 20800 x 8128 19.3 -> 20.1);
+// - cluster sizes that are not a power of two are slower (6144 x 4096: 3 ranges 11.9, 2 ranges 8.0).
 static int choose_ranks(int n_tiles, int k_tiles, int sms, int forced, int bt) {
     int r = 1;
     if (forced > 0) {
@@ -405,8 +414,10 @@ static int choose_ranks(int n_tiles, int k_tiles, int sms, int forced, int bt) {
     } else {
         // 128 tokens need a ring that leaves room for one CTA per SM: there the GPCs' room for clusters counts (119 x 2164 x 8448,
         // 17 tiles: 18.8 us with eight ranges, whose 16th cluster waits for the first to finish, 10.6 with four)
-        while (r < 8 && n_tiles * (2 * r) <= sms && (bt <= 64 || n_tiles <= resident_clusters(2 * r, 1, sms))) r *= 2;
+        const bool few = k_tiles <= 8 && n_tiles >= 40;
+        while (!few && r < 8 && n_tiles * (2 * r) <= sms && (bt <= 64 || n_tiles <= resident_clusters(2 * r, 1, sms))) r *= 2;
         if (bt <= 32 && r >= 2 && r < 8 && n_tiles * (2 * r) <= 2 * sms - 40 && k_tiles / (2 * r) >= 4) r *= 2;
+        if (bt <= 32 && r == 1 && k_tiles > 16 && n_tiles * 10 <= sms * (bt <= 16 ? 14 : 10)) r = 2;
     }
     if (r > 8) r = 8;
     while (r > 1 && r > k_tiles / 2) --r;
@@ -429,11 +440,11 @@ struct SkinnyItem {
 // Ring depth: the deepest ring with which the whole grid is resident at once (as many CTAs per SM as that takes, at
 // most what the TMEM columns allow), since a CTA that has to wait for a free SM starts its weight stream late.
 template <int BT>
-static int choose_stages(int clusters, int ranks, int sms, int max_per_sm) {
+static int choose_stages(int clusters, int ranks, int sms) {
     using C = SkinnyCfg<BT>;
     constexpr int kMaxPerSm = kTmemCols / C::kTmemCols;
     int per_sm = 1;
-    while (per_sm < kMaxPerSm && per_sm < max_per_sm && clusters > resident_clusters(ranks, per_sm, sms)) ++per_sm;
+    while (per_sm < kMaxPerSm && clusters > resident_clusters(ranks, per_sm, sms)) ++per_sm;
     // an SM has 233472 bytes of shared memory, of which 1 KiB per resident CTA is reserved; a CTA asks for its ring
     // plus 1 KiB of alignment slack plus 256 bytes of barriers
     int stages = (233472 / per_sm - 1024 - 1024 - 256) / C::kStageBytes;
@@ -443,6 +454,34 @@ static int choose_stages(int clusters, int ranks, int sms, int max_per_sm) {
     if (per_sm >= 2 && stages > 4) stages = 4;
     if (stages < 2) stages = 2;
     return stages;
+}
+
+// K ranges of products of different K, in clusters of four: each product's ranges by its own K, so that the longest tiles end
+// with the others.  The ranges are the finest for which the CTAs still fit the GPU at once, 13 for 4 SMs: a second wave pays
+// the kernel's whole latency again.  Where the shortest K is cut too, its many short ranges must leave room, 5 for 2 SMs (4
+// tokens, hidden 1280, FFN 9984, K of 5 and 39 stages: 13.7 with 432 CTAs, 11.6 with 236).  A layer's seven matrices with their
+// quantization, us, against the same number of ranges for all: hidden 4096, K / V 1024, FFN 14336, 1 token 26.2 -> 24.1, 16
+// tokens 30.4 -> 28.1; 2048 / 512 / 8192, 4 tokens 17.6 -> 12.4; 3072 / 3072 / 8192, 3 tokens 24.5 -> 15.1; clusters of eight are
+// no faster.
+template <int G>
+static int plan_mixed(SkinnyParams<G>& p, int n, int sms) {
+    constexpr int kCluster = 4;
+    for (int target = 2;; ++target) {
+        int64_t ctas = 0;
+        bool longer = false;   // a larger target would change something
+        bool all_cut = true;
+        for (int i = 0; i < n; ++i) {
+            const int k = (p.w[i].K + kBK - 1) / kBK;
+            int r = 1;
+            while (r < kCluster && (k + r - 1) / r > target) r *= 2;
+            while (r > 1 && (r - 1) * ((k + r - 1) / r) >= k) r /= 2;   // no empty range
+            p.w[i].ranks = r;
+            longer = longer || r > 1;
+            all_cut = all_cut && r > 1;
+            ctas += static_cast<int64_t>((p.w[i].N + 127) / 128) * r;
+        }
+        if (!longer || ctas * 4 <= static_cast<int64_t>(sms) * (all_cut ? 10 : 13)) return kCluster;
+    }
 }
 
 // Items are in order of descending K (the longest tiles start first).
@@ -469,42 +508,39 @@ static int launch_skinny_list(int M, const SkinnyItem* items, int n_items, int f
         p.w[i].N = static_cast<int>(it.N);
         p.w[i].K = static_cast<int>(it.K);
         p.w[i].sf_group_stride = round_up_i64(it.K / 16, 4) * 128;
-        p.w[i].tile_end = n_tiles;
     }
     if (st != NVFP4_OK) return st;
     const DeviceInfo di = device_info();
     const int sms = di.sms;
     const int longest = (p.w[0].K + kBK - 1) / kBK, shortest = (p.w[n_items - 1].K + kBK - 1) / kBK;
-    // Products of different K: enough ranges that the longest tile's are not much longer than what every SM has to stream
-    // (at two CTAs per SM), and three CTAs per SM.  The seven matrices of a Llama-3-8B layer at 1 token, K 4096 and 14336:
-    // 23.2 us with two ranges, 30.8 with one, 25.1 with three; 24.4 with two CTAs per SM, 27.1 with four (32.9 as four launches).
     const bool mixed = longest != shortest;
-    int ranks = 1;
+    auto stages_of = [&](int i, int r) { return ((p.w[i].K + kBK - 1) / kBK + r - 1) / r; };
+    // no empty K range: with every rank holding ceil(k / ranks) stages the last one must get some
+    auto fits = [&](int i, int r) { return (r - 1) * stages_of(i, r) < (p.w[i].K + kBK - 1) / kBK; };
+    int cluster;
     if (mixed && forced_ranks == 0) {
-        int64_t stages = 0;
-        for (int i = 0; i < n_items; ++i)
-            stages += static_cast<int64_t>((p.w[i].N + 127) / 128) * ((p.w[i].K + kBK - 1) / kBK);
-        while (ranks < 8 && ranks < shortest / 2 && static_cast<int64_t>(longest) * 8 * sms > stages * 5 * ranks) ranks *= 2;
+        cluster = plan_mixed(p, n_items, sms);
     } else {
-        ranks = choose_ranks(n_tiles, shortest, sms, forced_ranks, BT);
+        cluster = choose_ranks(n_tiles, shortest, sms, forced_ranks, BT);
+        for (int i = 0; i < n_items; ++i)
+            while (cluster > 1 && !fits(i, cluster)) --cluster;
+        for (int i = 0; i < n_items; ++i) p.w[i].ranks = cluster;
     }
-    // no empty K range in any item: with every rank holding ceil(k / ranks) stages the last one must get some
-    auto fits = [&](int r) {
-        for (int i = 0; i < n_items; ++i) {
-            const int k = (p.w[i].K + kBK - 1) / kBK;
-            if ((r - 1) * ((k + r - 1) / r) >= k) return false;
-        }
-        return true;
-    };
-    while (ranks > 1 && !fits(ranks)) --ranks;
-    for (int i = 0; i < n_items; ++i) p.w[i].k_tiles_per_rank = ((p.w[i].K + kBK - 1) / kBK + ranks - 1) / ranks;
+    int clusters = 0, per_rank = 1, max_ranks = 1;
+    for (int i = 0; i < n_items; ++i) {
+        const int tiles = static_cast<int>((items[i].N + 127) / 128), per = cluster / p.w[i].ranks;
+        clusters += (tiles + per - 1) / per;
+        p.w[i].cluster_end = clusters;
+        p.w[i].k_tiles_per_rank = stages_of(i, p.w[i].ranks);
+        if (p.w[i].k_tiles_per_rank > per_rank) per_rank = p.w[i].k_tiles_per_rank;
+        if (p.w[i].ranks > max_ranks) max_ranks = p.w[i].ranks;
+    }
     p.M = M;
     p.n_weights = n_items;
-    p.stages = choose_stages<BT>(n_tiles, ranks, sms, mixed ? 3 : kTmemCols);
-    const int per_rank = (longest + ranks - 1) / ranks;
+    p.stages = choose_stages<BT>(clusters, cluster, sms);
     if (p.stages > per_rank) p.stages = per_rank < 2 ? 2 : per_rank;
     // the ring doubles as the reduce-scatter buffers: the partial tile plus one slot per rank of the owned columns
-    while (ranks > 1 && (2 * BT + 8) * 512 > p.stages * C::kStageBytes) ++p.stages;
+    while (max_ranks > 1 && (2 * BT + 8) * 512 > p.stages * C::kStageBytes) ++p.stages;
     if (p.stages > C::kMaxStages) return NVFP4_ERR_UNSUPPORTED;
     // Co-resident CTAs must never want more than the 512 TMEM columns of an SM between them (a CTA that waits in
     // tcgen05.alloc while its cluster peers wait for it is a deadlock).  Shared memory is what bounds co-residency, so
@@ -518,13 +554,13 @@ static int launch_skinny_list(int M, const SkinnyItem* items, int n_items, int f
     cudaError_t e = allow_full_smem(skinny_kernel<BT, G>, attr_done, di.device);
     if (e != cudaSuccess) return static_cast<int>(e);
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(n_tiles * ranks, 1, 1);
+    cfg.gridDim = dim3(clusters * cluster, 1, 1);
     cfg.blockDim = dim3(kThreads, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = ranks;
+    attr[0].val.clusterDim.x = cluster;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     // programmatic dependent launch: this kernel may be scheduled while its predecessor on the stream is finishing

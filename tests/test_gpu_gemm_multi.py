@@ -53,6 +53,31 @@ def test_list_of_products_equals_one_by_one(cuda_lib, path, m, shapes):
             assert torch.allclose(g.float(), w.float(), rtol=2.0 ** -7, atol=float(w.abs().max()) * 2.0 ** -12)
 
 
+@pytest.mark.parametrize("m", [1, 15, 24, 33])
+@pytest.mark.parametrize("shapes", [
+    [(643, 10240), (384, 1344), (72, 128), (768, 1280)],       # 4, 2, 1 and 2 K ranges; clusters with tiles missing
+    [(2000, 4096), (12800, 512), (12800, 512), (12800, 576)],  # so many tiles that only the longest K is cut
+])
+def test_products_of_different_k_in_one_decode_launch(cuda_lib, m, shapes):
+    import nvfp4quant_test_b200.kernels as K
+    from nvfp4quant_test_b200 import helper as H
+    from nvfp4quant_test_b200.kernels.kernel_gemm import gemm_last_status
+
+    acts = [_operand(m, k, i) for i, (_, k) in enumerate(shapes)]
+    weights = [_operand(n, k, 50 + i) for i, (n, k) in enumerate(shapes)]
+    prepared = [K.PreparedWeight(c, s) for c, s, _ in weights]
+    scale = [w[2].reshape(1) for w in weights]
+    columns = [list(c) for c in zip(*acts)]
+    got = K.nvfp4_scaled_mm_multi(*columns, prepared, scale)
+    again = K.nvfp4_scaled_mm_multi(*columns, prepared, scale)
+    for (_, k), a, w, x, y in zip(shapes, acts, weights, got, again):
+        full = [H.dequantize("base", q, K.unswizzle_vllm_fp4_scale(s, q.shape[0], k), gs).double() for q, s, gs in (a, w)]
+        want = (full[0] @ full[1].T).float()
+        assert torch.allclose(x.float(), want, rtol=2.0 ** -7, atol=float(want.abs().max()) * 2.0 ** -12)
+        assert torch.equal(x, y)
+    assert gemm_last_status() == 0
+
+
 def test_list_arguments_are_checked(cuda_lib):
     import nvfp4quant_test_b200.kernels as K
 
