@@ -477,11 +477,13 @@ extern "C" int nvfp4_gemm_launch_multi(const nvfp4_gemm_item* items, int n_items
         if (st != NVFP4_OK) return st;
     }
     if (M == 0) return NVFP4_OK;
-    // with different K, beyond 24 tokens one launch of a tile kernel over the list is faster than the decode-sized kernel (Llama-3-8B layer, all
-    // seven matrices, us, tile kernel / decode-sized kernel: 16 tokens 26.2 / 24.5, 24: 26.6 / 25.7, 32: 26.5 / 26.9, 48: 25.9 / 31.6)
+    // With different K, beyond 32 tokens (where the decode-sized kernel's token tile doubles and two CTAs an SM have room for)
+    // one launch of a tile kernel over the list takes over.  A layer's seven matrices with their quantization, us, tile kernel /
+    // decode-sized kernel, hidden 4096, K / V 1024, FFN 14336: 24 tokens 35.7 / 29.3, 32 35.5 / 30.4, 64 33.6 / 37.5;
+    // 2048 / 2048 / 4096: 32 tokens 13.3 / 12.3, 36 14.4 / 18.9.
     bool mixed = false;
     for (int i = 1; i < n_items; ++i) mixed = mixed || list[i].K != list[0].K;
-    if (M > (mixed ? 24 : 64) || n_items == 1 || (g_gemm_force_path != 0 && g_gemm_force_path != 5))
+    if (M > (mixed ? 32 : 64) || n_items == 1 || (g_gemm_force_path != 0 && g_gemm_force_path != 5))
         return gemm_launch_list(list, wh, n_items, stream);
     // decode-sized: one launch of the decode-sized kernel per 8 products, longest K first
     gemm::skinny::SkinnyItem s_items[64];
