@@ -71,6 +71,8 @@ struct SkinnyWeight {
     int N, K;
     int k_tiles_per_rank;
     int ranks;            // K ranges of a tile: a power of two of the cluster's CTAs, or all of them
+    int tiles;            // tiles of a cluster: its CTAs / ranks
+    int rank_shift;       // a CTA's tile among the cluster's: its rank in the cluster >> rank_shift
     int64_t sf_group_stride;
     int cluster_end;      // clusters of this and all earlier weights of the group
 };
@@ -116,17 +118,18 @@ skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant_
     const int lane = threadIdx.x & 31;
     // Clusters run along x and are numbered through the weights of the group.  A cluster holds cluster / ranks weight tiles of
     // one weight, a tile's K ranges side by side.
-    uint32_t cluster;
-    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(cluster));
     const uint32_t crank = cluster_ctarank();
-    const int cluster_id = blockIdx.x / cluster;
+    uint32_t cluster, cluster_id;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(cluster));
+    asm volatile("mov.u32 %0, %%clusterid.x;" : "=r"(cluster_id));
     int gi = 0;
     if (G > 1)
-        while (gi + 1 < p.n_weights && cluster_id >= p.w[gi].cluster_end) ++gi;
+        while (gi + 1 < p.n_weights && static_cast<int>(cluster_id) >= p.w[gi].cluster_end) ++gi;
     const uint32_t ranks = G > 1 ? static_cast<uint32_t>(p.w[gi].ranks) : cluster;
-    const uint32_t sub = G > 1 ? crank / ranks : 0u;             // this tile among the cluster's
+    const uint32_t sub = G > 1 ? crank >> p.w[gi].rank_shift : 0u;
     const uint32_t rank = crank - sub * ranks, first_peer = sub * ranks;
-    const int nt = (cluster_id - (gi > 0 ? p.w[gi - 1].cluster_end : 0)) * static_cast<int>(cluster / ranks) + static_cast<int>(sub);
+    const int nt = G > 1 ? (static_cast<int>(cluster_id) - (gi > 0 ? p.w[gi - 1].cluster_end : 0)) * p.w[gi].tiles + static_cast<int>(sub)
+                         : static_cast<int>(cluster_id);
     const CUtensorMap* tmap_w = &maps.m[gi];
     const CUtensorMap* tmap_x = &maps.x[gi];
     const uint8_t *const sfw = p.w[gi].sfw, *const sfx = p.w[gi].sfx;
@@ -156,7 +159,7 @@ skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant_
     const int kt_begin = static_cast<int>(rank) * p.w[gi].k_tiles_per_rank;
     // never 0, but for a CTA of a weight's last cluster behind its last tile: that one streams nothing, takes part in the
     // barriers and stores nothing (its rows lie beyond N)
-    const int kcount = nt * 128 < N ? max(0, min(k_tiles, kt_begin + p.w[gi].k_tiles_per_rank) - kt_begin) : 0;
+    const int kcount = G == 1 || nt * 128 < N ? max(0, min(k_tiles, kt_begin + p.w[gi].k_tiles_per_rank) - kt_begin) : 0;
 
     // Producer state (warp 0).  The first ring-full of copies is issued BEFORE the CTA-wide barrier of the prologue:
     // the copies need the mbarriers (initialised by this warp's thread 0 just above) but neither TMEM nor the other
@@ -403,21 +406,23 @@ static int resident_clusters(int ranks, int per_sm, int sms) {
 // SM), with at least two K stages each and at most 8 (the portable cluster size); measured (us):
 // - a K of few stages is not cut where the tiles are many already (4 x 8512 x 1536, 67 tiles of 6 stages: one range 4.9, two 5.5);
 // - with small token tiles two CTAs fit on an SM, and where the K range is already cut, cutting it once more is faster
-//   (16 x 8192 x 8192: 12.2 -> 11.4), as it is for up to 1.4 tiles per SM (one at 17 to 32 tokens) with a long K, where one range
-//   leaves the last tiles alone on their SMs (24 x 10048 x 11008 17.4 -> 14.7, 2 x 10624 x 6720 12.3 -> 10.6, 4 x 26496 x 12928 34.3 ->
-//   32.7; but 16 x 28672 x 8192 23.4 -> 24.5, 31 x 20800 x 8128 19.3 -> 20.1);
+//   (16 x 8192 x 8192: 12.2 -> 11.4);
+// - one range becomes two where the tiles leave a third of the SMs without one, too few streams for HBM (16 x 9728 x 12288, 76
+//   tiles, 18.7 -> 15.8; at 92 tiles 2 to 9 % are left, at 112 tiles and K 8192 two are 5 % slower), and where a very long K
+//   would leave the last of up to 1.4 tiles per SM alone (16 x 23040 x 12288 30.5 -> 28.6; K 8192: no gain);
 // - cluster sizes that are not a power of two are slower (6144 x 4096: 3 ranges 11.9, 2 ranges 8.0).
 static int choose_ranks(int n_tiles, int k_tiles, int sms, int forced, int bt) {
     int r = 1;
     if (forced > 0) {
         r = forced;
     } else {
+        const bool few = k_tiles <= 8 && n_tiles >= 40;
         // 128 tokens need a ring that leaves room for one CTA per SM: there the GPCs' room for clusters counts (119 x 2164 x 8448,
         // 17 tiles: 18.8 us with eight ranges, whose 16th cluster waits for the first to finish, 10.6 with four)
-        const bool few = k_tiles <= 8 && n_tiles >= 40;
         while (!few && r < 8 && n_tiles * (2 * r) <= sms && (bt <= 64 || n_tiles <= resident_clusters(2 * r, 1, sms))) r *= 2;
         if (bt <= 32 && r >= 2 && r < 8 && n_tiles * (2 * r) <= 2 * sms - 40 && k_tiles / (2 * r) >= 4) r *= 2;
-        if (bt <= 32 && r == 1 && k_tiles > 16 && n_tiles * 10 <= sms * (bt <= 16 ? 14 : 10)) r = 2;
+        const bool thin = n_tiles * 8 <= sms * 5, tail = k_tiles >= 40 && n_tiles > sms && n_tiles * 10 <= sms * 14;
+        if (bt <= 32 && r == 1 && k_tiles > 16 && (thin || tail)) r = 2;
     }
     if (r > 8) r = 8;
     while (r > 1 && r > k_tiles / 2) --r;
@@ -529,6 +534,10 @@ static int launch_skinny_list(int M, const SkinnyItem* items, int n_items, int f
     int clusters = 0, per_rank = 1, max_ranks = 1;
     for (int i = 0; i < n_items; ++i) {
         const int tiles = static_cast<int>((items[i].N + 127) / 128), per = cluster / p.w[i].ranks;
+        p.w[i].tiles = per;
+        p.w[i].rank_shift = 31;   // one tile per cluster: the first
+        if (per > 1)
+            for (p.w[i].rank_shift = 0; 1 << p.w[i].rank_shift < p.w[i].ranks;) ++p.w[i].rank_shift;
         clusters += (tiles + per - 1) / per;
         p.w[i].cluster_end = clusters;
         p.w[i].k_tiles_per_rank = stages_of(i, p.w[i].ranks);
