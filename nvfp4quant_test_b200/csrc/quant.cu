@@ -19,9 +19,9 @@
 // candidates per trip whose FMA chains share one f32x2 instruction (each lane of
 // a packed instruction is an independent IEEE operation).
 //
-// Bodies 3 and 7 to 9 are the default loop over different grids: 3 and 9 number the slots of the real rows through (9 in
-// small CTAs, for a few tokens), 7 and 8 have a two-dimensional grid for rows of whole chunks (8 for tensors without any
-// padding, without predicates).  (5 is another name of 3 and 6 of 7, for callers that ask for a body by number.)
+// Bodies 3 and 6 to 9 are the default loop over different grids: 3 and 9 number the slots of the real rows through (9 in
+// small CTAs, for a few tokens), 6 the warps of rows, 7 and 8 have a two-dimensional grid, a row's chunks by a row's CTAs (8 for
+// tensors without any padding in rows of whole chunks, without predicates).  (5 is another name of 3.)
 //
 // Body 4 is the default loop with the tensor-wide global scale (helper.py:96-100: amax / (6 * fp8_max) and its reciprocal)
 // computed inside the same launch: every thread keeps its block in registers, the CTAs combine their maxima
@@ -52,12 +52,13 @@ constexpr int kSmallThreads = 64;
 // (against body 3).  Measured in a chain of launches (us, body 9 / the other): whole chunks, unweighted 4 x 8192 1.92 / 2.03,
 // 32 x 8192 2.10 / 3.23, 96 x 4096 2.48 / 3.00, 40 x 8192 3.28 / 3.06, 128 x 8192 3.52 / 3.14; weighted 32 x 8192 2.90 / 5.23,
 // 40 x 8192 3.52 / 4.73, 48 x 8192 5.69 / 4.91, 128 x 8192 6.30 / 5.33.  Ragged rows, unweighted 77 x 5104 2.86 / 3.69, 300 x
-// 5104 4.85 / 5.05, 200 x 10000 5.52 / 5.09; weighted 150 x 5104 6.29 / 7.98, 500 x 10000 17.47 / 17.60.
+// 5104 4.85 / 5.05, 200 x 10000 5.52 / 5.09; weighted 150 x 5104 6.29 / 7.98, 500 x 10000 17.47 / 17.60.  (Against body 6 or 7
+// on ragged rows the weighted line is the unweighted one: 120000 blocks 8.5 / 8.5, 250000 15.2 / 14.7.)
 constexpr int64_t kSmallBlocks = 24576;
 constexpr int64_t kSmallBlocksRagged = 98304;
 constexpr int64_t kSmallBlocksRaggedWeighted = 327680;
 __host__ __device__ constexpr int block_threads(int variant, int impl) {
-    return impl == 9 ? kSmallThreads : (variant != NVFP4_VARIANT_AMAX && (impl == 3 || impl == 7 || impl == 8 || impl == 10)) ? kSweepThreads : kThreads;
+    return impl == 9 ? kSmallThreads : (variant != NVFP4_VARIANT_AMAX && (impl == 3 || impl == 6 || impl == 7 || impl == 8 || impl == 10)) ? kSweepThreads : kThreads;
 }
 constexpr int min_blocks(int variant, int impl) {
     if (impl == 9) return 8;
@@ -88,16 +89,17 @@ struct QuantParams {
     uint32_t* fused_scratch;  // [4]: running maximum, arrivals, readers, unused; zero between calls
 };
 
-// n / width for n < 2^31, as (n * ceil(2^(32 + shift) / width)) >> (32 + shift) with 2^shift < width <= 2^(shift + 1): the
-// rounding of the multiplier adds less than n * width / 2^(32 + shift) < 1 / width to the quotient's fraction.
-inline void set_width_div(QuantParams& p) {
+// n / d for n < 2^31, as (n * ceil(2^(32 + shift) / d)) >> (32 + shift) with 2^shift < d <= 2^(shift + 1): the
+// rounding of the multiplier adds less than n * d / 2^(32 + shift) < 1 / d to the quotient's fraction.  d: the width, or the
+// warps of a row (body 6).
+inline void set_row_div(QuantParams& p, int64_t d) {
     p.div_mul = p.div_shift = 0;
-    if (p.width <= 1 || p.width > 0x7fffffffLL) return;
-    while ((2ll << p.div_shift) < p.width) ++p.div_shift;
-    p.div_mul = static_cast<uint32_t>(((1ull << (32 + p.div_shift)) + p.width - 1) / p.width);
+    if (d <= 1 || d > 0x7fffffffLL) return;
+    while ((2ll << p.div_shift) < d) ++p.div_shift;
+    p.div_mul = static_cast<uint32_t>(((1ull << (32 + p.div_shift)) + d - 1) / d);
 }
-__device__ __forceinline__ uint32_t width_div(const QuantParams& p, uint32_t n) {
-    return p.width == 1 ? n : __umulhi(n, p.div_mul) >> p.div_shift;
+__device__ __forceinline__ uint32_t row_div(const QuantParams& p, uint32_t n) {
+    return p.div_mul == 0 ? n : __umulhi(n, p.div_mul) >> p.div_shift;
 }
 
 __device__ uint32_t g_quant_status;   // 0 = ok; 1 = the grid-wide wait of the fused kernel gave up
@@ -449,14 +451,24 @@ quant_kernel(const __grid_constant__ Args args) {
     constexpr bool FLAT = IMPL == 3 || IMPL == 9 || IMPL == 10;   // real rows' slots numbered through, then CTAs that fill the padding rows
     const int64_t id = GRID2D ? 0 : static_cast<int64_t>(bx) * T + threadIdx.x;
     const int64_t slots = FLAT ? p.m * p.width : p.total;
-    const bool in_range = GRID2D ? true : id < slots;
+    constexpr bool WARPS = IMPL == 6;               // a row's columns by whole warps, numbered through the rows
+    const uint32_t row_warps = static_cast<uint32_t>((p.width + 31) >> 5);
+    const uint32_t warps = static_cast<uint32_t>(p.m) * row_warps;
+    bool in_range = GRID2D ? true : id < slots;
     int64_t row = 0, col = 0;
     if (GRID2D) {
         row = bx;
         col = static_cast<int64_t>(blockIdx.y) * T + threadIdx.x;
+        if (!WHOLE) in_range = col < p.width;
+    } else if (WARPS) {
+        const uint32_t w = bx * (T / 32) + __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
+        const uint32_t r32 = row_div(p, w);
+        row = r32;
+        col = (w - r32 * row_warps) * 32u + (threadIdx.x & 31u);
+        in_range = w < warps && col < p.width;
     } else if (in_range) {
         if (p.total <= 0x7fffffffLL) {
-            const uint32_t r32 = width_div(p, static_cast<uint32_t>(id));
+            const uint32_t r32 = row_div(p, static_cast<uint32_t>(id));
             row = r32;
             col = static_cast<uint32_t>(id) - r32 * static_cast<uint32_t>(p.width);
         } else {
@@ -466,17 +478,17 @@ quant_kernel(const __grid_constant__ Args args) {
     }
     const bool valid = WHOLE ? true : (in_range && row < p.m && col < p.bout);
     if (IMPL == 7 && row >= p.m) {   // a padding row of the tiled scale layout: zero words, nothing else
-        if ((threadIdx.x & 3) == 0) *reinterpret_cast<uint32_t*>(p.scales + swizzled_scale_offset(row, col, p.k_pad)) = 0u;
+        if (in_range && (threadIdx.x & 3) == 0) *reinterpret_cast<uint32_t*>(p.scales + swizzled_scale_offset(row, col, p.k_pad)) = 0u;
         return;
     }
-    if (FLAT && static_cast<int64_t>(bx) * T >= slots) {
+    const uint32_t real_ctas = WARPS ? (warps + T / 32 - 1) / (T / 32) : FLAT ? static_cast<uint32_t>((slots + T - 1) / T) : 0u;
+    if ((FLAT || WARPS) && bx >= real_ctas) {
         // A CTA behind the real rows' slots.  The rows m .. rows-1 of the tiled scale layout (127 of 128 for one token)
         // hold no data; these CTAs write their zero scale bytes, four 32-bit words (of four columns each) per thread,
         // and leave before the candidate table is built.  (Rows beyond m exist only in the tiled layout, whose width is
         // a multiple of 4; the launcher sizes this part of the grid, and at most 127 rows are padding.)
         const uint32_t words_per_row = static_cast<uint32_t>(p.width >> 2);
         const uint32_t words = static_cast<uint32_t>(p.rows - p.m) * words_per_row;
-        const uint32_t real_ctas = static_cast<uint32_t>((slots + T - 1) / T);
         const uint32_t fill_threads = (ctas - real_ctas) * T;
         for (uint32_t wi = (bx - real_ctas) * T + threadIdx.x; wi < words; wi += fill_threads) {
             const uint32_t r = wi / words_per_row;
@@ -580,7 +592,7 @@ quant_kernel(const __grid_constant__ Args args) {
 
     uint32_t sbyte = 0;
     float inv = 0.0f;
-    if (FLAT && !__any_sync(0xffffffffu, valid)) {   // only padding columns, or threads behind the last slot
+    if ((FLAT || WARPS || IMPL == 7) && !__any_sync(0xffffffffu, valid)) {   // only padding columns, or threads behind the last slot
         // nothing
     } else if (VARIANT == NVFP4_VARIANT_AMAX) {
         const float amax = max_abs16(v);
@@ -604,7 +616,7 @@ quant_kernel(const __grid_constant__ Args args) {
         sbyte = (IMPL == 1)   ? sweep_scalar<W>(v, w, first_idx, p.ncand, tab)
                 : (IMPL == 2) ? sweep_single<W>(v, w, first_idx, p.ncand, tab)
                 // the reference's own windows (11 candidates unweighted, 16 weighted) are compiled in, unrolled
-                : (WHOLE || ((IMPL == 7 || FLAT) && p.ncand == (W ? 16 : 11)))
+                : (WHOLE || ((IMPL == 7 || FLAT || WARPS) && p.ncand == (W ? 16 : 11)))
                     ? sweep_paired<W, W ? 16 : 11>(v, w, first_idx, p.ncand, tab)
                     : sweep_paired<W>(v, w, first_idx, p.ncand, tab);
         // sbyte is 0 only when no candidate had a comparable (non-NaN, < inf) error: 1/0 as the reference computes it
@@ -640,21 +652,36 @@ quant_kernel(const __grid_constant__ Args args) {
     }
 }
 
-// Grid of the bodies that number the real rows' slots through: CTAs for those, then CTAs that zero the padding rows' scale
+// Grid of the bodies that number the real rows' slots (or warps of rows) through: CTAs for those, then CTAs that zero the padding rows' scale
 // words (4 words per thread).
-int64_t flat_ctas(const QuantParams& p, int T) {
+int64_t flat_ctas(const QuantParams& p, int T, bool warps) {
     const int64_t pad_words = (p.rows - p.m) * (p.width >> 2);
     if (pad_words > 0x7fffffffLL) return INT64_MAX;   // at most 127 rows: a width beyond 2^26 columns
-    return (p.m * p.width + T - 1) / T + (pad_words + 4 * T - 1) / (4 * T);
+    const int64_t slots = warps ? p.m * ((p.width + 31) / 32 * 32) : p.m * p.width;
+    return (slots + T - 1) / T + (pad_words + 4 * T - 1) / (4 * T);
 }
 template <int DT, int VARIANT, int IMPL>
 cudaError_t launch_flat(const QuantParams& p, cudaStream_t stream) {
     constexpr int T = block_threads(VARIANT, IMPL);
-    const int64_t grid = flat_ctas(p, T);
+    const int64_t grid = flat_ctas(p, T, IMPL == 6);
     if (grid > 0x7fffffffLL) return cudaErrorInvalidValue;
     return launch_dependent(quant_kernel<DT, VARIANT, IMPL, QuantParams>, static_cast<unsigned>(grid), dim3(T), 0, stream, p);
 }
 
+// The grid of rows that are no whole chunks of T blocks: the slots numbered through (3) keeps every thread busy but divides
+// per thread, a row by whole warps (6) or by whole CTAs (7) leaves the last one partly idle; 7 divides nothing, 6 once per warp.
+// By the idle part; us, bodies 3 / 6 / 7, bf16, 1500000 blocks: unweighted, rows of 498 45.6 / 44.4 / 43.9, 575 45.5 / 43.3 /
+// 44.0, 643 45.5 / 45.0 / 45.7, 90 44.2 / 45.0 / 46.3; weighted, 498 73.9 / 73.7 / 73.2, 643 73.8 / 74.7 / 75.3; amax, 498 13.1 /
+// 11.6 / 11.1, 575 13.2 / 11.5 / 12.1, 85 13.2 / 12.4 / 19.8, 198 13.2 / 12.4 / 12.3, 65 13.3 / 14.8 / 25.3.
+int ragged_body(int variant, int64_t width, int T) {
+    const int64_t idle_warp = (width + 31) / 32 * 32 - width, idle_cta = (width + T - 1) / T * T - width;
+    if (variant == NVFP4_VARIANT_AMAX) {
+        if (idle_cta * 4 <= width) return 7;
+        return idle_warp * 7 <= width ? 6 : idle_cta * 2 <= width ? 7 : 3;
+    }
+    if (idle_warp * (variant == NVFP4_VARIANT_MSE ? 20 : 32) > width) return 3;
+    return idle_cta == idle_warp ? 7 : 6;
+}
 template <int DT, int VARIANT>
 cudaError_t launch_impl(int impl, const QuantParams& p, cudaStream_t stream) {
     constexpr bool kSweep = VARIANT != NVFP4_VARIANT_AMAX;
@@ -664,15 +691,27 @@ cudaError_t launch_impl(int impl, const QuantParams& p, cudaStream_t stream) {
         return impl == 1 ? launch_dependent(quant_kernel<DT, VARIANT, 1, QuantParams>, grid, dim3(kThreads), 0, stream, p)
                          : launch_dependent(quant_kernel<DT, VARIANT, 2, QuantParams>, grid, dim3(kThreads), 0, stream, p);
     }
-    const bool chunks = (p.width % T) == 0 && p.width / T <= 65535 && p.rows <= 0x7fffffffLL;
-    const bool small = kSweep && p.m * p.bout <= (chunks ? kSmallBlocks : VARIANT == NVFP4_VARIANT_WEIGHTED ? kSmallBlocksRaggedWeighted : kSmallBlocksRagged);
-    if (impl == 9 || (impl == 0 && small)) return launch_flat<DT, VARIANT, 9>(p, stream);
-    if (chunks && impl != 3 && impl != 5) {
-        const dim3 grid2(static_cast<unsigned>(p.rows), static_cast<unsigned>(p.width / T));
+    const bool chunks = p.width % T == 0;
+    int body = impl;
+    if (impl == 0 || impl == 8) body = chunks ? 7 : ragged_body(VARIANT, p.width, T);
+    if (impl == 0 && kSweep) {
+        const int64_t small = chunks ? kSmallBlocks : VARIANT == NVFP4_VARIANT_WEIGHTED && body == 3 ? kSmallBlocksRaggedWeighted : kSmallBlocksRagged;
+        if (p.m * p.bout <= small) body = 9;
+    }
+    if (body == 7 && ((p.width + T - 1) / T > 65535 || p.rows > 0x7fffffffLL)) body = 3;
+    if (body == 6 && p.m * ((p.width + 31) / 32) > 0x7fffffffLL) body = 3;
+    if (body == 9) return launch_flat<DT, VARIANT, 9>(p, stream);
+    if (body == 6) {
+        QuantParams q = p;
+        set_row_div(q, (p.width + 31) / 32);
+        return launch_flat<DT, VARIANT, 6>(q, stream);
+    }
+    if (body == 7) {
+        const dim3 grid2(static_cast<unsigned>(p.rows), static_cast<unsigned>((p.width + T - 1) / T));
         // no padding anywhere: every slot of the scale layout is a real block
-        const bool whole = p.rows == p.m && p.bin == p.bout && p.bout == p.width && p.ncand == (VARIANT == NVFP4_VARIANT_MSE ? 11 : 16);
+        const bool whole = chunks && p.rows == p.m && p.bin == p.bout && p.bout == p.width && p.ncand == (VARIANT == NVFP4_VARIANT_MSE ? 11 : 16);
         if constexpr (kSweep)
-            if (whole && (impl == 0 || impl == 8)) return launch_dependent(quant_kernel<DT, VARIANT, 8, QuantParams>, grid2, dim3(T), 0, stream, p);
+            if (whole && impl != 7) return launch_dependent(quant_kernel<DT, VARIANT, 8, QuantParams>, grid2, dim3(T), 0, stream, p);
         return launch_dependent(quant_kernel<DT, VARIANT, 7, QuantParams>, grid2, dim3(T), 0, stream, p);
     }
     return launch_flat<DT, VARIANT, 3>(p, stream);
@@ -709,7 +748,7 @@ int fill_params(QuantParams& p, int variant, const void* x, int x_dtype, const f
     p.width = swizzled ? p.k_pad : p.bout;
     p.rows = swizzled ? round_up_i64(m, 128) : m;
     p.total = p.rows * p.width;
-    set_width_div(p);
+    set_row_div(p, p.width);
     if (p.total == 0) return NVFP4_OK;
     if ((p.total + kThreads - 1) / kThreads > 0x7fffffffLL) return NVFP4_ERR_TOO_LARGE;
     if (!gs_inv || !codes || !scales || (!x && m * n > 0)) return NVFP4_ERR_NULL_POINTER;
@@ -797,7 +836,7 @@ cudaError_t launch_multi(const QuantParams* q, int n, cudaStream_t stream) {
     int64_t end = 0;
     for (int i = 0; i < n; ++i) {
         mp.q[i] = q[i];
-        end += flat_ctas(q[i], T);
+        end += flat_ctas(q[i], T, false);
         mp.cta_end[i] = static_cast<uint32_t>(end);
     }
     return launch_dependent(quant_kernel<DT, VARIANT, IMPL, MultiParams>, dim3(static_cast<unsigned>(end)), dim3(T), 0, stream, mp);

@@ -151,9 +151,10 @@ def test_scale_layouts_and_dequantization_equal_torch(cuda_lib, m, n, dtype):
 
 @pytest.mark.parametrize("m,n,padded_n,tiled", [(129, 16, None, False), (300, 32, None, True), (77, 48, None, False), (3, 112, 176, True),
                                                 (127, 2048, None, True), (129, 2048, 4096, True), (1, 6144, None, True),
-                                                (200, 2064, None, True), (45, 6128, 6144, False)])
+                                                (200, 2064, None, True), (45, 6128, 6144, False), (900, 1968, None, True), (900, 1952, 1968, False),
+                                                (401, 9200, None, False)])
 def test_quantizer_grids_equal_the_scalar_body(cuda_lib, m, n, padded_n, tiled):
-    """Every grid (slots numbered through in two CTA sizes, rows of whole chunks with and without padding) against the scalar
+    """Every grid (slots numbered through in two CTA sizes, rows of CTAs with and without idle threads and padding) against the scalar
     transcription, at widths where the division by the row length and the padding can go wrong."""
     from nvfp4quant_test_b200 import _lib
 
@@ -163,9 +164,9 @@ def test_quantizer_grids_equal_the_scalar_body(cuda_lib, m, n, padded_n, tiled):
     gs_inv = torch.tensor([37.5], device="cuda")
     p = padded_n or n
     size = (m + 127) // 128 * 128 * ((p // 16 + 3) // 4 * 4) if tiled else m * p // 16
-    for variant, lower, upper in ((0, -3, 7), (0, -2, 5), (1, -8, 7), (1, -1, 1)):
+    for variant, lower, upper in ((0, -3, 7), (0, -2, 5), (1, -8, 7), (1, -1, 1), (2, 0, 0)):
         want = None
-        for impl in (1, 0, 3, 7, 8, 9):
+        for impl in (3, 0, 7, 8, 9) if variant == 2 else (1, 0, 3, 7, 8, 9):
             codes = torch.full((m, p // 2), 0xA5, dtype=torch.uint8, device="cuda")
             scales = torch.full((size,), 0xA5, dtype=torch.uint8, device="cuda")
             _lib.check(cuda_lib.nvfp4_quant_launch_impl(impl, variant, x.data_ptr(), 0, imp.data_ptr(), gs_inv.data_ptr(), codes.data_ptr(),
