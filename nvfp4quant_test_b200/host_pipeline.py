@@ -28,10 +28,11 @@ def chunk_plan(rows: int, chunk_rows: int) -> list[tuple[int, int]]:
 
 # Upload per chunk: every copy costs the link ~4 us beside its bytes, and a large last chunk leaves its kernel and download
 # uncovered.  [4096, 4096] fp32 / bf16, us: 2 MB 1455 / 765, 4 MB 1339 / 718, 8 MB 1297 / 698, 16 MB 1284 / 701 (the link alone:
-# 1211 / 608).  Up to ONE_CHUNK_BYTES one chunk on the caller's stream beats the round trips between streams (3.2 MB: 100
-# against 109 us).
+# 1211 / 608).  The halving ends at 4 MB, small chunks cost more than they uncover ([1888, 2304] bf16 with 1 / 4 / 6 MB 229 / 219 /
+# 221, [1024, 4096] bf16 222 / 213 / 222).  Up to ONE_CHUNK_BYTES one chunk on the caller's stream beats the round trips between
+# streams (3.2 MB: 100 against 109 us).
 CHUNK_BYTES = 16 << 20
-LAST_CHUNK_BYTES = 1 << 20
+LAST_CHUNK_BYTES = 4 << 20
 ONE_CHUNK_BYTES = 4 << 20
 
 

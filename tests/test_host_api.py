@@ -246,6 +246,6 @@ def test_tapered_plan_covers_the_rows_once():
         assert [a for a, _ in plan] == ([0] + [b for _, b in plan])[: len(plan)] and (not plan or plan[-1][1] == rows)
         assert all(a % 128 == 0 and 0 <= b - a <= chunk for a, b in plan)
     sizes = [b - a for a, b in tapered_plan(4096, 16384, 1024)]
-    assert sizes == sorted(sizes, reverse=True) and sizes[-1] == 128
+    assert sizes == sorted(sizes, reverse=True) and sizes[-1] == 256
     with pytest.raises(ValueError):
         tapered_plan(1024, 64, 100)
