@@ -592,7 +592,10 @@ quant_kernel(const __grid_constant__ Args args) {
 
     uint32_t sbyte = 0;
     float inv = 0.0f;
-    if ((FLAT || WARPS || IMPL == 7) && !__any_sync(0xffffffffu, valid)) {   // only padding columns, or threads behind the last slot
+    // A warp with nothing but padding columns or threads behind the last slot has nothing to sweep.  (Body 6 has next to none of
+    // these and is 0.5 % faster without the vote, the weighted body 3 up to 3 %; the unweighted one is slower without it.)
+    constexpr bool VOTE = IMPL == 7 || (FLAT && !(IMPL == 3 && VARIANT == NVFP4_VARIANT_WEIGHTED));
+    if (VOTE && !__any_sync(0xffffffffu, valid)) {
         // nothing
     } else if (VARIANT == NVFP4_VARIANT_AMAX) {
         const float amax = max_abs16(v);
@@ -671,15 +674,16 @@ cudaError_t launch_flat(const QuantParams& p, cudaStream_t stream) {
 // The grid of rows that are no whole chunks of T blocks: the slots numbered through (3) keeps every thread busy but divides
 // per thread, a row by whole warps (6) or by whole CTAs (7) leaves the last one partly idle; 7 divides nothing, 6 once per warp.
 // By the idle part; us, bodies 3 / 6 / 7, bf16, 1500000 blocks: unweighted, rows of 498 45.6 / 44.4 / 43.9, 575 45.5 / 43.3 /
-// 44.0, 643 45.5 / 45.0 / 45.7, 90 44.2 / 45.0 / 46.3; weighted, 498 73.9 / 73.7 / 73.2, 643 73.8 / 74.7 / 75.3; amax, 498 13.1 /
+// 44.0, 643 45.5 / 45.0 / 45.7, 90 46.5 / 45.9 / 47.7 (not tiled,
+// where the address is cheap, 44.2 / 45.0 / 46.3); weighted, 498 73.9 / 73.7 / 73.2, 643 73.8 / 74.7 / 75.3; amax, 498 13.1 /
 // 11.6 / 11.1, 575 13.2 / 11.5 / 12.1, 85 13.2 / 12.4 / 19.8, 198 13.2 / 12.4 / 12.3, 65 13.3 / 14.8 / 25.3.
-int ragged_body(int variant, int64_t width, int T) {
+int ragged_body(int variant, int64_t width, bool tiled, int T) {
     const int64_t idle_warp = (width + 31) / 32 * 32 - width, idle_cta = (width + T - 1) / T * T - width;
     if (variant == NVFP4_VARIANT_AMAX) {
         if (idle_cta * 4 <= width) return 7;
         return idle_warp * 7 <= width ? 6 : idle_cta * 2 <= width ? 7 : 3;
     }
-    if (idle_warp * (variant == NVFP4_VARIANT_MSE ? 20 : 32) > width) return 3;
+    if (idle_warp * (variant == NVFP4_VARIANT_WEIGHTED ? 32 : tiled ? 15 : 20) > width) return 3;
     return idle_cta == idle_warp ? 7 : 6;
 }
 template <int DT, int VARIANT>
@@ -693,7 +697,7 @@ cudaError_t launch_impl(int impl, const QuantParams& p, cudaStream_t stream) {
     }
     const bool chunks = p.width % T == 0;
     int body = impl;
-    if (impl == 0 || impl == 8) body = chunks ? 7 : ragged_body(VARIANT, p.width, T);
+    if (impl == 0 || impl == 8) body = chunks ? 7 : ragged_body(VARIANT, p.width, p.swizzled != 0, T);
     if (impl == 0 && kSweep) {
         const int64_t small = chunks ? kSmallBlocks : VARIANT == NVFP4_VARIANT_WEIGHTED && body == 3 ? kSmallBlocksRaggedWeighted : kSmallBlocksRagged;
         if (p.m * p.bout <= small) body = 9;
