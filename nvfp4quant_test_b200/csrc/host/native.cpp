@@ -4,8 +4,8 @@
 // same checks, two torch.empty, a dtype view and a 15-argument ctypes call cost 13-15 us of interpreter time.  Every
 // function here does the whole common case and returns None for anything else (a wrong shape, a CPU tensor, a strided
 // or misaligned operand, a tensor subclass, a stream under capture where scratch words are needed, a failed launch); the
-// Python entry point then takes its own path, which holds the conversions and all error messages.  So there is one place
-// that decides what an error is, and this file never raises.
+// Python entry point then takes its own path, which holds the conversions and all error messages, so that there is one
+// place that decides what an error of a caller is.
 //
 // The kernels are reached through the C ABI of include/nvfp4_b200.h, like from any other caller.
 #include <Python.h>
