@@ -71,7 +71,14 @@ int nvfp4_quant_launch(int variant, const void* x, int x_dtype, const float* imp
                        const float* gs_inv, uint8_t* codes, uint8_t* scales, int64_t m, int64_t n,
                        int64_t padded_n, int lower, int upper, int swizzled, void* stream);
 
-/* Same, choosing the kernel body: 0 = default (9 for tensors of a few tokens, see there; else 5 when a quarter or more
+/* Same, for outputs that a prepared weight refers to (nvfp4_gemm_prepare; a weight requantized in place): no kernel behind
+ * this one on the stream starts before it has completed, so launches with the handle that follow it read what it wrote.  (After
+ * nvfp4_quant_launch a GEMM may be let in early, and streams a prepared weight at once.) */
+int nvfp4_quant_launch_in_place(int variant, const void* x, int x_dtype, const float* importance, const float* gs_inv,
+                                uint8_t* codes, uint8_t* scales, int64_t m, int64_t n, int64_t padded_n, int lower, int upper,
+                                int swizzled, void* stream);
+
+/* Same as nvfp4_quant_launch, choosing the kernel body: 0 = default (9 for tensors of a few tokens, see there; else 5 when a quarter or more
  * of the scale layout's rows are padding, else 8 / 7 / 6 where they apply, else 3), 1 = scalar (one candidate at a time, the plainest transcription), 2 = one candidate per trip with
  * packed multiplies and the mixed-precision subtract, 3 = two candidates per trip sharing one f32x2 FMA chain,
  * 5 = 3 with warps that hold only padding rows skipping the sweep, 6 = 3 on a two-dimensional grid (row =
@@ -202,8 +209,8 @@ size_t nvfp4_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K);
  * accepted).  It refers to b / sfb without owning them: keep both allocated at the same addresses with the same
  * shape while the handle lives.  A prepared weight is treated as a constant: a launch with the handle starts reading
  * b / sfb while kernels queued before it on the stream are still finishing (see nvfp4_gemm_tune_pdl), so their
- * contents must be complete before such a launch is issued - written before nvfp4_gemm_prepare, or rewritten in place
- * later and followed by a stream / event synchronisation on the host.  (nvfp4_gemm_launch, with raw pointers, makes no
+ * contents must be complete before such a launch can run: written by work that the host has waited for, or ordered before it by a
+ * kernel or copy that is no dependent launch, or written by nvfp4_quant_launch_in_place on the same stream.  (nvfp4_gemm_launch, with raw pointers, makes no
  * such assumption: its weights may come from the kernel just before it.)  A handle belongs to the device that was
  * current in nvfp4_gemm_prepare; launching it with another device current returns NVFP4_ERR_UNSUPPORTED.  Handles may
  * be used from several host threads at once (they are read-only after creation).

@@ -22,7 +22,7 @@ DT_BF16, DT_F16, DT_F32 = 0, 1, 2
 ERR_TOO_LARGE = -8
 
 EXPORTS = (
-    "nvfp4_quant_launch", "nvfp4_quant_launch_impl", "nvfp4_quant_fused_launch", "nvfp4_quant_chain_launch", "nvfp4_quant_chain_multi_launch",
+    "nvfp4_quant_launch", "nvfp4_quant_launch_impl", "nvfp4_quant_launch_in_place", "nvfp4_quant_fused_launch", "nvfp4_quant_chain_launch", "nvfp4_quant_chain_multi_launch",
     "nvfp4_quant_fused_last_status",
     "nvfp4_global_scale_launch", "nvfp4_global_scale_launch_static", "nvfp4_global_scale_static_max_bytes",
     "nvfp4_channel_sqnorm_launch", "nvfp4_channel_sqnorm_launch_strided", "nvfp4_gemm_peak_probe", "nvfp4_gemm_set_wait_limit_ns", "nvfp4_quant_fused_set_wait_limit_ns",
@@ -87,6 +87,8 @@ def lib() -> ctypes.CDLL:
         L.nvfp4_quant_launch.argtypes = [ci, vp, ci, vp, vp, vp, vp, i64, i64, i64, ci, ci, ci, vp]
         L.nvfp4_quant_launch_impl.restype = ci
         L.nvfp4_quant_launch_impl.argtypes = [ci, ci, vp, ci, vp, vp, vp, vp, i64, i64, i64, ci, ci, ci, vp]
+        L.nvfp4_quant_launch_in_place.restype = ci
+        L.nvfp4_quant_launch_in_place.argtypes = [ci, vp, ci, vp, vp, vp, vp, i64, i64, i64, ci, ci, ci, vp]
         L.nvfp4_quant_fused_launch.restype = ci
         L.nvfp4_quant_fused_launch.argtypes = [ci, vp, ci, vp, f32, vp, vp, vp, vp, i64, i64, i64, ci, ci, ci, vp]
         L.nvfp4_quant_chain_launch.restype = ci

@@ -250,7 +250,8 @@ PyObject* quant_impl(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     });
 }
 
-// quant_out(variant, input, importance | None, input_scale, tiled, output, output_scale, lower, upper) -> True
+// quant_out(variant, input, importance | None, input_scale, tiled, output, output_scale, lower, upper) -> True; the caller's buffers
+// may be a prepared weight's
 PyObject* quant_out(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     return guarded([&]() -> PyObject* {
         if (nargs != 9) return none();
@@ -272,9 +273,9 @@ PyObject* quant_out(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         const int variant = small_int(a[0]), lower = small_int(a[7]), upper = small_int(a[8]);
         const cudaStream_t s = current_stream(q.device);
         const int st = launch_on(q.device, [&] {
-            return nvfp4_quant_launch(variant, q.x->const_data_ptr(), q.dtype, q.importance, gs_inv,
-                                      static_cast<uint8_t*>(codes->mutable_data_ptr()), static_cast<uint8_t*>(scales->mutable_data_ptr()),
-                                      q.m, q.n, padded_n, lower, upper, tiled ? 1 : 0, s);
+            return nvfp4_quant_launch_in_place(variant, q.x->const_data_ptr(), q.dtype, q.importance, gs_inv,
+                                               static_cast<uint8_t*>(codes->mutable_data_ptr()), static_cast<uint8_t*>(scales->mutable_data_ptr()),
+                                               q.m, q.n, padded_n, lower, upper, tiled ? 1 : 0, s);
         });
         return st == NVFP4_OK ? truth() : none();
     });

@@ -83,6 +83,7 @@ struct QuantParams {
     uint32_t div_mul, div_shift;  // division by width: see width_div
     int lower, ncand;
     int swizzled;
+    int early;              // != 0: kernels behind this one may be scheduled while it runs (see the kernel's first lines)
     // fused global-scale variant only
     float fp8_max;
     float* gs_out;          // [2]: global scale, its reciprocal
@@ -436,8 +437,10 @@ quant_kernel(const __grid_constant__ Args args) {
     // the kernel before this one on the stream, so everything waits.  The kernel BEHIND this one may be scheduled right
     // away, even before that wait is over: whatever it does ahead of its own wait (a GEMM streams a prepared, constant
     // weight) depends on neither this kernel nor the ones before it, and its wait covers this kernel's completion,
-    // which in turn comes after this wait.
-    griddep_launch();
+    // which in turn comes after this wait.  That does not hold where this kernel writes such a weight: then (early == 0)
+    // nothing behind it starts before it is complete, not even a GEMM two launches on, which without this could be let in by
+    // a short kernel between them while this one still runs.
+    if (p.early) griddep_launch();
     if (!FUSED) griddep_wait();
     // everything the kernel before this one may have written is read through pointers taken behind the wait
     const void* const x_in = after_wait(p.x);
@@ -770,6 +773,7 @@ int fill_params(QuantParams& p, int variant, const void* x, int x_dtype, const f
     p.scales = scales;
     p.lower = lower;
     p.ncand = (variant == NVFP4_VARIANT_AMAX) ? 0 : upper - lower + 1;
+    p.early = 1;
     p.fp8_max = 0.0f;
     p.gs_out = nullptr;
     p.fused_scratch = nullptr;
@@ -778,14 +782,15 @@ int fill_params(QuantParams& p, int variant, const void* x, int x_dtype, const f
 }  // namespace
 }  // namespace nvfp4
 
-extern "C" int nvfp4_quant_launch_impl(int impl, int variant, const void* x, int x_dtype, const float* importance,
-                                       const float* gs_inv, uint8_t* codes, uint8_t* scales, int64_t m, int64_t n,
-                                       int64_t padded_n, int lower, int upper, int swizzled, void* stream) {
+static int quant_launch(int impl, int early, int variant, const void* x, int x_dtype, const float* importance, const float* gs_inv,
+                        uint8_t* codes, uint8_t* scales, int64_t m, int64_t n, int64_t padded_n, int lower, int upper, int swizzled,
+                        void* stream) {
     using namespace nvfp4;
     if (impl < 0 || impl > 9 || impl == 4) return NVFP4_ERR_BAD_ENUM;
     QuantParams p;
     const int st = fill_params(p, variant, x, x_dtype, importance, gs_inv, codes, scales, m, n, padded_n, lower, upper, swizzled);
     if (st != NVFP4_OK || p.total == 0) return st;
+    p.early = early;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     cudaError_t err;
     switch (x_dtype) {
@@ -794,6 +799,19 @@ extern "C" int nvfp4_quant_launch_impl(int impl, int variant, const void* x, int
         default: err = launch_variant<NVFP4_DT_F32>(variant, impl, p, s); break;
     }
     return static_cast<int>(err);
+}
+
+extern "C" int nvfp4_quant_launch_impl(int impl, int variant, const void* x, int x_dtype, const float* importance,
+                                       const float* gs_inv, uint8_t* codes, uint8_t* scales, int64_t m, int64_t n,
+                                       int64_t padded_n, int lower, int upper, int swizzled, void* stream) {
+    return quant_launch(impl, 1, variant, x, x_dtype, importance, gs_inv, codes, scales, m, n, padded_n, lower, upper, swizzled, stream);
+}
+
+// nvfp4_quant_launch into buffers that a prepared weight may refer to.
+extern "C" int nvfp4_quant_launch_in_place(int variant, const void* x, int x_dtype, const float* importance, const float* gs_inv,
+                                           uint8_t* codes, uint8_t* scales, int64_t m, int64_t n, int64_t padded_n, int lower,
+                                           int upper, int swizzled, void* stream) {
+    return quant_launch(0, 0, variant, x, x_dtype, importance, gs_inv, codes, scales, m, n, padded_n, lower, upper, swizzled, stream);
 }
 
 namespace nvfp4 {

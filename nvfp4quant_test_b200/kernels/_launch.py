@@ -79,7 +79,8 @@ def _raise(st: int, what: str) -> None:
 def quant_out(variant: int, input: torch.Tensor, importance: torch.Tensor | None, input_scale: torch.Tensor,
               is_sf_swizzled_layout: bool, output: torch.Tensor, output_scale: torch.Tensor,
               lower: int, upper: int, impl: int = 0) -> None:
-    """Validate, then launch on the current stream of input.device.  Writes output / output_scale in place."""
+    """Validate, then launch on the current stream of input.device.  Writes output / output_scale in place; where a
+    PreparedWeight refers to them, launches behind this one on the stream read what it wrote."""
     if impl == 0 and _lib.fast.quant_out(variant, input, importance, input_scale, is_sf_swizzled_layout, output,
                                          output_scale, lower, upper):
         return
@@ -90,9 +91,9 @@ def quant_out(variant: int, input: torch.Tensor, importance: torch.Tensor | None
     imp_ptr, _keep = _importance_ptr(variant, importance)
     if m == 0 or physical_n == 0:
         return
-    args = (impl, variant, input.data_ptr(), _lib.dtype_code(input.dtype), imp_ptr, input_scale.data_ptr(),
+    args = (variant, input.data_ptr(), _lib.dtype_code(input.dtype), imp_ptr, input_scale.data_ptr(),
             output.data_ptr(), output_scale.data_ptr(), m, n, physical_n, lower, upper,
             1 if is_sf_swizzled_layout else 0, _lib.current_stream_ptr(input.device))
     with _lib.device_guard(input.device):   # launch with the tensor's device current
-        st = _lib.lib().nvfp4_quant_launch_impl(*args)
+        st = _lib.lib().nvfp4_quant_launch_impl(impl, *args) if impl else _lib.lib().nvfp4_quant_launch_in_place(*args)
     _raise(st, "nvfp4_quant_launch")

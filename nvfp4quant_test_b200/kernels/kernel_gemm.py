@@ -77,7 +77,12 @@ class PreparedWeight:
     """A quantized weight [N, K] that will be multiplied many times (a model's linear layer).  Its tensor maps are
     encoded once (nvfp4_gemm_prepare); `nvfp4_scaled_mm_prepared` then costs less host time per call than
     `nvfp4_scaled_mm` and gives the same bits.  Keeps references to the two tensors, which must not be resized or
-    moved while this object lives (their contents may be overwritten in place)."""
+    moved while this object lives.
+
+    Products stream a prepared weight while launches before them are still running, so what writes it has to be complete by
+    then.  Work queued on the current stream when the object is made is ordered before its products.  Later the contents may be
+    overwritten in place, on the stream of the products, by the quantizers' `_out` entry points or by torch; not by an
+    ActivationQuantizer."""
 
     def __init__(self, b: torch.Tensor, block_scale_b: torch.Tensor):
         import ctypes
@@ -97,6 +102,9 @@ class PreparedWeight:
         with _lib.device_guard(b.device):
             st = _lib.lib().nvfp4_gemm_prepare(b.data_ptr(), block_scale_b.data_ptr(), self.n, self.k, ctypes.byref(self._handle))
         _lib.check(st, "nvfp4_gemm_prepare")
+        # An ordinary kernel, no dependent launch: it starts when everything before it has completed (the quantizer that has just
+        # been queued for this weight), and nothing behind it starts before it has.
+        torch.zeros(1, dtype=torch.uint8, device=b.device)
         self._fast = (self._handle.value, self.n, self.k, b.device.index)   # the form the compiled calls take
 
     def close(self) -> None:

@@ -1,0 +1,36 @@
+"""GPU: forms of calls at the edges of what the entry points take, and their order on a stream."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("tokens", [1, 256])
+def test_a_weight_is_complete_before_a_product_reads_it(cuda_lib, tokens):
+    """A weight whose quantizer runs for hundreds of microseconds, then a short quantization and the product with it in dependent
+    launches, nothing else between: the product must wait for the weight, freshly made and requantized in place."""
+    import nvfp4quant_test_b200.kernels as K
+    from nvfp4quant_test_b200 import helper as H
+
+    n, k = 28672, 8192
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    ws = [torch.randn((n, k), generator=g, device="cuda").bfloat16() * f for f in (1.0, 2.0, 0.5)]
+    pairs = [H.get_nvfp4_global_scale(w, 256.0) for w in ws]
+    vecs = [gs.reshape(1) for gs, _ in pairs]
+    x = torch.randn((tokens, k), generator=g, device="cuda").bfloat16()
+    used = torch.full((n, k // 2), 0x77, dtype=torch.uint8, device="cuda")   # the block the first codes are likely to get
+    K.scalesweep_mse_nvfp4_quant_impl(x, pairs[0][1])                        # modules loaded
+    torch.cuda.synchronize()
+    del used
+    codes, scales = K.scalesweep_mse_nvfp4_quant_impl(ws[0], pairs[0][1])
+    weight = K.PreparedWeight(codes, scales)
+    got = [K.nvfp4_linear_multi([x], [0], [weight], [vecs[0]], [0])[0]]
+    for i in (1, 2, 0):
+        K.scalesweep_mse_nvfp4_quant_out(ws[i], pairs[i][1], True, output=codes, output_scale=scales)
+        got.append(K.nvfp4_linear_multi([x], [0], [weight], [vecs[i]], [0])[0])
+    torch.cuda.synchronize()
+    for i, have in zip((0, 1, 2, 0), got):
+        K.scalesweep_mse_nvfp4_quant_out(ws[i], pairs[i][1], True, output=codes, output_scale=scales)
+        torch.cuda.synchronize()
+        assert torch.equal(have, K.nvfp4_linear_multi([x], [0], [weight], [vecs[i]], [0])[0])
+        torch.cuda.synchronize()
