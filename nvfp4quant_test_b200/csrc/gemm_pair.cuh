@@ -370,9 +370,9 @@ static int launch_pair_list(const GemmParams* list, const WeightHandle* const* w
     static_assert(C::kSmemBytes <= kGemmDynSmemBytes, "ring does not fit");
     PairParams<G> q;
     q.M = list[0].M;
-    q.raster_group = list[0].raster_group;
-    q.weights_ready = 1;
     const int m_tiles = (q.M + 255) / 256;
+    q.raster_group = band_rows(list[0].raster_group, m_tiles);
+    q.weights_ready = 1;
     for (int i = 0; i < n; ++i) {
         const GemmParams& p = list[i];
         int st = make_operand_map(&q.a[i], p.a, p.M, p.K / 2, 128);
@@ -390,6 +390,7 @@ static int launch_pair_list(const GemmParams* list, const WeightHandle* const* w
     }
     const DeviceInfo di = device_info();
     const int pairs = fill_group_table<G>(q.g, list, n, m_tiles, BN, di.sms / 2);
+    if (pairs == 0) return NVFP4_ERR_TOO_LARGE;
     static bool attr_done[64] = {false};
     cudaError_t e = allow_full_smem(gemm_pair_kernel<BN, G>, attr_done, di.device);
     if (e != cudaSuccess) return static_cast<int>(e);

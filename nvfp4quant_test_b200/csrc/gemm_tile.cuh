@@ -2,6 +2,7 @@
 #pragma once
 
 #include "tc_ptx.cuh"
+#include "tile_index.cuh"
 
 namespace nvfp4 {
 namespace gemm {
@@ -227,18 +228,6 @@ __device__ __forceinline__ float load_alpha(const float* alpha, const float* alp
     // called behind griddep_wait(): the scales may be the work of the kernels before this one
     const float a = load_f32_after_wait(alpha);
     return alpha2 ? __fmul_rn(a, load_f32_after_wait(alpha2)) : a;
-}
-
-// Tile index -> (m tile, n tile).  Tiles are numbered in bands of `group` m-tiles: inside a band the m index runs
-// fastest, then n.  The CTAs that run at the same time then cover a roughly square patch of the output, so every A
-// tile and every B tile is being fetched by a moderate number of CTAs at once instead of one B tile by all of them.
-__device__ __forceinline__ void tile_to_mn(int tile, int m_tiles, int n_tiles, int group, int& mt, int& nt) {
-    const int band = tile / (group * n_tiles);
-    const int first_m = band * group;
-    const int rows = min(group, m_tiles - first_m);
-    const int in_band = tile - band * group * n_tiles;
-    nt = in_band / rows;
-    mt = first_m + in_band - nt * rows;
 }
 
 // Operand maps and the work list of one launch over G products (G = 1: an ordinary GEMM, whose K may be cut into ranges).
@@ -662,7 +651,8 @@ struct WeightHandle {
 };
 constexpr uint32_t kWeightMagic = 0x4e56463u;
 
-// Fills the work list for `workers` CTAs (or CTA pairs) and returns how many are used (0: too few for the classes).
+// Fills the work list for `workers` CTAs (or CTA pairs) and returns how many are used (0: too few for the classes, or more
+// tiles than a launch can number).
 // A class is a run of items of equal K.  With one class every worker takes tiles of it; with several the smallest makespan
 // T (in K stages) is searched for which the classes' workers, ceil(tiles / floor(T / k)) each, fit.
 template <int G>
@@ -691,11 +681,13 @@ static int fill_group_table(GroupTable<G>& g, const GemmParams* list, int n, int
         tiles[c] += mine;
         stages += mine * k[c];
         if (k[c] > longest) longest = k[c];
+        if (tiles[c] > kMaxTiles) return 0;
         it.tile_end = static_cast<int>(tiles[c]);
         g.item_end[c] = i + 1;
     }
     if (g.n_classes == 1) {
         const int64_t all = tiles[0] * (G == 1 ? list[0].k_splits : 1);
+        if (all > kMaxTiles) return 0;
         return g.worker_end[0] = static_cast<int>(all < workers ? all : workers);
     }
     if (workers < g.n_classes) return 0;
@@ -740,7 +732,8 @@ static int launch_list(const GemmParams* list, const WeightHandle* const* wh, in
     q.k_tiles_per_split = p0.k_tiles_per_split;
     q.k_rotate = p0.k_rotate;
     q.partial = p0.partial;
-    q.raster_group = p0.raster_group;
+    const int m_tiles = (q.M + kBM - 1) / kBM;
+    q.raster_group = band_rows(p0.raster_group, m_tiles);
     q.weights_ready = 1;
     for (int i = 0; i < n; ++i) {
         const GemmParams& p = list[i];
@@ -755,7 +748,8 @@ static int launch_list(const GemmParams* list, const WeightHandle* const* wh, in
         if (st != NVFP4_OK) return st;
     }
     const DeviceInfo di = device_info();
-    const int grid = fill_group_table<G>(q.g, list, n, (q.M + kBM - 1) / kBM, BN, di.sms);
+    const int grid = fill_group_table<G>(q.g, list, n, m_tiles, BN, di.sms);
+    if (grid == 0) return NVFP4_ERR_TOO_LARGE;
     static bool attr_done[64] = {false};
     cudaError_t e = allow_full_smem(gemm_kernel<BN, G>, attr_done, di.device);
     if (e != cudaSuccess) return static_cast<int>(e);

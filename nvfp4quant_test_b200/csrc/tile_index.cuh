@@ -1,0 +1,33 @@
+// Numbering of output tiles: plain index arithmetic, for the kernels and the host.
+#pragma once
+
+#ifdef __CUDACC__
+#define NVFP4_HOST_DEVICE __host__ __device__ __forceinline__
+#else
+#define NVFP4_HOST_DEVICE inline
+#endif
+
+namespace nvfp4 {
+namespace gemm {
+
+// Most tiles of a launch: numbers of tiles, and the next tile of any worker, stay within an int.
+constexpr long long kMaxTiles = 0x7fff0000LL;
+
+// m-tiles per band for a wish of `group` (see tile_to_mn).  More than there are would be the same numbering, but group * n_tiles
+// must not leave the int range.
+NVFP4_HOST_DEVICE int band_rows(int group, int m_tiles) { return group < m_tiles ? group : m_tiles; }
+
+// Tile index -> (m tile, n tile).  Tiles are numbered in bands of `group` m-tiles (1 .. m_tiles): inside a band the m index runs
+// fastest, then n.  The CTAs that run at the same time then cover a roughly square patch of the output, so every A
+// tile and every B tile is being fetched by a moderate number of CTAs at once instead of one B tile by all of them.
+NVFP4_HOST_DEVICE void tile_to_mn(int tile, int m_tiles, int n_tiles, int group, int& mt, int& nt) {
+    const int band = tile / (group * n_tiles);
+    const int first_m = band * group;
+    const int rows = group < m_tiles - first_m ? group : m_tiles - first_m;
+    const int in_band = tile - band * group * n_tiles;
+    nt = in_band / rows;
+    mt = first_m + in_band - nt * rows;
+}
+
+}  // namespace gemm
+}  // namespace nvfp4

@@ -34,3 +34,24 @@ def test_a_weight_is_complete_before_a_product_reads_it(cuda_lib, tokens):
         torch.cuda.synchronize()
         assert torch.equal(have, K.nvfp4_linear_multi([x], [0], [weight], [vecs[i]], [0])[0])
         torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("path,n", [(6, 131072), (6, 262144), (6, 262208), (1, 524288)])
+def test_products_with_thousands_of_column_tiles(cuda_lib, path, n):
+    """Counts of column tiles at which (m-tiles of a band) x (column tiles) used to leave the int range, against 256-wide tiles."""
+    import nvfp4quant_test_b200.kernels as K
+
+    m, k = 130, 64
+    g = torch.Generator(device="cuda").manual_seed(n)
+    a, b = (torch.randint(0, 256, (rows, k // 2), dtype=torch.uint8, device="cuda", generator=g) for rows in (m, n))
+    sa, sb = (torch.randint(0x30, 0x40, ((rows + 127) // 128 * 128, 4), dtype=torch.uint8, device="cuda", generator=g) for rows in (m, n))
+    one = torch.ones(1, device="cuda")
+    got = []
+    try:
+        for p in (path, 2):
+            assert cuda_lib.nvfp4_gemm_force_path(p) == 0
+            got.append(K.nvfp4_scaled_mm(a, b, sa, sb, one, torch.bfloat16))
+            torch.cuda.synchronize()
+    finally:
+        cuda_lib.nvfp4_gemm_force_path(0)
+    assert torch.equal(*got)
