@@ -14,6 +14,9 @@
 #include <ATen/core/CachingHostAllocator.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/ops/zeros.h>
+#include <c10/core/GradMode.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cuda_runtime_api.h>
@@ -417,10 +420,16 @@ PyObject* channel_square_norm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     });
 }
 
+// The dequantizer and the scale layouts are torch operations anywhere but here, so what torch does beside computing them has to
+// go on: a tracer or a dispatch mode sees the operations, gradients and forward-mode tangents flow through them, a lazily negated
+// scale is read as its value.  (Inside torch.func transforms a wrapped tensor has no data to point at and falls out by itself.)
+inline bool observed() { return c10::impl::dispatch_mode_enabled() || c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::Tracer); }
+inline bool plain_value(const Tensor& t) { return !(c10::GradMode::is_enabled() && t.requires_grad()) && !t._fw_grad(0).defined() && !t.is_neg(); }
+
 // dequant(codes, block scales | None, global scale | None) -> float32 [m, n]
 PyObject* dequant(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     return guarded([&]() -> PyObject* {
-        if (nargs != 3) return none();
+        if (nargs != 3 || observed()) return none();
         const Tensor* q = tensor_of(a[0]);
         if (!q || !plain_cuda(*q) || q->dim() != 2 || q->scalar_type() != at::kByte || !q->is_contiguous() || !aligned(*q, 4)) return none();
         const int64_t m = q->size(0), n = q->size(1) * 2;
@@ -433,7 +442,7 @@ PyObject* dequant(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         } else {
             const Tensor *s = tensor_of(a[1]), *g = tensor_of(a[2]);
             if (!s || !g || s->device() != q->device() || s->scalar_type() != at::kFloat8_e4m3fn || s->dim() != 2 || s->size(0) != m ||
-                s->size(1) * 16 != n || !s->is_contiguous() || g->numel() != 1 || g->dim() > 2 || !scalar_input(a[2], dev, &gs))
+                s->size(1) * 16 != n || !s->is_contiguous() || g->numel() != 1 || g->dim() > 2 || !plain_value(*s) || !plain_value(*g) || !scalar_input(a[2], dev, &gs))
                 return none();
             scales = static_cast<const uint8_t*>(s->const_data_ptr());
         }
@@ -451,7 +460,7 @@ PyObject* dequant(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
 PyObject* scale_layout(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     return guarded([&]() -> PyObject* {
         int64_t m, k;
-        if (nargs != 4 || !int_or_none(a[1], 0, &m) || !int_or_none(a[2], 0, &k) || m <= 0 || k <= 0) return none();
+        if (nargs != 4 || observed() || !int_or_none(a[1], 0, &m) || !int_or_none(a[2], 0, &k) || m <= 0 || k <= 0) return none();
         const bool to_tiled = a[3] == Py_True;
         const Tensor* s = tensor_of(a[0]);
         const int64_t padded = round_up(m, 128) * round_up(k, 4);

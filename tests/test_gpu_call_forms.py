@@ -55,3 +55,56 @@ def test_products_with_thousands_of_column_tiles(cuda_lib, path, n):
     finally:
         cuda_lib.nvfp4_gemm_force_path(0)
     assert torch.equal(*got)
+
+
+def _quantized(m=32, n=256):
+    g = torch.Generator(device="cuda").manual_seed(3)
+    codes = torch.randint(0, 256, (m, n // 2), dtype=torch.uint8, device="cuda", generator=g)
+    scales = torch.randint(0x20, 0x70, (m, n // 16), dtype=torch.uint8, device="cuda", generator=g).view(torch.float8_e4m3fn)
+    return codes, scales, torch.tensor(0.5, device="cuda")
+
+
+def test_dequantization_stays_differentiable_in_the_global_scale(cuda_lib):
+    import torch.autograd.forward_ad as fwd
+
+    from nvfp4quant_test_b200 import helper as H
+
+    q, s, gs = _quantized()
+    unit = H.dequantize_base(q, s, torch.ones((), device="cuda"))
+    g = gs.clone().requires_grad_()
+    y = H.dequantize_base(q, s, g)
+    assert torch.equal(y.detach(), H.dequantize_base(q, s, gs))
+    (grad,) = torch.autograd.grad(y.sum(), g)
+    # two fp32 sums of the same n values in any order: n * 2^-24 of the sum of their magnitudes apart
+    assert abs(grad - unit.sum()) <= unit.abs().sum() * unit.numel() * 2.0 ** -24
+    with torch.no_grad():
+        assert not H.dequantize_base(q, s, g).requires_grad
+    with fwd.dual_level():
+        tangent = fwd.unpack_dual(H.dequantize_base(q, s, fwd.make_dual(gs, torch.ones_like(gs)))).tangent
+        assert tangent is not None and torch.equal(tangent, unit)
+    assert torch.equal(torch.func.grad(lambda v: H.dequantize_base(q, s, v).sum())(gs), grad)
+    both = torch.func.vmap(lambda v: H.dequantize_base(q, s, v))(torch.stack([gs, gs * 2]))
+    assert torch.equal(both[1], H.dequantize_base(q, s, gs * 2))
+    assert torch.equal(H.dequantize_base(q, s, torch._neg_view(gs)), -H.dequantize_base(q, s, gs))
+
+
+@pytest.mark.parametrize("trace", ["make_fx", "compile"])
+def test_dequantization_and_scale_layouts_can_be_traced(cuda_lib, trace):
+    import nvfp4quant_test_b200.kernels as K
+    from nvfp4quant_test_b200 import helper as H
+
+    q, s, gs = _quantized()
+
+    def f(q, s, gs):
+        tiled = K.swizzle_vllm_fp4_scale(s, 32, 256)
+        return H.dequantize_base(q, K.unswizzle_vllm_fp4_scale(tiled, 32, 256), gs), H.unpack_fp4_e2m1(q)
+
+    if trace == "make_fx":
+        from torch.fx.experimental.proxy_tensor import make_fx
+
+        traced = make_fx(f)(q, s, gs)
+    else:
+        traced = torch.compile(f, backend="eager", fullgraph=True)
+    other = (q.flip(0).contiguous(), s.view(torch.uint8).flip(0).contiguous().view(torch.float8_e4m3fn), gs * 2)
+    for got, want in zip(traced(*other), f(*other)):
+        assert torch.equal(got, want)
