@@ -191,7 +191,7 @@ def layer_gemms(qlayer: dict, acts: dict[int, torch.Tensor], act_importance: dic
     works under CUDA-graph capture)."""
     if weight_scales is None:
         weight_scales = stack_weight_scales(qlayer)
-    if prepared is not None:
+    if prepared is not None and all(x.shape[0] for x in acts.values()):     # an activation without rows has no maximum
         return _layer_gemms_prepared(qlayer, acts, act_importance, weight_scales, prepared)
     main = torch.cuda.current_stream()
     out = {}
@@ -218,6 +218,8 @@ def layer_gemms(qlayer: dict, acts: dict[int, torch.Tensor], act_importance: dic
         qa, sa, alphas, ready = qact[k]
         slot = weight_scales[k][1][name]
         def mm():
+            if prepared is not None:
+                return K.nvfp4_scaled_mm_prepared(qa, sa, alphas[slot:slot + 1], prepared[name])
             return K.nvfp4_scaled_mm(qa, codes, sa, scales, alphas[slot:slot + 1], torch.bfloat16)
 
         if side_streams:

@@ -108,3 +108,20 @@ def test_dequantization_and_scale_layouts_can_be_traced(cuda_lib, trace):
     other = (q.flip(0).contiguous(), s.view(torch.uint8).flip(0).contiguous().view(torch.float8_e4m3fn), gs * 2)
     for got, want in zip(traced(*other), f(*other)):
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("streams", [0, 2])
+@pytest.mark.parametrize("rows", [(0, 0), (3, 0)])
+def test_a_layer_of_prepared_weights_takes_an_activation_without_rows(cuda_lib, streams, rows):
+    import nvfp4quant_test_b200.kernels as K
+    from nvfp4quant_test_b200 import llama_stack as S
+
+    qlayer = {name: K.scalesweep_nvfp4_quant_with_global_scale(torch.randn(shape, device="cuda").bfloat16(), 256.0)[:3]
+              for name, shape in {"a": (64, 128), "b": (72, 256)}.items()}
+    acts = {k: torch.randn((m, k), device="cuda").bfloat16() for m, k in zip(rows, (128, 256))}
+    side = [torch.cuda.Stream() for _ in range(streams)] or None
+    scales = S.stack_weight_scales(qlayer)
+    got = S.layer_gemms(qlayer, acts, {}, scales, side, S.prepare_layer(qlayer))
+    want = S.layer_gemms(qlayer, acts, {}, scales)
+    assert {k: tuple(v.shape) for k, v in got.items()} == {"a": (rows[0], 64), "b": (rows[1], 72)}
+    assert all(torch.equal(got[k], want[k]) for k in got)
