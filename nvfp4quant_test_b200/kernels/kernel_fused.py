@@ -58,6 +58,8 @@ def scalesweep_nvfp4_quant_with_global_scale(
         raise ValueError("input must be a CUDA tensor: these kernels have no CPU path")
     if m == 0 or n == 0:
         raise ValueError("the global scale of an empty tensor is undefined")
+    if not float(fp8_max) > 0.0:
+        raise ValueError(f"fp8_max must be positive, got {fp8_max}")
     output, output_scale = create_fp4_output_tensors(m, n, input.device, is_sf_swizzled_layout, padded_n=padded_n)
     g, g_inv = _helper.get_nvfp4_global_scale(input, fp8_max)
     quant_out(variant, input, importance, g_inv, is_sf_swizzled_layout, output, output_scale, lower, upper)

@@ -125,3 +125,15 @@ def test_a_layer_of_prepared_weights_takes_an_activation_without_rows(cuda_lib, 
     want = S.layer_gemms(qlayer, acts, {}, scales)
     assert {k: tuple(v.shape) for k, v in got.items()} == {"a": (rows[0], 64), "b": (rows[1], 72)}
     assert all(torch.equal(got[k], want[k]) for k in got)
+
+
+@pytest.mark.parametrize("fp8_max", [0.0, -448.0, float("nan")])
+def test_a_maximum_that_is_not_positive_is_refused(cuda_lib, fp8_max):
+    import nvfp4quant_test_b200.kernels as K
+
+    x = torch.randn((4, 64), device="cuda").bfloat16()
+    for importance in (None, torch.ones((1, 64), device="cuda")):
+        with pytest.raises(ValueError, match="positive"):
+            K.scalesweep_nvfp4_quant_with_global_scale(x, fp8_max, importance)
+    with pytest.raises(ValueError, match="positive"):
+        K.scalesweep_nvfp4_quant_with_global_scales([x, x], fp8_max)
