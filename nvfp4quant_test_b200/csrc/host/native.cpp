@@ -1024,7 +1024,7 @@ PyObject* host_pipe_call(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
             return none();
         }
         if (x->dim() != 2 || x->size(0) != p->rows || x->size(1) != p->dim || dtype_code(x->scalar_type()) != p->dtype || !x->is_contiguous() ||
-            codes->scalar_type() != at::kByte || codes->numel() != p->rows * (p->dim / 2) || !codes->is_contiguous() || !scales->is_contiguous() ||
+            codes->scalar_type() != at::kByte || codes->dim() != 2 || codes->size(0) != p->rows || codes->size(1) != p->dim / 2 || !codes->is_contiguous() || !scales->is_contiguous() ||
             static_cast<int64_t>(scales->nbytes()) < round_up(p->rows, 128) * round_up(p->dim / 16, 4))
             return none();
         if (a[5] != Py_None) {

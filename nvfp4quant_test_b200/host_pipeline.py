@@ -89,25 +89,38 @@ class HostQuantizer:
             raise ValueError("input does not match the shape this quantizer was built for")
         if self.rows == 0 or self.dim == 0:
             return
-        if importance is not None:
-            _launch.check_importance(self.stage_in[0][:1], importance)
-            importance = importance.float().contiguous() if self.variant == _lib.VARIANT_WEIGHTED else None
+        if self.variant != _lib.VARIANT_WEIGHTED:
+            importance = None
+        elif importance is None:
+            raise ValueError("the weighted variant needs an importance vector")
+        else:
+            if importance.numel() < self.dim or importance.device != self.stage_in[0].device:
+                raise ValueError(f"importance must hold {self.dim} values on {self.stage_in[0].device}")
+            importance = importance.float().contiguous()
+            if importance.numel() > self.dim:
+                importance = importance.reshape(-1)[:self.dim]
         if _lib.fast.host_pipe_call(self._pipe, x_host, gs_inv, codes_host, scales_host, importance):
             return
         # something about the operands: name it, or bring it into the form the call takes
-        if self.variant == _lib.VARIANT_WEIGHTED and importance is None:
-            raise ValueError("the weighted variant needs an importance vector")
         _launch._check_common(self.stage_in[0], gs_inv)
-        if codes_host.dtype != torch.uint8 or tuple(codes_host.shape) != (self.rows, self.dim // 2):
-            raise ValueError(f"codes_host must be uint8 [{self.rows}, {self.dim // 2}]")
+        if codes_host.ndim != 2 or codes_host.shape[0] < self.rows or codes_host.shape[1] != self.dim // 2:
+            raise ValueError(f"codes_host must be [{self.rows}, {self.dim // 2}]")
         need = round_up(self.rows, 128) * self.k_pad
         if not scales_host.is_contiguous() or scales_host.numel() * scales_host.element_size() < need:
             raise ValueError(f"scales_host must be a contiguous buffer of {need} bytes")
-        codes = codes_host.contiguous()
-        if importance is not None and importance.data_ptr() & 15:
-            importance = importance.clone()
-        if not _lib.fast.host_pipe_call(self._pipe, x_host.detach().contiguous(), gs_inv, codes, scales_host.detach(), importance):
+
+        def plain(t):
+            return t.detach().as_subclass(torch.Tensor)
+
+        target = plain(codes_host)[:self.rows]
+        direct = target.dtype == torch.uint8 and target.is_contiguous()
+        codes = target if direct else torch.empty((self.rows, self.dim // 2), dtype=torch.uint8)
+        if importance is not None:
+            importance = plain(importance)
+            if importance.data_ptr() & 15:
+                importance = importance.clone()
+        if not _lib.fast.host_pipe_call(self._pipe, plain(x_host).contiguous(), plain(gs_inv), codes, plain(scales_host), importance):
             raise ValueError("operands the host pipeline does not take")
-        if codes.data_ptr() != codes_host.data_ptr():      # a strided output
+        if not direct:      # strided, or of another type
             torch.cuda.current_stream(self.device).synchronize()
-            codes_host.copy_(codes)
+            target.copy_(codes)

@@ -137,3 +137,48 @@ def test_a_maximum_that_is_not_positive_is_refused(cuda_lib, fp8_max):
             K.scalesweep_nvfp4_quant_with_global_scale(x, fp8_max, importance)
     with pytest.raises(ValueError, match="positive"):
         K.scalesweep_nvfp4_quant_with_global_scales([x, x], fp8_max)
+
+
+def _host_operands(m=200, n=96):
+    g = torch.Generator().manual_seed(1)
+    return torch.randn((m, n), generator=g).bfloat16(), torch.rand((1, n), generator=g).cuda(), torch.tensor([40.0], device="cuda")
+
+
+@pytest.mark.parametrize("form", ["flat importance", "longer importance", "importance of no use", "more rows", "int16 codes", "subclass"])
+def test_host_pipeline_takes_what_it_took(cuda_lib, form):
+    import nvfp4quant_test_b200.kernels as K
+    from nvfp4quant_test_b200 import _lib
+    from nvfp4quant_test_b200.host_pipeline import HostQuantizer
+
+    class Sub(torch.Tensor):
+        pass
+
+    x, imp, gs = _host_operands()
+    m, n = x.shape
+    if form == "importance of no use":
+        want, variant, window = K.scalesweep_mse_nvfp4_quant_impl(x.cuda(), gs), _lib.VARIANT_MSE, (-3, 7)
+    else:
+        want, variant, window = K.scalesweep_weighted_mse_nvfp4_quant_impl(x.cuda(), imp, gs), _lib.VARIANT_WEIGHTED, (-8, 7)
+    hq = HostQuantizer(m, n, torch.bfloat16, "cuda", chunk_rows=128, variant=variant, lower=window[0], upper=window[1])
+    codes = torch.zeros((m + 7 if form == "more rows" else m, n // 2), dtype=torch.int16 if form == "int16 codes" else torch.uint8)
+    scales = torch.zeros(want[1].numel(), dtype=torch.uint8)
+    imp = {"flat importance": imp[0], "longer importance": torch.cat([imp, imp], 1), "importance of no use": torch.ones(3)}.get(form, imp)
+    args = (x, gs, codes, scales, imp)
+    hq(*(t.as_subclass(Sub) for t in args) if form == "subclass" else args)
+    torch.cuda.synchronize()
+    assert torch.equal(codes[:m].to(torch.uint8), want[0].cpu()) and not codes[m:].any()
+    assert torch.equal(scales, want[1].view(torch.uint8).reshape(-1).cpu())
+
+
+def test_host_pipeline_refuses_codes_of_another_shape(cuda_lib):
+    from nvfp4quant_test_b200.host_pipeline import HostQuantizer
+
+    x, imp, gs = _host_operands()
+    m, n = x.shape
+    hq = HostQuantizer(m, n, torch.bfloat16, "cuda", chunk_rows=128)
+    scales = torch.zeros(256 * 8, dtype=torch.uint8)
+    for shape in ((m * n // 2,), (n // 2, m), (m - 1, n // 2)):
+        with pytest.raises(ValueError, match="codes_host"):
+            hq(x, gs, torch.zeros(shape, dtype=torch.uint8), scales)
+    with pytest.raises(ValueError, match="importance"):
+        HostQuantizer(m, n, torch.bfloat16, "cuda", variant=1, lower=-8, upper=7)(x, gs, torch.zeros((m, n // 2), dtype=torch.uint8), scales, imp[:, :-1])
