@@ -24,6 +24,7 @@
 
 #include <list>
 #include <memory>
+#include <mutex>
 #include <unordered_map>
 #include <vector>
 
@@ -916,6 +917,7 @@ struct HostPipe {
     std::vector<cudaEvent_t> ev_up, ev_run, ev_down;
     std::vector<bool> used;                    // slot j's events have been recorded, by this call or an earlier one
     cudaEvent_t begin = nullptr, end_run = nullptr, end_down = nullptr;
+    std::mutex mutex;                          // one call at a time: `used` and the events, which are queued without the interpreter lock
     ~HostPipe() {
         for (auto* v : {&ev_up, &ev_run, &ev_down})
             for (cudaEvent_t e : *v) cudaEventDestroy(e);
@@ -1040,6 +1042,7 @@ PyObject* host_pipe_call(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         const bool one = p->plan.size() == 1;
         int status = NVFP4_OK;
         const int e = launch_on(p->device, [&] {
+            const std::lock_guard<std::mutex> one_call(p->mutex);
             return static_cast<int>(host_pipe_run(*p, static_cast<const char*>(x->const_data_ptr()), gs_inv, importance,
                                                   static_cast<char*>(codes->mutable_data_ptr()), static_cast<char*>(scales->mutable_data_ptr()), cur, &status));
         });

@@ -84,7 +84,8 @@ class HostQuantizer:
                  scales_host: torch.Tensor, importance: torch.Tensor | None = None) -> None:
         """x_host [rows, dim] (pinned for real overlap); codes_host uint8 [rows, dim/2]; scales_host uint8
         [round_up(rows,128) * round_up(dim/16,4)] (tiled layout).  Returns once everything has been enqueued;
-        the caller synchronises (e.g. torch.cuda.synchronize()) before reading the host outputs."""
+        the caller synchronises (e.g. torch.cuda.synchronize()) before reading the host outputs.  Calls from several threads,
+        each on a stream of its own, go one after the other."""
         if tuple(x_host.shape) != (self.rows, self.dim) or x_host.dtype != self.dtype:
             raise ValueError("input does not match the shape this quantizer was built for")
         if self.rows == 0 or self.dim == 0:

@@ -182,3 +182,39 @@ def test_host_pipeline_refuses_codes_of_another_shape(cuda_lib):
             hq(x, gs, torch.zeros(shape, dtype=torch.uint8), scales)
     with pytest.raises(ValueError, match="importance"):
         HostQuantizer(m, n, torch.bfloat16, "cuda", variant=1, lower=-8, upper=7)(x, gs, torch.zeros((m, n // 2), dtype=torch.uint8), scales, imp[:, :-1])
+
+
+@pytest.mark.parametrize("rows,chunk", [(2000, 256), (300, 512)])     # several chunks, one chunk
+def test_host_pipeline_is_shared_by_threads(cuda_lib, rows, chunk):
+    import threading
+
+    import nvfp4quant_test_b200.kernels as K
+    from nvfp4quant_test_b200.host_pipeline import HostQuantizer
+
+    g = torch.Generator().manual_seed(rows)
+    gs = torch.tensor([40.0], device="cuda")
+    hq = HostQuantizer(rows, 4096, torch.bfloat16, "cuda", chunk_rows=chunk)
+    wrong = []
+
+    def work(x, want, stream):
+        codes, scales = torch.zeros_like(want[0]).pin_memory(), torch.zeros_like(want[1]).pin_memory()
+        with torch.cuda.stream(stream):
+            for _ in range(20):
+                codes.zero_(), scales.zero_()
+                hq(x, gs, codes, scales)
+                stream.synchronize()
+                if not (torch.equal(codes, want[0]) and torch.equal(scales, want[1])):
+                    wrong.append(1)
+
+    xs = [torch.randn((rows, 4096), generator=g).bfloat16().pin_memory() for _ in range(3)]
+    wants = []
+    for x in xs:
+        codes, scales = K.scalesweep_mse_nvfp4_quant_impl(x.cuda(), gs)
+        wants.append((codes.cpu(), scales.view(torch.uint8).reshape(-1).cpu()))
+    threads = [threading.Thread(target=work, args=(x, w, torch.cuda.Stream())) for x, w in zip(xs, wants)]
+    torch.cuda.synchronize()
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
