@@ -526,9 +526,15 @@ static int launch_skinny_list(int M, const SkinnyItem* items, int n_items, int f
     if (mixed && forced_ranks == 0) {
         cluster = plan_mixed(p, n_items, sms);
     } else {
+        // one number of ranges for all: the largest that leaves none of any item empty.  (A smaller one need not fit where a larger
+        // one did, 24 stages fit 6 ranges and 25 do not, so every item is asked again for each.)
         cluster = choose_ranks(n_tiles, shortest, sms, forced_ranks, BT);
-        for (int i = 0; i < n_items; ++i)
-            while (cluster > 1 && !fits(i, cluster)) --cluster;
+        auto all_fit = [&](int r) {
+            for (int i = 0; i < n_items; ++i)
+                if (!fits(i, r)) return false;
+            return true;
+        };
+        while (cluster > 1 && !all_fit(cluster)) --cluster;
         for (int i = 0; i < n_items; ++i) p.w[i].ranks = cluster;
     }
     int clusters = 0, per_rank = 1, max_ranks = 1;

@@ -218,3 +218,30 @@ def test_host_pipeline_is_shared_by_threads(cuda_lib, rows, chunk):
     for t in threads:
         t.join()
     assert not wrong
+
+
+@pytest.mark.parametrize("ranges", [3, 6, 7, 8])
+@pytest.mark.parametrize("stages", [(25, 24), (24, 25), (49, 13, 24), (9, 8)])
+def test_forced_k_ranges_of_products_of_different_k(cuda_lib, ranges, stages):
+    """A number of ranges that leaves none of any product empty: an empty one would add uninitialised TMEM."""
+    import nvfp4quant_test_b200.kernels as K
+    from nvfp4quant_test_b200 import helper as H
+    from nvfp4quant_test_b200.kernels.kernel_gemm import gemm_last_status
+
+    def operand(rows, k):
+        return K.scalesweep_nvfp4_quant_with_global_scale(torch.randn((rows, k), device="cuda").bfloat16(), 256.0)[:3]
+
+    acts, weights = [operand(16, 256 * s) for s in stages], [operand(200, 256 * s) for s in stages]
+    prepared = [K.PreparedWeight(c, s) for c, s, _ in weights]
+    try:
+        assert cuda_lib.nvfp4_gemm_force_path(5) == 0 and cuda_lib.nvfp4_gemm_tune(ranges, -1) == 0
+        got = K.nvfp4_scaled_mm_multi(*[list(c) for c in zip(*acts)], prepared, [w[2].reshape(1) for w in weights])
+        torch.cuda.synchronize()
+    finally:
+        cuda_lib.nvfp4_gemm_force_path(0)
+        cuda_lib.nvfp4_gemm_tune(0, -1)
+    assert gemm_last_status() == 0
+    for s, a, w, x in zip(stages, acts, weights, got):
+        full = [H.dequantize("base", q, K.unswizzle_vllm_fp4_scale(sc, q.shape[0], 256 * s), gs).double() for q, sc, gs in (a, w)]
+        want = full[0] @ full[1].T
+        assert ((x.double() - want).abs() <= want.abs() * 2.0 ** -7 + want.abs().max() * 2.0 ** -16).all()
