@@ -396,7 +396,7 @@ PyObject* channel_square_norm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         const int64_t m = x->size(0), n = x->size(1);
         // a column slice of a wider batch is read in place through its row pitch
         const int64_t ld = m > 1 ? x->stride(0) : n;
-        if (dt < 0 || (m > 1 && (x->stride(1) != 1 || ld < n || ld % 4))) return none();
+        if (dt < 0 || x->stride(1) != 1 || (m > 1 && (ld < n || ld % 4))) return none();
         const c10::DeviceIndex dev = x->device().index();
         Tensor out;
         if (a[1] == Py_None) {

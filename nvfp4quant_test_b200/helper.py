@@ -61,7 +61,7 @@ def channel_square_norm(x: torch.Tensor, out: torch.Tensor | None = None) -> tor
     if x.shape[1] % 4:
         raise ValueError("x.shape[1] must be divisible by 4")
     # a column slice of a wider batch (x_full[:, c0:c1]) is read in place through its row pitch
-    in_place = x.shape[0] <= 1 or (x.stride(1) == 1 and x.stride(0) >= x.shape[1] and x.stride(0) % 4 == 0)
+    in_place = x.stride(1) == 1 and (x.shape[0] <= 1 or (x.stride(0) >= x.shape[1] and x.stride(0) % 4 == 0))
     if not in_place or x.data_ptr() & 15:
         x = x.contiguous()
         if x.data_ptr() & 15:

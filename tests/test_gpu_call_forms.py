@@ -245,3 +245,12 @@ def test_forced_k_ranges_of_products_of_different_k(cuda_lib, ranges, stages):
         full = [H.dequantize("base", q, K.unswizzle_vllm_fp4_scale(sc, q.shape[0], 256 * s), gs).double() for q, sc, gs in (a, w)]
         want = full[0] @ full[1].T
         assert ((x.double() - want).abs() <= want.abs() * 2.0 ** -7 + want.abs().max() * 2.0 ** -16).all()
+
+
+def test_channel_norms_of_one_strided_row(cuda_lib):
+    from nvfp4quant_test_b200 import helper as H
+
+    x = torch.randn((1, 128), device="cuda").bfloat16()
+    assert torch.equal(H.channel_square_norm(x[:, ::2]), H.channel_square_norm(x[:, ::2].contiguous()))
+    column = torch.randn((64, 4), device="cuda").bfloat16()
+    assert torch.equal(H.channel_square_norm(column.t()[1:2]), column.float().square().t()[1:2])
