@@ -110,7 +110,14 @@ inline bool as_float(PyObject* o, float* out) {
     *out = static_cast<float>(d);
     return true;
 }
-inline int small_int(PyObject* o) { return static_cast<int>(PyLong_AsLong(o)); }
+// An int of the candidate window; false for anything else and for what does not fit.
+inline bool window_int(PyObject* o, int* out) {
+    int overflow = 0;
+    const long v = PyLong_CheckExact(o) ? PyLong_AsLongAndOverflow(o, &overflow) : 0;
+    *out = static_cast<int>(v);
+    return PyLong_CheckExact(o) && overflow == 0 && *out == v;
+}
+inline int small_int(PyObject* o) { return static_cast<int>(PyLong_AsLong(o)); }   // a constant of the package's own
 
 PyObject* pack(std::initializer_list<Tensor> ts) {
     PyObject* t = PyTuple_New(static_cast<Py_ssize_t>(ts.size()));
@@ -237,10 +244,11 @@ PyObject* quant_impl(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         QuantIn q;
         const float* gs_inv;
         int64_t padded_n;
+        int lower, upper;
         if (!quant_input(a[1], a[2], &q) || !scalar_input(a[3], q.device, &gs_inv) || !PyBool_Check(a[4]) ||
-            !int_or_none(a[5], q.n, &padded_n) || padded_n < q.n || padded_n % 16 || !PyLong_CheckExact(a[6]) || !PyLong_CheckExact(a[7]))
+            !int_or_none(a[5], q.n, &padded_n) || padded_n < q.n || padded_n % 16 || !window_int(a[6], &lower) || !window_int(a[7], &upper))
             return none();
-        const int variant = small_int(a[0]), lower = small_int(a[6]), upper = small_int(a[7]);
+        const int variant = small_int(a[0]);
         const bool tiled = a[4] == Py_True;
         Tensor codes = empty({q.m, padded_n / 2}, at::kByte, q.device);
         Tensor scales = empty_scales(q.m, padded_n, tiled, q.device);
@@ -261,8 +269,9 @@ PyObject* quant_out(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         if (nargs != 9) return none();
         QuantIn q;
         const float* gs_inv;
-        if (!quant_input(a[1], a[2], &q) || !scalar_input(a[3], q.device, &gs_inv) || !PyBool_Check(a[4]) || !PyLong_CheckExact(a[7]) ||
-            !PyLong_CheckExact(a[8]))
+        int lower, upper;
+        if (!quant_input(a[1], a[2], &q) || !scalar_input(a[3], q.device, &gs_inv) || !PyBool_Check(a[4]) || !window_int(a[7], &lower) ||
+            !window_int(a[8], &upper))
             return none();
         const Tensor *codes = tensor_of(a[5]), *scales = tensor_of(a[6]);
         if (!codes || !scales || !plain_cuda(*codes) || !plain_cuda(*scales) || codes->device() != q.x->device() ||
@@ -274,7 +283,7 @@ PyObject* quant_out(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         const bool tiled = a[4] == Py_True;
         const int64_t need = tiled ? round_up(q.m, 128) * round_up(padded_n / 16, 4) : q.m * (padded_n / 16);
         if (static_cast<int64_t>(scales->nbytes()) < need) return none();
-        const int variant = small_int(a[0]), lower = small_int(a[7]), upper = small_int(a[8]);
+        const int variant = small_int(a[0]);
         const cudaStream_t s = current_stream(q.device);
         const int st = launch_on(q.device, [&] {
             return nvfp4_quant_launch_in_place(variant, q.x->const_data_ptr(), q.dtype, q.importance, gs_inv,
@@ -323,10 +332,11 @@ PyObject* quant_dynamic(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         QuantIn q;
         float fp8_max;
         int64_t padded_n;
+        int lower, upper;
         if (!quant_input(a[1], a[2], &q) || !as_float(a[3], &fp8_max) || !PyBool_Check(a[4]) || !int_or_none(a[5], q.n, &padded_n) ||
-            padded_n < q.n || padded_n % 16 || !PyLong_CheckExact(a[6]) || !PyLong_CheckExact(a[7]))
+            padded_n < q.n || padded_n % 16 || !window_int(a[6], &lower) || !window_int(a[7], &upper))
             return none();
-        const int variant = small_int(a[0]), lower = small_int(a[6]), upper = small_int(a[7]);
+        const int variant = small_int(a[0]);
         const bool tiled = a[4] == Py_True;
         const cudaStream_t s = current_stream(q.device);
         uint32_t* scratch = scratch_words(q.device, s);
@@ -348,7 +358,8 @@ PyObject* quant_dynamic(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
 PyObject* quant_dynamic_multi(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     return guarded([&]() -> PyObject* {
         float fp8_max;
-        if (nargs != 5 || !PyList_CheckExact(a[1]) || !as_float(a[2], &fp8_max) || !PyLong_CheckExact(a[3]) || !PyLong_CheckExact(a[4])) return none();
+        int lower, upper;
+        if (nargs != 5 || !PyList_CheckExact(a[1]) || !as_float(a[2], &fp8_max) || !window_int(a[3], &lower) || !window_int(a[4], &upper)) return none();
         const Py_ssize_t n = PyList_GET_SIZE(a[1]);
         constexpr Py_ssize_t kMost = 16;
         if (n < 1 || n > kMost) return none();
@@ -368,7 +379,7 @@ PyObject* quant_dynamic_multi(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
             items[i] = {q[i].x->const_data_ptr(), nullptr, static_cast<float*>(gs[i].mutable_data_ptr()), scratch + 2 * i,
                         static_cast<uint8_t*>(codes[i].mutable_data_ptr()), static_cast<uint8_t*>(scales[i].mutable_data_ptr()), q[i].m, q[i].n, q[i].n};
         }
-        const int variant = small_int(a[0]), lower = small_int(a[3]), upper = small_int(a[4]);
+        const int variant = small_int(a[0]);
         const int st = launch_on(dev, [&] {
             return nvfp4_quant_chain_multi_launch(variant, q[0].dtype, fp8_max, items, static_cast<int>(n), lower, upper, 1, s);
         });
@@ -676,7 +687,8 @@ PyObject* linear_multi(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     return guarded([&]() -> PyObject* {
         constexpr Py_ssize_t kMostActs = 16, kMost = 64;
         float fp8_max;
-        if (nargs != 9 || !PyList_CheckExact(a[1]) || !as_float(a[2], &fp8_max) || !PyLong_CheckExact(a[3]) || !PyLong_CheckExact(a[4])) return none();
+        int lower, upper;
+        if (nargs != 9 || !PyList_CheckExact(a[1]) || !as_float(a[2], &fp8_max) || !window_int(a[3], &lower) || !window_int(a[4], &upper)) return none();
         for (int i = 5; i < 9; ++i)
             if (!PyList_CheckExact(a[i]) || PyList_GET_SIZE(a[i]) != PyList_GET_SIZE(a[5])) return none();
         const Py_ssize_t acts = PyList_GET_SIZE(a[1]), count = PyList_GET_SIZE(a[5]);
@@ -717,7 +729,7 @@ PyObject* linear_multi(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         nvfp4_chain_item chain[kMostActs];
         for (Py_ssize_t i = 0; i < acts; ++i)
             chain[i] = {q[i].x->const_data_ptr(), nullptr, gs + 2 * i, scratch + 2 * i, base + at[i][0], base + at[i][1], q[i].m, q[i].n, q[i].n};
-        const int variant = small_int(a[0]), lower = small_int(a[3]), upper = small_int(a[4]);
+        const int variant = small_int(a[0]);
         const int st = launch_on(dev, [&] {
             const int c = nvfp4_quant_chain_multi_launch(variant, q[0].dtype, fp8_max, chain, static_cast<int>(acts), lower, upper, 1, s);
             return c != NVFP4_OK ? c : nvfp4_gemm_launch_multi(items, static_cast<int>(count), q[0].m, s);

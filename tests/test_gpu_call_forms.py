@@ -254,3 +254,17 @@ def test_channel_norms_of_one_strided_row(cuda_lib):
     assert torch.equal(H.channel_square_norm(x[:, ::2]), H.channel_square_norm(x[:, ::2].contiguous()))
     column = torch.randn((64, 4), device="cuda").bfloat16()
     assert torch.equal(H.channel_square_norm(column.t()[1:2]), column.float().square().t()[1:2])
+
+
+@pytest.mark.parametrize("lower", [-(1 << 70), (1 << 32) - 3])
+def test_window_bounds_beyond_an_int_go_the_way_of_ctypes(cuda_lib, lower):
+    """ctypes keeps the low 32 bits of an int argument: 0 and -3 here."""
+    import nvfp4quant_test_b200.kernels as K
+
+    x, imp = torch.randn((4, 64), device="cuda").bfloat16(), torch.rand((1, 64), device="cuda")
+    gs_inv = torch.ones(1, device="cuda")
+    same = 0 if lower < 0 else -3
+    for call in (lambda b: K.scalesweep_weighted_mse_nvfp4_quant_impl(x, imp, gs_inv, lower_bound=b, upper_bound=7),
+                 lambda b: K.scalesweep_nvfp4_quant_with_global_scale(x, 256.0, imp, lower_bound=b, upper_bound=7)):
+        for got, want in zip(call(lower), call(same)):
+            assert torch.equal(got.reshape(-1).view(torch.uint8), want.reshape(-1).view(torch.uint8))
