@@ -52,8 +52,8 @@ def nvfp4_scaled_mm(a: torch.Tensor, b: torch.Tensor, block_scale_a: torch.Tenso
             raise ValueError(f"{name} holds {have} bytes, the tiled layout for [{rows}, {k}] needs {_scale_bytes(rows, k)}")
     if out is None:
         out = torch.empty((m, n), dtype=torch.bfloat16, device=a.device)
-    elif out.shape != (m, n) or out.dtype != torch.bfloat16 or not out.is_contiguous():
-        raise ValueError("out must be a contiguous bfloat16 [M, N] tensor")
+    elif out.shape != (m, n) or out.dtype != torch.bfloat16 or not out.is_contiguous() or out.device != a.device:
+        raise ValueError("out must be a contiguous bfloat16 [M, N] tensor on a's device")
     if m == 0 or n == 0:
         return out
     L = _lib.lib()
@@ -131,6 +131,8 @@ def nvfp4_scaled_mm_prepared(a: torch.Tensor, block_scale_a: torch.Tensor, alpha
         raise ValueError(f"a and the weight disagree on K: {a.shape[1] * 2} vs {weight.k}")
     if alpha.dtype != torch.float32 or alpha.device != a.device:
         raise ValueError("alpha must be a float32 tensor on a's device")
+    if block_scale_a.device != a.device:
+        raise ValueError("block_scale_a must be on a's device")
     if not a.is_contiguous():
         a = a.contiguous()
     sfa = block_scale_a if block_scale_a.is_contiguous() else block_scale_a.contiguous()
@@ -139,8 +141,8 @@ def nvfp4_scaled_mm_prepared(a: torch.Tensor, block_scale_a: torch.Tensor, alpha
         raise ValueError("block_scale_a is smaller than the tiled layout of a needs")
     if out is None:
         out = torch.empty((m, weight.n), dtype=torch.bfloat16, device=a.device)
-    elif out.shape != (m, weight.n) or out.dtype != torch.bfloat16 or not out.is_contiguous():
-        raise ValueError("out must be a contiguous bfloat16 [M, N] tensor")
+    elif out.shape != (m, weight.n) or out.dtype != torch.bfloat16 or not out.is_contiguous() or out.device != a.device:
+        raise ValueError("out must be a contiguous bfloat16 [M, N] tensor on a's device")
     if m == 0:
         return out
     if not weight._handle:
@@ -183,6 +185,8 @@ def nvfp4_scaled_mm_grouped(a: torch.Tensor, block_scale_a: torch.Tensor, alpha_
         raise ValueError("a must be a uint8 [M, K/2] tensor on the weights' device")
     if a.shape[1] * 2 != k:
         raise ValueError(f"a and the weights disagree on K: {a.shape[1] * 2} vs {k}")
+    if block_scale_a.device != dev:
+        raise ValueError("block_scale_a must be on a's device")
     if not a.is_contiguous():
         a = a.contiguous()
     sfa = block_scale_a if block_scale_a.is_contiguous() else block_scale_a.contiguous()

@@ -98,6 +98,10 @@ class LinearGroup:
             raise ValueError(f"codes must be a contiguous uint8 [{self.tokens}, {self.k // 2}] tensor on {self.device}")
         if scales.numel() * scales.element_size() < self._min_scale_bytes or not scales.is_contiguous():
             raise ValueError("scales are smaller than the tiled layout of the activation needs")
+        if scales.device != self.device:
+            raise ValueError(f"scales must be on {self.device}")
+        if alpha_a is not None and (alpha_a.dtype != torch.float32 or alpha_a.device != self.device or alpha_a.numel() < 1):
+            raise ValueError(f"alpha_a must be a float32 tensor on {self.device}")
         with _lib.device_guard(self.device):
             st = _lib.lib().nvfp4_gemm_launch_grouped(self._handles, self._n, codes.data_ptr(), scales.data_ptr(),
                                                       None if alpha_a is None else alpha_a.data_ptr(), self._alphas,

@@ -268,3 +268,29 @@ def test_window_bounds_beyond_an_int_go_the_way_of_ctypes(cuda_lib, lower):
                  lambda b: K.scalesweep_nvfp4_quant_with_global_scale(x, 256.0, imp, lower_bound=b, upper_bound=7)):
         for got, want in zip(call(lower), call(same)):
             assert torch.equal(got.reshape(-1).view(torch.uint8), want.reshape(-1).view(torch.uint8))
+
+
+def test_products_refuse_operands_in_host_memory(cuda_lib):
+    """Every operand of every form: what is not on the weight's device is an error of the call, not of the GPU."""
+    import nvfp4quant_test_b200.kernels as K
+
+    x, w = (torch.randn((rows, 128), device="cuda").bfloat16() for rows in (4, 64))
+    (a, sa, ga, _), (b, sb, gb, _) = (K.scalesweep_nvfp4_quant_with_global_scale(t) for t in (x, w))
+    ga, gb, out = ga.reshape(1), gb.reshape(1), torch.empty((4, 64), dtype=torch.bfloat16, device="cuda")
+    weight = K.PreparedWeight(b, sb)
+    group, quantizer = K.LinearGroup([weight], [gb], 4), K.ActivationQuantizer(4, 128, "cuda")
+    forms = [(K.nvfp4_scaled_mm, [a, b, sa, sb, ga, torch.bfloat16, out]), (K.nvfp4_scaled_mm_prepared, [a, sa, ga, weight, out]),
+             (K.nvfp4_scaled_mm_grouped, [a, sa, ga, [weight], [gb], [out]]), (K.nvfp4_scaled_mm_multi, [[a], [sa], [ga], [weight], [gb]]),
+             (K.nvfp4_linear_multi, [[x], [0], [weight], [gb], [0]]), (group, [a, sa, ga]), (quantizer, [x])]
+    for call, args in forms:
+        for i, arg in enumerate(args):
+            if isinstance(arg, torch.Tensor):
+                moved = arg.cpu()
+            elif isinstance(arg, list) and isinstance(arg[0], torch.Tensor):
+                moved = [arg[0].cpu()]
+            else:
+                continue
+            with pytest.raises(ValueError):
+                call(*args[:i], moved, *args[i + 1:])
+        call(*args)
+    torch.cuda.synchronize()
