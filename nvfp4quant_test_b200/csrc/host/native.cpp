@@ -168,13 +168,15 @@ std::unordered_map<ScratchKey, std::list<std::pair<ScratchKey, Tensor>>::iterato
     return *m;
 }
 
-uint32_t* scratch_words(c10::DeviceIndex device, cudaStream_t stream) {
+// Undefined where the caller takes the Python path.  The caller keeps the tensor until its launch is queued: it gives up the
+// interpreter lock for that, and other threads may drop the block from the list meanwhile.
+Tensor scratch_words(c10::DeviceIndex device, cudaStream_t stream) {
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) {
         cudaGetLastError();   // e.g. the legacy stream while another stream captures: the Python path decides
-        return nullptr;
+        return Tensor();
     }
-    if (status != cudaStreamCaptureStatusNone) return nullptr;
+    if (status != cudaStreamCaptureStatusNone) return Tensor();
     auto& l = scratch_list();
     auto& m = scratch_map();
     const ScratchKey key{device, stream};
@@ -190,8 +192,9 @@ uint32_t* scratch_words(c10::DeviceIndex device, cudaStream_t stream) {
             l.pop_back();
         }
     }
-    return static_cast<uint32_t*>(l.front().second.mutable_data_ptr());
+    return l.front().second;
 }
+inline uint32_t* words_of(const Tensor& scratch) { return static_cast<uint32_t*>(scratch.mutable_data_ptr()); }
 
 // ---- quantizers -----------------------------------------------------------------------------------------------------
 
@@ -314,10 +317,10 @@ PyObject* global_scale(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
             out = *o;
         }
         const cudaStream_t s = current_stream(dev);
-        uint32_t* scratch = scratch_words(dev, s);
-        if (!scratch) return none();
+        const Tensor scratch = scratch_words(dev, s);
+        if (!scratch.defined()) return none();
         const int st = launch_on(dev, [&] {
-            return nvfp4_global_scale_launch(x->const_data_ptr(), dt, x->numel(), fp8_max, static_cast<float*>(out.mutable_data_ptr()), scratch, s);
+            return nvfp4_global_scale_launch(x->const_data_ptr(), dt, x->numel(), fp8_max, static_cast<float*>(out.mutable_data_ptr()), words_of(scratch), s);
         });
         return st == NVFP4_OK ? pack({scalar_view(out, 0), scalar_view(out, 1)}) : none();
     });
@@ -339,14 +342,14 @@ PyObject* quant_dynamic(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         const int variant = small_int(a[0]);
         const bool tiled = a[4] == Py_True;
         const cudaStream_t s = current_stream(q.device);
-        uint32_t* scratch = scratch_words(q.device, s);
-        if (!scratch) return none();
+        const Tensor scratch = scratch_words(q.device, s);
+        if (!scratch.defined()) return none();
         Tensor codes = empty({q.m, padded_n / 2}, at::kByte, q.device);
         Tensor scales = empty_scales(q.m, padded_n, tiled, q.device);
         Tensor gs = empty({2}, at::kFloat, q.device);
         const int st = launch_on(q.device, [&] {
             return nvfp4_quant_chain_launch(variant, q.x->const_data_ptr(), q.dtype, q.importance, fp8_max,
-                                            static_cast<float*>(gs.mutable_data_ptr()), scratch, static_cast<uint8_t*>(codes.mutable_data_ptr()),
+                                            static_cast<float*>(gs.mutable_data_ptr()), words_of(scratch), static_cast<uint8_t*>(codes.mutable_data_ptr()),
                                             static_cast<uint8_t*>(scales.mutable_data_ptr()), q.m, q.n, padded_n, lower, upper, tiled ? 1 : 0, s);
         });
         return st == NVFP4_OK ? pack({codes, scales, scalar_view(gs, 0), scalar_view(gs, 1)}) : none();
@@ -368,15 +371,15 @@ PyObject* quant_dynamic_multi(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
             if (!quant_input(PyList_GET_ITEM(a[1], i), Py_None, &q[i]) || q[i].device != q[0].device || q[i].dtype != q[0].dtype) return none();
         const c10::DeviceIndex dev = q[0].device;
         const cudaStream_t s = current_stream(dev);
-        uint32_t* scratch = scratch_words(dev, s);
-        if (!scratch) return none();
+        const Tensor scratch = scratch_words(dev, s);
+        if (!scratch.defined()) return none();
         nvfp4_chain_item items[kMost];
         Tensor codes[kMost], scales[kMost], gs[kMost];
         for (Py_ssize_t i = 0; i < n; ++i) {
             codes[i] = empty({q[i].m, q[i].n / 2}, at::kByte, dev);
             scales[i] = empty_scales(q[i].m, q[i].n, true, dev);
             gs[i] = empty({2}, at::kFloat, dev);
-            items[i] = {q[i].x->const_data_ptr(), nullptr, static_cast<float*>(gs[i].mutable_data_ptr()), scratch + 2 * i,
+            items[i] = {q[i].x->const_data_ptr(), nullptr, static_cast<float*>(gs[i].mutable_data_ptr()), words_of(scratch) + 2 * i,
                         static_cast<uint8_t*>(codes[i].mutable_data_ptr()), static_cast<uint8_t*>(scales[i].mutable_data_ptr()), q[i].m, q[i].n, q[i].n};
         }
         const int variant = small_int(a[0]);
@@ -705,8 +708,8 @@ PyObject* linear_multi(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         const int64_t gs_at = bytes;
         const c10::DeviceIndex dev = q[0].device;
         const cudaStream_t s = current_stream(dev);
-        uint32_t* scratch = scratch_words(dev, s);
-        if (!scratch) return none();
+        const Tensor scratch = scratch_words(dev, s);
+        if (!scratch.defined()) return none();
         nvfp4_gemm_item items[kMost];
         std::vector<Tensor> out(static_cast<size_t>(count));
         Tensor work = empty({gs_at + 256}, at::kByte, dev);
@@ -728,7 +731,7 @@ PyObject* linear_multi(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         }
         nvfp4_chain_item chain[kMostActs];
         for (Py_ssize_t i = 0; i < acts; ++i)
-            chain[i] = {q[i].x->const_data_ptr(), nullptr, gs + 2 * i, scratch + 2 * i, base + at[i][0], base + at[i][1], q[i].m, q[i].n, q[i].n};
+            chain[i] = {q[i].x->const_data_ptr(), nullptr, gs + 2 * i, words_of(scratch) + 2 * i, base + at[i][0], base + at[i][1], q[i].m, q[i].n, q[i].n};
         const int variant = small_int(a[0]);
         const int st = launch_on(dev, [&] {
             const int c = nvfp4_quant_chain_multi_launch(variant, q[0].dtype, fp8_max, chain, static_cast<int>(acts), lower, upper, 1, s);

@@ -294,3 +294,33 @@ def test_products_refuse_operands_in_host_memory(cuda_lib):
                 call(*args[:i], moved, *args[i + 1:])
         call(*args)
     torch.cuda.synchronize()
+
+
+def test_scratch_words_of_many_streams_and_threads(cuda_lib):
+    """More streams than scratch words are kept for, used by several threads at once."""
+    import threading
+
+    from nvfp4quant_test_b200 import helper as H
+
+    x = torch.randn((300, 8192), device="cuda").bfloat16()
+    xs = [x * (i + 1) for i in range(8)]
+    want = [H.get_nvfp4_global_scale(t)[0].item() for t in xs]
+    wrong = []
+
+    def work(i):
+        streams = [torch.cuda.Stream() for _ in range(6)]
+        for _ in range(30):
+            got = []
+            for s in streams:
+                with torch.cuda.stream(s):
+                    got.append(H.get_nvfp4_global_scale(xs[i])[0])
+            torch.cuda.synchronize()
+            wrong.extend(1 for g in got if g.item() != want[i])
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(8)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
