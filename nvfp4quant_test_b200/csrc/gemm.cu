@@ -134,6 +134,22 @@ static double tile_time(const TileCost& c, int64_t M, int64_t N, int64_t K, int 
     return t;
 }
 
+// tile_time with two corrections the fit does not see: with a long K the pair that shares its weight rows is ahead of what the model
+// says when those come from HBM (256 x 8192 x 8192, weights cold: 18.0 us against 21.1 with 128x128 or 256x192 tiles),
+// and 256x192 tiles, whose two accumulators overlap, lose less than 256x256 ones to the power cap over long launches
+// (8192 x 16384 x 4096 211 against 225 us, 20000 x 8192 x 8192 603 against 623).
+static double planned_time(const TileCost& c, int64_t M, int64_t N, int64_t K, int sms) {
+    const double t = tile_time(c, M, N, K, sms);
+    if (M <= 128) return t;
+    return c.path == 7 && (K + 255) / 256 >= 28 ? 0.9 * t : c.path == 4 ? 0.95 * t : t;
+}
+
+// A row's kernel was fastest at the row's M; how the tiles fill the waves at the launch's own M may favour another (600 x 7168 x 8192
+// takes the 1024-token row's 256x256 tiles in two waves, 25.2 us, and 128x256 ones in one, 16.1).  The model errs by less than this
+// on nearly every row of the table.  Over 165 shapes with random M between the rows: the row always 2.6 % behind the fastest kernel
+// on average and up to 56 %, the model always 1.3 % and 46 %, the row unless the model sees another this far ahead 0.6 % and 11 %.
+constexpr double kRowMargin = 1.1;
+
 // The decode-sized kernel, 33 to 128 tokens: it streams the weights whatever its K ranges, and its epilogue grows with the
 // token tile.
 static double skinny_time(int64_t M, int64_t N, int64_t K) {
@@ -150,13 +166,7 @@ static void plan_gemm(int64_t M, int64_t N, int64_t K, int sms, int k_splits, in
     double best_time = 0.0;
     for (const TileCost& c : kTileCosts) {
         if (c.pair && N <= 128) continue;
-        double t = tile_time(c, M, N, K, sms);
-        // Two corrections the fit does not see: with a long K the pair that shares its weight rows is ahead of what the model
-        // says when those come from HBM (256 x 8192 x 8192, weights cold: 18.0 us against 21.1 with 128x128 or 256x192 tiles),
-        // and 256x192 tiles, whose two accumulators overlap, lose less than 256x256 ones to the power cap over long launches
-        // (8192 x 16384 x 4096 211 against 225 us, 20000 x 8192 x 8192 603 against 623).
-        if (c.path == 7 && M > 128 && k_tiles_total >= 28) t *= 0.9;
-        if (c.path == 4 && M > 128) t *= 0.95;
+        const double t = planned_time(c, M, N, K, sms);
         if (best == 0 || t < best_time) {
             best = c.path;
             best_time = t;
@@ -183,7 +193,11 @@ static void plan_gemm(int64_t M, int64_t N, int64_t K, int sms, int k_splits, in
     }
     int path = g_gemm_force_path == 5 ? 0 : g_gemm_force_path;   // 0 = choose by shape
     // shapes of the measured table (on the GPU it was measured on) take the kernel that was fastest there
-    if (path == 0 && k_splits == 1 && sms == 148) path = table_path(M, N, K);
+    if (path == 0 && k_splits == 1 && sms == 148) {
+        path = table_path(M, N, K);
+        for (const TileCost& c : kTileCosts)
+            if (c.path == path && planned_time(c, M, N, K, sms) > kRowMargin * best_time) path = 0;
+    }
     if (path == 0) path = best;
     if (k_splits > 1 && path != 1 && path != 2 && path != 6) path = 1;
     *path_out = path;
