@@ -150,10 +150,19 @@ static double planned_time(const TileCost& c, int64_t M, int64_t N, int64_t K, i
 // on average and up to 56 %, the model always 1.3 % and 46 %, the row unless the model sees another this far ahead 0.6 % and 11 %.
 constexpr double kRowMargin = 1.1;
 
-// The decode-sized kernel, 33 to 128 tokens: it streams the weights whatever its K ranges, and its epilogue grows with the
+// The decode-sized kernel, 49 to 128 tokens: it streams the weights whatever its K ranges, and its epilogue grows with the
 // token tile.
 static double skinny_time(int64_t M, int64_t N, int64_t K) {
     return 4.1 + static_cast<double>(M + N) * static_cast<double>(K) * (9.0 / 16.0) / 5.4e6 + 0.03 * static_cast<double>(M);
+}
+
+// 33 to 48 tokens, where the decode-sized kernel's token tile has doubled to 64.  Up to about half as many weight tiles as SMs it
+// can cut K across a cluster, which pays the more stages there are for the tiles: 48 tokens, its time over the best tile kernel's,
+// 48 tiles 1.05 at K = 4096 and 0.94 at 6144, 32 tiles 1.23 at 2048 and 0.76 at 14336.  With more tiles it has one range and is a
+// plain stream of the weights: 112 tiles 1.13 at K = 2048, 0.94 at 4608, 1.08 at 8192, where the tile kernels' own streams are long
+// enough.  650 shapes: 0.5 % behind the fastest on average (by the model, and always from 64 tiles on: 2.1 %).
+static bool skinny_ahead(int n_tiles, int k_tiles) {
+    return n_tiles <= 72 ? 5 * k_tiles >= 2 * n_tiles : k_tiles >= 12 && k_tiles < 24;
 }
 
 // Kernel choice for one shape: host arithmetic only.  *path: 1 = 128x128 tiles, 2 = 128x256, 3 = pair 256x256,
@@ -173,13 +182,12 @@ static void plan_gemm(int64_t M, int64_t N, int64_t K, int sms, int k_splits, in
         }
     }
     // Decode-sized batches: weight rows on the MMA's 128 rows, tokens on its N dimension, K ranges across a cluster.  Up to 32
-    // tokens always; up to 48 where more than 64 weight tiles make it a plain stream, which the tile kernels sustain less well
-    // than the model says (45 x 27520 x 4352: 15.0 us against 17.3); up to 128 where the model puts it clearly ahead.
+    // tokens always; up to 48 by skinny_ahead; up to 128 where the model puts it clearly ahead.
     bool skinny = false;
     if (g_gemm_force_path == 5) {
         skinny = M <= kSkinnyMaxM;
     } else if (g_gemm_force_path == 0 && g_gemm_force_splits == 0 && M <= kSkinnyMaxM) {
-        skinny = M <= kSkinnyAutoM || (M <= 48 && n_tiles > 64) || skinny_time(M, N, K) < 0.95 * best_time;
+        skinny = M <= kSkinnyAutoM || (M <= 48 ? skinny_ahead(n_tiles, k_tiles_total) : skinny_time(M, N, K) < 0.95 * best_time);
     }
     if (skinny) {
         const int forced = g_gemm_force_path == 5 ? g_gemm_force_splits : 0;

@@ -33,3 +33,11 @@ def test_a_row_gives_way_where_its_kernel_needs_another_wave(plan, m, n, k, fast
 def test_rows_hold_at_their_own_sizes(plan):
     rows = [tuple(map(int, r)) for r in re.findall(r"^\{(\d+), (\d+), (\d+), (\d+)\}", TABLE.read_text(), re.M)]
     assert all(plan(m, n, k) in (path, 5) for m, n, k, path in rows)
+
+
+@pytest.mark.parametrize("m,tiles,k,decode", [(33, 48, 7168, True), (48, 48, 4096, False), (48, 56, 7168, True), (40, 64, 8192, True),
+                                              (48, 32, 2048, False), (48, 32, 14336, True), (48, 112, 2048, False), (48, 112, 4608, True),
+                                              (46, 112, 8192, False), (48, 148, 2048, False), (33, 224, 4096, True)])
+def test_decode_sized_kernel_at_33_to_48_tokens(plan, m, tiles, k, decode):
+    """Measured at least 1 % apart, in this order (33 x 224 tiles x 4096: 6 %; 48 x 32 x 2048: 23 %)."""
+    assert (plan(m, tiles * 128, k) == 5) == decode
