@@ -25,10 +25,9 @@ struct Cfg {
     // ring depth: as many stages as fit in shared memory (the bytes in flight per SM are what keeps HBM busy when
     // few CTAs stream a long K)
     static constexpr int kStages = (BN == 64) ? 7 : (BN == 128) ? 6 : 4;
-    // staged output pieces per epilogue warp; 0: the ring is worth more than they are (with 5 stages and two pieces 128 x 128
-    // tiles gain 7 % at K = 1088 and lose 5 % at K = 2880), so rows go out of the registers
-    static constexpr int kOutBufs = 0;
-    static constexpr int kEpilogueBytes = 4 * (kOutBufs > 0 ? kOutBufs * kPieceBytes : kTurnBytes);
+    // no staged output pieces: the ring is worth more than they are (with 5 stages and two pieces 128 x 128 tiles gain 7 % at
+    // K = 1088 and lose 5 % at K = 2880), so rows go out of the registers
+    static constexpr int kEpilogueBytes = 4 * kTurnBytes;
     static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*align*/ + 256 /*barriers*/ + kEpilogueBytes;
 
     // scale factors sit behind the accumulators, in two sets used by alternate K tiles so that the
@@ -233,7 +232,7 @@ __device__ __forceinline__ float load_alpha(const float* alpha, const float* alp
 // Operand maps and the work list of one launch over G products (G = 1: an ordinary GEMM, whose K may be cut into ranges).
 template <int G>
 struct TileParams {
-    CUtensorMap a[G], b[G], out[G];
+    CUtensorMap a[G], b[G];
     GroupTable<G> g;
     int M;
     int k_splits, k_tiles_per_split, k_rotate;   // G = 1 only, see GemmParams
@@ -503,7 +502,7 @@ gemm_kernel(const __grid_constant__ TileParams<G> p) {
                 if (lane == 0) mbar_arrive(tempty_bar(acc));
             };
             if (splits == 1) {
-                store_accumulator<BN, C::kOutBufs>(taddr, it.out, &p.out[cur.item], p.M, N, row0, nt * BN, alpha, epilogue_stage, out_turn, release);
+                store_accumulator<BN, 0>(taddr, it.out, nullptr, p.M, N, row0, nt * BN, alpha, epilogue_stage, out_turn, release);
             } else {
                 // fp32 partials of this K range; alpha and the bf16 rounding happen in the reduction kernel
 #pragma unroll 1
@@ -532,7 +531,6 @@ gemm_kernel(const __grid_constant__ TileParams<G> p) {
         }
     }
 
-    if (warp >= 2 && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     if (lane == 0) trace_mark(0, warp == 0 ? 3 : warp == 1 ? 4 : 5);
     // ---------------------------------------------------------------------- teardown
     if (*abort_flag) {
@@ -738,7 +736,6 @@ static int launch_list(const GemmParams* list, const WeightHandle* const* wh, in
     for (int i = 0; i < n; ++i) {
         const GemmParams& p = list[i];
         int st = make_operand_map(&q.a[i], p.a, p.M, p.K / 2, kBM);
-        if (st == NVFP4_OK) st = make_output_map(&q.out[i], p.out, p.M, p.N);
         if (wh[i]) {
             q.b[i] = *wh[i]->by_rows(BN);
         } else {
