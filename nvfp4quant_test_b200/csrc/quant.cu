@@ -19,9 +19,10 @@
 // candidates per trip whose FMA chains share one f32x2 instruction (each lane of
 // a packed instruction is an independent IEEE operation).
 //
-// Bodies 3 and 6 to 9 are the default loop over different grids: 3 and 9 number the slots of the real rows through (9 in
-// small CTAs, for a few tokens), 6 the warps of rows, 7 and 8 have a two-dimensional grid, a row's chunks by a row's CTAs (8 for
-// tensors without any padding in rows of whole chunks, without predicates).  (5 is another name of 3.)
+// Bodies 3 and 5 to 9 are the default loop over different grids: 3, 5 and 9 number the slots of the real rows through (5 in
+// CTAs of 256 threads with the loop rolled, for large ragged unweighted 16-bit tensors; 9 in small CTAs, for a few tokens), 6 the
+// warps of rows, 7 and 8 have a two-dimensional grid, a row's chunks by a row's CTAs (8 for rows of whole chunks: sweeps of tensors
+// without any padding, without predicates, and amax).
 //
 // Body 4 is the default loop with the tensor-wide global scale (helper.py:96-100: amax / (6 * fp8_max) and its reciprocal)
 // computed inside the same launch: every thread keeps its block in registers, the CTAs combine their maxima
@@ -57,6 +58,9 @@ constexpr int kSmallThreads = 64;
 constexpr int64_t kSmallBlocks = 24576;
 constexpr int64_t kSmallBlocksRagged = 98304;
 constexpr int64_t kSmallBlocksRaggedWeighted = 327680;
+// Real blocks from which body 5 takes the place of 3 (unweighted, 16-bit), us bodies 3 / 5: 300000 blocks, 2325 x 2064 10.69 / 10.94;
+// 400000, 1111 x 5760 13.76 / 13.50; 1500000, 7575 x 3168 45.99 / 44.97; 3700000, 8191 x 7216 110.1 / 107.5.  fp32 gains nothing.
+constexpr int64_t kLargeBlocksRagged = 393216;
 __host__ __device__ constexpr int block_threads(int variant, int impl) {
     return impl == 9 ? kSmallThreads : (variant != NVFP4_VARIANT_AMAX && (impl == 3 || impl == 6 || impl == 7 || impl == 8 || impl == 10)) ? kSweepThreads : kThreads;
 }
@@ -450,8 +454,9 @@ quant_kernel(const __grid_constant__ Args args) {
     // the division below, the row part of the addresses and most of the tiled scale offset leave the per-thread
     // instruction stream (8192 x 8192 sweep: 126 us numbered through, 112 us with this grid).
     constexpr bool GRID2D = IMPL == 7 || IMPL == 8;
-    constexpr bool WHOLE = IMPL == 8;
-    constexpr bool FLAT = IMPL == 3 || IMPL == 9 || IMPL == 10;   // real rows' slots numbered through, then CTAs that fill the padding rows
+    constexpr bool WHOLE = IMPL == 8 && VARIANT != NVFP4_VARIANT_AMAX;
+    constexpr bool CHUNKS = IMPL == 8;   // rows of whole chunks: every column is in range
+    constexpr bool FLAT = IMPL == 3 || IMPL == 5 || IMPL == 9 || IMPL == 10;   // real rows' slots numbered through, then CTAs that fill the padding rows
     const int64_t id = GRID2D ? 0 : static_cast<int64_t>(bx) * T + threadIdx.x;
     const int64_t slots = FLAT ? p.m * p.width : p.total;
     constexpr bool WARPS = IMPL == 6;               // a row's columns by whole warps, numbered through the rows
@@ -462,7 +467,7 @@ quant_kernel(const __grid_constant__ Args args) {
     if (GRID2D) {
         row = bx;
         col = static_cast<int64_t>(blockIdx.y) * T + threadIdx.x;
-        if (!WHOLE) in_range = col < p.width;
+        if (!CHUNKS) in_range = col < p.width;
     } else if (WARPS) {
         const uint32_t w = bx * (T / 32) + __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
         const uint32_t r32 = row_div(p, w);
@@ -596,8 +601,11 @@ quant_kernel(const __grid_constant__ Args args) {
     uint32_t sbyte = 0;
     float inv = 0.0f;
     // A warp with nothing but padding columns or threads behind the last slot has nothing to sweep.  (Body 6 has next to none of
-    // these and is 0.5 % faster without the vote, the weighted body 3 up to 3 %; the unweighted one is slower without it.)
-    constexpr bool VOTE = IMPL == 7 || (FLAT && !(IMPL == 3 && VARIANT == NVFP4_VARIANT_WEIGHTED));
+    // these and is 0.5 % faster without the vote, the weighted body 3 up to 3 %, body 5 2.5 %; the unweighted body 3 is slower without
+    // it.)  Amax has little to skip: 16-bit 7575 x 3168 13.1 us with the vote, 11.9 without; fp32, whose warps wait for twice the
+    // bytes, 17.6 and 18.3.
+    constexpr bool VOTE = VARIANT == NVFP4_VARIANT_AMAX ? FLAT && DT == NVFP4_DT_F32
+                                                        : IMPL == 7 || (FLAT && IMPL != 5 && !(IMPL == 3 && VARIANT == NVFP4_VARIANT_WEIGHTED));
     if (VOTE && !__any_sync(0xffffffffu, valid)) {
         // nothing
     } else if (VARIANT == NVFP4_VARIANT_AMAX) {
@@ -622,7 +630,7 @@ quant_kernel(const __grid_constant__ Args args) {
         sbyte = (IMPL == 1)   ? sweep_scalar<W>(v, w, first_idx, p.ncand, tab)
                 : (IMPL == 2) ? sweep_single<W>(v, w, first_idx, p.ncand, tab)
                 // the reference's own windows (11 candidates unweighted, 16 weighted) are compiled in, unrolled
-                : (WHOLE || ((IMPL == 7 || FLAT || WARPS) && p.ncand == (W ? 16 : 11)))
+                : (WHOLE || ((IMPL == 7 || (FLAT && IMPL != 5) || WARPS) && p.ncand == (W ? 16 : 11)))
                     ? sweep_paired<W, W ? 16 : 11>(v, w, first_idx, p.ncand, tab)
                     : sweep_paired<W>(v, w, first_idx, p.ncand, tab);
         // sbyte is 0 only when no candidate had a comparable (non-NaN, < inf) error: 1/0 as the reference computes it
@@ -678,15 +686,16 @@ cudaError_t launch_flat(const QuantParams& p, cudaStream_t stream) {
 // per thread, a row by whole warps (6) or by whole CTAs (7) leaves the last one partly idle; 7 divides nothing, 6 once per warp.
 // By the idle part; us, bodies 3 / 6 / 7, bf16, 1500000 blocks: unweighted, rows of 498 45.6 / 44.4 / 43.9, 575 45.5 / 43.3 /
 // 44.0, 643 45.5 / 45.0 / 45.7, 90 46.5 / 45.9 / 47.7 (not tiled,
-// where the address is cheap, 44.2 / 45.0 / 46.3); weighted, 498 73.9 / 73.7 / 73.2, 643 73.8 / 74.7 / 75.3; amax, 498 13.1 /
-// 11.6 / 11.1, 575 13.2 / 11.5 / 12.1, 85 13.2 / 12.4 / 19.8, 198 13.2 / 12.4 / 12.3, 65 13.3 / 14.8 / 25.3.
-int ragged_body(int variant, int64_t width, bool tiled, int T) {
+// where the address is cheap, 44.2 / 45.0 / 46.3); weighted, 498 73.9 / 73.7 / 73.2, 643 73.8 / 74.7 / 75.3; amax, 200000 blocks, rows of 200
+// 2.95 / 2.82 / 2.69, 564 3.07 / 2.88 / 2.62, 1500000, 200 11.9 / 12.2 / 12.1, 320 11.8 / 11.3 / 13.4, 716 11.7 / 11.4 / 11.2, 4000000, 836
+// 30.5 / 29.4 / 31.0, 500 29.7 / 29.4 / 28.9.  Fp32 amax is bound by its loads: the grid without an idle thread is ahead (4000000, 836
+// 43.3 / 43.8 / 46.3) but for a short launch, which its division delays (60000, 512 2.88 / 2.50 / 2.93, 716 3.33 / 3.14 / 3.33).
+int ragged_body(int variant, bool fp32, int64_t blocks, int64_t width, bool tiled, int T) {
     const int64_t idle_warp = (width + 31) / 32 * 32 - width, idle_cta = (width + T - 1) / T * T - width;
-    if (variant == NVFP4_VARIANT_AMAX) {
-        if (idle_cta * 4 <= width) return 7;
-        return idle_warp * 7 <= width ? 6 : idle_cta * 2 <= width ? 7 : 3;
-    }
-    if (idle_warp * (variant == NVFP4_VARIANT_WEIGHTED ? 32 : tiled ? 15 : 20) > width) return 3;
+    if (variant == NVFP4_VARIANT_AMAX && fp32) return blocks >= 131072 ? 3 : 6;
+    if (variant == NVFP4_VARIANT_AMAX)
+        return idle_cta * (blocks < 524288 ? 2 : 8) <= width ? 7 : idle_warp * 10 <= width ? 6 : 3;
+    if (idle_warp * (variant == NVFP4_VARIANT_WEIGHTED ? 32 : tiled ? 17 : 20) > width) return 3;
     return idle_cta == idle_warp ? 7 : 6;
 }
 template <int DT, int VARIANT>
@@ -700,10 +709,13 @@ cudaError_t launch_impl(int impl, const QuantParams& p, cudaStream_t stream) {
     }
     const bool chunks = p.width % T == 0;
     int body = impl;
-    if (impl == 0 || impl == 8) body = chunks ? 7 : ragged_body(VARIANT, p.width, p.swizzled != 0, T);
+    const int64_t blocks = p.m * p.bout;
+    constexpr bool kFp32 = DT == NVFP4_DT_F32;
+    if (impl == 0 || impl == 8) body = chunks && !(!kSweep && kFp32 && blocks >= 131072) ? 7 : ragged_body(VARIANT, kFp32, blocks, p.width, p.swizzled != 0, T);
     if (impl == 0 && kSweep) {
         const int64_t small = chunks ? kSmallBlocks : VARIANT == NVFP4_VARIANT_WEIGHTED && body == 3 ? kSmallBlocksRaggedWeighted : kSmallBlocksRagged;
-        if (p.m * p.bout <= small) body = 9;
+        if (blocks <= small) body = 9;
+        if (body == 3 && VARIANT == NVFP4_VARIANT_MSE && !kFp32 && blocks >= kLargeBlocksRagged) body = 5;
     }
     if (body == 7 && ((p.width + T - 1) / T > 65535 || p.rows > 0x7fffffffLL)) body = 3;
     if (body == 6 && p.m * ((p.width + 31) / 32) > 0x7fffffffLL) body = 3;
@@ -717,10 +729,14 @@ cudaError_t launch_impl(int impl, const QuantParams& p, cudaStream_t stream) {
         const dim3 grid2(static_cast<unsigned>(p.rows), static_cast<unsigned>((p.width + T - 1) / T));
         // no padding anywhere: every slot of the scale layout is a real block
         const bool whole = chunks && p.rows == p.m && p.bin == p.bout && p.bout == p.width && p.ncand == (VARIANT == NVFP4_VARIANT_MSE ? 11 : 16);
+        if constexpr (!kSweep)
+            if (chunks && impl != 7) return launch_dependent(quant_kernel<DT, VARIANT, 8, QuantParams>, grid2, dim3(T), 0, stream, p);
         if constexpr (kSweep)
             if (whole && impl != 7) return launch_dependent(quant_kernel<DT, VARIANT, 8, QuantParams>, grid2, dim3(T), 0, stream, p);
         return launch_dependent(quant_kernel<DT, VARIANT, 7, QuantParams>, grid2, dim3(T), 0, stream, p);
     }
+    if constexpr (VARIANT == NVFP4_VARIANT_MSE && !kFp32)
+        if (body == 5) return launch_flat<DT, VARIANT, 5>(p, stream);
     return launch_flat<DT, VARIANT, 3>(p, stream);
 }
 

@@ -324,3 +324,44 @@ def test_scratch_words_of_many_streams_and_threads(cuda_lib):
     for t in threads:
         t.join()
     assert not wrong
+
+
+@pytest.mark.parametrize("m,n,padded_n,tiled", [(129, 16, None, True), (3, 112, 176, True), (300, 48, None, False), (77, 4096, None, True), (130, 4096, 8192, True),
+                                                (129, 8192, None, False), (401, 7216, 7232, True)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_quantizer_bodies_by_size_equal_the_plain_ones(cuda_lib, m, n, padded_n, tiled, dtype):
+    """Slots in large CTAs with the loop rolled (5), warps of rows (6), amax on rows of whole chunks (8): padding rows, padding columns,
+    rows longer and shorter than a CTA."""
+    from nvfp4quant_test_b200 import _lib
+
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    x = torch.randn((m, n), generator=g, device="cuda").to(dtype)
+    gs_inv, p = torch.tensor([37.5], device="cuda"), padded_n or n
+    size = (m + 127) // 128 * 128 * ((p // 16 + 3) // 4 * 4) if tiled else m * p // 16
+    for variant, lower, upper, plain, bodies in ((0, -3, 7, 1, (5, 6)), (0, -2, 5, 1, (5, 6)), (2, 0, 0, 3, (5, 6, 7, 8))):
+        want = None
+        for impl in (plain, *bodies):
+            codes, scales = (torch.full(s, 0xA5, dtype=torch.uint8, device="cuda") for s in ((m, p // 2), (size,)))
+            _lib.check(cuda_lib.nvfp4_quant_launch_impl(impl, variant, x.data_ptr(), _lib.dtype_code(dtype), None, gs_inv.data_ptr(), codes.data_ptr(),
+                                                        scales.data_ptr(), m, n, p, lower, upper, int(tiled), None), "launch")
+            torch.cuda.synchronize()
+            want = want or (codes, scales)
+            assert torch.equal(codes, want[0]) and torch.equal(scales, want[1]), (impl, variant, lower)
+
+
+@pytest.mark.parametrize("variant,dtype,blocks", [(0, torch.bfloat16, 393216), (0, torch.float16, 393216), (2, torch.float32, 131072), (2, torch.bfloat16, 524288)])
+def test_quantizer_choice_by_size_equals_the_plain_body(cuda_lib, variant, dtype, blocks):
+    """Either side of the sizes at which the default changes: whole chunks and three kinds of ragged rows."""
+    import nvfp4quant_test_b200.kernels as K
+    from nvfp4quant_test_b200 import _lib
+
+    gs_inv = torch.tensor([37.5], device="cuda")
+    call = K.amax_nvfp4_quant_impl if variant == 2 else K.scalesweep_mse_nvfp4_quant_impl
+    for n in (4096, 4176, 7216, 13328):
+        for m in (blocks * 16 // n, -(-blocks * 16 // n)):
+            x = torch.randn((m, n), device="cuda").to(dtype)
+            got = call(x, gs_inv)
+            codes, scales = torch.empty_like(got[0]), torch.empty_like(got[1])
+            _lib.check(cuda_lib.nvfp4_quant_launch_impl(1 if variant == 0 else 3, variant, x.data_ptr(), _lib.dtype_code(dtype), None, gs_inv.data_ptr(),
+                                                        codes.data_ptr(), scales.data_ptr(), m, n, n, -3, 7, 1, None), "launch")
+            assert torch.equal(codes, got[0]) and torch.equal(scales.view(torch.uint8), got[1].view(torch.uint8)), (n, m)
