@@ -60,11 +60,6 @@ except ImportError:     # not built yet: lib() says so when something is to be l
     pass
 
 
-def compiling() -> bool:
-    """Inside torch.compile or torch.export: the functions that are plain torch off the GPU stay plain torch there."""
-    return torch.compiler.is_compiling()
-
-
 class Nvfp4Error(RuntimeError):
     """A launch was rejected or failed; `.status` holds the C ABI status code."""
 

@@ -7,6 +7,7 @@ tensors and as plain torch elsewhere; the error metrics are plain torch.
 from __future__ import annotations
 
 import torch
+from torch.compiler import is_compiling
 
 from . import _lib
 
@@ -92,7 +93,7 @@ _E2M1 = (0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0)
 def unpack_fp4_e2m1(packed: torch.Tensor) -> torch.Tensor:
     """uint8 [m, k/2] -> float32 [m, k]; low nibble first."""
     assert packed.dtype == torch.uint8
-    got = None if _lib.compiling() else _lib.fast.dequant(packed, None, None)
+    got = None if is_compiling() else _lib.fast.dequant(packed, None, None)   # torch.compile and torch.export see plain torch
     if got is not None:
         return got
     lut = torch.tensor(_E2M1 + tuple(-v for v in _E2M1), dtype=torch.float32, device=packed.device)
@@ -102,7 +103,7 @@ def unpack_fp4_e2m1(packed: torch.Tensor) -> torch.Tensor:
 
 def dequantize_base(q, scale_fp8, global_scale):
     """q uint8 [m, k/2], scale_fp8 float8_e4m3fn [m, k/16] (row-major, i.e. already unswizzled)."""
-    got = None if scale_fp8 is None or _lib.compiling() else _lib.fast.dequant(q, scale_fp8, global_scale)
+    got = None if scale_fp8 is None or is_compiling() else _lib.fast.dequant(q, scale_fp8, global_scale)
     if got is not None:
         return got
     scales = scale_fp8.to(torch.float32).repeat_interleave(16, dim=1)

@@ -15,6 +15,7 @@ torch, on any device.
 from __future__ import annotations
 
 import torch
+from torch.compiler import is_compiling
 
 from .. import _lib
 
@@ -35,7 +36,7 @@ def swizzle_vllm_fp4_scale(scale: torch.Tensor, m: int, n: int, block_size: int 
     assert n % block_size == 0
     k = n // block_size
     assert tuple(scale.shape) == (m, k)
-    got = None if _lib.compiling() else _lib.fast.scale_layout(scale, m, k, True)
+    got = None if is_compiling() else _lib.fast.scale_layout(scale, m, k, True)   # torch.compile and torch.export see plain torch
     if got is not None:
         return got
     m_pad, k_pad = round_up(m, 128), round_up(k, 4)
@@ -50,7 +51,7 @@ def unswizzle_vllm_fp4_scale(scale_swizzled: torch.Tensor, m: int, n: int, block
     """Flat (or [m_pad, k_pad]-shaped) tiled buffer -> [m, n/block_size] row-major scales."""
     assert n % block_size == 0
     k = n // block_size
-    got = None if _lib.compiling() else _lib.fast.scale_layout(scale_swizzled, m, k, False)
+    got = None if is_compiling() else _lib.fast.scale_layout(scale_swizzled, m, k, False)
     if got is not None:
         return got
     m_pad, k_pad = round_up(m, 128), round_up(k, 4)
