@@ -78,20 +78,20 @@ int nvfp4_quant_launch_in_place(int variant, const void* x, int x_dtype, const f
                                 uint8_t* codes, uint8_t* scales, int64_t m, int64_t n, int64_t padded_n, int lower, int upper,
                                 int swizzled, void* stream);
 
-/* Same as nvfp4_quant_launch, choosing the kernel body: 0 = default (9 for tensors of a few tokens, see there; else 5 when a quarter or more
- * of the scale layout's rows are padding, else 8 / 7 / 6 where they apply, else 3), 1 = scalar (one candidate at a time, the plainest transcription), 2 = one candidate per trip with
- * packed multiplies and the mixed-precision subtract, 3 = two candidates per trip sharing one f32x2 FMA chain,
- * 5 = 3 with warps that hold only padding rows skipping the sweep, 6 = 3 on a two-dimensional grid (row =
- * blockIdx.x, uniform over the CTA; taken by default when the row is a whole number of 256-block chunks wide,
- * otherwise 6 means 3), 7 = 6 with the reference's candidate count (11 unweighted, 16 weighted) compiled in and
- * the sweep unrolled (default for the unweighted sweep with the reference's window; other windows make it 6),
- * 8 = 7 without any validity predicate, for tensors in which every slot of the scale layout is a real block (m a
- * multiple of 128 in the tiled layout, padded_n == n, rows a whole number of 256-block chunks wide, the reference's
- * window); the default there, elsewhere 8 means the default; 9 = 3 in CTAs of 64 threads over the real rows' slots,
- * which spreads a tensor of a few tokens over four times as many SMs, plus a few CTAs that zero the padding rows of the
- * tiled scale layout (the default up to 32768 real blocks, e.g. 64 tokens x 8192; 24576 for the weighted sweep).
- * 4 is the fused form, which has its own entry point below.  All give identical bytes; exposed for testing and
- * timing. */
+/* Same as nvfp4_quant_launch, choosing the kernel body.  All give identical bytes; exposed for testing and timing.
+ *   0  the default: chosen by size, type and row width (launch_impl in csrc/quant.cu says where the lines lie and why)
+ *   1  scalar, one candidate at a time: the plainest transcription
+ *   2  one candidate per trip with packed multiplies and the mixed-precision subtract
+ *   3  two candidates per trip sharing one f32x2 FMA chain; the real rows' slots numbered through the CTAs, further CTAs write the
+ *      zero words of the padding rows
+ *   5  3 in CTAs of 256 threads with the loop rolled (unweighted 16-bit input; elsewhere 3)
+ *   6  3 with whole warps per row, numbered through the rows
+ *   7  3 on a two-dimensional grid: row = blockIdx.x, chunk of 128 blocks (amax: 256) = blockIdx.y
+ *   8  rows of whole chunks: 7 without predicates for sweeps of tensors without any padding in the reference's window, 7 without a
+ *      range check for amax; elsewhere the default's choice among 3, 6 and 7
+ *   9  3 in CTAs of 64 threads (the sweeps' default up to 24576 real blocks, 98304 on ragged rows, weighted 327680 where 3 is
+ *      the alternative)
+ * 4 is the fused form, which has its own entry point below; 10, the form that takes its global scale itself, is part of the chain. */
 int nvfp4_quant_launch_impl(int impl, int variant, const void* x, int x_dtype, const float* importance,
                             const float* gs_inv, uint8_t* codes, uint8_t* scales, int64_t m, int64_t n,
                             int64_t padded_n, int lower, int upper, int swizzled, void* stream);
@@ -223,8 +223,8 @@ int nvfp4_gemm_release(void* handle);
 /*
  * Several products of equal M in one call, each with its own activation, prepared weight (any K), scales and output:
  *   out_bf16[M, N] = alpha_w[0] * alpha_a[0] * dq(a) dq(weight)^T      (alpha_a may be NULL: factor 1)
- * for the matrices of a layer whose inputs are all at hand.  Up to 8 of them become one launch of a tile kernel; at
- * decode-sized M those that share an activation become one grouped launch (below).  n_items <= 64.  Each output has the
+ * for the matrices of a layer whose inputs are all at hand.  Up to 8 of them become one launch: of the decode-sized kernel up to 32
+ * tokens (64 where all have the same K), of a tile or pair kernel beyond.  n_items <= 64.  Each output has the
  * bits of nvfp4_gemm_launch_prepared, up to the order of the fp32 sums at decode-sized M.  No counterpart in the reference.
  */
 typedef struct {
@@ -247,7 +247,7 @@ int nvfp4_gemm_launch_multi(const nvfp4_gemm_item* items_host, int n_items, int6
  * separate fp32 multiplication, without that extra launch.  handles / alpha_w / outs_bf16 are HOST arrays read during the call.
  * Up to 64 tokens (and wherever the kernel choice takes the decode-sized kernel for the group's total N), up to 8 weights
  * go out as ONE launch whose weight tiles are numbered through the group (fixed costs paid once, every SM on the
- * combined weight stream); otherwise one launch per weight.  Outputs agree with the one-by-one calls to fp32 rounding before the bf16 store (bit for bit when
+ * combined weight stream); beyond, up to 8 weights are one launch of a tile or pair kernel over the list.  Outputs agree with the one-by-one calls to fp32 rounding before the bf16 store (bit for bit when
  * the K ranges per tile agree; they are chosen from the group's total tile count).  No workspace.
  */
 int nvfp4_gemm_launch_grouped(void* const* handles, int n_weights, const uint8_t* a, const uint8_t* sfa,

@@ -56,7 +56,6 @@ extern "C" size_t nvfp4_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K) {
     return splits > 1 ? static_cast<size_t>(splits) * static_cast<size_t>(M) * static_cast<size_t>(N) * sizeof(float) : 0;
 }
 
-// Testing hook: K ranges (0 = by shape) and K-loop rotation (-1 = by shape, 0 = off, 1 = on) of the single-CTA kernel.
 // Testing hook: m-tiles per band of the tile numbering (0 = default).
 extern "C" int nvfp4_gemm_tune_raster(int group) {
     if (group < 0 || group > 4096) return NVFP4_ERR_BAD_ENUM;
@@ -71,6 +70,7 @@ extern "C" int nvfp4_gemm_tune_pdl(int enabled) {
     return NVFP4_OK;
 }
 
+// Testing hook: K ranges (0 = by shape) and K-loop rotation (-1 = by shape, 0 = off, 1 = on) of the single-CTA kernel.
 extern "C" int nvfp4_gemm_tune(int k_splits, int k_rotate) {
     if (k_splits < 0 || k_splits > 16 || k_rotate < -1 || k_rotate > 1) return NVFP4_ERR_BAD_ENUM;
     g_gemm_force_splits = k_splits;

@@ -1,4 +1,4 @@
-// CTA-pair kernels of the NVFP4 GEMM (cta_group::2, 256 x 192 / 256 x 256 output tiles).
+// CTA-pair kernels of the NVFP4 GEMM (cta_group::2, 256 x 128 / 256 x 192 / 256 x 256 output tiles).
 #pragma once
 
 #include "gemm_tile.cuh"

@@ -157,7 +157,7 @@ skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant_
     }
     const int k_tiles = (K + kBK - 1) / kBK;
     const int kt_begin = static_cast<int>(rank) * p.w[gi].k_tiles_per_rank;
-    // never 0, but for a CTA of a weight's last cluster behind its last tile: that one streams nothing, takes part in the
+    // never 0 (the launcher leaves no K range empty), but for a CTA of a weight's last cluster behind its last tile: that one streams nothing, takes part in the
     // barriers and stores nothing (its rows lie beyond N)
     const int kcount = G == 1 || nt * 128 < N ? max(0, min(k_tiles, kt_begin + p.w[gi].k_tiles_per_rank) - kt_begin) : 0;
 

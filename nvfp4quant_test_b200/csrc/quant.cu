@@ -40,8 +40,9 @@ namespace {
 constexpr int kThreads = 256;
 // The sweeps' bodies 3, 7 and 8 run in CTAs of 128 threads with up to 72 registers (7 CTAs, 28 warps per SM).  A large
 // sweep takes the same time with anything from 20 to 48 warps per SM (8192 x 8192, us, unweighted / weighted: 256 threads
-// at 40 registers 110.4 / 237, at 64 114.4 / 191; 128 threads at 96 registers 110.7 / 193, at 72 110.5 / 190.5): operand
-// reads from the register file bound it, not latency.  Below a few hundred tokens latency does, and there more registers
+// at 40 registers 110.4 / 237, at 64 114.4 / 191; 128 threads at 96 registers 110.7 / 193, at 72 110.5 / 190.5): instruction
+// issue (79 % of the active cycles unweighted, 73 % weighted) and the FMA and ALU pipes (61 and 63 %, 72 and 48 %) bound it together,
+// not latency.  Below a few hundred tokens latency does, and there more registers
 // (independent work in flight per warp) and smaller CTAs (an even spread over the SMs) decide: 256 x 8192 7.2 -> 4.9 us
 // unweighted and 9.1 -> 7.9 weighted against 256 threads at 40 and 64 registers, 128 x 8192 5.4 -> 3.3 and 7.0 -> 5.1.
 constexpr int kSweepThreads = 128;
@@ -84,7 +85,7 @@ struct QuantParams {
     int64_t width, rows;    // slot grid: scale columns / rows that get written
     int64_t k_pad;          // padded scale columns (swizzled layout)
     int64_t total;          // rows * width
-    uint32_t div_mul, div_shift;  // division by width: see width_div
+    uint32_t div_mul, div_shift;  // division by width: see set_row_div
     int lower, ncand;
     int swizzled;
     int early;              // != 0: kernels behind this one may be scheduled while it runs (see the kernel's first lines)
@@ -94,9 +95,9 @@ struct QuantParams {
     uint32_t* fused_scratch;  // [4]: running maximum, arrivals, readers, unused; zero between calls
 };
 
-// n / d for n < 2^31, as (n * ceil(2^(32 + shift) / d)) >> (32 + shift) with 2^shift < d <= 2^(shift + 1): the
-// rounding of the multiplier adds less than n * d / 2^(32 + shift) < 1 / d to the quotient's fraction.  d: the width, or the
-// warps of a row (body 6).
+// n / d for n < 2^31, as (n * ceil(2^(32 + shift) / d)) >> (32 + shift) with 2^shift < d <= 2^(shift + 1): the rounding of the
+// multiplier is e / d with e < d and adds n * e / (d * 2^(32 + shift)) < n / 2^(32 + shift) to the quotient, less than the 1 / d that
+// its fraction is at least away from the next integer because n * e < 2^31 * 2^(shift + 1).  d: the width, or the warps of a row (body 6).
 inline void set_row_div(QuantParams& p, int64_t d) {
     p.div_mul = p.div_shift = 0;
     if (d <= 1 || d > 0x7fffffffLL) return;

@@ -25,9 +25,10 @@ extern "C" const char* nvfp4_status_string(int status) {
     return "unknown status";
 }
 
-// 2: grouped GEMM launch, one-call quantizer chain, strided importance reduction, capture id (additions only: every
-// version-1 entry point keeps its signature and meaning)
-extern "C" int nvfp4_abi_version(void) { return 3; }
+// 2: grouped GEMM launch, one-call quantizer chain, strided importance reduction, capture id; 3: chains and products of several
+// tensors, dequantization and scale layouts; 4: nvfp4_quant_launch_in_place (additions only: every version-1 entry point keeps its
+// signature and meaning)
+extern "C" int nvfp4_abi_version(void) { return 4; }
 
 // 0 while `stream` is not being captured into a CUDA graph, else the id of the capture (unique per capture sequence of the
 // process).  Host bookkeeping only: callers that hand out scratch buffers per stream use it to tell captures apart, because

@@ -2,8 +2,8 @@
 
 `nvfp4_scaled_mm_grouped` and the quantizer entry points allocate their outputs, check their arguments and build
 their argument arrays on every call; that is tens of microseconds of Python per call, several times what the GPU
-needs for a decode-sized launch.  The two classes here do that work once: buffers are allocated and arguments are
-checked at construction, a call is one C ABI call.  Outputs are reused from call to call (copy what must be kept), and
+needs for a decode-sized launch.  The classes here do that work once: buffers are allocated and arguments are
+checked at construction, a call is one call into the library.  Outputs are reused from call to call (copy what must be kept), and
 an instance serves one stream at a time.  Bits equal the allocating entry points'.
 """
 from __future__ import annotations
@@ -22,7 +22,8 @@ from .kernel_vllm import create_fp4_output_tensors
 
 class ActivationQuantizer:
     """global scale -> ScaleSweep_MSE quantization of an activation [tokens, k] with one host call
-    (nvfp4_quant_chain_launch: two kernels, the second a programmatic dependent launch of the first)."""
+    (nvfp4_quant_chain_launch: two dependent launches, one up to 128 KiB).  Its buffers are an activation's: a PreparedWeight on
+    them would be read while a later call rewrites them."""
 
     def __init__(self, tokens: int, k: int, device, fp8_max: float = _helper.FP8_E4M3_MAX_4OVER6,
                  dtype: torch.dtype = torch.bfloat16):

@@ -100,7 +100,7 @@ def prepare_layer(qlayer: dict) -> dict:
 # matrices that read the same activation in a decoder layer (q / k / v the normed hidden state, gate / up the normed
 # post-attention state); o and down have inputs of their own
 WEIGHT_GROUPS = (("q", "k", "v"), ("o",), ("gate", "up"), ("down",))
-GROUPED_MAX_TOKENS = 64    # beyond, the per-matrix kernels on forked streams are faster (96 tokens: 1.95 against 2.05 ms)
+GROUPED_MAX_TOKENS = 64    # up to this many tokens `run` goes through DecodeLayer, beyond through layer_gemms
 
 
 def layer_gemms_grouped(qlayer: dict, acts: dict[int, torch.Tensor], weight_scales: dict, prepared: dict):
@@ -127,9 +127,10 @@ def layer_gemms_grouped(qlayer: dict, acts: dict[int, torch.Tensor], weight_scal
 
 class DecodeLayer:
     """layer_gemms_grouped with everything that does not depend on the activations done once: buffers allocated,
-    arguments checked, argument arrays built (kernels.ActivationQuantizer / LinearGroup / DecodeStep).  The activations of
-    a call are all given, so it is one host call that quantizes them and multiplies with every matrix, two launches at a
-    few tokens.  Outputs are overwritten by the next call."""
+    arguments checked, argument arrays built (kernels.ActivationQuantizer / LinearGroup / DecodeStep).  A call is given one
+    activation per input width, all of them at once, so it is one host call that quantizes them and multiplies with every matrix,
+    two launches at a few tokens.  (In a decoder `o` and `down` wait for what the matrices before them feed; such a loop
+    calls the quantizers and groups one behind the other.)  Outputs are overwritten by the next call."""
 
     def __init__(self, qlayer: dict, weight_scales: dict, prepared: dict, tokens: int, device):
         self.quantizers = {}
@@ -184,7 +185,7 @@ def layer_gemms(qlayer: dict, acts: dict[int, torch.Tensor], act_importance: dic
     """y = x @ W.T for every matrix of the layer with NVFP4 operands; activations quantized with the unweighted sweep
     unless an importance vector for them is given.  Returns {name: bf16 [tokens, N]}.
 
-    The GEMMs of a layer are independent of one another.  With `prepared` weights they go out as one launch of a
+    One activation per input width, all of them given.  With `prepared` weights the products go out as one launch of a
     persistent kernel over all of them (nvfp4_scaled_mm_multi; 256 tokens of a Llama-3-8B layer, quantization included: 180 us with
     seven launches dealt out over four streams, 61 us as one).  Raw weights are launched one by
     one, with `side_streams` dealt out over those streams (forked from and joined back into the current stream, which also
@@ -351,8 +352,9 @@ def run(n_layers: int, token_batches: list[int], seed: int = 0, use_graph: bool 
         flops = 2.0 * tokens * weights_per_layer() * n_layers
         result["gemm"].append({"tokens": tokens, "ms_all_layers": ms, "eager_ms_all_layers": eager_ms,
                                "tflops": flops / (ms * 1e-3) / 1e12,
+                               # streams the layer calls were offered; with prepared weights all launches go to the current one
                                "cuda_graph": graph is not None, "streams": 1 if grouped else n_streams,
-                               "launches": "grouped (q+k+v, o, gate+up, down), one stream" if grouped else "one per matrix",
+                               "launches": "a layer's activations quantized together, then its matrices multiplied together, one stream",
                                "includes": "activation global scale + quantization + 7 GEMMs per layer"})
     if own_group:
         dist.destroy_process_group()
@@ -365,7 +367,7 @@ def main() -> None:
     ap.add_argument("--batches", type=int, nargs="*", default=[1, 32, 256, 4096])
     ap.add_argument("--seed", type=int, default=0)
     ap.add_argument("--streams", type=int, default=4,
-                    help="streams the GEMMs of a layer are dealt out over (1 = all on the current stream)")
+                    help="streams offered to layer_gemms (prepared weights, as here, go out together on the current stream)")
     ap.add_argument("--no-graph", action="store_true", help="launch the GEMM phase eagerly instead of replaying a CUDA graph")
     args = ap.parse_args()
     res = run(args.layers, args.batches, args.seed, use_graph=not args.no_graph, n_streams=args.streams)
