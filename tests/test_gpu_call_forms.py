@@ -365,3 +365,18 @@ def test_quantizer_choice_by_size_equals_the_plain_body(cuda_lib, variant, dtype
             _lib.check(cuda_lib.nvfp4_quant_launch_impl(1 if variant == 0 else 3, variant, x.data_ptr(), _lib.dtype_code(dtype), None, gs_inv.data_ptr(),
                                                         codes.data_ptr(), scales.data_ptr(), m, n, n, -3, 7, 1, None), "launch")
             assert torch.equal(codes, got[0]) and torch.equal(scales.view(torch.uint8), got[1].view(torch.uint8)), (n, m)
+
+
+@pytest.mark.parametrize("dtype,n", [(torch.bfloat16, 4096), (torch.float32, 2048)])
+@pytest.mark.parametrize("m", [8, 9])
+def test_scale_inside_the_quantizer_up_to_its_limit(cuda_lib, dtype, n, m):
+    """64 KiB and one row more: one launch and two, same bytes."""
+    import nvfp4quant_test_b200.kernels as K
+    from nvfp4quant_test_b200 import helper as H
+
+    x = torch.randn((m, n), device="cuda").to(dtype)
+    codes, scales, gs, gs_inv = K.scalesweep_nvfp4_quant_with_global_scale(x, 256.0)
+    want = H.get_nvfp4_global_scale(x, 256.0)
+    plain = K.scalesweep_mse_nvfp4_quant_impl(x, want[1])
+    assert gs == want[0] and gs_inv == want[1] and torch.equal(codes, plain[0])
+    assert torch.equal(scales.view(torch.uint8), plain[1].view(torch.uint8))
