@@ -454,7 +454,7 @@ def main():
                 "peak_source": "probe kernel of this run: back-to-back tcgen05.mma kind::mxf4nvf4 on shared-memory operands, ~0.4 s under the power cap",
                 "burst": {"achieved": tf / world, "peak": peak["burst_tflops"], "frac": tf / world / peak["burst_tflops"]},
                 "nominal_dense_fp4": NOMINAL_FP4_TFLOPS, "frac_of_nominal": sus_tf / NOMINAL_FP4_TFLOPS,
-                "peak_probe": peak, "kernel": "gemm::pair::gemm_pair_kernel<192>",
+                "peak_probe": peak, "kernel": "gemm::pair::gemm_pair_kernel<256>",
                 "algorithmic_flop_per_launch": flop}
 
         del qa, qb, sa, sb, out
