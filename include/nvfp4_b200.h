@@ -125,13 +125,14 @@ int nvfp4_quant_fused_launch(int variant, const void* x, int x_dtype, const floa
                              int64_t padded_n, int lower, int upper, int swizzled, void* stream);
 /*
  * The same two steps from ONE host call, for callers that pay per host call, e.g. an eager decode loop: global scale
- * kernel, then the quantizer reading gs_out[1]; a tensor of a few tokens takes one launch.  Any variant (amax included), any
+ * kernel, then the quantizer reading gs_out[1]; a tensor of up to 128 KiB takes one launch.  Any variant (amax included), any
  * size; `scratch` = the 2 zeroed uint32 of nvfp4_global_scale_launch.  Bytes and scales equal the two separate calls.
  */
 int nvfp4_quant_chain_launch(int variant, const void* x, int x_dtype, const float* importance, float fp8_max,
                              float* gs_out, uint32_t* scratch, uint8_t* codes, uint8_t* scales, int64_t m, int64_t n,
                              int64_t padded_n, int lower, int upper, int swizzled, void* stream);
-/* nvfp4_quant_chain_launch over several tensors of one dtype (a layer's activations), up to four per launch.  n_items <= 64.
+/* nvfp4_quant_chain_launch over several tensors of one dtype (a layer's activations, products behind them), up to four per launch;
+ * one launch does both steps where each takes up to 64 KiB.  n_items <= 64.
  * Each item has the arguments of the single form and its own scratch words. */
 typedef struct {
     const void* x;

@@ -825,9 +825,9 @@ PyObject* chain_call(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
             return none();
         }
         const cudaStream_t s = current_stream(c->device);
-        const int st = launch_on(c->device, [&] {
-            return nvfp4_quant_chain_launch(c->variant, x->const_data_ptr(), c->dtype, nullptr, c->fp8_max, c->gs, c->scratch, c->codes,
-                                            c->scales, c->m, c->n, c->n, c->lower, c->upper, 1, s);
+        const nvfp4_chain_item item = {x->const_data_ptr(), nullptr, c->gs, c->scratch, c->codes, c->scales, c->m, c->n, c->n};
+        const int st = launch_on(c->device, [&] {   // products follow: the layer's form, see quant.cu
+            return nvfp4_quant_chain_multi_launch(c->variant, c->dtype, c->fp8_max, &item, 1, c->lower, c->upper, 1, s);
         });
         return st == NVFP4_OK ? truth() : none();
     });

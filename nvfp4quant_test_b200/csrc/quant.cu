@@ -861,9 +861,12 @@ namespace {
 // Tensors of up to this many bytes take their global scale inside the quantizer: every CTA reads the whole tensor (from L2,
 // 16 loads per thread in flight at once) instead of waiting for a kernel before it.  One launch instead of two: chain of
 // launches, 1 x 4096 bf16 3.2 -> 2.4 us, 4 x 8192 (64 KiB) 4.8 -> 3.5, 16 x 4096 (128 KiB) 5.0 -> 4.8, but 16 x 8192 5.4 -> 8.0.
-// Beyond 64 KiB the pass over all of it delays the products behind it more than a launch does: a Llama-3-8B-shaped layer as four
-// quantizers and the products with each, 8 tokens 51.7 us, 12 tokens 54.6 with two launches and 56.8 with one, 16 tokens 57.9 and 62.8.
-constexpr int64_t kOwnScaleBytes = 65536;
+// A quantization on its own is bound by the host up to there (5 x 13024 from Python, 127 KiB: 5.8 us with one launch, 7.6 with two).
+// With products behind it the pass over all of the tensor delays them more than a launch does from 64 KiB on: a Llama-3-8B-shaped layer
+// as four quantizers and the products with each, 8 tokens 51.7 us, 12 tokens 54.6 with two launches and 56.8 with one, 16 tokens 57.9
+// and 62.8; launched eagerly, 16 tokens 62.6 and 65.7.
+constexpr int64_t kOwnScaleBytes = 131072;        // nvfp4_quant_chain_launch
+constexpr int64_t kOwnScaleBytesLayer = 65536;    // nvfp4_quant_chain_multi_launch: a layer's activations
 // Several tensors with up to this many blocks in all share their launches, slots numbered through; beyond it the
 // two-dimensional grids of separate launches gain more than the launches cost.
 constexpr int64_t kMultiBlocks = 524288;
@@ -900,8 +903,8 @@ cudaError_t launch_chain(int variant, bool own_scale, bool small, const QuantPar
 // Global scale, then the quantizer with that scale, of up to kMaxChain tensors per launch: what get_nvfp4_global_scale
 // followed by scalesweep_*_quant_out do (helper.py:96-100, bench.py:57-67 of the reference), for callers that pay per
 // launch and per host call (an eager decode loop).  Bytes equal the separate calls.
-extern "C" int nvfp4_quant_chain_multi_launch(int variant, int x_dtype, float fp8_max, const nvfp4_chain_item* items, int n_items,
-                                              int lower, int upper, int swizzled, void* stream) {
+static int chain_launch(int64_t own_scale_bytes, int variant, int x_dtype, float fp8_max, const nvfp4_chain_item* items, int n_items,
+                        int lower, int upper, int swizzled, void* stream) {
     using namespace nvfp4;
     if (n_items < 0 || n_items > 64) return NVFP4_ERR_BAD_RANGE;
     if (n_items == 0) return NVFP4_OK;
@@ -927,7 +930,7 @@ extern "C" int nvfp4_quant_chain_multi_launch(int variant, int x_dtype, float fp
             q[i].fp8_max = fp8_max;
             q[i].gs_out = it[i].gs_out;
             blocks += q[i].m * q[i].width;
-            own_scale = own_scale && it[i].m * it[i].n * (x_dtype == NVFP4_DT_F32 ? 4 : 2) <= kOwnScaleBytes;
+            own_scale = own_scale && it[i].m * it[i].n * (x_dtype == NVFP4_DT_F32 ? 4 : 2) <= own_scale_bytes;
         }
         const bool together = own_scale || (n > 1 && variant != NVFP4_VARIANT_AMAX && blocks <= kMultiBlocks);
         if (!own_scale) {
@@ -956,12 +959,17 @@ extern "C" int nvfp4_quant_chain_multi_launch(int variant, int x_dtype, float fp
     return NVFP4_OK;
 }
 
+extern "C" int nvfp4_quant_chain_multi_launch(int variant, int x_dtype, float fp8_max, const nvfp4_chain_item* items, int n_items,
+                                              int lower, int upper, int swizzled, void* stream) {
+    return chain_launch(nvfp4::kOwnScaleBytesLayer, variant, x_dtype, fp8_max, items, n_items, lower, upper, swizzled, stream);
+}
+
 extern "C" int nvfp4_quant_chain_launch(int variant, const void* x, int x_dtype, const float* importance, float fp8_max,
                                         float* gs_out, uint32_t* scratch, uint8_t* codes, uint8_t* scales, int64_t m,
                                         int64_t n, int64_t padded_n, int lower, int upper, int swizzled, void* stream) {
     const nvfp4_chain_item item = {x, importance, gs_out, scratch, codes, scales, m, n, padded_n};
     if (m <= 0 || n <= 0) return NVFP4_ERR_BAD_SHAPE;
-    return nvfp4_quant_chain_multi_launch(variant, x_dtype, fp8_max, &item, 1, lower, upper, swizzled, stream);
+    return chain_launch(nvfp4::kOwnScaleBytes, variant, x_dtype, fp8_max, &item, 1, lower, upper, swizzled, stream);
 }
 
 extern "C" int nvfp4_quant_fused_launch(int variant, const void* x, int x_dtype, const float* importance, float fp8_max,

@@ -2,7 +2,7 @@
 
 The reference computes the tensor-wide scale first (`get_nvfp4_global_scale`, helper.py:96-100 of
 efsotr/nvfp4quant_test) and hands its reciprocal to the quantizer (bench.py:57-67): two passes over the tensor
-and two launches from two host calls.  Here it is one host call: two dependent launches, or one for a tensor of up to 64 KiB,
+and two launches from two host calls.  Here it is one host call: two dependent launches, or one for a tensor of up to 128 KiB,
 whose CTAs each take the scale themselves.  (One cooperative launch that keeps the tensor in registers across a grid-wide wait
 is in the C ABI, nvfp4_quant_fused_launch, for tensors that fit the resident grid; it takes longer than two launches, 1 x
 4096: 5.6 against 5.1 us, 16 x 8192: 7.3 against 6.3.)

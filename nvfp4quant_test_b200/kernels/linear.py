@@ -22,7 +22,7 @@ from .kernel_vllm import create_fp4_output_tensors
 
 class ActivationQuantizer:
     """global scale -> ScaleSweep_MSE quantization of an activation [tokens, k] with one host call
-    (nvfp4_quant_chain_launch: two dependent launches, one up to 64 KiB).  Its buffers are an activation's: a PreparedWeight on
+    (nvfp4_quant_chain_multi_launch: two dependent launches, one up to 64 KiB).  Its buffers are an activation's: a PreparedWeight on
     them would be read while a later call rewrites them."""
 
     def __init__(self, tokens: int, k: int, device, fp8_max: float = _helper.FP8_E4M3_MAX_4OVER6,

@@ -368,9 +368,9 @@ def test_quantizer_choice_by_size_equals_the_plain_body(cuda_lib, variant, dtype
 
 
 @pytest.mark.parametrize("dtype,n", [(torch.bfloat16, 4096), (torch.float32, 2048)])
-@pytest.mark.parametrize("m", [8, 9])
+@pytest.mark.parametrize("m", [8, 9, 16, 17])
 def test_scale_inside_the_quantizer_up_to_its_limit(cuda_lib, dtype, n, m):
-    """64 KiB and one row more: one launch and two, same bytes."""
+    """64 and 128 KiB and one row more: one launch and two, same bytes."""
     import nvfp4quant_test_b200.kernels as K
     from nvfp4quant_test_b200 import helper as H
 
@@ -380,3 +380,5 @@ def test_scale_inside_the_quantizer_up_to_its_limit(cuda_lib, dtype, n, m):
     plain = K.scalesweep_mse_nvfp4_quant_impl(x, want[1])
     assert gs == want[0] and gs_inv == want[1] and torch.equal(codes, plain[0])
     assert torch.equal(scales.view(torch.uint8), plain[1].view(torch.uint8))
+    codes, scales, gs = K.ActivationQuantizer(m, n, "cuda", dtype=dtype)(x)
+    assert gs[0] == want[0] and torch.equal(codes, plain[0]) and torch.equal(scales.view(torch.uint8), plain[1].view(torch.uint8))
