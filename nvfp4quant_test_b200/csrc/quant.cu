@@ -65,6 +65,11 @@ constexpr int64_t kLargeBlocksRagged = 393216;
 __host__ __device__ constexpr int block_threads(int variant, int impl) {
     return impl == 9 ? kSmallThreads : (variant != NVFP4_VARIANT_AMAX && (impl == 3 || impl == 6 || impl == 7 || impl == 8 || impl == 10)) ? kSweepThreads : kThreads;
 }
+// The reference's windows: 11 candidates, unweighted; 16 from eight below the base, weighted.  The unrolled sweeps are compiled for these.
+constexpr int kWindow = 11, kWindowWeighted = 16, kWeightedLower = -8;
+__host__ __device__ constexpr bool own_window(int variant, int lower, int ncand) {
+    return variant == NVFP4_VARIANT_WEIGHTED ? lower == kWeightedLower && ncand == kWindowWeighted : ncand == kWindow;
+}
 constexpr int min_blocks(int variant, int impl) {
     if (impl == 9) return 8;
     if (impl == 10) return 4;
@@ -160,11 +165,12 @@ __device__ __forceinline__ float max_abs16(const float v[16]) {
     return fmaxf(fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3])), fmaxf(fmaxf(m[4], m[5]), fmaxf(m[6], m[7])));
 }
 
-// Candidate table: entry k describes raw code clamp(k - kTabPad, 1, 126), so a sweep that starts at
-// tab[first + kTabPad] reads consecutive entries and needs no per-candidate clamping.
-// .x = .y = 1/s (div.full.f32), .z = s*s, .w = the raw code (bit pattern).
+// Candidate table: entry k describes raw code table_raw(k), so a sweep that starts at tab[first + kTabPad] reads consecutive
+// entries and needs no per-candidate clamping.  .x = .y = 1/s (div.full.f32), .z = s*s, .w = s*s of entry k + 1: a trip's two
+// factors are a register pair as they are loaded.
 constexpr int kTabPad = 64;
 constexpr int kTabSize = 256;
+__device__ __forceinline__ uint32_t table_raw(int k) { return static_cast<uint32_t>(min(max(k - kTabPad, 1), 126)); }
 
 // ---- scalar transcription: one candidate at a time --------------------------------------
 template <bool WEIGHTED>
@@ -176,7 +182,7 @@ __device__ __forceinline__ uint32_t sweep_scalar(const float v[16], const float 
     for (int i = 0; i < ncand; ++i) {
         const float4 e4 = tab[first_idx + i];
         const float2 e = make_float2(e4.x, e4.z);
-        const uint32_t raw = __float_as_uint(e4.w);
+        const uint32_t raw = table_raw(first_idx + i);
         float err;
         if (!WEIGHTED) {
             float acc = 0.0f;
@@ -227,58 +233,87 @@ __device__ __forceinline__ void e2m1_diff_pair(uint64_t x2, float& d0, float& d1
         : "l"(x2));
 }
 
+// Both lanes' sums of a trip: candidate a in the low lane, b in the high lane.
+__device__ __forceinline__ uint64_t trip_sum(const uint64_t vp[8], uint64_t inv_a, uint64_t inv_b) {
+    uint64_t acc2 = 0;
+#pragma unroll
+    for (int p = 0; p < 8; ++p) {
+        float a0, a1, b0, b1;
+        e2m1_diff_pair(mul_f32x2(vp[p], inv_a), a0, a1);
+        e2m1_diff_pair(mul_f32x2(vp[p], inv_b), b0, b1);
+        const uint64_t d0 = pack_f32x2(a0, b0), d1 = pack_f32x2(a1, b1);
+        acc2 = fma_f32x2(d0, d0, acc2);
+        acc2 = fma_f32x2(d1, d1, acc2);
+    }
+    return acc2;
+}
+__device__ __forceinline__ uint64_t trip_sum_weighted(const uint64_t vp[8], const float w[16], uint64_t inv_a, uint64_t inv_b) {
+    uint64_t pe[8];
+#pragma unroll
+    for (int p = 0; p < 8; ++p) {
+        float a0, a1, b0, b1;
+        e2m1_diff_pair(mul_f32x2(vp[p], inv_a), a0, a1);
+        e2m1_diff_pair(mul_f32x2(vp[p], inv_b), b0, b1);
+        const uint64_t d0 = pack_f32x2(a0, b0), d1 = pack_f32x2(a1, b1);
+        const uint64_t t = mul_f32x2(mul_f32x2(d0, d0), pack_f32x2(w[2 * p], w[2 * p]));
+        pe[p] = fma_f32x2(mul_f32x2(d1, d1), pack_f32x2(w[2 * p + 1], w[2 * p + 1]), t);
+    }
+    return add_f32x2(add_f32x2(add_f32x2(pe[0], pe[1]), add_f32x2(pe[2], pe[3])),
+                     add_f32x2(add_f32x2(pe[4], pe[5]), add_f32x2(pe[6], pe[7])));
+}
+// One candidate alone (an odd count's last one).
+template <bool WEIGHTED>
+__device__ __forceinline__ float single_sum(const uint64_t vp[8], const float w[16], uint64_t inv2) {
+    if (!WEIGHTED) {
+        float acc = 0.0f;
+#pragma unroll
+        for (int p = 0; p < 8; ++p) {
+            float d0, d1;
+            e2m1_diff_pair(mul_f32x2(vp[p], inv2), d0, d1);
+            acc = __fmaf_rn(d0, d0, acc);
+            acc = __fmaf_rn(d1, d1, acc);
+        }
+        return acc;
+    }
+    float pe[8];
+#pragma unroll
+    for (int p = 0; p < 8; ++p) {
+        float d0, d1;
+        e2m1_diff_pair(mul_f32x2(vp[p], inv2), d0, d1);
+        const float a = __fmul_rn(__fmul_rn(d0, d0), w[2 * p]);
+        pe[p] = __fmaf_rn(__fmul_rn(d1, d1), w[2 * p + 1], a);
+    }
+    return __fadd_rn(__fadd_rn(__fadd_rn(pe[0], pe[1]), __fadd_rn(pe[2], pe[3])),
+                     __fadd_rn(__fadd_rn(pe[4], pe[5]), __fadd_rn(pe[6], pe[7])));
+}
+
 // NC > 0: the candidate count is the compile-time constant NC and the trips are unrolled (the table index and the
 // loop control leave the instruction stream); NC = 0: `ncand` at run time, one rolled loop.
+// A trip keeps the least error so far (one three-way minimum, which passes over NaN), its own index if that fell, and its first
+// candidate's error, by which the winner of the pair is told at the end.
+// (Two compares, two error and two code selects per trip before, and the factors packed: us, 8192 x 8192 111.2 -> 109.7, 1024 x 8192
+// 15.74 -> 15.50, 3000 x 5104 28.82 -> 28.23, weighted 8191 x 7216 178.6 -> 175.0.)
 template <bool WEIGHTED, int NC = 0>
-__device__ __forceinline__ uint32_t sweep_paired(const float v[16], const float w[16], int first_idx, int ncand_rt,
-                                                 const float4* tab) {
+__device__ __forceinline__ uint32_t sweep_paired(const float v[16], const float w[16], int first_idx, int ncand_rt, const float4* tab) {
     const int ncand = NC > 0 ? NC : ncand_rt;
     uint64_t vp[8];  // (v[2p], v[2p+1])
 #pragma unroll
     for (int p = 0; p < 8; ++p) vp[p] = pack_f32x2(v[2 * p], v[2 * p + 1]);
-    float best = __int_as_float(0x7f800000);
-    uint32_t best_raw = 0;
+    float best = __int_as_float(0x7f800000), err_first = 0.0f;
+    int pos = -2;   // of the best trip's first candidate; below 0: no error was comparable
     auto trip = [&](int i) {
-        const float4 ea = tab[first_idx + i], eb = tab[first_idx + i + 1];
-        const uint32_t raw_a = __float_as_uint(ea.w), raw_b = __float_as_uint(eb.w);
-        const uint64_t inv_a = pack_f32x2(ea.x, ea.y), inv_b = pack_f32x2(eb.x, eb.y);
-        uint64_t tot2;
-        if (!WEIGHTED) {
-            uint64_t acc2 = 0;  // (+0, +0): candidate a in the low lane, b in the high lane
-#pragma unroll
-            for (int p = 0; p < 8; ++p) {
-                float a0, a1, b0, b1;
-                e2m1_diff_pair(mul_f32x2(vp[p], inv_a), a0, a1);
-                e2m1_diff_pair(mul_f32x2(vp[p], inv_b), b0, b1);
-                const uint64_t d0 = pack_f32x2(a0, b0), d1 = pack_f32x2(a1, b1);
-                acc2 = fma_f32x2(d0, d0, acc2);
-                acc2 = fma_f32x2(d1, d1, acc2);
-            }
-            tot2 = acc2;
-        } else {
-            uint64_t pe[8];
-#pragma unroll
-            for (int p = 0; p < 8; ++p) {
-                float a0, a1, b0, b1;
-                e2m1_diff_pair(mul_f32x2(vp[p], inv_a), a0, a1);
-                e2m1_diff_pair(mul_f32x2(vp[p], inv_b), b0, b1);
-                const uint64_t d0 = pack_f32x2(a0, b0), d1 = pack_f32x2(a1, b1);
-                const uint64_t t = mul_f32x2(mul_f32x2(d0, d0), pack_f32x2(w[2 * p], w[2 * p]));
-                pe[p] = fma_f32x2(mul_f32x2(d1, d1), pack_f32x2(w[2 * p + 1], w[2 * p + 1]), t);
-            }
-            tot2 = add_f32x2(add_f32x2(add_f32x2(pe[0], pe[1]), add_f32x2(pe[2], pe[3])),
-                             add_f32x2(add_f32x2(pe[4], pe[5]), add_f32x2(pe[6], pe[7])));
-        }
+        const float4 ea = tab[first_idx + i];
+        const float2 eb = *reinterpret_cast<const float2*>(tab + first_idx + i + 1);
         float err_a, err_b;
-        unpack_f32x2(mul_f32x2(tot2, pack_f32x2(ea.z, eb.z)), err_a, err_b);
-        if (err_a < best) {
-            best = err_a;
-            best_raw = raw_a;
+        const uint64_t inv_a = pack_f32x2(ea.x, ea.y), inv_b = pack_f32x2(eb.x, eb.y);
+        const uint64_t sum = WEIGHTED ? trip_sum_weighted(vp, w, inv_a, inv_b) : trip_sum(vp, inv_a, inv_b);
+        unpack_f32x2(mul_f32x2(sum, pack_f32x2(ea.z, ea.w)), err_a, err_b);
+        const float least = fminf(fminf(best, err_a), err_b);
+        if (least < best) {
+            pos = i;
+            err_first = err_a;
         }
-        if (err_b < best) {
-            best = err_b;
-            best_raw = raw_b;
-        }
+        best = least;
     };
     if (NC > 0 && !WEIGHTED) {
 #pragma unroll
@@ -290,41 +325,13 @@ __device__ __forceinline__ uint32_t sweep_paired(const float v[16], const float 
 #pragma unroll 1
         for (int i = 0; i + 1 < ncand; i += 2) trip(i);
     }
-    if (ncand & 1) {  // odd count: the last candidate alone, scalar chain
+    pos += err_first == best ? 0 : 1;
+    if (ncand & 1) {
         const float4 e4 = tab[first_idx + ncand - 1];
-        const float2 e = make_float2(e4.x, e4.z);
-        const uint32_t raw = __float_as_uint(e4.w);
-        const uint64_t inv2 = pack_f32x2(e4.x, e4.y);
-        float err;
-        if (!WEIGHTED) {
-            float acc = 0.0f;
-#pragma unroll
-            for (int p = 0; p < 8; ++p) {
-                float d0, d1;
-                e2m1_diff_pair(mul_f32x2(vp[p], inv2), d0, d1);
-                acc = __fmaf_rn(d0, d0, acc);
-                acc = __fmaf_rn(d1, d1, acc);
-            }
-            err = __fmul_rn(acc, e.y);
-        } else {
-            float pe[8];
-#pragma unroll
-            for (int p = 0; p < 8; ++p) {
-                float d0, d1;
-                e2m1_diff_pair(mul_f32x2(vp[p], inv2), d0, d1);
-                const float a = __fmul_rn(__fmul_rn(d0, d0), w[2 * p]);
-                pe[p] = __fmaf_rn(__fmul_rn(d1, d1), w[2 * p + 1], a);
-            }
-            const float t = __fadd_rn(__fadd_rn(__fadd_rn(pe[0], pe[1]), __fadd_rn(pe[2], pe[3])),
-                                      __fadd_rn(__fadd_rn(pe[4], pe[5]), __fadd_rn(pe[6], pe[7])));
-            err = __fmul_rn(t, e.y);
-        }
-        if (err < best) {
-            best = err;
-            best_raw = raw;
-        }
+        const float err = __fmul_rn(single_sum<WEIGHTED>(vp, w, pack_f32x2(e4.x, e4.y)), e4.z);
+        if (err < best) pos = ncand - 1;
     }
-    return best_raw;
+    return pos < 0 ? 0u : table_raw(first_idx + pos);
 }
 
 // ---- one candidate per trip, element pairs share the multiply, scalar FMA chain ----------------
@@ -340,7 +347,7 @@ __device__ __forceinline__ uint32_t sweep_single(const float v[16], const float 
     for (int i = 0; i < ncand; ++i) {
         const float4 e4 = tab[first_idx + i];
         const float2 e = make_float2(e4.x, e4.z);
-        const uint32_t raw = __float_as_uint(e4.w);
+        const uint32_t raw = table_raw(first_idx + i);
         const uint64_t inv2 = pack_f32x2(e4.x, e4.y);
         float err;
         if (!WEIGHTED) {
@@ -536,12 +543,11 @@ quant_kernel(const __grid_constant__ Args args) {
     if (VARIANT != NVFP4_VARIANT_AMAX) {
 #pragma unroll
         for (int t = threadIdx.x; t < kTabSize; t += T) {   // one entry per thread with 256 threads, four with 64
-            const uint32_t raw = static_cast<uint32_t>(min(max(t - kTabPad, 1), 126));
-            const float s = e4m3_to_f32(raw);
+            const float s = e4m3_to_f32(table_raw(t)), s_next = e4m3_to_f32(table_raw(t + 1));
             float4 e;
             e.x = e.y = div_full(1.0f, s);
             e.z = __fmul_rn(s, s);
-            e.w = __uint_as_float(raw);
+            e.w = __fmul_rn(s_next, s_next);
             tab[t] = e;
         }
         __syncthreads();
@@ -628,12 +634,16 @@ quant_kernel(const __grid_constant__ Args args) {
         constexpr bool W = VARIANT == NVFP4_VARIANT_WEIGHTED;
         // clamping the start once is enough: with it below -kTabPad every candidate is raw 1, above 127 every one 126
         const int first_idx = min(max(base_raw + p.lower, -kTabPad), 127) + kTabPad;
-        sbyte = (IMPL == 1)   ? sweep_scalar<W>(v, w, first_idx, p.ncand, tab)
-                : (IMPL == 2) ? sweep_single<W>(v, w, first_idx, p.ncand, tab)
-                // the reference's own windows (11 candidates unweighted, 16 weighted) are compiled in, unrolled
-                : (WHOLE || ((IMPL == 7 || (FLAT && IMPL != 5) || WARPS) && p.ncand == (W ? 16 : 11)))
-                    ? sweep_paired<W, W ? 16 : 11>(v, w, first_idx, p.ncand, tab)
-                    : sweep_paired<W>(v, w, first_idx, p.ncand, tab);
+        if constexpr (IMPL == 1) {
+            sbyte = sweep_scalar<W>(v, w, first_idx, p.ncand, tab);
+        } else if constexpr (IMPL == 2) {
+            sbyte = sweep_single<W>(v, w, first_idx, p.ncand, tab);
+        } else {
+            // the reference's own windows are compiled in, unrolled
+            constexpr int NC = W ? kWindowWeighted : kWindow;
+            const bool compiled = WHOLE || ((IMPL == 7 || (FLAT && IMPL != 5) || WARPS) && own_window(VARIANT, p.lower, p.ncand));
+            sbyte = compiled ? sweep_paired<W, NC>(v, w, first_idx, p.ncand, tab) : sweep_paired<W>(v, w, first_idx, p.ncand, tab);
+        }
         // sbyte is 0 only when no candidate had a comparable (non-NaN, < inf) error: 1/0 as the reference computes it
         inv = (sbyte == 0) ? div_full(1.0f, 0.0f) : tab[sbyte + kTabPad].x;
     }
@@ -729,7 +739,7 @@ cudaError_t launch_impl(int impl, const QuantParams& p, cudaStream_t stream) {
     if (body == 7) {
         const dim3 grid2(static_cast<unsigned>(p.rows), static_cast<unsigned>((p.width + T - 1) / T));
         // no padding anywhere: every slot of the scale layout is a real block
-        const bool whole = chunks && p.rows == p.m && p.bin == p.bout && p.bout == p.width && p.ncand == (VARIANT == NVFP4_VARIANT_MSE ? 11 : 16);
+        const bool whole = chunks && p.rows == p.m && p.bin == p.bout && p.bout == p.width && own_window(VARIANT, p.lower, p.ncand);
         if constexpr (!kSweep)
             if (chunks && impl != 7) return launch_dependent(quant_kernel<DT, VARIANT, 8, QuantParams>, grid2, dim3(T), 0, stream, p);
         if constexpr (kSweep)

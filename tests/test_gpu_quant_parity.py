@@ -596,3 +596,42 @@ def test_global_scale_in_graphs_replayed_at_the_same_time(cuda_lib):
         assert all(torch.equal(o, w) for o in out)
     for x, w in zip(xs, want):
         assert torch.equal(H.get_nvfp4_global_scale(x, 256.0)[0], w)
+
+
+def _hard_rows():
+    """Blocks on which candidates tie, saturate, underflow or have no comparable error, [384, 2048] fp32."""
+    rng = np.random.default_rng(17)
+    grid = np.array([0, .5, 1, 1.5, 2, 3, 4, 6])
+    n = 2048
+
+    def spread(lo, hi):
+        return 10.0 ** rng.uniform(lo, hi, (n, 1))
+
+    kinds = [rng.standard_normal((n, 16)) * spread(-2, 3), rng.choice(grid, (n, 16)) * 2.0 ** rng.integers(-9, 9, (n, 1)),
+             np.repeat(spread(-4, 4), 16, 1), np.eye(16)[rng.integers(0, 16, n)] * spread(-3, 4),
+             rng.standard_normal((n, 16)) * spread(-44, -2), rng.standard_normal((n, 16)) * spread(3, 37)]
+    x = np.tile(np.concatenate(kinds).astype(np.float32).reshape(-1), 4).reshape(384, 2048)
+    x[5, ::37] = np.nan
+    x[6, ::53] = np.inf
+    x[7, :64] = 0.0
+    return torch.from_numpy(x)
+
+
+@pytest.mark.parametrize("variant, importance", [("mse", None), ("weighted", "even"), ("weighted", "spread"), ("weighted", "zeros"),
+                                                 ("weighted", "negative"), ("weighted", "nan")])
+@pytest.mark.parametrize("window", [None, (-8, 7), (-3, 7), (-11, 4), (-20, -5), (0, 0)])
+def test_bodies_choose_the_plain_sweeps_scales_on_hard_blocks(cuda_lib, variant, importance, window):
+    x = _hard_rows()
+    n = x.shape[1]
+    rng = np.random.default_rng(3)
+    w = {None: None, "even": 1 + 0.05 * rng.standard_normal(n), "spread": np.exp(2 * rng.standard_normal(n)), "zeros": rng.integers(0, 2, n),
+         "negative": rng.standard_normal(n), "nan": np.where(np.arange(n) % 97 == 0, np.nan, 1.0)}[importance]
+    lower, upper = window or (None, None)
+    for dtype in (torch.float32, torch.bfloat16):
+        for m, cols in ((384, n), (200, 1296)):     # rows of whole chunks; ragged rows with padding
+            c = {"x": x[:m, :cols].contiguous().to(dtype), "padded_n": 0, "swizzled": True, "variant": variant, "lower": lower, "upper": upper,
+                 "importance": None if w is None else torch.from_numpy(w.astype(np.float32))[:cols].reshape(1, -1)}
+            want = _run_cuda(c, 1.0, 1)
+            for impl in (0, 3, 6, 7, 8, 9):
+                codes, scales, intact = _run_cuda(c, 1.0, impl)
+                assert intact and np.array_equal(scales, want[1]) and np.array_equal(codes, want[0]), (impl, dtype, m, cols)
