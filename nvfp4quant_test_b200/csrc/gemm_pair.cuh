@@ -175,7 +175,8 @@ gemm_pair_kernel(const __grid_constant__ PairParams<G> p) {
             uint32_t phase = 0;
             bool ok = true;
             // weight half (B rows and their scales: independent of whatever ran before this kernel) and token half (A rows
-            // and their scales) of a stage; the weight halves of the first ring-full are issued before griddep_wait()
+            // and their scales) of a stage; the weight halves of the first ring-full are issued before griddep_wait(), if they are
+            // prepared (raw: side by side with the tokens, see gemm_kernel)
             auto issue = [&](int st, int mt, int nt, int kt, bool weights, bool tokens) {
                 const uint32_t lead_full = map_to_cta(full_bar(st), 0);
                 const uint32_t sbase = base + st * C::kStageBytes;
@@ -192,8 +193,7 @@ gemm_pair_kernel(const __grid_constant__ PairParams<G> p) {
                 }
             };
             int early = 0;
-            if (!p.weights_ready) griddep_wait();
-            if (cur.local < cur.total) {
+            if (p.weights_ready && cur.local < cur.total) {
                 early = min((p.g.item[cur.item].K + kBK - 1) / kBK, C::kStages);
                 if (issuer)
                     for (int i = 0; i < early; ++i) issue(i, mt, nt, i, true, false);

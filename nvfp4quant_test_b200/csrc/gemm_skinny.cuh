@@ -26,6 +26,13 @@ using pair::cluster_sync_all;
 using pair::map_to_cta;
 
 constexpr int kMaxStages = 8;
+// Stages of prepared weights that are requested ahead of the wait for the kernel before this one.  A CTA's copies are carried out in
+// order: the token tile of the first stage, without which none is consumed and none is requested again, comes behind them all.
+// Raw weights have none ahead and each stage's operands side by side; all weights of a ring of eight first, then the tokens: us, raw, 16
+// x 14336 x 8192 15.23 -> 14.38, 1 x 14336 x 4096 9.99 -> 9.04, 16 x 16384 x 2048 7.62 -> 6.69, 4 x 11000 x 4096 9.46 -> 8.48; prepared, eight
+// ahead / five, behind a product 14.09 / 13.78, 8.49 / 8.25, 6.48 / 6.29, 8.09 / 7.87, behind the quantizer 15.66 / 15.57, 10.00 / 9.47, 8.09 /
+// 7.55, 9.26 / 9.20 (three 16.08, 9.90, 7.23, 9.71).
+constexpr int kAhead = 5;
 // TMEM: accumulator in columns 0..BT-1, then two scale sets of 32 columns
 
 template <int BT>
@@ -167,26 +174,27 @@ skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant_
     int p_stage = 0, p_next = 0;
     uint32_t p_phase = 0;
     bool p_ok = true;
+    // copies of one stage, by the elected lane: the weight tile and its scales, the token tile and its scales
+    auto copy_stage = [&](int stage, int kt, bool weights, bool tokens) {
+        const uint32_t sf_bytes = 512u * min(4, (K - kt * kBK + 63) / 64);
+        const uint32_t sbase = base + stage * C::kStageBytes;
+        if (weights) {
+            mbar_expect_tx(full_bar(stage), C::kWBytes + C::kXBytes + 2 * sf_bytes);
+            tma_load_2d(sbase, tmap_w, kt * kBKBytes, nt * 128, full_bar(stage));
+        }
+        if (tokens) tma_load_2d(sbase + C::kWBytes, tmap_x, kt * kBKBytes, 0, full_bar(stage));
+        if (weights)
+            bulk_load_1d(sbase + C::kWBytes + C::kXBytes, sfw + static_cast<int64_t>(nt) * sf_group_stride + static_cast<int64_t>(kt) * 2048,
+                         sf_bytes, full_bar(stage));
+        if (tokens)
+            bulk_load_1d(sbase + C::kWBytes + C::kXBytes + C::kSfBytes, sfx + static_cast<int64_t>(kt) * 2048, sf_bytes, full_bar(stage));
+    };
     auto produce = [&](int end) {
         const bool issuer = elect_one();
         for (; p_ok && p_next < end; ++p_next) {
             const int kt = kt_begin + p_next;
-            const int stage = p_stage;
-            const uint32_t phase = p_phase;
-            if (!(p_ok = mbar_wait_warp(empty_bar(stage), phase ^ 1u, abort_flag, (7u << 24) | kt))) break;
-            const int kb_count = min(4, (K - kt * kBK + 63) / 64);
-            const uint32_t sf_bytes = 512u * kb_count;
-            const uint32_t sbase = base + stage * C::kStageBytes;
-            if (issuer) {
-                mbar_expect_tx(full_bar(stage), C::kWBytes + C::kXBytes + 2 * sf_bytes);
-                tma_load_2d(sbase, tmap_w, kt * kBKBytes, nt * 128, full_bar(stage));
-                tma_load_2d(sbase + C::kWBytes, tmap_x, kt * kBKBytes, 0, full_bar(stage));
-                bulk_load_1d(sbase + C::kWBytes + C::kXBytes,
-                             sfw + static_cast<int64_t>(nt) * sf_group_stride + static_cast<int64_t>(kt) * 2048, sf_bytes,
-                             full_bar(stage));
-                bulk_load_1d(sbase + C::kWBytes + C::kXBytes + C::kSfBytes, sfx + static_cast<int64_t>(kt) * 2048, sf_bytes,
-                             full_bar(stage));
-            }
+            if (!(p_ok = mbar_wait_warp(empty_bar(p_stage), p_phase ^ 1u, abort_flag, (7u << 24) | kt))) break;
+            if (issuer) copy_stage(p_stage, kt, true, true);
             __syncwarp();
             if (++p_stage == nstages) {
                 p_stage = 0;
@@ -201,33 +209,17 @@ skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant_
             asm volatile("prefetch.tensormap [%0];" ::"l"(tmap_x) : "memory");
         }
         // First ring-full.  The weights do not depend on whatever ran before this kernel on the stream, the token tile
-        // and its scales (the quantizer's output) do: with a programmatic dependent launch the weight copies go out
+        // and its scales (the quantizer's output) do: with a programmatic dependent launch up to kAhead stages' prepared weights go out
         // at once, the rest after griddep_wait().
         const int first = min(kcount, nstages);
         const bool issuer = elect_one();
-        if (!p.weights_ready) griddep_wait();   // raw weight pointers: they may be the previous kernel's output too
-        if (issuer) {
-            for (int i = 0; i < first; ++i) {
-                const int kt = kt_begin + i;
-                const uint32_t sf_bytes = 512u * min(4, (K - kt * kBK + 63) / 64);
-                const uint32_t sbase = base + i * C::kStageBytes;
-                mbar_expect_tx(full_bar(i), C::kWBytes + C::kXBytes + 2 * sf_bytes);
-                tma_load_2d(sbase, tmap_w, kt * kBKBytes, nt * 128, full_bar(i));
-                bulk_load_1d(sbase + C::kWBytes + C::kXBytes,
-                             sfw + static_cast<int64_t>(nt) * sf_group_stride + static_cast<int64_t>(kt) * 2048, sf_bytes,
-                             full_bar(i));
-            }
-        }
+        const int ahead = p.weights_ready ? min(first, kAhead) : 0;   // raw weight pointers may be the previous kernel's output too
+        if (issuer)
+            for (int i = 0; i < ahead; ++i) copy_stage(i, kt_begin + i, true, false);
         griddep_wait();
         if (issuer) {
-            for (int i = 0; i < first; ++i) {
-                const int kt = kt_begin + i;
-                const uint32_t sf_bytes = 512u * min(4, (K - kt * kBK + 63) / 64);
-                const uint32_t sbase = base + i * C::kStageBytes;
-                tma_load_2d(sbase + C::kWBytes, tmap_x, kt * kBKBytes, 0, full_bar(i));
-                bulk_load_1d(sbase + C::kWBytes + C::kXBytes + C::kSfBytes, sfx + static_cast<int64_t>(kt) * 2048, sf_bytes,
-                             full_bar(i));
-            }
+            for (int i = 0; i < ahead; ++i) copy_stage(i, kt_begin + i, false, true);
+            for (int i = ahead; i < first; ++i) copy_stage(i, kt_begin + i, true, true);
         }
         __syncwarp();
         p_next = first;
@@ -457,6 +449,10 @@ static int choose_stages(int clusters, int ranks, int sms) {
     // with CTAs sharing an SM a fifth stage, which would still fit, measured slower than four (Llama-3-8B-shaped decode
     // chain of 32 layers at 1 / 16 tokens: 1.30 / 1.48 ms against 1.25 / 1.43; 16 x 28672 x 8192: 23.3 against 23.0 us)
     if (per_sm >= 2 && stages > 4) stages = 4;
+    // a cluster's CTAs need room at the same time, which they find sooner beside the launch before them with six stages than with
+    // eight (30 x 9000 x 5120, raw / prepared / behind the quantizer: 9.36 / 8.82 / 11.75 -> 9.10 / 8.40 / 10.35; 16 x 9216 x 4096 8.16 / 7.49 /
+    // 8.96 -> 7.95 / 7.13 / 8.62); single CTAs gain 1-4 % with raw weights and lose 1-8 % behind the quantizer
+    if (ranks > 1 && stages > 6) stages = 6;
     if (stages < 2) stages = 2;
     return stages;
 }
