@@ -27,7 +27,10 @@ struct PairCfg {
     static constexpr int kABytes = 128 * kBKBytes;          // this CTA's 128 rows of A
     static constexpr int kBBytes = (BN / 2) * kBKBytes;     // this CTA's half of the B rows
     static constexpr int kSfaBytes = 2048;                  // scales of this CTA's A rows
-    static constexpr int kSfbBytes = 4096;                  // two 128-row scale groups cover the B tile
+    // 128-row scale groups that a B tile touches: a 128-wide one exactly one (with two loaded for it, us, before / after: 256 x 4096 x 14336
+    // 15.08 / 14.71, 700 x 1500 x 14336 14.99 / 14.43, 300 x 1024 x 8192 9.86 / 9.54)
+    static constexpr int kSfbGroups = BN == 128 ? 1 : 2;
+    static constexpr int kSfbBytes = 2048 * kSfbGroups;
     static constexpr int kStageBytes = kABytes + kBBytes + kSfaBytes + kSfbBytes;
     // ring stages against staged output pieces per epilogue warp: as deep a ring as leaves one piece (256 x 192 tiles with 5
     // stages and two pieces: 5 % faster at K = 1024, 4 % slower at K = 8192)
@@ -35,9 +38,9 @@ struct PairCfg {
     static constexpr int kOutBufs = (BN == 256) ? 2 : 1;
     static constexpr int kEpilogueBytes = 4 * kOutBufs * kPieceBytes;
     static constexpr int kSmemBytes = kStages * kStageBytes + kEpilogueBytes + 256;
-    static constexpr int kSfaCol = kAcc * BN;               // scale set 0; set 1 follows 48 columns later
+    static constexpr int kSfaCol = kAcc * BN;               // scale set 0; set 1 follows
     static constexpr int kSfbCol = kSfaCol + 16;
-    static constexpr int kSfSetCols = 48;
+    static constexpr int kSfSetCols = 16 + 16 * kSfbGroups;
     static_assert(kSfaCol + 2 * kSfSetCols <= kTmemCols, "TMEM budget");
     static_assert(kStageBytes % 1024 == 0, "stage alignment for the 128-byte swizzle");
 };
@@ -52,9 +55,12 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
     return r;
 }
+// every thread of the cluster arrives and waits in turn
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cluster_arrive();
+    cluster_wait();
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
@@ -133,6 +139,10 @@ gemm_pair_kernel(const __grid_constant__ PairParams<G> p) {
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
+    __syncwarp();
+    // Two phases of the cluster barrier: the barriers of both CTAs exist (nothing is signalled across CTAs before), which is all that
+    // the producers need; TMEM is allocated in both, which the other warps wait for as well while the first copies are on their way.
+    cluster_arrive();
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                          smem_u32(const_cast<uint32_t*>(tmem_slot))),
@@ -141,11 +151,12 @@ gemm_pair_kernel(const __grid_constant__ PairParams<G> p) {
         if (lane == 0) trace_mark(1, 1);
     }
     tc_fence_before();
-    __syncthreads();
+    cluster_wait();
     if (threadIdx.x == 0) trace_mark(1, 9);
-    cluster_sync_all();   // the peer's barriers exist before anything is signalled across CTAs
+    cluster_arrive();
+    if (warp != 0) cluster_wait();   // the producer warps wait at their end
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = *tmem_slot;   // meaningful in warps 1..5 only
     if (threadIdx.x == 0) trace_mark(1, 2);
     if (warp >= 2) griddep_wait();    // the epilogue reads alpha and writes the output: only after the previous kernel
 
@@ -184,8 +195,10 @@ gemm_pair_kernel(const __grid_constant__ PairParams<G> p) {
                     if (rank == 0) mbar_expect_tx(full_bar(st), 2u * C::kStageBytes);
                     tma_load_2d_pair(sbase + C::kABytes, &p.b[cur.item], kt * kBKBytes, nt * BN + static_cast<int>(rank) * (BN / 2), lead_full);
                     // scale tiles: x counts 8-byte elements (2048 B per K tile), y = 128-row group
-                    tma_load_2d_pair(sbase + C::kABytes + C::kBBytes + C::kSfaBytes, &p.sfb[cur.item], kt * 256, (nt * BN) / 128, lead_full);
-                    tma_load_2d_pair(sbase + C::kABytes + C::kBBytes + C::kSfaBytes + 2048, &p.sfb[cur.item], kt * 256, (nt * BN) / 128 + 1, lead_full);
+#pragma unroll
+                    for (int g = 0; g < C::kSfbGroups; ++g)
+                        tma_load_2d_pair(sbase + C::kABytes + C::kBBytes + C::kSfaBytes + 2048 * g, &p.sfb[cur.item], kt * 256, (nt * BN) / 128 + g,
+                                         lead_full);
                 }
                 if (tokens) {
                     tma_load_2d_pair(sbase, &p.a[cur.item], kt * kBKBytes, mt * 256 + static_cast<int>(rank) * 128, lead_full);
@@ -254,21 +267,23 @@ gemm_pair_kernel(const __grid_constant__ PairParams<G> p) {
 #pragma unroll
                         for (int kb = 0; kb < 4; ++kb) {
                             tc_cp_pair(sfa_t + 4 * kb, sfa_lo + 32 * kb);
-                            tc_cp_pair(sfb_t + 8 * kb, sfb_lo + 32 * kb);
-                            tc_cp_pair(sfb_t + 8 * kb + 4, sfb_lo + 128 + 32 * kb);
+#pragma unroll
+                            for (int g = 0; g < C::kSfbGroups; ++g)
+                                tc_cp_pair(sfb_t + 4 * C::kSfbGroups * kb + 4 * g, sfb_lo + 128 * g + 32 * kb);
                         }
 #pragma unroll
                         for (int kb = 0; kb < 4; ++kb)
-                            tc_mma_pair(d_tmem, a_lo + 2 * kb, b_lo + 2 * kb, idesc, sfa_t + 4 * kb, sfb_t + 8 * kb + sfb_shift,
+                            tc_mma_pair(d_tmem, a_lo + 2 * kb, b_lo + 2 * kb, idesc, sfa_t + 4 * kb, sfb_t + 4 * C::kSfbGroups * kb + sfb_shift,
                                         kb == 0 ? first : 1u);
                     } else {
                         for (int kb = 0; kb < kb_count; ++kb) {
                             tc_cp_pair(sfa_t + 4 * kb, sfa_lo + 32 * kb);
-                            tc_cp_pair(sfb_t + 8 * kb, sfb_lo + 32 * kb);
-                            tc_cp_pair(sfb_t + 8 * kb + 4, sfb_lo + 128 + 32 * kb);
+#pragma unroll
+                            for (int g = 0; g < C::kSfbGroups; ++g)
+                                tc_cp_pair(sfb_t + 4 * C::kSfbGroups * kb + 4 * g, sfb_lo + 128 * g + 32 * kb);
                         }
                         for (int kb = 0; kb < kb_count; ++kb)
-                            tc_mma_pair(d_tmem, a_lo + 2 * kb, b_lo + 2 * kb, idesc, sfa_t + 4 * kb, sfb_t + 8 * kb + sfb_shift,
+                            tc_mma_pair(d_tmem, a_lo + 2 * kb, b_lo + 2 * kb, idesc, sfa_t + 4 * kb, sfb_t + 4 * C::kSfbGroups * kb + sfb_shift,
                                         kb == 0 ? first : 1u);
                     }
                     if (issuer) tc_commit_pair(empty_bar(stage));   // frees this slot in both CTAs
@@ -324,7 +339,13 @@ gemm_pair_kernel(const __grid_constant__ PairParams<G> p) {
         }
     }
 
-    if (warp >= 2 && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    if (warp == 0) {
+        __syncwarp();
+        cluster_wait();
+    }
+    // the staged output has been read; the writes themselves are complete when the grid is
+    if (warp >= 2 && lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+    __syncwarp();
     if (lane == 0) trace_mark(1, warp == 0 ? 3 : warp == 1 ? 4 : 5);
     // ---------------------------------------------------------------------- teardown
     if (*abort_flag) {
