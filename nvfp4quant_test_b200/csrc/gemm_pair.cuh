@@ -174,52 +174,59 @@ gemm_pair_kernel(const __grid_constant__ PairParams<G> p) {
         // ------------------------------------------------------------------ producer (both CTAs)
         {
             const bool issuer = elect_one();
-            int mt, nt;
-            if (cur.local < cur.total) locate(cur.local, mt, nt);
+            int mt = 0, nt = 0, k_tiles = 0;
+            auto set_tile = [&](int tile) {
+                locate(tile, mt, nt);
+                k_tiles = (p.g.item[cur.item].K + kBK - 1) / kBK;
+            };
+            const uint32_t lead_full = map_to_cta(full_bar(0), 0);
+            // weight half (B rows and their scales: independent of whatever ran before this kernel) and token half (A rows
+            // and their scales) of a stage; the weight halves of the first ring-full are issued before griddep_wait(), if they are
+            // prepared (raw: side by side with the tokens, see gemm_kernel)
+            auto issue = [&](int st, int kt, bool weights, bool tokens) {
+                const uint32_t bar = lead_full + 8u * st;
+                const uint32_t sbase = base + st * C::kStageBytes;
+                if (weights) {
+                    if (rank == 0) mbar_expect_tx(full_bar(st), 2u * C::kStageBytes);
+                    tma_load_2d_pair(sbase + C::kABytes, &p.b[cur.item], kt * kBKBytes, nt * BN + static_cast<int>(rank) * (BN / 2), bar);
+                }
+                if (tokens) tma_load_2d_pair(sbase, &p.a[cur.item], kt * kBKBytes, mt * 256 + static_cast<int>(rank) * 128, bar);
+                if (weights) {
+                    // scale tiles: x counts 8-byte elements (2048 B per K tile), y = 128-row group
+#pragma unroll
+                    for (int g = 0; g < C::kSfbGroups; ++g)
+                        tma_load_2d_pair(sbase + C::kABytes + C::kBBytes + C::kSfaBytes + 2048 * g, &p.sfb[cur.item], kt * 256, (nt * BN) / 128 + g, bar);
+                }
+                if (tokens)
+                    tma_load_2d_pair(sbase + C::kABytes + C::kBBytes, &p.sfa[cur.item], kt * 256, mt * 2 + static_cast<int>(rank), bar);
+            };
+            const bool any = cur.local < cur.total;
+            if (any) set_tile(cur.local);
             if (issuer) {
                 asm volatile("prefetch.tensormap [%0];" ::"l"(&p.a[cur.item]) : "memory");
                 asm volatile("prefetch.tensormap [%0];" ::"l"(&p.b[cur.item]) : "memory");
                 asm volatile("prefetch.tensormap [%0];" ::"l"(&p.sfa[cur.item]) : "memory");
                 asm volatile("prefetch.tensormap [%0];" ::"l"(&p.sfb[cur.item]) : "memory");
             }
-            int stage = 0;
-            uint32_t phase = 0;
-            bool ok = true;
-            // weight half (B rows and their scales: independent of whatever ran before this kernel) and token half (A rows
-            // and their scales) of a stage; the weight halves of the first ring-full are issued before griddep_wait(), if they are
-            // prepared (raw: side by side with the tokens, see gemm_kernel)
-            auto issue = [&](int st, int mt, int nt, int kt, bool weights, bool tokens) {
-                const uint32_t lead_full = map_to_cta(full_bar(st), 0);
-                const uint32_t sbase = base + st * C::kStageBytes;
-                if (weights) {
-                    if (rank == 0) mbar_expect_tx(full_bar(st), 2u * C::kStageBytes);
-                    tma_load_2d_pair(sbase + C::kABytes, &p.b[cur.item], kt * kBKBytes, nt * BN + static_cast<int>(rank) * (BN / 2), lead_full);
-                    // scale tiles: x counts 8-byte elements (2048 B per K tile), y = 128-row group
-#pragma unroll
-                    for (int g = 0; g < C::kSfbGroups; ++g)
-                        tma_load_2d_pair(sbase + C::kABytes + C::kBBytes + C::kSfaBytes + 2048 * g, &p.sfb[cur.item], kt * 256, (nt * BN) / 128 + g,
-                                         lead_full);
-                }
-                if (tokens) {
-                    tma_load_2d_pair(sbase, &p.a[cur.item], kt * kBKBytes, mt * 256 + static_cast<int>(rank) * 128, lead_full);
-                    tma_load_2d_pair(sbase + C::kABytes + C::kBBytes, &p.sfa[cur.item], kt * 256, mt * 2 + static_cast<int>(rank), lead_full);
-                }
-            };
-            int early = 0;
-            if (p.weights_ready && cur.local < cur.total) {
-                early = min((p.g.item[cur.item].K + kBK - 1) / kBK, C::kStages);
-                if (issuer)
-                    for (int i = 0; i < early; ++i) issue(i, mt, nt, i, true, false);
-                __syncwarp();
-            }
+            const int early = any ? min(k_tiles, C::kStages) : 0;   // stages requested without a wait
+            if (issuer && p.weights_ready)
+                for (int i = 0; i < early; ++i) issue(i, i, true, false);
             griddep_wait();
+            if (issuer)
+                for (int i = 0; i < early; ++i) issue(i, i, !p.weights_ready, true);
+            __syncwarp();
+            int stage = early == C::kStages ? 0 : early;
+            uint32_t phase = early == C::kStages ? 1u : 0u;
+            bool ok = true;
             for (int tile = cur.local; ok && tile < cur.total; tile += cur.workers) {
-                locate(tile, mt, nt);
-                const int k_tiles = (p.g.item[cur.item].K + kBK - 1) / kBK;
-                for (int kt = 0; kt < k_tiles; ++kt) {
+                int kt = early;
+                if (tile != cur.local) {
+                    set_tile(tile);
+                    kt = 0;
+                }
+                for (; kt < k_tiles; ++kt) {
                     if (!(ok = mbar_wait_warp(empty_bar(stage), phase ^ 1u, abort_flag, (1u << 24) | kt))) break;
-                    if (issuer) issue(stage, mt, nt, kt, early == 0, true);
-                    if (early > 0) --early;
+                    if (issuer) issue(stage, kt, true, true);
                     __syncwarp();
                     if (++stage == C::kStages) {
                         stage = 0;

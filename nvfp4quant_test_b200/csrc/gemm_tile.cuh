@@ -329,67 +329,78 @@ gemm_kernel(const __grid_constant__ TileParams<G> p) {
         // ------------------------------------------------------------------ producer
         {
             const bool issuer = elect_one();
-            int ks, mt, nt, kt_begin, kcount, rot;
-            if (cur.local < total_tiles) locate(cur.local, ks, mt, nt);
+            // One lane requests four copies per stage, and how long it takes over them bounds these kernels (with the addresses, the K
+            // range and the number of scale groups worked out for every stage, us: 128 x 64 tiles 128 x 4096 x 4096 7.27 -> 5.48, 512 x 4096 x
+            // 4096 12.5 -> 9.7; 128 x 128 tiles 333 x 5000 x 2880 7.16 -> 6.28, 300 x 1024 x 8192 12.1 -> 9.3, 2048 x 4096 x 4096 24.9 -> 18.8).
+            // So all that is constant over a tile is worked out once per tile.
+            // The current tile: coordinates, K range (see k_range), where its scales are.
+            int ks, mt = 0, nt = 0, kt_begin = 0, kcount = 0, rot = 0, kt_last = 0;
+            uint32_t last_bytes = 0, groups = 0;
+            const uint8_t *sfa = nullptr, *sfb = nullptr;
+            int64_t group_stride = 0;
+            auto set_tile = [&](int tile) {
+                locate(tile, ks, mt, nt);
+                k_range(ks, tile, kt_begin, kcount, rot);
+                const GemmItem& it = p.g.item[cur.item];
+                group_stride = it.sf_group_stride;
+                const int grp0 = BN == 64 ? (nt >> 1) : nt * C::kNG;   // first 128-row scale group of this B tile
+                groups = static_cast<uint32_t>(min(C::kNG, it.sfb_groups - grp0));
+                sfa = it.sfa + static_cast<int64_t>(mt) * group_stride;
+                sfb = it.sfb + static_cast<int64_t>(grp0) * group_stride;
+                kt_last = (it.K + kBK - 1) / kBK - 1;
+                last_bytes = 512u * static_cast<uint32_t>((it.K - kt_last * kBK + 63) / 64);   // 64-element K blocks of the last stage
+            };
+            // Stage copies come in two halves: the weight half (B tile and its scales) of a prepared weight depends on nothing that ran
+            // before this kernel, the token half (A tile and its scales) may be the previous kernel's output.  The
+            // weight halves of the first ring-full go out before griddep_wait(), so that with a programmatic dependent
+            // launch the weight stream starts while the previous kernel is still finishing.  A raw weight has to
+            // wait itself, and its first ring-full goes side by side with the tokens: copies are carried out in order, and behind a ring-full
+            // of weights the first stage's tokens come late (us, 100 x 14336 x 4096 10.01 -> 8.87, 150 x 3000 x 1024 4.22 -> 3.62, 1000 x 2048 x
+            // 2048 6.05 -> 5.54).
+            auto issue = [&](int st, int kt, bool weights, bool tokens) {
+                const uint32_t sf_bytes = kt == kt_last ? last_bytes : 2048u;
+                const uint32_t sbase = base + st * C::kStageBytes;
+                const int64_t sf_at = static_cast<int64_t>(kt) * 2048;
+                if (weights) {
+                    mbar_expect_tx(full_bar(st), C::kABytes + C::kBBytes + sf_bytes * (1 + groups));
+                    tma_load_2d(sbase + C::kABytes, &p.b[cur.item], kt * kBKBytes, nt * BN, full_bar(st));
+                }
+                if (tokens) tma_load_2d(sbase, &p.a[cur.item], kt * kBKBytes, mt * kBM, full_bar(st));
+                if (weights) {
+                    bulk_load_1d(sbase + C::kABytes + C::kBBytes + C::kSfaBytes, sfb + sf_at, sf_bytes, full_bar(st));
+                    if (C::kNG > 1 && groups > 1)
+                        bulk_load_1d(sbase + C::kABytes + C::kBBytes + C::kSfaBytes + 2048, sfb + group_stride + sf_at, sf_bytes, full_bar(st));
+                }
+                if (tokens) bulk_load_1d(sbase + C::kABytes + C::kBBytes, sfa + sf_at, sf_bytes, full_bar(st));
+            };
+            const bool any = cur.local < total_tiles;
+            if (any) set_tile(cur.local);
             if (issuer) {
                 asm volatile("prefetch.tensormap [%0];" ::"l"(&p.a[cur.item]) : "memory");
                 asm volatile("prefetch.tensormap [%0];" ::"l"(&p.b[cur.item]) : "memory");
             }
-            int stage = 0;
-            uint32_t phase = 0;
-            bool ok = true;
-            // Stage copies come in two halves: the weight half (B tile and its scales) of a prepared weight depends on nothing that ran
-            // before this kernel, the token half (A tile and its scales) may be the previous kernel's output.  The
-            // weight halves of the first ring-full go out before griddep_wait(), so that with a programmatic dependent
-            // launch the weight stream starts while the previous kernel is still finishing; `early` counts them.  A raw weight has to
-            // wait itself, and then goes side by side with the tokens: copies are carried out in order, and behind a ring-full of weights
-            // the first stage's tokens come late (us, 100 x 14336 x 4096 10.36 -> 9.42, 150 x 3000 x 1024 4.49 -> 4.07, 1000 x 2048 x 2048 6.36 ->
-            // 5.87, 333 x 5000 x 2880 7.84 -> 7.59).
-            auto issue = [&](int st, int mt, int nt, int kt, bool weights, bool tokens) {
-                const GemmItem& it = p.g.item[cur.item];
-                const int kb_count = min(4, (it.K - kt * kBK + 63) / 64);  // 64-element K blocks in this stage
-                const uint32_t sf_bytes = 512u * kb_count;
-                int sfb_present = 0;
-                const int grp0 = BN == 64 ? (nt >> 1) : nt * C::kNG;   // first 128-row scale group of this B tile
-                for (int g = 0; g < C::kNG; ++g) sfb_present += (grp0 + g < it.sfb_groups) ? 1 : 0;
-                const uint32_t sbase = base + st * C::kStageBytes;
-                if (weights) {
-                    mbar_expect_tx(full_bar(st), C::kABytes + C::kBBytes + sf_bytes * (1 + sfb_present));
-                    tma_load_2d(sbase + C::kABytes, &p.b[cur.item], kt * kBKBytes, nt * BN, full_bar(st));
-                    for (int g = 0; g < C::kNG; ++g) {
-                        const int grp = grp0 + g;
-                        if (grp < it.sfb_groups)
-                            bulk_load_1d(sbase + C::kABytes + C::kBBytes + C::kSfaBytes + g * 2048,
-                                         it.sfb + static_cast<int64_t>(grp) * it.sf_group_stride +
-                                             static_cast<int64_t>(kt) * 2048,
-                                         sf_bytes, full_bar(st));
-                    }
-                }
-                if (tokens) {
-                    tma_load_2d(sbase, &p.a[cur.item], kt * kBKBytes, mt * kBM, full_bar(st));
-                    bulk_load_1d(sbase + C::kABytes + C::kBBytes,
-                                 it.sfa + static_cast<int64_t>(mt) * it.sf_group_stride + static_cast<int64_t>(kt) * 2048,
-                                 sf_bytes, full_bar(st));
-                }
-            };
-            int early = 0;
-            if (p.weights_ready && cur.local < total_tiles && !(G == 1 && p.k_rotate)) {
-                k_range(ks, cur.local, kt_begin, kcount, rot);
-                early = min(kcount, C::kStages);
-                if (issuer)
-                    for (int i = 0; i < early; ++i) issue(i, mt, nt, kt_begin + i, true, false);
-                __syncwarp();
-            }
+            const int early = any && !(G == 1 && p.k_rotate) ? min(kcount, C::kStages) : 0;   // stages requested without a wait
+            if (issuer && p.weights_ready)
+                for (int i = 0; i < early; ++i) issue(i, kt_begin + i, true, false);
             griddep_wait();
+            if (issuer)
+                for (int i = 0; i < early; ++i) issue(i, kt_begin + i, !p.weights_ready, true);
+            __syncwarp();
+            int stage = early == C::kStages ? 0 : early;
+            uint32_t phase = early == C::kStages ? 1u : 0u;
+            bool ok = true;
             for (int tile = cur.local; ok && tile < total_tiles; tile += cur.workers) {
-                locate(tile, ks, mt, nt);
-                k_range(ks, tile, kt_begin, kcount, rot);
-                for (int i = 0; i < kcount; ++i) {
-                    const int kt = kt_begin + (i + rot) % kcount;
+                int i = early;
+                if (tile != cur.local) {
+                    set_tile(tile);
+                    i = 0;
+                }
+                int kt = kt_begin + i + rot;
+                for (; i < kcount; ++i) {
                     if (!(ok = mbar_wait_warp(empty_bar(stage), phase ^ 1u, abort_flag, (1u << 24) | kt))) break;
-                    if (issuer) issue(stage, mt, nt, kt, early == 0, true);
-                    if (early > 0) --early;
+                    if (issuer) issue(stage, kt, true, true);
                     __syncwarp();
+                    if (++kt == kt_begin + kcount) kt = kt_begin;
                     if (++stage == C::kStages) {
                         stage = 0;
                         phase ^= 1u;
@@ -417,8 +428,8 @@ gemm_kernel(const __grid_constant__ TileParams<G> p) {
                 const int K = p.g.item[cur.item].K;
                 // a 64-row B tile is one half of a 128-row scale group: rows 64..127 sit two TMEM columns further on
                 const uint32_t sfb_half = BN == 64 ? 2u * (nt & 1) : 0u;
+                int kt = kt_begin + rot;
                 for (int i = 0; i < kcount; ++i) {
-                    const int kt = kt_begin + (i + rot) % kcount;
                     if (!(ok = mbar_wait_warp(full_bar(stage), phase, abort_flag, (2u << 24) | kt))) break;
                     tc_fence_after();
                     const int kb_count = min(4, (K - kt * kBK + 63) / 64);
@@ -458,6 +469,7 @@ gemm_kernel(const __grid_constant__ TileParams<G> p) {
                     }
                     if (issuer) tc_commit(empty_bar(stage));  // slot reusable once these MMAs have read it
                     __syncwarp();
+                    if (++kt == kt_begin + kcount) kt = kt_begin;
                     if (++stage == C::kStages) {
                         stage = 0;
                         phase ^= 1u;
