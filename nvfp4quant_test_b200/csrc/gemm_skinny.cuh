@@ -15,17 +15,20 @@ namespace gemm {
 // The partial accumulators are combined by a reduce-scatter through distributed shared memory: the token
 // columns are dealt out to the ranks, every rank writes its partial tile to its own shared memory and sends
 // each other rank the columns that rank owns with one bulk copy (cp.async.bulk shared::cta -> shared::cluster,
-// completion counted on the receiver's mbarrier); the owner adds the partials in ascending rank order, applies
+// completion counted on the receiver's mbarrier) into an area that nothing else uses; the owner adds the partials in ascending rank order, applies
 // alpha and stores bf16.  One kernel, no workspace, and the result does not depend on timing.  Every copy has
 // one destination CTA (no multicast).
 // =============================================================================================
 namespace skinny {
 
+using pair::cluster_arrive;
 using pair::cluster_ctarank;
-using pair::cluster_sync_all;
+using pair::cluster_wait;
 using pair::map_to_cta;
 
 constexpr int kMaxStages = 8;
+constexpr int kBarrierBytes = 256;
+constexpr int kSlack = 1024;   // a ring that starts at a rounded address of the launch measured 2 to 5 % faster than one at a fixed offset
 // Stages of prepared weights that are requested ahead of the wait for the kernel before this one.  A CTA's copies are carried out in
 // order: the token tile of the first stage, without which none is consumed and none is requested again, comes behind them all.
 // Raw weights have none ahead and each stage's operands side by side; all weights of a ring of eight first, then the tokens: us, raw, 16
@@ -158,9 +161,14 @@ skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant_
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        // (ranks - 1) senders x my columns x 128 rows x 4 bytes; armed before any rank can send (they send after
-        // the cluster barrier below the main loop)
+        // (ranks - 1) senders x my columns x 128 rows x 4 bytes; armed before any rank can send
         if (ranks > 1 && my_cols > 0) mbar_expect_tx(recv_bar, (ranks - 1) * my_cols * 512u);
+    }
+    // Two phases of the cluster barrier: the barriers of all CTAs exist and are armed (waited for before the first copy to another
+    // CTA), and all copies have landed (waited for at the end).
+    if (cluster > 1) {
+        __syncwarp();
+        cluster_arrive();
     }
     const int k_tiles = (K + kBK - 1) / kBK;
     const int kt_begin = static_cast<int>(rank) * p.w[gi].k_tiles_per_rank;
@@ -312,38 +320,46 @@ skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant_
             }
         }
     } else {
-        // The ring is idle once the accumulator is complete (all copies landed and were consumed), so it is reused:
-        // `part` [token column][128 rows] fp32 = this rank's partial tile, `recv` [sending rank][owned column][128 rows].
+        // The ring is idle once the accumulator is complete (all copies landed and were consumed) and takes this rank's partial tile:
+        // `part` [token column][128 rows] fp32.  `recv` [sending rank][owned column][128 rows], behind the barriers, is nobody's ring: a
+        // rank sends as soon as it is done, whether or not the owner still multiplies.  us, with `recv` in the ring, behind a cluster barrier
+        // and with another one after the exchange / this, prepared: 16 x 4096 x 4096 5.12 / 4.54, 1 x 4096 x 4096 4.85 / 4.36, 16 x 8192 x 8192
+        // 9.85 / 9.19, 32 x 2048 x 2048 4.55 / 4.00, 48 x 4096 x 14336 10.42 / 10.03, 24 x 7168 x 14336 12.87 / 13.12.  (Partials stored straight
+        // into the owner's shared memory, 4 bytes per lane, instead of bulk copies: 4 x 1024 x 8192 4.64 for 4.42, 48 x 7168 x 7168 10.64 for 9.92.)
         float* part = reinterpret_cast<float*>(aligned);
-        float* recv = part + BT * 128;
-        if (warp >= 2 && have) {
+        const float* const recv = reinterpret_cast<const float*>(reinterpret_cast<uint8_t*>(bars) + kBarrierBytes);
+        if (warp >= 2) {
+            if (have) {
 #pragma unroll 1
-            for (int c = 0; c < BT / 16 && c * 16 < p.M; ++c) {
-                uint32_t v[16];
-                tc_ld_32x32b_x16(t_lane + c * 16, v);
-                tc_ld_wait();
+                for (int c = 0; c < BT / 16 && c * 16 < p.M; ++c) {
+                    uint32_t v[16];
+                    tc_ld_32x32b_x16(t_lane + c * 16, v);
+                    tc_ld_wait();
 #pragma unroll
-                for (int e = 0; e < 16; ++e)
-                    if (c * 16 + e < p.M) part[(c * 16 + e) * 128 + n_local] = __uint_as_float(v[e]);
+                    for (int e = 0; e < 16; ++e)
+                        if (c * 16 + e < p.M) part[(c * 16 + e) * 128 + n_local] = __uint_as_float(v[e]);
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the bulk copies below read `part`
             }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the bulk copies below read `part`
-        }
-        // every rank has left its main loop: the `recv` areas may be written
-        cluster_sync_all();
-        if (warp == 2 && have && elect_one()) {
-            for (uint32_t o = 0; o < ranks; ++o) {
-                const uint32_t first = o * cols_per_rank;
-                if (o == rank || first >= m_cols) continue;
-                const uint32_t cols = min(cols_per_rank, m_cols - first);
-                bulk_copy_to_cta(map_to_cta(smem_u32(recv + (rank * cols_per_rank) * 128), first_peer + o),
-                                 smem_u32(part + first * 128), cols * 512u, map_to_cta(recv_bar, first_peer + o));
+            cluster_wait();
+            asm volatile("bar.sync 2, 128;" ::: "memory");   // the four warps' rows are staged
+            if (warp == 2 && have && elect_one()) {
+                for (uint32_t i = 1; i < ranks; ++i) {   // this rank's successor first
+                    const uint32_t o = rank + i < ranks ? rank + i : rank + i - ranks, first = o * cols_per_rank;
+                    if (first >= m_cols) continue;
+                    const uint32_t cols = min(cols_per_rank, m_cols - first);
+                    bulk_copy_to_cta(map_to_cta(smem_u32(recv + (rank * cols_per_rank) * 128), first_peer + o),
+                                     smem_u32(part + first * 128), cols * 512u, map_to_cta(recv_bar, first_peer + o));
+                }
             }
+            __syncwarp();
         }
         if (warp >= 2 && have && my_cols > 0) {
+            const float alpha = load_alpha(p.w[gi].alpha, p.w[gi].alpha_x);
             bool ok = mbar_wait(recv_bar, 0, abort_flag, (10u << 24) | nt);
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+            cluster_arrive();
             if (ok && n < N) {
-                const float alpha = load_alpha(p.w[gi].alpha, p.w[gi].alpha_x);
                 // this rank's own partial sits in `recv` terms at part[my_first ..]; eight columns at a time so that
                 // the shared-memory loads of one rank's partials are in flight together
                 const float* own = part + my_first * 128 + n_local;
@@ -367,8 +383,14 @@ skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant_
                 }
             }
         }
-        // no rank may leave while another still copies out of its `part`
-        cluster_sync_all();
+        if (warp >= 2 && !(have && my_cols > 0)) cluster_arrive();
+    }
+    if (cluster > 1) {
+        __syncwarp();
+        if (warp < 2 || ranks == 1) {   // the others have done this around the exchange
+            cluster_wait();
+            cluster_arrive();
+        }
     }
 
     // ---------------------------------------------------------------------- teardown
@@ -381,6 +403,10 @@ skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant_
     if (warp == 1) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(C::kTmemCols) : "memory");
+    }
+    if (cluster > 1) {   // no rank may leave while another still copies out of its `part` or into its `recv`
+        __syncwarp();
+        cluster_wait();
     }
 }
 
@@ -437,14 +463,14 @@ struct SkinnyItem {
 // Ring depth: the deepest ring with which the whole grid is resident at once (as many CTAs per SM as that takes, at
 // most what the TMEM columns allow), since a CTA that has to wait for a free SM starts its weight stream late.
 template <int BT>
-static int choose_stages(int clusters, int ranks, int sms) {
+static int choose_stages(int clusters, int ranks, int sms, int recv_bytes) {
     using C = SkinnyCfg<BT>;
     constexpr int kMaxPerSm = kTmemCols / C::kTmemCols;
     int per_sm = 1;
     while (per_sm < kMaxPerSm && clusters > resident_clusters(ranks, per_sm, sms)) ++per_sm;
-    // an SM has 233472 bytes of shared memory, of which 1 KiB per resident CTA is reserved; a CTA asks for its ring
-    // plus 1 KiB of alignment slack plus 256 bytes of barriers
-    int stages = (233472 / per_sm - 1024 - 1024 - 256) / C::kStageBytes;
+    // an SM has 233472 bytes of shared memory, of which 1 KiB per resident CTA is reserved; a CTA asks for its ring with
+    // alignment slack, its barriers and the area of the other ranks' partials
+    int stages = (233472 / per_sm - 1024 - kSlack - kBarrierBytes - recv_bytes) / C::kStageBytes;
     if (stages > C::kMaxStages) stages = C::kMaxStages;
     // with CTAs sharing an SM a fifth stage, which would still fit, measured slower than four (Llama-3-8B-shaped decode
     // chain of 32 layers at 1 / 16 tokens: 1.30 / 1.48 ms against 1.25 / 1.43; 16 x 28672 x 8192: 23.3 against 23.0 us)
@@ -533,7 +559,7 @@ static int launch_skinny_list(int M, const SkinnyItem* items, int n_items, int f
         while (cluster > 1 && !all_fit(cluster)) --cluster;
         for (int i = 0; i < n_items; ++i) p.w[i].ranks = cluster;
     }
-    int clusters = 0, per_rank = 1, max_ranks = 1;
+    int clusters = 0, per_rank = 1;
     for (int i = 0; i < n_items; ++i) {
         const int tiles = static_cast<int>((items[i].N + 127) / 128), per = cluster / p.w[i].ranks;
         p.w[i].tiles = per;
@@ -544,23 +570,27 @@ static int launch_skinny_list(int M, const SkinnyItem* items, int n_items, int f
         p.w[i].cluster_end = clusters;
         p.w[i].k_tiles_per_rank = stages_of(i, p.w[i].ranks);
         if (p.w[i].k_tiles_per_rank > per_rank) per_rank = p.w[i].k_tiles_per_rank;
-        if (p.w[i].ranks > max_ranks) max_ranks = p.w[i].ranks;
     }
     p.M = M;
     p.n_weights = n_items;
-    p.stages = choose_stages<BT>(clusters, cluster, sms);
+    int recv_bytes = 0;   // ranks x owned columns x 128 rows
+    for (int i = 0; i < n_items; ++i) {
+        const int r = p.w[i].ranks;
+        if (r > 1) recv_bytes = std::max(recv_bytes, ((M < BT ? M : BT) + r - 1) / r * r * 512);
+    }
+    p.stages = choose_stages<BT>(clusters, cluster, sms, recv_bytes);
     if (p.stages > per_rank) p.stages = per_rank < 2 ? 2 : per_rank;
-    // the ring doubles as the reduce-scatter buffers: the partial tile plus one slot per rank of the owned columns
-    while (max_ranks > 1 && (2 * BT + 8) * 512 > p.stages * C::kStageBytes) ++p.stages;
-    if (p.stages > C::kMaxStages) return NVFP4_ERR_UNSUPPORTED;
+    // the ring doubles as `part`
+    while (recv_bytes > 0 && BT * 512 > p.stages * C::kStageBytes) ++p.stages;
     // Co-resident CTAs must never want more than the 512 TMEM columns of an SM between them (a CTA that waits in
     // tcgen05.alloc while its cluster peers wait for it is a deadlock).  Shared memory is what bounds co-residency, so
     // every CTA asks for at least the share of the SM's shared memory that matches its share of the TMEM columns
     // (1 KiB per CTA is reserved by the system): whatever mix of these kernels fits an SM then fits its TMEM too.
     constexpr int kMinSmem = 233472 / (kTmemCols / C::kTmemCols) - 1024;   // 128 columns: 57344 (4 CTAs), 256: 115712 (2)
-    int smem = p.stages * C::kStageBytes + 1024 + 256;
+    int smem = p.stages * C::kStageBytes + kSlack + kBarrierBytes + recv_bytes;
     if (smem < kMinSmem) smem = kMinSmem;
-    static_assert(C::kMaxStages * C::kStageBytes + 1024 + 256 <= kGemmDynSmemBytes, "ring does not fit");
+    static_assert(C::kMaxStages * C::kStageBytes + kSlack + kBarrierBytes <= kGemmDynSmemBytes, "ring does not fit");
+    static_assert(2 * C::kStageBytes + kSlack + kBarrierBytes + (BT + 7) * 512 <= kGemmDynSmemBytes && BT * 512 <= 2 * C::kStageBytes, "partials do not fit");
     static bool attr_done[64] = {false};
     cudaError_t e = allow_full_smem(skinny_kernel<BT, G>, attr_done, di.device);
     if (e != cudaSuccess) return static_cast<int>(e);
