@@ -372,10 +372,9 @@ extern "C" int nvfp4_gemm_prepare(const uint8_t* b, const uint8_t* sfb, int64_t 
     h->sfb = sfb;
     h->N = N;
     h->K = K;
-    int st = gemm::make_operand_map(&h->rows64, b, N, K / 2, 64);
-    if (st == NVFP4_OK) st = gemm::make_operand_map(&h->rows96, b, N, K / 2, 96);
-    if (st == NVFP4_OK) st = gemm::make_operand_map(&h->rows128, b, N, K / 2, 128);
-    if (st == NVFP4_OK) st = gemm::make_operand_map(&h->rows256, b, N, K / 2, 256);
+    int st = NVFP4_OK;
+    for (int i = 0; i < 4 && st == NVFP4_OK; ++i)
+        st = gemm::make_operand_maps(&h->rows[i], &h->rest[i], b, N, K / 2, gemm::WeightHandle::kHeights[i]);
     if (st == NVFP4_OK)
         st = gemm::pair::make_scale_map(&h->scales, sfb, (N + 127) / 128, round_up_i64(K / 16, 4) * 128);
     if (st != NVFP4_OK) {

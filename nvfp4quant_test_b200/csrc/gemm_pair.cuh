@@ -407,7 +407,7 @@ static int launch_pair_list(const GemmParams* list, const WeightHandle* const* w
         if (st == NVFP4_OK) st = make_scale_map(&q.sfa[i], p.sfa, p.sfa_groups, p.sf_group_stride);
         if (st == NVFP4_OK) st = make_output_map(&q.out[i], p.out, p.M, p.N);
         if (wh[i]) {
-            q.b[i] = *wh[i]->by_rows(BN / 2);
+            q.b[i] = wh[i]->rows[WeightHandle::index(BN / 2)];
             q.sfb[i] = wh[i]->scales;
         } else {
             q.weights_ready = 0;

@@ -99,8 +99,9 @@ struct SkinnyParams {
 
 template <int G>
 struct SkinnyMaps {
-    CUtensorMap m[G];   // one per weight: [N, K/2] bytes in boxes of 128 rows x 128 bytes
-    CUtensorMap x[G];   // its activation: [M, K/2] bytes in boxes of BT rows
+    CUtensorMap m[G];        // one per weight: [N, K/2] bytes in boxes of 128 rows x 128 bytes
+    CUtensorMap m_rest[G];   // and of the N % 128 last rows (see TileParams)
+    CUtensorMap x[G];        // its activation: [M, K/2] bytes in boxes of M rows
 };
 
 template <int BT, int G>
@@ -140,10 +141,12 @@ skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant_
     const uint32_t rank = crank - sub * ranks, first_peer = sub * ranks;
     const int nt = G > 1 ? (static_cast<int>(cluster_id) - (gi > 0 ? p.w[gi - 1].cluster_end : 0)) * p.w[gi].tiles + static_cast<int>(sub)
                          : static_cast<int>(cluster_id);
-    const CUtensorMap* tmap_w = &maps.m[gi];
-    const CUtensorMap* tmap_x = &maps.x[gi];
     const uint8_t *const sfw = p.w[gi].sfw, *const sfx = p.w[gi].sfx;
     const int N = p.w[gi].N, K = p.w[gi].K;
+    const int w_rows = min(128, N - nt * 128);
+    const CUtensorMap* tmap_w = w_rows == 128 ? &maps.m[gi] : &maps.m_rest[gi];
+    const CUtensorMap* tmap_x = &maps.x[gi];
+    const uint32_t operand_bytes = static_cast<uint32_t>(w_rows + p.M) * kBKBytes;
     const int64_t sf_group_stride = p.w[gi].sf_group_stride;
     // reduce-scatter: token column c belongs to rank c / cols_per_rank
     const uint32_t m_cols = static_cast<uint32_t>(min(p.M, BT));
@@ -187,7 +190,7 @@ skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant_
         const uint32_t sf_bytes = 512u * min(4, (K - kt * kBK + 63) / 64);
         const uint32_t sbase = base + stage * C::kStageBytes;
         if (weights) {
-            mbar_expect_tx(full_bar(stage), C::kWBytes + C::kXBytes + 2 * sf_bytes);
+            mbar_expect_tx(full_bar(stage), operand_bytes + 2 * sf_bytes);
             tma_load_2d(sbase, tmap_w, kt * kBKBytes, nt * 128, full_bar(stage));
         }
         if (tokens) tma_load_2d(sbase + C::kWBytes, tmap_x, kt * kBKBytes, 0, full_bar(stage));
@@ -522,10 +525,14 @@ static int launch_skinny_list(int M, const SkinnyItem* items, int n_items, int f
     for (int i = 0; i < n_items && st == NVFP4_OK; ++i) {
         const SkinnyItem& it = items[i];
         if (!it.wh) p.weights_ready = 0;
-        if (it.wh) maps.m[i] = it.wh->rows128;
-        else st = make_operand_map(&maps.m[i], it.w, it.N, it.K / 2, 128);
+        if (it.wh) {
+            maps.m[i] = it.wh->rows[WeightHandle::index(128)];
+            maps.m_rest[i] = it.wh->rest[WeightHandle::index(128)];
+        } else {
+            st = make_operand_maps(&maps.m[i], &maps.m_rest[i], it.w, it.N, it.K / 2, 128);
+        }
         if (i > 0 && it.x == items[i - 1].x && it.K == items[i - 1].K) maps.x[i] = maps.x[i - 1];
-        else if (st == NVFP4_OK) st = make_operand_map(&maps.x[i], it.x, M, it.K / 2, BT);
+        else if (st == NVFP4_OK) st = make_operand_map(&maps.x[i], it.x, M, it.K / 2, M);
         n_tiles += static_cast<int>((it.N + 127) / 128);
         p.w[i].sfw = it.sfw;
         p.w[i].sfx = it.sfx;

@@ -230,9 +230,15 @@ __device__ __forceinline__ float load_alpha(const float* alpha, const float* alp
 }
 
 // Operand maps and the work list of one launch over G products (G = 1: an ordinary GEMM, whose K may be cut into ranges).
+//
+// A copy of a box that reaches beyond the matrix fills the rows outside with zeros, and takes longer over a row of zeros than over one
+// that it fetches.  So a last tile that is not whole has a map of its own (`a_rest`, `b_rest`), whose box ends with the matrix.  The rows
+// behind it in shared memory hold what was there before: bytes that are valid codes, for outputs that do not exist.  us, whole boxes /
+// this, prepared: 128 x 64 tiles 17 x 6208 x 4224 10.1 / 5.9, 48 x 14336 x 4096 13.5 / 9.3, 150 x 3000 x 1024 3.45 / 3.15, 128 x 128 tiles 48 x 14336 x 4096 8.8 /
+// 7.9.  (The pair kernels, which take larger launches, gain nothing by it and lose 1 to 3 % to the choice.)
 template <int G>
 struct TileParams {
-    CUtensorMap a[G], b[G];
+    CUtensorMap a[G], b[G], a_rest[G], b_rest[G];
     GroupTable<G> g;
     int M;
     int k_splits, k_tiles_per_split, k_rotate;   // G = 1 only, see GemmParams
@@ -333,15 +339,20 @@ gemm_kernel(const __grid_constant__ TileParams<G> p) {
             // range and the number of scale groups worked out for every stage, us: 128 x 64 tiles 128 x 4096 x 4096 7.27 -> 5.48, 512 x 4096 x
             // 4096 12.5 -> 9.7; 128 x 128 tiles 333 x 5000 x 2880 7.16 -> 6.28, 300 x 1024 x 8192 12.1 -> 9.3, 2048 x 4096 x 4096 24.9 -> 18.8).
             // So all that is constant over a tile is worked out once per tile.
-            // The current tile: coordinates, K range (see k_range), where its scales are.
+            // The current tile: coordinates, K range (see k_range), its operands' maps, where its scales are.
             int ks, mt = 0, nt = 0, kt_begin = 0, kcount = 0, rot = 0, kt_last = 0;
-            uint32_t last_bytes = 0, groups = 0;
+            uint32_t last_bytes = 0, groups = 0, operand_bytes = 0;
+            const CUtensorMap *map_a = &p.a[0], *map_b = &p.b[0];
             const uint8_t *sfa = nullptr, *sfb = nullptr;
             int64_t group_stride = 0;
             auto set_tile = [&](int tile) {
                 locate(tile, ks, mt, nt);
                 k_range(ks, tile, kt_begin, kcount, rot);
                 const GemmItem& it = p.g.item[cur.item];
+                const int a_rows = min(kBM, p.M - mt * kBM), b_rows = min(BN, it.N - nt * BN);
+                map_a = a_rows == kBM ? &p.a[cur.item] : &p.a_rest[cur.item];
+                map_b = b_rows == BN ? &p.b[cur.item] : &p.b_rest[cur.item];
+                operand_bytes = static_cast<uint32_t>(a_rows + b_rows) * kBKBytes;
                 group_stride = it.sf_group_stride;
                 const int grp0 = BN == 64 ? (nt >> 1) : nt * C::kNG;   // first 128-row scale group of this B tile
                 groups = static_cast<uint32_t>(min(C::kNG, it.sfb_groups - grp0));
@@ -362,10 +373,10 @@ gemm_kernel(const __grid_constant__ TileParams<G> p) {
                 const uint32_t sbase = base + st * C::kStageBytes;
                 const int64_t sf_at = static_cast<int64_t>(kt) * 2048;
                 if (weights) {
-                    mbar_expect_tx(full_bar(st), C::kABytes + C::kBBytes + sf_bytes * (1 + groups));
-                    tma_load_2d(sbase + C::kABytes, &p.b[cur.item], kt * kBKBytes, nt * BN, full_bar(st));
+                    mbar_expect_tx(full_bar(st), operand_bytes + sf_bytes * (1 + groups));
+                    tma_load_2d(sbase + C::kABytes, map_b, kt * kBKBytes, nt * BN, full_bar(st));
                 }
-                if (tokens) tma_load_2d(sbase, &p.a[cur.item], kt * kBKBytes, mt * kBM, full_bar(st));
+                if (tokens) tma_load_2d(sbase, map_a, kt * kBKBytes, mt * kBM, full_bar(st));
                 if (weights) {
                     bulk_load_1d(sbase + C::kABytes + C::kBBytes + C::kSfaBytes, sfb + sf_at, sf_bytes, full_bar(st));
                     if (C::kNG > 1 && groups > 1)
@@ -376,8 +387,8 @@ gemm_kernel(const __grid_constant__ TileParams<G> p) {
             const bool any = cur.local < total_tiles;
             if (any) set_tile(cur.local);
             if (issuer) {
-                asm volatile("prefetch.tensormap [%0];" ::"l"(&p.a[cur.item]) : "memory");
-                asm volatile("prefetch.tensormap [%0];" ::"l"(&p.b[cur.item]) : "memory");
+                asm volatile("prefetch.tensormap [%0];" ::"l"(map_a) : "memory");
+                asm volatile("prefetch.tensormap [%0];" ::"l"(map_b) : "memory");
             }
             const int early = any && !(G == 1 && p.k_rotate) ? min(kcount, C::kStages) : 0;   // stages requested without a wait
             if (issuer && p.weights_ready)
@@ -655,12 +666,26 @@ struct WeightHandle {
     const uint8_t* b;
     const uint8_t* sfb;
     int64_t N, K;
-    CUtensorMap rows64, rows96, rows128, rows256;   // operand maps by box height
-    CUtensorMap scales;                             // scale groups as rows of 8-byte words (pair kernels)
-    const CUtensorMap* by_rows(int rows) const {
-        return rows == 64 ? &rows64 : rows == 96 ? &rows96 : rows == 128 ? &rows128 : &rows256;
-    }
+    CUtensorMap rows[4], rest[4];   // operand maps by box height (kHeights), and of a last box that is not whole (N % height rows)
+    CUtensorMap scales;             // scale groups as rows of 8-byte words (pair kernels)
+    static constexpr int kHeights[4] = {64, 96, 128, 256};
+    static constexpr int index(int height) { return height == 64 ? 0 : height == 96 ? 1 : height == 128 ? 2 : 3; }
 };
+// Maps of a [rows, k_bytes] operand in boxes of `height` rows: whole ones, and the one of the rows % height last rows where there are
+// any.
+static int make_operand_maps(CUtensorMap* whole, CUtensorMap* rest, const void* ptr, int64_t rows, int64_t k_bytes, int height) {
+    int st = make_operand_map(whole, ptr, rows, k_bytes, height);
+    if (st == NVFP4_OK && rows % height) st = make_operand_map(rest, ptr, rows, k_bytes, static_cast<int>(rows % height));
+    return st;
+}
+// A weight's maps for a launch: the prepared ones, or encoded now.
+static int weight_maps(CUtensorMap* whole, CUtensorMap* rest, const GemmParams& p, const WeightHandle* wh, int height) {
+    if (!wh) return make_operand_maps(whole, rest, p.b, p.N, p.K / 2, height);
+    const int i = WeightHandle::index(height);
+    *whole = wh->rows[i];
+    if (p.N % height) *rest = wh->rest[i];
+    return NVFP4_OK;
+}
 constexpr uint32_t kWeightMagic = 0x4e56463u;
 
 // Fills the work list for `workers` CTAs (or CTA pairs) and returns how many are used (0: too few for the classes, or more
@@ -749,13 +774,9 @@ static int launch_list(const GemmParams* list, const WeightHandle* const* wh, in
     q.weights_ready = 1;
     for (int i = 0; i < n; ++i) {
         const GemmParams& p = list[i];
-        int st = make_operand_map(&q.a[i], p.a, p.M, p.K / 2, kBM);
-        if (wh[i]) {
-            q.b[i] = *wh[i]->by_rows(BN);
-        } else {
-            q.weights_ready = 0;
-            if (st == NVFP4_OK) st = make_operand_map(&q.b[i], p.b, p.N, p.K / 2, BN);
-        }
+        if (!wh[i]) q.weights_ready = 0;
+        int st = make_operand_maps(&q.a[i], &q.a_rest[i], p.a, p.M, p.K / 2, kBM);
+        if (st == NVFP4_OK) st = weight_maps(&q.b[i], &q.b_rest[i], p, wh[i], BN);
         if (st != NVFP4_OK) return st;
     }
     const DeviceInfo di = device_info();
