@@ -23,6 +23,7 @@ namespace skinny {
 
 using pair::cluster_arrive;
 using pair::cluster_ctarank;
+using pair::cluster_sync_all;
 using pair::cluster_wait;
 using pair::map_to_cta;
 
@@ -108,6 +109,8 @@ template <int BT, int G>
 __global__ void __launch_bounds__(kThreads)
 skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant__ SkinnyParams<G> p) {
     using C = SkinnyCfg<BT>;
+    // Where the ranks' partials meet: behind the ring (`apart`), or in it.  See the epilogue.
+    constexpr bool kApart = G == 1;
     extern __shared__ uint8_t smem_raw[];
     // The kernel queued behind this one may be scheduled at once: ahead of its own wait it reads nothing but a
     // prepared (constant) weight, and that wait covers this kernel's completion.
@@ -169,7 +172,7 @@ skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant_
     }
     // Two phases of the cluster barrier: the barriers of all CTAs exist and are armed (waited for before the first copy to another
     // CTA), and all copies have landed (waited for at the end).
-    if (cluster > 1) {
+    if (kApart && ranks > 1) {
         __syncwarp();
         cluster_arrive();
     }
@@ -224,13 +227,17 @@ skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant_
         // at once, the rest after griddep_wait().
         const int first = min(kcount, nstages);
         const bool issuer = elect_one();
-        const int ahead = p.weights_ready ? min(first, kAhead) : 0;   // raw weight pointers may be the previous kernel's output too
+        const int ahead = !p.weights_ready ? 0 : G > 1 ? first : min(first, kAhead);   // raw weight pointers may be the previous kernel's output too
         if (issuer)
             for (int i = 0; i < ahead; ++i) copy_stage(i, kt_begin + i, true, false);
         griddep_wait();
         if (issuer) {
-            for (int i = 0; i < ahead; ++i) copy_stage(i, kt_begin + i, false, true);
-            for (int i = ahead; i < first; ++i) copy_stage(i, kt_begin + i, true, true);
+            if (G > 1) {
+                for (int i = 0; i < first; ++i) copy_stage(i, kt_begin + i, !p.weights_ready, true);
+            } else {
+                for (int i = 0; i < ahead; ++i) copy_stage(i, kt_begin + i, false, true);
+                for (int i = ahead; i < first; ++i) copy_stage(i, kt_begin + i, true, true);
+            }
         }
         __syncwarp();
         p_next = first;
@@ -324,44 +331,56 @@ skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant_
         }
     } else {
         // The ring is idle once the accumulator is complete (all copies landed and were consumed) and takes this rank's partial tile:
-        // `part` [token column][128 rows] fp32.  `recv` [sending rank][owned column][128 rows], behind the barriers, is nobody's ring: a
-        // rank sends as soon as it is done, whether or not the owner still multiplies.  us, with `recv` in the ring, behind a cluster barrier
-        // and with another one after the exchange / this, prepared: 16 x 4096 x 4096 5.12 / 4.54, 1 x 4096 x 4096 4.85 / 4.36, 16 x 8192 x 8192
-        // 9.85 / 9.19, 32 x 2048 x 2048 4.55 / 4.00, 48 x 4096 x 14336 10.42 / 10.03, 24 x 7168 x 14336 12.87 / 13.12.  (Partials stored straight
-        // into the owner's shared memory, 4 bytes per lane, instead of bulk copies: 4 x 1024 x 8192 4.64 for 4.42, 48 x 7168 x 7168 10.64 for 9.92.)
+        // `part` [token column][128 rows] fp32.  `recv` [sending rank][owned column][128 rows] holds the other ranks' partials of the
+        // columns that this one owns.
+        //
+        // A launch of one product has room for `recv` behind the barriers: a rank sends as soon as it is done, whether or not the owner
+        // still multiplies, and the cluster meets once, at the end.  us, with `recv` in the ring, behind a cluster barrier and with another
+        // one after the exchange / this, prepared: 16 x 4096 x 4096 5.12 / 4.54, 1 x 4096 x 4096 4.85 / 4.36, 16 x 8192 x 8192 9.85 / 9.19, 32 x
+        // 2048 x 2048 4.55 / 4.00, 48 x 4096 x 14336 10.42 / 10.03, 24 x 7168 x 14336 12.87 / 13.12.  (Partials stored straight into the owner's
+        // shared memory, 4 bytes per lane, instead of bulk copies: 4 x 1024 x 8192 4.64 for 4.42, 48 x 7168 x 7168 10.64 for 9.92.)
+        //
+        // A launch of many products has three or four CTAs on an SM, which hide one another's waits and whose rings have no stage to
+        // spare: there `recv` stays in the ring (the seven matrices of a layer of hidden 5120, FFN 13824, 16 tokens, with their
+        // quantization: 34.5 us, 35.1 apart; 32 tokens 36.2 and 43.9).
         float* part = reinterpret_cast<float*>(aligned);
-        const float* const recv = reinterpret_cast<const float*>(reinterpret_cast<uint8_t*>(bars) + kBarrierBytes);
-        if (warp >= 2) {
-            if (have) {
+        const float* const recv = kApart ? reinterpret_cast<const float*>(reinterpret_cast<uint8_t*>(bars) + kBarrierBytes) : part + BT * 128;
+        if (warp >= 2 && have) {
 #pragma unroll 1
-                for (int c = 0; c < BT / 16 && c * 16 < p.M; ++c) {
-                    uint32_t v[16];
-                    tc_ld_32x32b_x16(t_lane + c * 16, v);
-                    tc_ld_wait();
+            for (int c = 0; c < BT / 16 && c * 16 < p.M; ++c) {
+                uint32_t v[16];
+                tc_ld_32x32b_x16(t_lane + c * 16, v);
+                tc_ld_wait();
 #pragma unroll
-                    for (int e = 0; e < 16; ++e)
-                        if (c * 16 + e < p.M) part[(c * 16 + e) * 128 + n_local] = __uint_as_float(v[e]);
-                }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the bulk copies below read `part`
+                for (int e = 0; e < 16; ++e)
+                    if (c * 16 + e < p.M) part[(c * 16 + e) * 128 + n_local] = __uint_as_float(v[e]);
             }
-            cluster_wait();
-            asm volatile("bar.sync 2, 128;" ::: "memory");   // the four warps' rows are staged
-            if (warp == 2 && have && elect_one()) {
-                for (uint32_t i = 1; i < ranks; ++i) {   // this rank's successor first
-                    const uint32_t o = rank + i < ranks ? rank + i : rank + i - ranks, first = o * cols_per_rank;
-                    if (first >= m_cols) continue;
-                    const uint32_t cols = min(cols_per_rank, m_cols - first);
-                    bulk_copy_to_cta(map_to_cta(smem_u32(recv + (rank * cols_per_rank) * 128), first_peer + o),
-                                     smem_u32(part + first * 128), cols * 512u, map_to_cta(recv_bar, first_peer + o));
-                }
-            }
-            __syncwarp();
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the bulk copies below read `part`
         }
+        if (kApart) {
+            if (warp >= 2) {
+                cluster_wait();
+                asm volatile("bar.sync 2, 128;" ::: "memory");   // the four warps' rows are staged
+            }
+        } else {
+            __syncwarp();
+            cluster_sync_all();   // every rank has left its main loop: the `recv` areas may be written
+        }
+        if (warp == 2 && have && elect_one()) {
+            for (uint32_t i = 1; i < ranks; ++i) {   // this rank's successor first
+                const uint32_t o = rank + i < ranks ? rank + i : rank + i - ranks, first = o * cols_per_rank;
+                if (first >= m_cols) continue;
+                const uint32_t cols = min(cols_per_rank, m_cols - first);
+                bulk_copy_to_cta(map_to_cta(smem_u32(recv + (rank * cols_per_rank) * 128), first_peer + o),
+                                 smem_u32(part + first * 128), cols * 512u, map_to_cta(recv_bar, first_peer + o));
+            }
+        }
+        __syncwarp();
         if (warp >= 2 && have && my_cols > 0) {
             const float alpha = load_alpha(p.w[gi].alpha, p.w[gi].alpha_x);
             bool ok = mbar_wait(recv_bar, 0, abort_flag, (10u << 24) | nt);
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-            cluster_arrive();
+            if (kApart) cluster_arrive();
             if (ok && n < N) {
                 // this rank's own partial sits in `recv` terms at part[my_first ..]; eight columns at a time so that
                 // the shared-memory loads of one rank's partials are in flight together
@@ -385,14 +404,17 @@ skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant_
                             dst[static_cast<int64_t>(c0 + j) * N] = __float2bfloat16_rn(__fmul_rn(acc[j], alpha));
                 }
             }
-        }
-        if (warp >= 2 && !(have && my_cols > 0)) cluster_arrive();
-    }
-    if (cluster > 1) {
-        __syncwarp();
-        if (warp < 2 || ranks == 1) {   // the others have done this around the exchange
-            cluster_wait();
+        } else if (kApart && warp >= 2) {
             cluster_arrive();
+        }
+        __syncwarp();
+        if (kApart) {
+            if (warp < 2) {   // the others have done this around the exchange
+                cluster_wait();
+                cluster_arrive();
+            }
+        } else {
+            cluster_sync_all();   // no rank may leave while another still copies out of its `part`
         }
     }
 
@@ -407,7 +429,7 @@ skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant_
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(C::kTmemCols) : "memory");
     }
-    if (cluster > 1) {   // no rank may leave while another still copies out of its `part` or into its `recv`
+    if (kApart && ranks > 1) {   // no rank may leave while another still copies out of its `part` or into its `recv`
         __syncwarp();
         cluster_wait();
     }
@@ -566,7 +588,7 @@ static int launch_skinny_list(int M, const SkinnyItem* items, int n_items, int f
         while (cluster > 1 && !all_fit(cluster)) --cluster;
         for (int i = 0; i < n_items; ++i) p.w[i].ranks = cluster;
     }
-    int clusters = 0, per_rank = 1;
+    int clusters = 0, per_rank = 1, max_ranks = 1;
     for (int i = 0; i < n_items; ++i) {
         const int tiles = static_cast<int>((items[i].N + 127) / 128), per = cluster / p.w[i].ranks;
         p.w[i].tiles = per;
@@ -577,18 +599,16 @@ static int launch_skinny_list(int M, const SkinnyItem* items, int n_items, int f
         p.w[i].cluster_end = clusters;
         p.w[i].k_tiles_per_rank = stages_of(i, p.w[i].ranks);
         if (p.w[i].k_tiles_per_rank > per_rank) per_rank = p.w[i].k_tiles_per_rank;
+        if (p.w[i].ranks > max_ranks) max_ranks = p.w[i].ranks;
     }
     p.M = M;
     p.n_weights = n_items;
-    int recv_bytes = 0;   // ranks x owned columns x 128 rows
-    for (int i = 0; i < n_items; ++i) {
-        const int r = p.w[i].ranks;
-        if (r > 1) recv_bytes = std::max(recv_bytes, ((M < BT ? M : BT) + r - 1) / r * r * 512);
-    }
+    int recv_bytes = 0;   // a launch of one product: ranks x owned columns x 128 rows behind the ring
+    if (G == 1 && p.w[0].ranks > 1) recv_bytes = ((M < BT ? M : BT) + p.w[0].ranks - 1) / p.w[0].ranks * p.w[0].ranks * 512;
     p.stages = choose_stages<BT>(clusters, cluster, sms, recv_bytes);
     if (p.stages > per_rank) p.stages = per_rank < 2 ? 2 : per_rank;
-    // the ring doubles as `part`
-    while (recv_bytes > 0 && BT * 512 > p.stages * C::kStageBytes) ++p.stages;
+    // the ring doubles as `part`, and for several products as `recv` (the size of `part` and a rounding)
+    while (max_ranks > 1 && (G == 1 ? BT : 2 * BT + 8) * 512 > p.stages * C::kStageBytes) ++p.stages;
     // Co-resident CTAs must never want more than the 512 TMEM columns of an SM between them (a CTA that waits in
     // tcgen05.alloc while its cluster peers wait for it is a deadlock).  Shared memory is what bounds co-residency, so
     // every CTA asks for at least the share of the SM's shared memory that matches its share of the TMEM columns
