@@ -36,7 +36,6 @@
 
 static int g_gemm_force_path = 0;
 constexpr int64_t kSkinnyMaxM = 128;   // what the skinny kernel accepts
-constexpr int64_t kSkinnyAutoM = 32;   // what it is chosen for by default
 static int g_gemm_force_splits = 0;    // 0 = by shape
 static int g_gemm_force_rotate = -1;   // -1 = by shape
 static int g_gemm_raster_group = 0;    // 0 = default
@@ -109,17 +108,18 @@ static int table_path(int64_t M, int64_t N, int64_t K) {
 
 // Microseconds of one launch, by kernel.  A tile (or a pair's tile) takes the longer of its K stages and its share of the
 // weights, tokens and output at the rate the kernel streams them; tiles go over the SMs in waves, of which the first hides
-// no epilogue and is otherwise the same.  The constants are a fit to 930 random shapes (17 .. 8192 tokens, N 512 .. 28672, K
-// 1024 .. 14336), a third of them with the weights coming from HBM every time: rms error 8-12 %, and the kernel chosen by it
-// is on average 0.5 % slower than the fastest one from 65 tokens on (the cost model before it: 3-5 %, up to 55 % at 65-128).
+// no epilogue and is otherwise the same.  The constants are a fit to 2900 random shapes (17 .. 8192 tokens, N 512 .. 28672, K
+// 1024 .. 14336), the weights coming from HBM every time: rms error 7-15 %, and the kernel chosen by it is on average 1.1 % slower
+// than the fastest one (with the constants of the kernels as they were before their producers were made lean: 5.8 %).
 struct TileCost {
     int path, rows, cols, pair;
-    double launch, first_stage, stage, epilogue, rate, out_weight;   // us, us per K stage, us, KB per us
+    // us; us per K stage of a launch's first tiles, alone and (beside one another) on all SMs; us per K stage further on; us; KB per us
+    double launch, first_stage, first_stage_full, stage, epilogue, rate, out_weight;
 };
 static const TileCost kTileCosts[] = {
-    {1, 128, 128, 0, 3.49, 0.294, 0.304, 0.60, 5437.0, 2.06}, {2, 128, 256, 0, 4.09, 0.380, 0.464, 1.52, 5371.0, 1.49},
-    {3, 256, 256, 1, 5.16, 0.299, 0.371, 1.37, 5863.0, 2.14}, {4, 256, 192, 1, 5.07, 0.230, 0.300, 0.81, 5397.0, 1.42},
-    {6, 128, 64, 0, 3.28, 0.285, 0.282, 0.52, 3663.0, 0.39},  {7, 256, 128, 1, 4.72, 0.191, 0.235, 0.89, 4850.0, 1.36}};
+    {1, 128, 128, 0, 2.49, 0.223, 0.346, 0.233, 0.89, 6289.9, 2.22}, {2, 128, 256, 0, 2.97, 0.369, 0.515, 0.372, 1.89, 5513.7, 1.69},
+    {3, 256, 256, 1, 4.66, 0.293, 0.447, 0.258, 2.39, 5104.0, 1.43}, {4, 256, 192, 1, 4.68, 0.223, 0.340, 0.216, 1.43, 5148.6, 1.37},
+    {6, 128, 64, 0, 2.31, 0.202, 0.257, 0.190, 0.52, 5557.2, 2.40},  {7, 256, 128, 1, 4.36, 0.170, 0.267, 0.171, 1.19, 4744.0, 1.46}};
 
 static double tile_time(const TileCost& c, int64_t M, int64_t N, int64_t K, int sms) {
     const double workers = c.pair ? (sms > 1 ? sms / 2 : 1) : sms;
@@ -128,7 +128,8 @@ static double tile_time(const TileCost& c, int64_t M, int64_t N, int64_t K, int 
     const double kbytes = (static_cast<double>(M + N) * static_cast<double>(K) * 9.0 / 16.0 + c.out_weight * 2.0 * M * N) / 1000.0;
     const double share = kbytes / tiles / c.rate, steady = k * c.stage + c.epilogue;
     const double full = std::floor(tiles / workers), rest = tiles - full * workers;
-    double t = c.launch + std::max(k * c.first_stage, share * std::min(tiles, workers));
+    const double active = std::min(tiles, workers);
+    double t = c.launch + std::max(k * std::max(c.first_stage, c.first_stage_full * active / workers), share * active);
     if (full > 1.0) t += (full - 1.0) * std::max(steady, share * workers);
     if (full > 0.0 && rest > 0.0) t += std::max(steady, share * rest);
     return t;
@@ -145,24 +146,30 @@ static double planned_time(const TileCost& c, int64_t M, int64_t N, int64_t K, i
 }
 
 // A row's kernel was fastest at the row's M; how the tiles fill the waves at the launch's own M may favour another (600 x 7168 x 8192
-// takes the 1024-token row's 256x256 tiles in two waves, 25.2 us, and 128x256 ones in one, 16.1).  The model errs by less than this
-// on nearly every row of the table.  Over 165 shapes with random M between the rows: the row always 2.6 % behind the fastest kernel
-// on average and up to 56 %, the model always 1.3 % and 46 %, the row unless the model sees another this far ahead 0.6 % and 11 %.
-constexpr double kRowMargin = 1.1;
+// would take the 1024-token row's 256x256 tiles in two waves, 27 us, and takes 128x256 ones in one, 17).  The model errs by less than this
+// on every row of the table, so that a row holds at its own size.
+constexpr double kRowMargin = 1.2;
 
-// The decode-sized kernel, 49 to 128 tokens: it streams the weights whatever its K ranges, and its epilogue grows with the
-// token tile.
-static double skinny_time(int64_t M, int64_t N, int64_t K) {
-    return 4.1 + static_cast<double>(M + N) * static_cast<double>(K) * (9.0 / 16.0) / 5.4e6 + 0.03 * static_cast<double>(M);
+// The decode-sized kernel: its longest K range or the stream of the weights, the exchange of partials, and an epilogue that grows with
+// the tokens.  Fit to 2700 random shapes of up to 128 tokens, rms error 7 %.
+static double skinny_time(int64_t M, int64_t N, int64_t K, int k_tiles, int ranks) {
+    const double kbytes = static_cast<double>(M + N) * static_cast<double>(K) * 9.0 / 16000.0;
+    return 2.5 + (ranks > 1 ? 0.84 : 0.0) + 0.035 * static_cast<double>(M) +
+           std::max((k_tiles + ranks - 1) / ranks * (M <= 64 ? 0.024 : 0.090), kbytes / 5728.0);
 }
 
-// 33 to 48 tokens, where the decode-sized kernel's token tile has doubled to 64.  Up to about half as many weight tiles as SMs it
-// can cut K across a cluster, which pays the more stages there are for the tiles: 48 tokens, its time over the best tile kernel's,
-// 48 tiles 1.05 at K = 4096 and 0.94 at 6144, 32 tiles 1.23 at 2048 and 0.76 at 14336.  With more tiles it has one range and is a
-// plain stream of the weights: 112 tiles 1.13 at K = 2048, 0.94 at 4608, 1.08 at 8192, where the tile kernels' own streams are long
-// enough.  650 shapes: 0.5 % behind the fastest on average (by the model, and always from 64 tiles on: 2.1 %).
-static bool skinny_ahead(int n_tiles, int k_tiles) {
-    return n_tiles <= 72 ? 5 * k_tiles >= 2 * n_tiles : k_tiles >= 12 && k_tiles < 24;
+// Whether a launch of up to 128 tokens goes to the decode-sized kernel; `best_time`: of the tile and pair kernels.  By the model from 17
+// tokens on, 17 to 32 only for K of less than 28 stages and where it is clearly behind.  Average loss against the fastest kernel, over
+// 2700 random shapes, by the choice before (always up to 32 tokens, by tiles and K up to 48) / now: 17-24 tokens 7.7 / 1.3 %, 25-32 9.9 / 1.3,
+// 33-48 8.9 / 1.1, 49-64 4.1 / 1.4, 65-128 4.8 / 0.9.  Up to 16 tokens it always goes there (3.2 %; by the model 1.4).  Two bands of 33 to 48 tokens stay with
+// it as well, where it was ahead of the tile kernels as they were: 48 to 64 tiles of 28 to 32 stages (now 10-20 % behind), and 112
+// or more of 16 to 18 (0-20 %).
+static bool take_skinny(int64_t M, int64_t N, int64_t K, int n_tiles, int k_tiles, int ranks, double best_time) {
+    if (M <= 16) return true;
+    const double t = skinny_time(M, N, K, k_tiles, ranks);
+    if (M <= 32) return k_tiles >= 28 || t < 1.06 * best_time;
+    if (M <= 48 && ((n_tiles >= 48 && n_tiles <= 64 && k_tiles >= 28 && k_tiles <= 32) || (n_tiles >= 112 && k_tiles >= 16 && k_tiles <= 18))) return true;
+    return t < (M <= 48 ? 1.0 : 1.02) * best_time;
 }
 
 // Kernel choice for one shape: host arithmetic only.  *path: 1 = 128x128 tiles, 2 = 128x256, 3 = pair 256x256,
@@ -181,23 +188,18 @@ static void plan_gemm(int64_t M, int64_t N, int64_t K, int sms, int k_splits, in
             best_time = t;
         }
     }
-    // Decode-sized batches: weight rows on the MMA's 128 rows, tokens on its N dimension, K ranges across a cluster.  Up to 32
-    // tokens always; up to 48 by skinny_ahead; up to 128 where the model puts it clearly ahead.
-    bool skinny = false;
-    if (g_gemm_force_path == 5) {
-        skinny = M <= kSkinnyMaxM;
-    } else if (g_gemm_force_path == 0 && g_gemm_force_splits == 0 && M <= kSkinnyMaxM) {
-        skinny = M <= kSkinnyAutoM || (M <= 48 ? skinny_ahead(n_tiles, k_tiles_total) : skinny_time(M, N, K) < 0.95 * best_time);
-    }
-    if (skinny) {
+    // Decode-sized batches: weight rows on the MMA's 128 rows, tokens on its N dimension, K ranges across a cluster.
+    if (M <= kSkinnyMaxM && (g_gemm_force_path == 5 || (g_gemm_force_path == 0 && g_gemm_force_splits == 0))) {
         const int forced = g_gemm_force_path == 5 ? g_gemm_force_splits : 0;
         const int bt = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
         int ranks = nvfp4::gemm::skinny::choose_ranks(n_tiles, k_tiles_total, sms, forced, bt);
         const int per = (k_tiles_total + ranks - 1) / ranks;
         ranks = (k_tiles_total + per - 1) / per;   // no empty range
-        *path_out = 5;
-        *ranges_out = ranks;
-        return;
+        if (g_gemm_force_path == 5 || take_skinny(M, N, K, n_tiles, k_tiles_total, ranks, best_time)) {
+            *path_out = 5;
+            *ranges_out = ranks;
+            return;
+        }
     }
     int path = g_gemm_force_path == 5 ? 0 : g_gemm_force_path;   // 0 = choose by shape
     // shapes of the measured table (on the GPU it was measured on) take the kernel that was fastest there
@@ -296,12 +298,11 @@ static int plan_list(const nvfp4::gemm::GemmParams* list, int n, int sms) {
     using namespace nvfp4::gemm;
     if (g_gemm_force_splits != 0) return 0;
     if (g_gemm_force_path != 0)
-        return g_gemm_force_path == 1 || g_gemm_force_path == 3 || g_gemm_force_path == 4 || g_gemm_force_path == 7 ? g_gemm_force_path : 0;
+        return g_gemm_force_path == 5 ? 0 : g_gemm_force_path;
     double best = 0.0, kbytes = 0.0;
     for (int i = 0; i < n; ++i) kbytes += static_cast<double>(list[i].M + list[i].N) * list[i].K * 9.0 / 16000.0 + 2.0 * list[i].M * list[i].N / 1000.0;
     int path = 0;
     for (const TileCost& c : kTileCosts) {
-        if (c.path == 2 || c.path == 6) continue;   // no form for lists
         // one token tile: the second CTA of a pair has no rows (Llama-3-8B layer, 128 tokens: 24.8 us with 128x128 tiles, 29.0
         // with 256x192, 30.1 with 256x256)
         if (c.pair && list[0].M <= 128) continue;
@@ -335,6 +336,8 @@ static int gemm_launch_list(nvfp4::gemm::GemmParams* list, const nvfp4::gemm::We
         const int path = m > 1 ? plan_list(l, m, device_info().sms) : 0;
         int st = NVFP4_OK;
         if (path == 1) st = launch_list<128, kMaxItems>(l, w, m, s);
+        else if (path == 2) st = launch_list<256, kMaxItems>(l, w, m, s);
+        else if (path == 6) st = launch_list<64, kMaxItems>(l, w, m, s);
         else if (path == 7) st = pair::launch_pair_list<128, kMaxItems>(l, w, m, s);
         else if (path == 4) st = pair::launch_pair_list<192, kMaxItems>(l, w, m, s);
         else if (path == 3) st = pair::launch_pair_list<256, kMaxItems>(l, w, m, s);
