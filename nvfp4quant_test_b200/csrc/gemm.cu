@@ -109,8 +109,9 @@ static int table_path(int64_t M, int64_t N, int64_t K) {
 // Microseconds of one launch, by kernel.  A tile (or a pair's tile) takes the longer of its K stages and its share of the
 // weights, tokens and output at the rate the kernel streams them; tiles go over the SMs in waves, of which the first hides
 // no epilogue and is otherwise the same.  The constants are a fit to 2900 random shapes (17 .. 8192 tokens, N 512 .. 28672, K
-// 1024 .. 14336), the weights coming from HBM every time: rms error 7-15 %, and the kernel chosen by it is on average 1.1 % slower
-// than the fastest one (with the constants of the kernels as they were before their producers were made lean: 5.8 %).
+// 1024 .. 14336), the weights coming from HBM every time: rms error 7-15 %.  The kernel chosen by it is on average
+// 1.1 to 1.4 % slower than the fastest one (with the constants of the kernels as they were before their producers were made
+// lean: 129 to 512 tokens 5.5 %, more 3.1 %).
 struct TileCost {
     int path, rows, cols, pair;
     // us; us per K stage of a launch's first tiles, alone and (beside one another) on all SMs; us per K stage further on; us; KB per us
@@ -135,14 +136,17 @@ static double tile_time(const TileCost& c, int64_t M, int64_t N, int64_t K, int 
     return t;
 }
 
-// tile_time with two corrections the fit does not see: with a long K the pair that shares its weight rows is ahead of what the model
-// says when those come from HBM (256 x 8192 x 8192, weights cold: 18.0 us against 21.1 with 128x128 or 256x192 tiles),
-// and 256x192 tiles, whose two accumulators overlap, lose less than 256x256 ones to the power cap over long launches
-// (8192 x 16384 x 4096 211 against 225 us, 20000 x 8192 x 8192 603 against 623).
+// tile_time with a correction the fit does not see: 256x192 tiles, whose two accumulators overlap, lose less than the others to the
+// power cap over launches of several waves (8192 x 16384 x 4096 211 against 225 us with 256x256).  Average loss against the fastest
+// kernel with it, 129 to 512 tokens / more: 1.1 / 1.4 % (without 1.2 / 1.4).  The second line was measured with the tile kernels as
+// they were, before their producers were made lean; on 148 SMs it would now cost 1.2 and 0.5 % (1690 x 2368 x 11456: 28 us
+// for 21 with 256x256 tiles), so that only other SM counts, which are not measured, keep it.
 static double planned_time(const TileCost& c, int64_t M, int64_t N, int64_t K, int sms) {
     const double t = tile_time(c, M, N, K, sms);
     if (M <= 128) return t;
-    return c.path == 7 && (K + 255) / 256 >= 28 ? 0.9 * t : c.path == 4 ? 0.95 * t : t;
+    if (c.path == 7 && (K + 255) / 256 >= 28 && sms != 148) return 0.9 * t;
+    const int64_t tiles = ((M + c.rows - 1) / c.rows) * ((N + c.cols - 1) / c.cols);
+    return c.path == 4 && tiles > sms / 2 ? 0.97 * t : t;
 }
 
 // A row's kernel was fastest at the row's M; how the tiles fill the waves at the launch's own M may favour another (600 x 7168 x 8192
@@ -161,7 +165,7 @@ static double skinny_time(int64_t M, int64_t N, int64_t K, int k_tiles, int rank
 // Whether a launch of up to 128 tokens goes to the decode-sized kernel; `best_time`: of the tile and pair kernels.  By the model from 17
 // tokens on, 17 to 32 only for K of less than 28 stages and where it is clearly behind.  Average loss against the fastest kernel, over
 // 2700 random shapes, by the choice before (always up to 32 tokens, by tiles and K up to 48) / now: 17-24 tokens 7.7 / 1.3 %, 25-32 9.9 / 1.3,
-// 33-48 8.9 / 1.1, 49-64 4.1 / 1.4, 65-128 4.8 / 0.9.  Up to 16 tokens it always goes there (3.2 %; by the model 1.4).  Two bands of 33 to 48 tokens stay with
+// 33-48 8.9 / 1.1, 49-64 4.1 / 1.7, 65-128 4.8 / 1.0.  Up to 16 tokens it always goes there (3.2 %; by the model 1.4).  Two bands of 33 to 48 tokens stay with
 // it as well, where it was ahead of the tile kernels as they were: 48 to 64 tiles of 28 to 32 stages (now 10-20 % behind), and 112
 // or more of 16 to 18 (0-20 %).
 static bool take_skinny(int64_t M, int64_t N, int64_t K, int n_tiles, int k_tiles, int ranks, double best_time) {
@@ -293,7 +297,8 @@ static int gemm_launch_impl(const uint8_t* a, const uint8_t* b, const uint8_t* s
     return gemm::launch<128>(p, s, wh);
 }
 
-// Kernel of a launch over several products (sorted by K): the tile costs of plan_gemm over the busiest worker's tiles.  0 = launch them one by one (a kernel is forced that has no form for lists).
+// Kernel of a launch over several products (sorted by K): the tile costs of plan_gemm over the busiest worker's tiles.  0 = launch
+// them one by one (a kernel is forced that has no form for lists).
 static int plan_list(const nvfp4::gemm::GemmParams* list, int n, int sms) {
     using namespace nvfp4::gemm;
     if (g_gemm_force_splits != 0) return 0;
