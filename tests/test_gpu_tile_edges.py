@@ -1,0 +1,102 @@
+"""GPU: the GEMM kernels at the edges of their boxes and rings, and every form of the channel square norm at the ends of its batches."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+TILES = (1, 2, 6)      # copy boxes that end with the matrix
+PAIRS = (3, 4, 7)      # zero-filled boxes
+RANGES_OF_ONE = 1
+
+
+def _operand(rows, k, g):
+    codes = torch.randint(0, 256, (rows, k // 2), dtype=torch.uint8, device="cuda", generator=g)
+    scales = torch.randint(0x28, 0x48, ((rows + 127) // 128 * 128, k // 16), dtype=torch.uint8, device="cuda", generator=g)
+    return codes, scales
+
+
+# K: below one 256-wide stage, one, around the four to eight stages of the rings, and once more round them; M and N: one row, one less and
+# one more than a tile of 64 / 128 / 256, a whole tile
+@pytest.mark.parametrize("k", [64, 256, 1024, 1344, 2048, 3136])
+@pytest.mark.parametrize("m,n", [(1, 8), (17, 127 * 8), (64, 264), (65, 64), (127, 65 * 8), (128, 128), (129, 136), (255, 200), (257, 392)])
+def test_boxes_and_rings_at_their_ends(cuda_lib, m, n, k):
+    """Exact: all tile and pair kernels accumulate in one K order, from a raw and from a prepared weight, whatever the boxes;
+    the rows behind the output stay as they were.  The decode-sized kernel with one K range keeps that order too."""
+    import nvfp4quant_test_b200.kernels as K
+    from nvfp4quant_test_b200.kernels.kernel_gemm import gemm_last_status
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(m * 7919 + n * 31 + k)
+    (a, sa), (b, sb) = _operand(m, k, g), _operand(n, k, g)
+    alpha = torch.full((1,), 0.011, dtype=torch.float32, device="cuda")
+    pw = K.PreparedWeight(b, sb)
+    want = None
+    try:
+        for path in (*PAIRS, *TILES, 5):
+            if path in PAIRS and n <= 128 or path == 5 and m > 128:
+                continue
+            assert cuda_lib.nvfp4_gemm_force_path(path) == 0
+            cuda_lib.nvfp4_gemm_tune(RANGES_OF_ONE if path == 5 else 0, -1)
+            for prepared in (False, True):
+                whole = torch.full((m + 4, n), float("nan"), dtype=torch.bfloat16, device="cuda")
+                if prepared:
+                    K.nvfp4_scaled_mm_prepared(a, sa, alpha, pw, out=whole[:m])
+                else:
+                    K.nvfp4_scaled_mm(a, b, sa, sb, alpha, torch.bfloat16, out=whole[:m])
+                assert gemm_last_status() == 0, (path, prepared)
+                assert torch.isnan(whole[m:]).all() and not torch.isnan(whole[:m]).any(), (path, prepared)
+                want = whole[:m] if want is None else want
+                assert torch.equal(whole[:m], want), (path, prepared)
+    finally:
+        cuda_lib.nvfp4_gemm_force_path(0)
+        cuda_lib.nvfp4_gemm_tune(0, -1)
+        pw.close()
+
+
+@pytest.mark.parametrize("m", [33, 80, 129, 300])
+def test_lists_in_every_tile(cuda_lib, m):
+    """Products of different K and N in one launch of each tile kernel equal the one-by-one calls bit for bit."""
+    import nvfp4quant_test_b200.kernels as K
+    from nvfp4quant_test_b200.kernels.kernel_gemm import gemm_last_status
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(m)
+    shapes = [(512, 1024), (136, 1024), (1000, 320), (264, 2752), (2048, 1024), (72, 64), (3000, 320)]
+    acts = {k: _operand(m, k, g) for _, k in shapes}
+    pws = [K.PreparedWeight(*_operand(n, k, g)) for n, k in shapes]
+    alphas = [torch.rand(1, device="cuda", generator=g) * 0.01 + 0.01 for _ in shapes]
+    one = torch.ones(1, device="cuda")
+    try:
+        cuda_lib.nvfp4_gemm_force_path(1)
+        single = [K.nvfp4_scaled_mm_prepared(*acts[k], al, pw) for (_, k), al, pw in zip(shapes, alphas, pws)]
+        for path in (0, 1, 2, 6):
+            assert cuda_lib.nvfp4_gemm_force_path(path) == 0
+            got = K.nvfp4_scaled_mm_multi([acts[k][0] for _, k in shapes], [acts[k][1] for _, k in shapes], [one] * len(shapes), pws, alphas)
+            assert gemm_last_status() == 0, path
+            for i, (x, y) in enumerate(zip(got, single)):
+                assert torch.equal(x, y), (path, i)
+    finally:
+        cuda_lib.nvfp4_gemm_force_path(0)
+
+
+# columns: one CTA, at most one / two / three / four and five / more an SM; rows: none of a group's, one, around the batches of 4, 8, 16, 32
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("n", [4, 1072, 4736, 7104, 9488, 12288])
+def test_square_norm_batches(cuda_lib, n, dtype):
+    """All terms are positive, so that a sum over ceil(m / 64) rows and six levels of a tree is within that many roundings (one more for
+    the square) of the exact one.  The rows behind the matrix and the columns beside it are NaN: nothing of them gets into a sum.
+    Slices of 1072 columns take another form than the whole and give the same bits."""
+    from nvfp4quant_test_b200 import helper as H
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    for m in (1, 63, 65, 256, 257, 64 * 7 + 3, 64 * 8, 64 * 9 + 1, 64 * 15 + 63, 64 * 31 + 1, 64 * 32, 64 * 33 + 5, 64 * 47 + 2):
+        whole = torch.full((m + 3, n + 8), float("nan"), dtype=dtype, device="cuda")
+        whole[:m, :n] = torch.randn((m, n), device="cuda", generator=g).to(dtype)
+        x = whole[:m, :n]
+        got = H.channel_square_norm(x)
+        want = (x.double() ** 2).sum(0, keepdim=True)
+        bound = ((m + 63) // 64 + 7) * 2.0 ** -24
+        assert bool(((got.double() - want).abs() <= bound * want).all()), (m, n)
+        if n > 1072:
+            assert torch.equal(H.channel_square_norm(x[:, 16:1088]), got[:, 16:1088]), (m, n)
