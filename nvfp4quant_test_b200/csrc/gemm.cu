@@ -6,7 +6,8 @@
 //
 // Structure (one persistent CTA per SM, 192 threads):
 //   warp 0      producer: TMA tile loads of A / B (128-byte swizzle) and bulk copies of the
-//               scale tiles into a shared-memory ring (6 stages with 128-wide tiles, 4 with 256-wide)
+//               scale tiles into a shared-memory ring (6 stages with 128-wide tiles, 4 with 256-wide); what is constant over a tile
+//               is worked out once per tile, and the first ring-full is requested without a wait
 //   warp 1      MMA issuer: tcgen05.cp scale tiles smem -> TMEM, then
 //               tcgen05.mma.kind::mxf4nvf4.block_scale (K = 64 per instruction) into a TMEM
 //               accumulator; tcgen05.commit releases ring slots / publishes the accumulator

@@ -40,7 +40,7 @@ namespace {
 
 constexpr int kThreads = 256;
 // The sweeps' bodies 3, 7 and 8 run in CTAs of 128 threads with up to 72 registers (7 CTAs, 28 warps per SM).  A large
-// sweep takes the same time with anything from 20 to 48 warps per SM (8192 x 8192, us, unweighted / weighted: 256 threads
+// sweep takes the same time with anything from 20 to 48 warps per SM (8192 x 8192, us, unweighted / weighted with all its candidates: 256 threads
 // at 40 registers 110.4 / 237, at 64 114.4 / 191; 128 threads at 96 registers 110.7 / 193, at 72 110.5 / 190.5): instruction
 // issue (79 % of the active cycles unweighted, 73 % weighted) and the FMA and ALU pipes (61 and 63 %, 72 and 48 %) bound it together,
 // not latency.  Below a few hundred tokens latency does, and there more registers
