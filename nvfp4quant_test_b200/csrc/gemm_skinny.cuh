@@ -146,8 +146,9 @@ skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant_
                          : static_cast<int>(cluster_id);
     const uint8_t *const sfw = p.w[gi].sfw, *const sfx = p.w[gi].sfx;
     const int N = p.w[gi].N, K = p.w[gi].K;
-    const int w_rows = min(128, N - nt * 128);
-    const CUtensorMap* tmap_w = w_rows == 128 ? &maps.m[gi] : &maps.m_rest[gi];
+    const int w_rows = box_rows(N, nt, 128);   // 0 behind a weight's last tile
+    const BoxMap w_map = box_map(w_rows, 128);
+    const CUtensorMap* tmap_w = w_map == kRestMap ? &maps.m_rest[gi] : &maps.m[gi];
     const CUtensorMap* tmap_x = &maps.x[gi];
     const uint32_t operand_bytes = static_cast<uint32_t>(w_rows + p.M) * kBKBytes;
     const int64_t sf_group_stride = p.w[gi].sf_group_stride;
@@ -180,7 +181,7 @@ skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant_
     const int kt_begin = static_cast<int>(rank) * p.w[gi].k_tiles_per_rank;
     // never 0 (the launcher leaves no K range empty), but for a CTA of a weight's last cluster behind its last tile: that one streams nothing, takes part in the
     // barriers and stores nothing (its rows lie beyond N)
-    const int kcount = G == 1 || nt * 128 < N ? max(0, min(k_tiles, kt_begin + p.w[gi].k_tiles_per_rank) - kt_begin) : 0;
+    const int kcount = w_map != kNoMap ? max(0, min(k_tiles, kt_begin + p.w[gi].k_tiles_per_rank) - kt_begin) : 0;
 
     // Producer state (warp 0).  The first ring-full of copies is issued BEFORE the CTA-wide barrier of the prologue:
     // the copies need the mbarriers (initialised by this warp's thread 0 just above) but neither TMEM nor the other
@@ -218,7 +219,7 @@ skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant_
     };
     if (warp == 0) {
         __syncwarp();   // thread 0's barrier initialisation above, before any lane of this warp uses the barriers
-        if (elect_one()) {
+        if (w_map != kNoMap && elect_one()) {
             asm volatile("prefetch.tensormap [%0];" ::"l"(tmap_w) : "memory");
             asm volatile("prefetch.tensormap [%0];" ::"l"(tmap_x) : "memory");
         }

@@ -349,9 +349,9 @@ gemm_kernel(const __grid_constant__ TileParams<G> p) {
                 locate(tile, ks, mt, nt);
                 k_range(ks, tile, kt_begin, kcount, rot);
                 const GemmItem& it = p.g.item[cur.item];
-                const int a_rows = min(kBM, p.M - mt * kBM), b_rows = min(BN, it.N - nt * BN);
-                map_a = a_rows == kBM ? &p.a[cur.item] : &p.a_rest[cur.item];
-                map_b = b_rows == BN ? &p.b[cur.item] : &p.b_rest[cur.item];
+                const int a_rows = box_rows(p.M, mt, kBM), b_rows = box_rows(it.N, nt, BN);
+                map_a = box_map(a_rows, kBM) == kRestMap ? &p.a_rest[cur.item] : &p.a[cur.item];
+                map_b = box_map(b_rows, BN) == kRestMap ? &p.b_rest[cur.item] : &p.b[cur.item];
                 operand_bytes = static_cast<uint32_t>(a_rows + b_rows) * kBKBytes;
                 group_stride = it.sf_group_stride;
                 const int grp0 = BN == 64 ? (nt >> 1) : nt * C::kNG;   // first 128-row scale group of this B tile

@@ -29,5 +29,17 @@ NVFP4_HOST_DEVICE void tile_to_mn(int tile, int m_tiles, int n_tiles, int group,
     mt = first_m + in_band - nt * rows;
 }
 
+// Rows of the copy box of tile `tile` in a matrix of `rows` rows: `height`, fewer in a last tile that is not whole, none behind
+// the last tile (a CTA of a launch of several products may lie there).
+NVFP4_HOST_DEVICE int box_rows(int rows, int tile, int height) {
+    const int left = rows - tile * height;
+    return left < 0 ? 0 : left < height ? left : height;
+}
+
+// The tensor map that copies a box of so many rows.  A map that no box of the matrix needs is not encoded (see make_operand_maps),
+// and nothing may be read from it.
+enum BoxMap : int { kNoMap, kWholeMap, kRestMap };
+NVFP4_HOST_DEVICE BoxMap box_map(int box_rows, int height) { return box_rows == height ? kWholeMap : box_rows > 0 ? kRestMap : kNoMap; }
+
 }  // namespace gemm
 }  // namespace nvfp4

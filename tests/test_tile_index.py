@@ -1,4 +1,5 @@
-"""CPU: the numbering of output tiles, compiled for the host, for column counts at which a product of ints used to overflow."""
+"""CPU: the numbering of output tiles and the copy boxes of operands, compiled for the host, for column counts at which a product of
+ints used to overflow and for tiles at and behind the end of a matrix."""
 import ctypes
 import pathlib
 import subprocess
@@ -9,17 +10,22 @@ CSRC = pathlib.Path(__file__).resolve().parents[1] / "nvfp4quant_test_b200" / "c
 
 
 @pytest.fixture(scope="module")
-def locate(tmp_path_factory):
+def shim(tmp_path_factory):
     d = tmp_path_factory.mktemp("tile_index")
     (d / "shim.cpp").write_text('#include "tile_index.cuh"\nextern "C" void locate(int tile, int m_tiles, int n_tiles, int wish, int* out) '
-                                "{ nvfp4::gemm::tile_to_mn(tile, m_tiles, n_tiles, nvfp4::gemm::band_rows(wish, m_tiles), out[0], out[1]); }\n")
+                                "{ nvfp4::gemm::tile_to_mn(tile, m_tiles, n_tiles, nvfp4::gemm::band_rows(wish, m_tiles), out[0], out[1]); }\n"
+                                'extern "C" int box_rows(int rows, int tile, int height) { return nvfp4::gemm::box_rows(rows, tile, height); }\n'
+                                'extern "C" int box_map(int box_rows, int height) { return nvfp4::gemm::box_map(box_rows, height); }\n')
     subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-fsanitize=signed-integer-overflow,integer-divide-by-zero",
                     "-fsanitize-undefined-trap-on-error", f"-I{CSRC}", str(d / "shim.cpp"), "-o", str(d / "shim.so")], check=True)
-    lib = ctypes.CDLL(str(d / "shim.so"))
+    return ctypes.CDLL(str(d / "shim.so"))
 
+
+@pytest.fixture
+def locate(shim):
     def call(tile, m_tiles, n_tiles, wish):
         out = (ctypes.c_int * 2)()
-        lib.locate(tile, m_tiles, n_tiles, wish, out)
+        shim.locate(tile, m_tiles, n_tiles, wish, out)
         return tuple(out)
 
     return call
@@ -38,3 +44,17 @@ def test_tiles_are_numbered_in_bands(locate, m_tiles, n_tiles, wish):
         assert locate(tile, m_tiles, n_tiles, wish) == (band * min(wish, m_tiles) + rest % rows, rest // rows)
     if total <= 5000:
         assert len({locate(t, m_tiles, n_tiles, wish) for t in range(total)}) == total
+
+
+@pytest.mark.parametrize("height", [64, 96, 128, 256])
+@pytest.mark.parametrize("rows", [1, 63, 64, 96, 127, 128, 129, 192, 256, 257, 1000, 1280, 4096])
+def test_no_tile_takes_a_map_that_its_matrix_has_no_box_for(shim, rows, height):
+    """A matrix of whole boxes has no map of a last one that is not whole.  A tile behind the last one, of which launches of
+    several products in clusters of up to eight have some, copies nothing and takes no map."""
+    no_map, whole, rest = range(3)
+    tiles = -(-rows // height)
+    for tile in range(tiles + 8):
+        n = shim.box_rows(rows, tile, height)
+        assert n == max(0, min(height, rows - tile * height))
+        took = shim.box_map(n, height)
+        assert took == (no_map if tile >= tiles else rest if tile == tiles - 1 and rows % height else whole)
