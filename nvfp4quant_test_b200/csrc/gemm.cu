@@ -386,8 +386,12 @@ extern "C" int nvfp4_gemm_prepare(const uint8_t* b, const uint8_t* sfb, int64_t 
     h->N = N;
     h->K = K;
     int st = NVFP4_OK;
-    for (int i = 0; i < 4 && st == NVFP4_OK; ++i)
-        st = gemm::make_operand_maps(&h->rows[i], &h->rest[i], b, N, K / 2, gemm::WeightHandle::kHeights[i]);
+    for (int i = 0; i < 4 && st == NVFP4_OK; ++i) {
+        const int height = gemm::WeightHandle::kHeights[i];
+        st = gemm::make_operand_maps(&h->rows[i], &h->rest[i], b, N, K / 2, height);
+        // the pair kernels' boxes are whole ones, whatever N is
+        if (st == NVFP4_OK && !gemm::has_map(N, height, gemm::kWholeMap)) st = gemm::make_operand_map(&h->rows[i], b, N, K / 2, height);
+    }
     if (st == NVFP4_OK)
         st = gemm::pair::make_scale_map(&h->scales, sfb, (N + 127) / 128, round_up_i64(K / 16, 4) * 128);
     if (st != NVFP4_OK) {

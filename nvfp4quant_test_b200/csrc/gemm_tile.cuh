@@ -386,7 +386,7 @@ gemm_kernel(const __grid_constant__ TileParams<G> p) {
             };
             const bool any = cur.local < total_tiles;
             if (any) set_tile(cur.local);
-            if (issuer) {
+            if (any && issuer) {
                 asm volatile("prefetch.tensormap [%0];" ::"l"(map_a) : "memory");
                 asm volatile("prefetch.tensormap [%0];" ::"l"(map_b) : "memory");
             }
@@ -666,24 +666,25 @@ struct WeightHandle {
     const uint8_t* b;
     const uint8_t* sfb;
     int64_t N, K;
-    CUtensorMap rows[4], rest[4];   // operand maps by box height (kHeights), and of a last box that is not whole (N % height rows)
+    CUtensorMap rows[4], rest[4];   // operand maps by box height (kHeights), and of a last box that is not whole (N % height rows, if any)
     CUtensorMap scales;             // scale groups as rows of 8-byte words (pair kernels)
     static constexpr int kHeights[4] = {64, 96, 128, 256};
     static constexpr int index(int height) { return height == 64 ? 0 : height == 96 ? 1 : height == 128 ? 2 : 3; }
 };
-// Maps of a [rows, k_bytes] operand in boxes of `height` rows: whole ones, and the one of the rows % height last rows where there are
-// any.
+// Maps of a [rows, k_bytes] operand in boxes of `height` rows: of whole ones and of the rows % height last rows, each where there are
+// any.  (Encoding one takes the host a while, and a launch of a few microseconds does not hide it.)
 static int make_operand_maps(CUtensorMap* whole, CUtensorMap* rest, const void* ptr, int64_t rows, int64_t k_bytes, int height) {
-    int st = make_operand_map(whole, ptr, rows, k_bytes, height);
-    if (st == NVFP4_OK && rows % height) st = make_operand_map(rest, ptr, rows, k_bytes, static_cast<int>(rows % height));
+    int st = NVFP4_OK;
+    if (has_map(rows, height, kWholeMap)) st = make_operand_map(whole, ptr, rows, k_bytes, height);
+    if (st == NVFP4_OK && has_map(rows, height, kRestMap)) st = make_operand_map(rest, ptr, rows, k_bytes, static_cast<int>(rows % height));
     return st;
 }
 // A weight's maps for a launch: the prepared ones, or encoded now.
 static int weight_maps(CUtensorMap* whole, CUtensorMap* rest, const GemmParams& p, const WeightHandle* wh, int height) {
     if (!wh) return make_operand_maps(whole, rest, p.b, p.N, p.K / 2, height);
     const int i = WeightHandle::index(height);
-    *whole = wh->rows[i];
-    if (p.N % height) *rest = wh->rest[i];
+    if (has_map(p.N, height, kWholeMap)) *whole = wh->rows[i];
+    if (has_map(p.N, height, kRestMap)) *rest = wh->rest[i];
     return NVFP4_OK;
 }
 constexpr uint32_t kWeightMagic = 0x4e56463u;
@@ -775,7 +776,13 @@ static int launch_list(const GemmParams* list, const WeightHandle* const* wh, in
     for (int i = 0; i < n; ++i) {
         const GemmParams& p = list[i];
         if (!wh[i]) q.weights_ready = 0;
-        int st = make_operand_maps(&q.a[i], &q.a_rest[i], p.a, p.M, p.K / 2, kBM);
+        int st = NVFP4_OK;
+        if (i > 0 && p.a == list[i - 1].a && p.K == list[i - 1].K) {   // products of one activation share its maps
+            q.a[i] = q.a[i - 1];
+            q.a_rest[i] = q.a_rest[i - 1];
+        } else {
+            st = make_operand_maps(&q.a[i], &q.a_rest[i], p.a, p.M, p.K / 2, kBM);
+        }
         if (st == NVFP4_OK) st = weight_maps(&q.b[i], &q.b_rest[i], p, wh[i], BN);
         if (st != NVFP4_OK) return st;
     }

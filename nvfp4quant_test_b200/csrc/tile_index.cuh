@@ -40,6 +40,8 @@ NVFP4_HOST_DEVICE int box_rows(int rows, int tile, int height) {
 // and nothing may be read from it.
 enum BoxMap : int { kNoMap, kWholeMap, kRestMap };
 NVFP4_HOST_DEVICE BoxMap box_map(int box_rows, int height) { return box_rows == height ? kWholeMap : box_rows > 0 ? kRestMap : kNoMap; }
+// Whether some box of a matrix of `rows` rows needs the map.
+NVFP4_HOST_DEVICE bool has_map(long long rows, int height, BoxMap map) { return map == kWholeMap ? rows >= height : rows % height != 0; }
 
 }  // namespace gemm
 }  // namespace nvfp4

@@ -15,7 +15,8 @@ def shim(tmp_path_factory):
     (d / "shim.cpp").write_text('#include "tile_index.cuh"\nextern "C" void locate(int tile, int m_tiles, int n_tiles, int wish, int* out) '
                                 "{ nvfp4::gemm::tile_to_mn(tile, m_tiles, n_tiles, nvfp4::gemm::band_rows(wish, m_tiles), out[0], out[1]); }\n"
                                 'extern "C" int box_rows(int rows, int tile, int height) { return nvfp4::gemm::box_rows(rows, tile, height); }\n'
-                                'extern "C" int box_map(int box_rows, int height) { return nvfp4::gemm::box_map(box_rows, height); }\n')
+                                'extern "C" int box_map(int box_rows, int height) { return nvfp4::gemm::box_map(box_rows, height); }\n'
+                                'extern "C" int has_map(int rows, int height, int map) { return nvfp4::gemm::has_map(rows, height, nvfp4::gemm::BoxMap(map)); }\n')
     subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-fsanitize=signed-integer-overflow,integer-divide-by-zero",
                     "-fsanitize-undefined-trap-on-error", f"-I{CSRC}", str(d / "shim.cpp"), "-o", str(d / "shim.so")], check=True)
     return ctypes.CDLL(str(d / "shim.so"))
@@ -48,13 +49,16 @@ def test_tiles_are_numbered_in_bands(locate, m_tiles, n_tiles, wish):
 
 @pytest.mark.parametrize("height", [64, 96, 128, 256])
 @pytest.mark.parametrize("rows", [1, 63, 64, 96, 127, 128, 129, 192, 256, 257, 1000, 1280, 4096])
-def test_no_tile_takes_a_map_that_its_matrix_has_no_box_for(shim, rows, height):
-    """A matrix of whole boxes has no map of a last one that is not whole.  A tile behind the last one, of which launches of
-    several products in clusters of up to eight have some, copies nothing and takes no map."""
+def test_tiles_take_the_maps_that_are_encoded_and_no_others(shim, rows, height):
+    """A matrix of whole boxes has no map of a last one that is not whole, one shorter than a box no other.  A tile behind the last
+    one, of which launches of several products in clusters of up to eight have some, copies nothing and takes no map."""
     no_map, whole, rest = range(3)
     tiles = -(-rows // height)
+    taken = set()
     for tile in range(tiles + 8):
         n = shim.box_rows(rows, tile, height)
         assert n == max(0, min(height, rows - tile * height))
         took = shim.box_map(n, height)
         assert took == (no_map if tile >= tiles else rest if tile == tiles - 1 and rows % height else whole)
+        taken.add(took)
+    assert taken - {no_map} == {m for m in (whole, rest) if shim.has_map(rows, height, m)}
