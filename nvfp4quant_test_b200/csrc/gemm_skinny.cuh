@@ -94,6 +94,7 @@ struct SkinnyParams {
     int M;
     int stages;
     int n_weights;
+    int apart;            // one product only: the other ranks' partials have a place behind the ring
     int weights_ready;    // != 0: all weights are prepared weights (constant while in use): read them before griddep_wait()
     SkinnyWeight w[G];
 };
@@ -109,8 +110,8 @@ template <int BT, int G>
 __global__ void __launch_bounds__(kThreads)
 skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant__ SkinnyParams<G> p) {
     using C = SkinnyCfg<BT>;
-    // Where the ranks' partials meet: behind the ring (`apart`), or in it.  See the epilogue.
-    constexpr bool kApart = G == 1;
+    // Where the ranks' partials meet: behind the ring, or in it.  See the epilogue.
+    const bool apart = G == 1 && p.apart;
     extern __shared__ uint8_t smem_raw[];
     // The kernel queued behind this one may be scheduled at once: ahead of its own wait it reads nothing but a
     // prepared (constant) weight, and that wait covers this kernel's completion.
@@ -173,7 +174,7 @@ skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant_
     }
     // Two phases of the cluster barrier: the barriers of all CTAs exist and are armed (waited for before the first copy to another
     // CTA), and all copies have landed (waited for at the end).
-    if (kApart && ranks > 1) {
+    if (apart && ranks > 1) {
         __syncwarp();
         cluster_arrive();
     }
@@ -335,17 +336,17 @@ skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant_
         // `part` [token column][128 rows] fp32.  `recv` [sending rank][owned column][128 rows] holds the other ranks' partials of the
         // columns that this one owns.
         //
-        // A launch of one product has room for `recv` behind the barriers: a rank sends as soon as it is done, whether or not the owner
+        // With room for `recv` behind the barriers (`apart`) a rank sends as soon as it is done, whether or not the owner
         // still multiplies, and the cluster meets once, at the end.  us, with `recv` in the ring, behind a cluster barrier and with another
-        // one after the exchange / this, prepared: 16 x 4096 x 4096 5.12 / 4.54, 1 x 4096 x 4096 4.85 / 4.36, 16 x 8192 x 8192 9.85 / 9.19, 32 x
-        // 2048 x 2048 4.55 / 4.00, 48 x 4096 x 14336 10.42 / 10.03, 24 x 7168 x 14336 12.87 / 13.12.  (Partials stored straight into the owner's
-        // shared memory, 4 bytes per lane, instead of bulk copies: 4 x 1024 x 8192 4.64 for 4.42, 48 x 7168 x 7168 10.64 for 9.92.)
+        // one after the exchange / this, prepared: 16 x 4096 x 4096 5.26 / 4.75, 1 x 4096 x 4096 5.08 / 4.56, 16 x 8192 x 8192 9.96 / 9.46,
+        // raw 6.26 / 6.00, 5.87 / 5.73, 10.39 / 10.39, behind the quantizer 7.57 / 7.25, 6.65 / 6.15, 11.65 / 11.00.  (Partials stored straight
+        // into the owner's shared memory, 4 bytes per lane, instead of bulk copies: 4 x 1024 x 8192 4.64 for 4.42, 48 x 7168 x 7168 10.64 for 9.92.)
         //
-        // A launch of many products has three or four CTAs on an SM, which hide one another's waits and whose rings have no stage to
-        // spare: there `recv` stays in the ring (the seven matrices of a layer of hidden 5120, FFN 13824, 16 tokens, with their
-        // quantization: 34.5 us, 35.1 apart; 32 tokens 36.2 and 43.9).
+        // CTAs that share an SM hide one another's waits, and their rings have no stage to spare: where the room would cost one (see
+        // launch_skinny_list) `recv` stays in the ring, as it does in launches of many products, three or four CTAs on an SM (the seven
+        // matrices of a layer of hidden 5120, FFN 13824, 16 tokens, with their quantization: 34.5 us, 35.1 apart; 32 tokens 36.2 and 43.9).
         float* part = reinterpret_cast<float*>(aligned);
-        const float* const recv = kApart ? reinterpret_cast<const float*>(reinterpret_cast<uint8_t*>(bars) + kBarrierBytes) : part + BT * 128;
+        const float* const recv = apart ? reinterpret_cast<const float*>(reinterpret_cast<uint8_t*>(bars) + kBarrierBytes) : part + BT * 128;
         if (warp >= 2 && have) {
 #pragma unroll 1
             for (int c = 0; c < BT / 16 && c * 16 < p.M; ++c) {
@@ -358,7 +359,7 @@ skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant_
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the bulk copies below read `part`
         }
-        if (kApart) {
+        if (apart) {
             if (warp >= 2) {
                 cluster_wait();
                 asm volatile("bar.sync 2, 128;" ::: "memory");   // the four warps' rows are staged
@@ -381,7 +382,7 @@ skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant_
             const float alpha = load_alpha(p.w[gi].alpha, p.w[gi].alpha_x);
             bool ok = mbar_wait(recv_bar, 0, abort_flag, (10u << 24) | nt);
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-            if (kApart) cluster_arrive();
+            if (apart) cluster_arrive();
             if (ok && n < N) {
                 // this rank's own partial sits in `recv` terms at part[my_first ..]; eight columns at a time so that
                 // the shared-memory loads of one rank's partials are in flight together
@@ -405,11 +406,11 @@ skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant_
                             dst[static_cast<int64_t>(c0 + j) * N] = __float2bfloat16_rn(__fmul_rn(acc[j], alpha));
                 }
             }
-        } else if (kApart && warp >= 2) {
+        } else if (apart && warp >= 2) {
             cluster_arrive();
         }
         __syncwarp();
-        if (kApart) {
+        if (apart) {
             if (warp < 2) {   // the others have done this around the exchange
                 cluster_wait();
                 cluster_arrive();
@@ -430,7 +431,7 @@ skinny_kernel(const __grid_constant__ SkinnyMaps<G> maps, const __grid_constant_
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(C::kTmemCols) : "memory");
     }
-    if (kApart && ranks > 1) {   // no rank may leave while another still copies out of its `part` or into its `recv`
+    if (apart && ranks > 1) {   // no rank may leave while another still copies out of its `part` or into its `recv`
         __syncwarp();
         cluster_wait();
     }
@@ -489,10 +490,10 @@ struct SkinnyItem {
 // Ring depth: the deepest ring with which the whole grid is resident at once (as many CTAs per SM as that takes, at
 // most what the TMEM columns allow), since a CTA that has to wait for a free SM starts its weight stream late.
 template <int BT>
-static int choose_stages(int clusters, int ranks, int sms, int recv_bytes) {
+static int choose_stages(int clusters, int ranks, int sms, int recv_bytes, int& per_sm) {
     using C = SkinnyCfg<BT>;
     constexpr int kMaxPerSm = kTmemCols / C::kTmemCols;
-    int per_sm = 1;
+    per_sm = 1;
     while (per_sm < kMaxPerSm && clusters > resident_clusters(ranks, per_sm, sms)) ++per_sm;
     // an SM has 233472 bytes of shared memory, of which 1 KiB per resident CTA is reserved; a CTA asks for its ring with
     // alignment slack, its barriers and the area of the other ranks' partials
@@ -604,12 +605,29 @@ static int launch_skinny_list(int M, const SkinnyItem* items, int n_items, int f
     }
     p.M = M;
     p.n_weights = n_items;
-    int recv_bytes = 0;   // a launch of one product: ranks x owned columns x 128 rows behind the ring
-    if (G == 1 && p.w[0].ranks > 1) recv_bytes = ((M < BT ? M : BT) + p.w[0].ranks - 1) / p.w[0].ranks * p.w[0].ranks * 512;
-    p.stages = choose_stages<BT>(clusters, cluster, sms, recv_bytes);
-    if (p.stages > per_rank) p.stages = per_rank < 2 ? 2 : per_rank;
-    // the ring doubles as `part`, and for several products as `recv` (the size of `part` and a rounding)
-    while (max_ranks > 1 && (G == 1 ? BT : 2 * BT + 8) * 512 > p.stages * C::kStageBytes) ++p.stages;
+    int per_sm = 1;
+    // Stages with `recv` bytes for the other ranks' partials behind the ring; without, the ring holds them beside this rank's own (the
+    // size of `part` and a rounding).
+    auto stages_with = [&](int recv) {
+        int st = choose_stages<BT>(clusters, cluster, sms, recv, per_sm);
+        if (st > per_rank) st = per_rank < 2 ? 2 : per_rank;
+        while (max_ranks > 1 && (recv > 0 ? BT : 2 * BT + 8) * 512 > st * C::kStageBytes) ++st;
+        return st;
+    };
+    int recv_bytes = 0;
+    p.stages = stages_with(0);
+    if (G == 1 && max_ranks > 1) {
+        // ranks x owned columns x 128 rows behind the ring, unless CTAs that share an SM would lose a stage by it (us, in the ring / behind
+        // it, prepared, raw, behind the quantizer: 19 x 20672 x 10624 24.4 / 25.2, 24.6 / 25.6, 26.0 / 27.1, 31 x 4288 x 14016 10.4 / 10.8, 10.9 /
+        // 11.6, 13.4 / 14.0; over 115 random launches the ring is 2.0, 2.7 and 3.1 % ahead.  Over 4645 others it is 4.8, 2.7 and 3.4 % behind,
+        // also where CTAs alone on their SM lose a stage, 965 of them: 1.9, 0.9 and 1.9 %.)
+        const int columns = (M < BT ? M : BT) + max_ranks - 1, bytes = columns / max_ranks * max_ranks * 512, left = stages_with(bytes);
+        if (per_sm < 2 || left >= p.stages) {
+            p.stages = left;
+            recv_bytes = bytes;
+        }
+    }
+    p.apart = recv_bytes > 0;
     // Co-resident CTAs must never want more than the 512 TMEM columns of an SM between them (a CTA that waits in
     // tcgen05.alloc while its cluster peers wait for it is a deadlock).  Shared memory is what bounds co-residency, so
     // every CTA asks for at least the share of the SM's shared memory that matches its share of the TMEM columns

@@ -1,4 +1,4 @@
-"""GPU: the GEMM kernels at the edges of their boxes and rings, and every form of the channel square norm at the ends of its batches."""
+"""GPU: the GEMM kernels at the edges of their boxes and rings, the decode-sized kernel's exchange of partials, and every form of the channel square norm at the ends of its batches."""
 import pytest
 import torch
 
@@ -51,6 +51,49 @@ def test_boxes_and_rings_at_their_ends(cuda_lib, m, n, k):
         cuda_lib.nvfp4_gemm_force_path(0)
         cuda_lib.nvfp4_gemm_tune(0, -1)
         pw.close()
+
+
+E2M1 = (0, .5, 1, 1.5, 2, 3, 4, 6, -0., -.5, -1, -1.5, -2, -3, -4, -6)
+
+
+def _values(codes, scales, rows):
+    """What `rows` rows of codes and tiled scales stand for, in fp64."""
+    low_first = torch.stack([codes & 15, codes >> 4], 2).reshape(rows, -1).long()
+    v = torch.tensor(E2M1, dtype=torch.float64, device="cuda")[low_first]
+    s = scales.reshape(scales.shape[0] // 128, -1, 32, 4, 4).permute(0, 3, 2, 1, 4).reshape(scales.shape[0], -1)[:rows]
+    return v * s.view(torch.float8_e4m3fn).double().repeat_interleave(16, 1)
+
+
+# N: one tile, 32 (partials behind the ring), 34 (31 and 17 tokens in four ranges: two CTAs on an SM, partials in the ring), 150 (in two
+# ranges of many stages: three CTAs on an SM)
+@pytest.mark.parametrize("n", [128, 32 * 128, 34 * 128 - 8, 150 * 128])
+@pytest.mark.parametrize("m,ranks", [(1, 8), (2, 3), (5, 4), (9, 8), (16, 2), (17, 4), (31, 4), (33, 2), (63, 4), (65, 2), (100, 3)])
+def test_partials_meet_whatever_the_tokens_of_a_rank(cuda_lib, m, n, ranks):
+    """Token counts that the K ranges do not divide, ranks without a token, and both places of the exchange.  |sum of the fp32 sums'
+    roundings| <= K 2^-24 sum |a b|, and one rounding to bf16."""
+    import nvfp4quant_test_b200.kernels as K
+    from nvfp4quant_test_b200.kernels.kernel_gemm import gemm_last_status
+
+    k = 4096
+    g = torch.Generator(device="cuda")
+    g.manual_seed(m * 31 + n + ranks)
+    (a, sa), (b, sb) = _operand(m, k, g), _operand(n, k, g)
+    alpha = torch.full((1,), 0.0078125, dtype=torch.float32, device="cuda")
+    va, vb = _values(a, sa, m), _values(b, sb, n)
+    want = va @ vb.T * 0.0078125
+    bound = (va.abs() @ vb.abs().T) * 0.0078125 * (k * 2.0 ** -24) + want.abs() * 2.0 ** -8
+    pw = K.PreparedWeight(b, sb)
+    try:
+        assert cuda_lib.nvfp4_gemm_force_path(5) == 0 and cuda_lib.nvfp4_gemm_tune(ranks, -1) == 0
+        raw = K.nvfp4_scaled_mm(a, b, sa, sb, alpha, torch.bfloat16)
+        prepared = K.nvfp4_scaled_mm_prepared(a, sa, alpha, pw)
+        assert gemm_last_status() == 0
+    finally:
+        cuda_lib.nvfp4_gemm_force_path(0)
+        cuda_lib.nvfp4_gemm_tune(0, -1)
+        pw.close()
+    assert torch.equal(raw, prepared)
+    assert bool(((raw.double() - want).abs() <= bound).all())
 
 
 @pytest.mark.parametrize("m", [33, 80, 129, 300])
