@@ -330,8 +330,9 @@ __device__ __forceinline__ uint32_t sweep_paired(const float v[16], int first_id
     return pos < 0 ? 0u : table_raw(first_idx + pos);
 }
 
-// Lanes of a warp that may still need smaller scales after the first test for the tests to go on.
-constexpr int kWorthLanes = 8;
+// Lanes of a warp that may still need smaller scales at the first test: by the bound with the least weight of each block, for the
+// bound with the largest element's own weight to be tried; by that one, for the tests to go on.
+constexpr int kLookupLanes = 28, kWorthLanes = 10;
 
 // The weighted sweep, from the largest scale down: `<=` against a finite start chooses what `<` against infinity chooses
 // upwards, the lowest raw code of the least comparable error.
@@ -343,10 +344,14 @@ constexpr int kWorthLanes = 8;
 // one.  Strictly above the least error so far, the candidate cannot win (equality is kept).  Neither can a smaller scale: amax -
 // 6 s grows by at least 6 s / 16 >= y s / 2731 for y <= 1024, far more than the roundings, while the product with s^2 stays normal
 // (least error >= 1e-30).  A lane whose candidates have come down to raw code 1 has seen the rest.  When all lanes of a warp are
-// done, it stops.  With importance from activations (weights within a few per cent) ten of the sixteen candidates are evaluated;
-// with spread weights the largest element's own weight takes the place of the least one, and a warp of which more than kWorthLanes
-// lanes go on after the first test tests no further.  us, sixteen candidates / this, 8192 x 8192: 190.7 / 135.0; log-normal weights,
-// sigma 0.3 145.5, 0.6 160.6, 1 186.4, 2 (a factor of 50 within a block) 204; 3000 x 5104 46.7 / 34.9, 1024 x 4096 13.9 / 10.9.
+// done, it stops.  Where the weights of a block lie within a few per cent of one another, ten of the sixteen candidates are evaluated;
+// with spread weights the largest element's own weight takes the place of the least one, and a warp whose lanes have too many
+// candidates left (see the constants above) tests no further.  Importances that differ by a factor of five within a block and more
+// gain nothing and pay for the first test.  us, sixteen candidates / this, 8192 x 8192: weights within 3 % 191.1 / 134.9; log-normal ones,
+// sigma 0.3 191.3 / 145.0, 0.6 191.5 / 159.8, 1 191.6 / 188.0, 1.5 191.7 / 196.5, 3 191.6 / 196.5; 1 % of the channels a hundred times the
+// others' 191.4 / 156.9, one in sixteen 191.6 / 190.1; 3000 x 5104, within 3 % 46.5 / 34.6, sigma 2 46.5 / 47.9, 1024 x 4096 14.1 / 10.6, 14.1 /
+// 14.3.  (With the trips that are left in a loop where the tests do not pay, and the largest element always looked up: sigma 1 189.5,
+// sigma 2 204.4, one channel in sixteen 194.2.  Without any test, the trips unrolled: 191.9.)
 template <int NC = 0>
 __device__ __forceinline__ uint32_t sweep_weighted(const float v[16], const float w[16], float w_min, float amax, int first_idx, int ncand_rt,
                                                    int lower_rt, const float4* tab) {
@@ -370,36 +375,47 @@ __device__ __forceinline__ uint32_t sweep_weighted(const float v[16], const floa
         }
     };
     // Down to two codes below the base every trip is needed by some lane of nearly every warp, and is not tested.
-    const int tested = min(-3 - lower, ncand - 3);
+    constexpr int kTested = -3 - kWeightedLower;
+    constexpr int kFirstTested = kTested - 1 - ((NC + kTested + 1) & 1);   // counts down from NC - 2 in twos
+    const int tested = NC > 0 ? kTested : min(-3 - lower, ncand - 3);
     int i = ncand - 2;
     if (NC > 0) {
 #pragma unroll 2
-        for (; i >= min(-3 - kWeightedLower, NC - 3); i -= 2) trip(i);
+        for (; i >= tested; i -= 2) trip(i);
     } else {
 #pragma unroll 1
         for (; i >= 0 && i >= tested; i -= 2) trip(i);
     }
-    float w_top = w_min;
-    bool looked_up = false, worth = true;
+    float w_bound = w_min;
+    bool first = true;
 #pragma unroll 1
     for (; i >= 0; i -= 2) {
-        if (!worth) {
-            trip(i);
-            continue;
-        }
         const float4 e = tab[first_idx + i + 1];   // the trip's larger scale
         const float y = __fmul_rn(amax, e.x), d = __fsub_rn(6.0f, y), dd = __fmul_rn(d, d);
         const bool last_code = first_idx + i + 2 <= kTabPad + 1;
         const bool bounded = w_min >= 0.0f && y >= 6.0f && y <= 1024.0f && best >= 1e-30f;
-        auto done = [&] { return last_code || (bounded && __fmul_rn(__fmul_rn(dd, w_top), e.z) > best); };
-        if (__all_sync(0xffffffffu, done())) break;
-        if (!looked_up) {
-            looked_up = true;
+        auto undecided = [&] { return __ballot_sync(0xffffffffu, !(last_code || (bounded && __fmul_rn(__fmul_rn(dd, w_bound), e.z) > best))); };
+        uint32_t lanes = undecided();
+        if (lanes == 0) break;
+        if (first) {
+            first = false;
+            if (__popc(lanes) <= kLookupLanes) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) w_top = fabsf(v[j]) == amax ? w[j] : w_top;
-            const uint32_t left = __ballot_sync(0xffffffffu, !done());
-            if (left == 0) break;
-            worth = __popc(left) <= kWorthLanes;
+                for (int j = 0; j < 16; ++j) w_bound = fabsf(v[j]) == amax ? w[j] : w_bound;
+                lanes = undecided();
+                if (lanes == 0) break;
+            }
+            if (__popc(lanes) > kWorthLanes) {   // the rest untested
+                if (NC > 0) {
+#pragma unroll
+                    for (int k = kFirstTested; k >= 0; k -= 2) trip(k);
+                    i = NC & 1 ? -1 : -2;
+                } else {
+#pragma unroll 1
+                    for (; i >= 0; i -= 2) trip(i);
+                }
+                break;
+            }
         }
         trip(i);
     }

@@ -635,3 +635,38 @@ def test_bodies_choose_the_plain_sweeps_scales_on_hard_blocks(cuda_lib, variant,
             for impl in (0, 3, 6, 7, 8, 9):
                 codes, scales, intact = _run_cuda(c, 1.0, impl)
                 assert intact and np.array_equal(scales, want[1]) and np.array_equal(codes, want[0]), (impl, dtype, m, cols)
+
+
+@pytest.mark.parametrize("variant, importance", [("mse", None), ("weighted", "even"), ("weighted", "spread"), ("weighted", "zeros"),
+                                                 ("weighted", "negative")])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_bodies_that_take_the_scale_themselves_on_hard_blocks(cuda_lib, variant, importance, dtype):
+    """The quantizers that work out the tensor's scale in the same launch (up to 128 KiB, and the cooperative one) against the plain
+    sweep with the scale that they give, for each kind of hard block, in whole rows and in ragged ones."""
+    from nvfp4quant_test_b200 import _lib
+
+    rng = np.random.default_rng(4)
+    n = 2048
+    w = {None: None, "even": 1 + 0.05 * rng.standard_normal(n), "spread": np.exp(2 * rng.standard_normal(n)), "zeros": rng.integers(0, 2, n),
+         "negative": rng.standard_normal(n)}[importance]
+    stream = torch.cuda.current_stream().cuda_stream
+    hard = torch.nan_to_num(_hard_rows()[:96].to(dtype), nan=1.0, posinf=2.0)
+    for first in range(0, 96, 16):      # a kind each
+        for m, cols in ((16, n), (13, 1296)):
+            x = hard[first:first + m, :cols].contiguous().cuda()
+            imp = None if w is None else torch.from_numpy(w.astype(np.float32))[:cols].reshape(1, -1)
+            c = {"x": x.cpu(), "padded_n": 0, "swizzled": True, "variant": variant, "lower": None, "upper": None, "importance": imp}
+            lo, up = util.window(c)
+            got = []
+            for launch in (cuda_lib.nvfp4_quant_chain_launch, cuda_lib.nvfp4_quant_fused_launch):
+                codes = torch.full((m, cols // 2), 0xA5, dtype=torch.uint8, device="cuda")
+                scales = torch.full((128 * ((cols // 16 + 3) // 4 * 4),), 0xA5, dtype=torch.uint8, device="cuda")
+                gs, scratch = torch.zeros(2, device="cuda"), torch.zeros(64, dtype=torch.int32, device="cuda")
+                d_imp = None if imp is None else imp.cuda()
+                _lib.check(launch(util.VARIANT[variant], x.data_ptr(), _lib.dtype_code(dtype), None if imp is None else d_imp.data_ptr(), 256.0,
+                                  gs.data_ptr(), scratch.data_ptr(), codes.data_ptr(), scales.data_ptr(), m, cols, cols, lo, up, 1, stream), "launch")
+                got.append((codes.cpu().numpy(), scales.cpu().numpy(), gs.cpu()))
+            want = _run_cuda(c, float(got[0][2][1]), 1)
+            for codes, scales, gs in got:
+                assert torch.equal(gs, got[0][2])
+                assert np.array_equal(scales, want[1]) and np.array_equal(codes, want[0]), (first, m, cols)
