@@ -107,115 +107,132 @@ static int table_path(int64_t M, int64_t N, int64_t K) {
     return path;
 }
 
-// Microseconds of one launch, by kernel.  A tile (or a pair's tile) takes the longer of its K stages and its share of the
-// weights, tokens and output at the rate the kernel streams them; tiles go over the SMs in waves, of which the first hides
-// no epilogue and is otherwise the same.  The constants are a fit to 2900 random shapes (17 .. 8192 tokens, N 512 .. 28672, K
-// 1024 .. 14336), the weights coming from HBM every time: rms error 7-15 %.  The kernel chosen by it is on average
-// 1.1 to 1.4 % slower than the fastest one (with the constants of the kernels as they were before their producers were made
-// lean: 129 to 512 tokens 5.5 %, more 3.1 %).
+// Microseconds of one launch, by kernel.  A K stage takes as long as it does alone or as the fetches of all SMs at work let it, tiles go
+// over the SMs in waves, and a wave takes the longer of its stages and its share of the weights, tokens and output at the rate the
+// kernel streams them.  The constants are a fit to 25000 random products (1 .. 8192 tokens, pairs from 129 on, N 512 .. 28672, a sixth of
+// them no multiple of 8, K 1024 .. 14336) and 13000 launches over the products of a decoder layer, or its q / k / v, or gate / up (17 .. 1024
+// tokens), launches back to back and weights from HBM every time: rms error 5-10 %.  How far the kernel chosen is behind the fastest one on
+// average, over 15700 other products: back to back up to 32 tokens 0.5 %, 33 to 128 0.7, 129 to 512 0.3, up to 1024 0.7, more 1.2; behind the quantizer
+// 0.4, 1.0, 0.9, 0.6, 0.6.  (By the fit to waves and one time per stage that this one replaces 1.5 %, 1.8 % where N is no multiple of 8, and
+// up to 20 % behind the choice before that one: 190 x 28288 x 10304, 1432 x 2266 x 13824, 30 x 12797 x 1024.)
 struct TileCost {
     int path, rows, cols, pair;
-    // us; us per K stage of a launch's first tiles, alone and (beside one another) on all SMs; us per K stage further on; us; KB per us
-    double launch, first_stage, first_stage_full, stage, epilogue, rate, out_weight;
+    // us: a launch, and with a whole tile's tokens; a K stage alone; relative to it, one behind a worker's first tile; us: an epilogue that
+    // the next tile waits for, in a list and in many waves of one product (128x128 tiles with a K of less than 1900 fell 8 to 16 % short there by
+    // the other: 2000 x 23616 x 1472); relative to it, one at the end of a last wave that is not full
+    double launch, tokens, stage, later, epilogue, wave_epilogue, last_epilogue;
+    // KB per us: operands of all SMs, streamed bytes; relative to their bytes: output, and in pairs a box's rows of zeros
+    double fabric, memory, out_weight, empty_rows;
+    // us, where the rows of the output are no multiple of 16 bytes: a launch, a tile
+    double ragged_launch, ragged_tile;
 };
 static const TileCost kTileCosts[] = {
-    {1, 128, 128, 0, 2.49, 0.223, 0.346, 0.233, 0.89, 6289.9, 2.22}, {2, 128, 256, 0, 2.97, 0.369, 0.515, 0.372, 1.89, 5513.7, 1.69},
-    {3, 256, 256, 1, 4.66, 0.293, 0.447, 0.258, 2.39, 5104.0, 1.43}, {4, 256, 192, 1, 4.68, 0.223, 0.340, 0.216, 1.43, 5148.6, 1.37},
-    {6, 128, 64, 0, 2.31, 0.202, 0.257, 0.190, 0.52, 5557.2, 2.40},  {7, 256, 128, 1, 4.36, 0.170, 0.267, 0.171, 1.19, 4744.0, 1.46}};
+    {1, 128, 128, 0, 2.21, 0.88, 0.214, 0.893, 0.35, 0.50, 1.02, 19342, 6567, 1.00, 0.00, 1.10, 0.79},
+    {2, 128, 256, 0, 2.31, 1.45, 0.352, 0.926, 1.41, 1.41, 1.04, 20034, 5881, 1.00, 0.00, 2.15, 1.84},
+    {3, 256, 256, 1, 4.88, 0.09, 0.287, 0.828, 2.04, 2.04, 0.64, 14042, 6849, 1.64, 0.90, 2.48, 2.60},
+    {4, 256, 192, 1, 4.29, 0.64, 0.228, 0.768, 1.19, 1.19, 0.41, 14572, 7654, 1.89, 0.43, 1.61, 1.58},
+    {6, 128, 64, 0, 1.97, 0.51, 0.205, 0.876, 0.45, 0.45, 1.22, 23086, 6200, 1.52, 0.00, 0.65, 0.14},
+    {7, 256, 128, 1, 3.75, 0.61, 0.188, 0.705, 0.95, 0.95, 0.53, 15500, 8378, 2.78, 0.65, 1.13, 1.09}};
+
+// A launch whose workers take several tiles each, products of one K: what is queued behind it does not get in while the last ones
+// end (2 x 14336 x 4096, 32 tokens, behind the quantizer: 128x128 tiles, 224 of them, 17.3 us, the decode-sized kernel 14.8; back to
+// back 13.5 and 13.0).
+constexpr double kTail = 0.8;
+
+// Of two things that go on at the same time; they are in one another's way where both take about as long.
+static double longer(double a, double b) {
+    const double a2 = a * a, b2 = b * b;
+    return std::sqrt(std::sqrt(a2 * a2 + b2 * b2));
+}
+// A K stage with `active` workers at it, tiles of `cols` columns on average.
+static double stage_time(const TileCost& c, int64_t M, double cols, double active) {
+    const double rows = static_cast<double>(M) / static_cast<double>((M + c.rows - 1) / c.rows);
+    const double kbytes = (rows + (c.pair ? c.empty_rows * (c.rows - rows) : 0.0) + cols) * 0.128 + 4.0;   // operands, scales
+    return longer(c.stage, kbytes * active / c.fabric);
+}
+static double launch_time(const TileCost& c, int64_t M, bool ragged) {
+    return c.launch + c.tokens * std::min(static_cast<double>(M) / 128.0, 1.0) + (ragged ? c.ragged_launch : 0.0);
+}
+static double streamed_kbytes(const TileCost& c, int64_t M, int64_t N, int64_t K) {
+    return (static_cast<double>(M + N) * static_cast<double>(K) * 9.0 / 16.0 + c.out_weight * 2.0 * static_cast<double>(M) * static_cast<double>(N)) / 1000.0;
+}
 
 static double tile_time(const TileCost& c, int64_t M, int64_t N, int64_t K, int sms) {
     const double workers = c.pair ? (sms > 1 ? sms / 2 : 1) : sms;
-    const double tiles = static_cast<double>((M + c.rows - 1) / c.rows) * static_cast<double>((N + c.cols - 1) / c.cols);
-    const double k = static_cast<double>((K + 255) / 256);
-    const double kbytes = (static_cast<double>(M + N) * static_cast<double>(K) * 9.0 / 16.0 + c.out_weight * 2.0 * M * N) / 1000.0;
-    const double share = kbytes / tiles / c.rate, steady = k * c.stage + c.epilogue;
-    const double full = std::floor(tiles / workers), rest = tiles - full * workers;
-    const double active = std::min(tiles, workers);
-    double t = c.launch + std::max(k * std::max(c.first_stage, c.first_stage_full * active / workers), share * active);
-    if (full > 1.0) t += (full - 1.0) * std::max(steady, share * workers);
-    if (full > 0.0 && rest > 0.0) t += std::max(steady, share * rest);
+    const double n_tiles = static_cast<double>((N + c.cols - 1) / c.cols), tiles = static_cast<double>((M + c.rows - 1) / c.rows) * n_tiles;
+    const double k = static_cast<double>((K + 255) / 256), cols = static_cast<double>(N) / n_tiles;
+    const bool ragged = N % 8 != 0;
+    const double share = streamed_kbytes(c, M, N, K) / tiles / c.memory, epilogue = c.wave_epilogue + (ragged ? c.ragged_tile : 0.0);
+    const double full = std::floor(tiles / workers), rest = tiles - full * workers, first = std::min(tiles, workers);
+    double t = launch_time(c, M, ragged) + longer(k * stage_time(c, M, cols, first), share * first);
+    if (full > 1.0) t += (full - 1.0) * longer(k * c.later * stage_time(c, M, cols, workers) + epilogue, share * workers);
+    if (tiles > workers) t += kTail;
+    if (full > 0.0 && rest > 0.0) t += longer(k * c.later * stage_time(c, M, cols, rest) + epilogue * c.last_epilogue, share * rest);
     return t;
-}
-
-// tile_time with a correction the fit does not see: 256x192 tiles, whose two accumulators overlap, lose less than the others to the
-// power cap over launches of several waves (8192 x 16384 x 4096 211 against 225 us with 256x256).  Average loss against the fastest
-// kernel with it, 129 to 512 tokens / more: 1.1 / 1.4 % (without 1.2 / 1.4).  The second line was measured with the tile kernels as
-// they were, before their producers were made lean; on 148 SMs it would now cost 1.2 and 0.5 % (1690 x 2368 x 11456: 28 us
-// for 21 with 256x256 tiles), so that only other SM counts, which are not measured, keep it.
-static double planned_time(const TileCost& c, int64_t M, int64_t N, int64_t K, int sms) {
-    const double t = tile_time(c, M, N, K, sms);
-    if (M <= 128) return t;
-    if (c.path == 7 && (K + 255) / 256 >= 28 && sms != 148) return 0.9 * t;
-    const int64_t tiles = ((M + c.rows - 1) / c.rows) * ((N + c.cols - 1) / c.cols);
-    return c.path == 4 && tiles > sms / 2 ? 0.97 * t : t;
 }
 
 // A row's kernel was fastest at the row's M; how the tiles fill the waves at the launch's own M may favour another (600 x 7168 x 8192
 // would take the 1024-token row's 256x256 tiles in two waves, 27 us, and takes 128x256 ones in one, 17).  The model errs by less than this
 // on every row of the table, so that a row holds at its own size.
-constexpr double kRowMargin = 1.2;
+constexpr double kRowMargin = 1.18;
 
-// The decode-sized kernel: its longest K range or the stream of the weights, the exchange of partials, and an epilogue that grows with
-// the tokens.  Fit to 2700 random shapes of up to 128 tokens, rms error 7 %.
-static double skinny_time(int64_t M, int64_t N, int64_t K, int k_tiles, int ranks) {
-    const double kbytes = static_cast<double>(M + N) * static_cast<double>(K) * 9.0 / 16000.0;
-    return 2.5 + (ranks > 1 ? 0.84 : 0.0) + 0.035 * static_cast<double>(M) +
-           std::max((k_tiles + ranks - 1) / ranks * (M <= 64 ? 0.024 : 0.090), kbytes / 5728.0);
+// The decode-sized kernel: the stages of its K ranges, with the fetches of up to two CTAs an SM, or the stream of the weights; the
+// exchange of partials; and an epilogue that grows with the tokens.  Fit to 13900 random products of up to 128 tokens, rms error
+// 6 %.
+static double skinny_time(int64_t M, int64_t K, int n_tiles, int ranks) {
+    const double m = static_cast<double>(M), n = 128.0 * n_tiles;
+    const int k_tiles = static_cast<int>((K + 255) / 256);
+    const double stage = longer(0.284, (16.384 + 0.128 * m + 4.096) * std::min(1.0 * n_tiles * ranks, 296.0) / 10417.0);
+    return 2.06 + (ranks > 1 ? 0.98 : 0.0) + 0.0316 * m +
+           longer((k_tiles + ranks - 1) / ranks * stage, (m + n) * static_cast<double>(K) * 9.0 / 16000.0 / 6264.0);
 }
-
-// Whether a launch of up to 128 tokens goes to the decode-sized kernel; `best_time`: of the tile and pair kernels.  By the model from 17
-// tokens on, 17 to 32 only for K of less than 28 stages and where it is clearly behind.  Average loss against the fastest kernel, over
-// 2700 random shapes, by the choice before (always up to 32 tokens, by tiles and K up to 48) / now: 17-24 tokens 7.7 / 1.3 %, 25-32 9.9 / 1.3,
-// 33-48 8.9 / 1.1, 49-64 4.1 / 1.7, 65-128 4.8 / 1.0.  Up to 16 tokens it always goes there (3.2 %; by the model 1.4).  Two bands of 33 to 48 tokens stay with
-// it as well, where it was ahead of the tile kernels as they were: 48 to 64 tiles of 28 to 32 stages (now 10-20 % behind), and 112
-// or more of 16 to 18 (0-20 %).
-static bool take_skinny(int64_t M, int64_t N, int64_t K, int n_tiles, int k_tiles, int ranks, double best_time) {
-    if (M <= 16) return true;
-    const double t = skinny_time(M, N, K, k_tiles, ranks);
-    if (M <= 32) return k_tiles >= 28 || t < 1.06 * best_time;
-    if (M <= 48 && ((n_tiles >= 48 && n_tiles <= 64 && k_tiles >= 28 && k_tiles <= 32) || (n_tiles >= 112 && k_tiles >= 16 && k_tiles <= 18))) return true;
-    return t < (M <= 48 ? 1.0 : 1.02) * best_time;
+// Whether it is chosen, against the time of the best tile or pair kernel.  How far the kernel chosen is behind the fastest one on average,
+// over 7300 random products of up to 128 tokens, prepared back to back / raw / behind the quantizer, %: up to 16 tokens 0.5 / 0.2 / 0.4, 17 to
+// 32 0.8 / 0.3 / 0.8 (without the factor 1.0 / 0.3 / 1.2), 33 to 64 0.8 / 0.2 / 1.5 (with it 1.4 / 0.6 / 1.8), 65 to 128 0.6 / 0.2 / 1.5.  Always in
+// this kernel, up to 16 tokens 3.4 to 4.4 / 3.6 to 4.8 / 1.7 to 2.8, 17 to 32 10 / 11 / 7.
+static bool skinny_ahead(int64_t M, double skinny, double tiles) { return skinny < (M <= 32 ? 1.06 : 1.0) * tiles; }
+// Its K ranges for so many weight tiles: none of them empty.
+static int skinny_ranges(int64_t M, int n_tiles, int k_tiles, int sms, int forced) {
+    const int bt = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
+    const int ranks = nvfp4::gemm::skinny::choose_ranks(n_tiles, k_tiles, sms, forced, bt), per = (k_tiles + ranks - 1) / ranks;
+    return (k_tiles + per - 1) / per;
 }
 
 // Kernel choice for one shape: host arithmetic only.  *path: 1 = 128x128 tiles, 2 = 128x256, 3 = pair 256x256,
 // 4 = pair 256x192, 5 = skinny, 6 = 128x64, 7 = pair 256x128; *k_ranges: cluster size of the skinny kernel (1 for the others).
 static void plan_gemm(int64_t M, int64_t N, int64_t K, int sms, int k_splits, int* path_out, int* ranges_out) {
-    const int k_tiles_total = static_cast<int>((K + 255) / 256);
+    const int k_tiles = static_cast<int>((K + 255) / 256);
     const int n_tiles = static_cast<int>((N + 127) / 128);
-    *ranges_out = 1;
     int best = 0;
     double best_time = 0.0;
     for (const TileCost& c : kTileCosts) {
-        if (c.pair && N <= 128) continue;
-        const double t = planned_time(c, M, N, K, sms);
+        if (c.pair && (M <= 128 || N <= 128)) continue;   // half of the pair would have no rows: never the fastest
+        const double t = tile_time(c, M, N, K, sms);
         if (best == 0 || t < best_time) {
             best = c.path;
             best_time = t;
         }
     }
     // Decode-sized batches: weight rows on the MMA's 128 rows, tokens on its N dimension, K ranges across a cluster.
-    if (M <= kSkinnyMaxM && (g_gemm_force_path == 5 || (g_gemm_force_path == 0 && g_gemm_force_splits == 0))) {
-        const int forced = g_gemm_force_path == 5 ? g_gemm_force_splits : 0;
-        const int bt = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
-        int ranks = nvfp4::gemm::skinny::choose_ranks(n_tiles, k_tiles_total, sms, forced, bt);
-        const int per = (k_tiles_total + ranks - 1) / ranks;
-        ranks = (k_tiles_total + per - 1) / per;   // no empty range
-        if (g_gemm_force_path == 5 || take_skinny(M, N, K, n_tiles, k_tiles_total, ranks, best_time)) {
-            *path_out = 5;
-            *ranges_out = ranks;
-            return;
-        }
+    const bool decode = M <= kSkinnyMaxM && (g_gemm_force_path == 5 || (g_gemm_force_path == 0 && g_gemm_force_splits == 0));
+    const int ranges = decode ? skinny_ranges(M, n_tiles, k_tiles, sms, g_gemm_force_path == 5 ? g_gemm_force_splits : 0) : 1;
+    const double decode_time = decode ? skinny_time(M, K, n_tiles, ranges) : 0.0;
+    if (decode && skinny_ahead(M, decode_time, best_time)) {
+        best = 5;
+        best_time = decode_time;
     }
-    int path = g_gemm_force_path == 5 ? 0 : g_gemm_force_path;   // 0 = choose by shape
+    int path = g_gemm_force_path == 5 && !decode ? 0 : g_gemm_force_path;   // 0 = choose by shape
     // shapes of the measured table (on the GPU it was measured on) take the kernel that was fastest there
     if (path == 0 && k_splits == 1 && sms == 148) {
         path = table_path(M, N, K);
+        if (path == 5 && (!decode || decode_time > kRowMargin * best_time)) path = 0;
         for (const TileCost& c : kTileCosts)
-            if (c.path == path && planned_time(c, M, N, K, sms) > kRowMargin * best_time) path = 0;
+            if (c.path == path && tile_time(c, M, N, K, sms) > kRowMargin * best_time) path = 0;
     }
     if (path == 0) path = best;
-    if (k_splits > 1 && path != 1 && path != 2 && path != 6) path = 1;
+    if (k_splits > 1 && path != 1 && path != 2 && path != 5 && path != 6) path = 1;
     *path_out = path;
+    *ranges_out = path == 5 ? ranges : 1;
 }
 
 // Testing hook: the kernel nvfp4_gemm_launch would pick for this shape on a GPU with `sms` SMs (under the current
@@ -298,31 +315,41 @@ static int gemm_launch_impl(const uint8_t* a, const uint8_t* b, const uint8_t* s
     return gemm::launch<128>(p, s, wh);
 }
 
-// Kernel of a launch over several products (sorted by K): the tile costs of plan_gemm over the busiest worker's tiles.  0 = launch
-// them one by one (a kernel is forced that has no form for lists).
-static int plan_list(const nvfp4::gemm::GemmParams* list, int n, int sms) {
+// Kernel of a launch over several products (sorted by K), and its time: the tile costs of plan_gemm over the busiest worker's tiles.  0 =
+// launch them one by one (K ranges are forced, or a kernel that has no form for lists).  How far the kernel chosen is behind the fastest
+// one on average, back to back / behind the quantizer, %: layers up to 128 tokens 0.0 / 1.2, 129 to 256 0.2 / 0.3, more 0.3 / 0.2; q / k / v up to 128 0.0 /
+// 1.0, more 0.3 / 1.0; gate / up 33 to 128 2.0 / 1.2, more 0.8 / 0.6.  (By the makespan at one time per stage, 128x64 tiles weighed 1.3 and 256x256
+// pairs 1.1, which this replaces, back to back: layers 65 to 128 tokens 2.2, 129 to 256 2.4, more 0.6; q / k / v 2 to 13; gate / up 1 to 2.)
+static int plan_list(const nvfp4::gemm::GemmParams* list, int n, int sms, double* time) {
     using namespace nvfp4::gemm;
+    *time = 0.0;
     if (g_gemm_force_splits != 0) return 0;
-    if (g_gemm_force_path != 0)
-        return g_gemm_force_path == 5 ? 0 : g_gemm_force_path;
-    double best = 0.0, kbytes = 0.0;
-    for (int i = 0; i < n; ++i) kbytes += static_cast<double>(list[i].M + list[i].N) * list[i].K * 9.0 / 16000.0 + 2.0 * list[i].M * list[i].N / 1000.0;
+    if (g_gemm_force_path != 0) return g_gemm_force_path == 5 ? 0 : g_gemm_force_path;
+    const int64_t M = list[0].M;
     int path = 0;
     for (const TileCost& c : kTileCosts) {
         // one token tile: the second CTA of a pair has no rows (Llama-3-8B layer, 128 tokens: 24.8 us with 128x128 tiles, 29.0
         // with 256x192, 30.1 with 256x256)
-        if (c.pair && list[0].M <= 128) continue;
+        if (c.pair && M <= 128) continue;
+        const int workers = c.pair ? sms / 2 : sms;
         GroupTable<kMaxItems> g;
-        const int used = fill_group_table<kMaxItems>(g, list, n, (list[0].M + c.rows - 1) / c.rows, c.cols, c.pair ? sms / 2 : sms);
+        const int used = fill_group_table<kMaxItems>(g, list, n, static_cast<int>((M + c.rows - 1) / c.rows), c.cols, workers);
         if (used == 0) continue;
-        double t = c.launch + std::max(list_makespan(g, list, c.stage, c.epilogue), kbytes / c.rate);
-        // Fit to 1154 random decoder layers (33 to 1024 tokens): with these two the kernel chosen is on average 0.7 % slower than the
-        // fastest one, over quantization and products, 1.3 % without (2048 wide, 7168 FFN, 80 tokens: 25.2 us in 128x64 tiles, 23.2 in
-        // 128x128).  Many short tiles on a worker hide less of their epilogues than the makespan says.
-        if (c.path == 6) t *= 1.3;
-        if (c.path == 3) t *= 1.1;
-        if (path == 0 || t < best) {
-            best = t;
+        double kbytes = 0.0, columns = 0.0, n_tiles = 0.0;
+        bool ragged = false;
+        for (int i = 0; i < n; ++i) {
+            kbytes += streamed_kbytes(c, M, list[i].N, list[i].K);
+            columns += list[i].N;
+            n_tiles += static_cast<double>((static_cast<int64_t>(list[i].N) + c.cols - 1) / c.cols);
+            ragged = ragged || list[i].N % 8 != 0;
+        }
+        const double cols = columns / n_tiles;
+        const double span = list_makespan(g, list, stage_time(c, M, cols, used), c.later * stage_time(c, M, cols, workers),
+                                          c.epilogue + (ragged ? c.ragged_tile : 0.0));
+        const bool tail = g.n_classes == 1 && g.item[n - 1].tile_end > workers;
+        const double t = launch_time(c, M, ragged) + longer(span, kbytes / c.memory) + (tail ? kTail : 0.0);
+        if (path == 0 || t < *time) {
+            *time = t;
             path = c.path;
         }
     }
@@ -343,7 +370,8 @@ static int gemm_launch_list(nvfp4::gemm::GemmParams* list, const nvfp4::gemm::We
         const int m = n - first < kMaxItems ? n - first : kMaxItems;
         const GemmParams* l = list + first;
         const WeightHandle* const* w = wh + first;
-        const int path = m > 1 ? plan_list(l, m, device_info().sms) : 0;
+        double t = 0.0;
+        const int path = m > 1 ? plan_list(l, m, device_info().sms, &t) : 0;
         int st = NVFP4_OK;
         if (path == 1) st = launch_list<128, kMaxItems>(l, w, m, s);
         else if (path == 2) st = launch_list<256, kMaxItems>(l, w, m, s);

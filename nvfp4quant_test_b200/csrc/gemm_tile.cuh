@@ -744,15 +744,15 @@ static int fill_group_table(GroupTable<G>& g, const GemmParams* list, int n, int
     }
 }
 
-// Time of the busiest worker, at `stage` per K stage and `epilogue` per tile.
+// Time of the busiest worker, at so much per K stage of its first tile, of the others, and per tile that follows another.
 template <int G>
-static double list_makespan(const GroupTable<G>& g, const GemmParams* list, double stage, double epilogue) {
+static double list_makespan(const GroupTable<G>& g, const GemmParams* list, double first_stage, double stage, double epilogue) {
     double longest = 0.0;
     for (int c = 0; c < g.n_classes; ++c) {
         const int workers = g.worker_end[c] - (c > 0 ? g.worker_end[c - 1] : 0);
         const int last = g.item_end[c] - 1;
-        const int tiles = (g.item[last].tile_end + workers - 1) / workers;
-        const double mine = tiles * ((list[last].K + kBK - 1) / kBK * stage + epilogue);
+        const int tiles = (g.item[last].tile_end + workers - 1) / workers, k = (list[last].K + kBK - 1) / kBK;
+        const double mine = k * first_stage + (tiles - 1) * (k * stage + epilogue);
         if (mine > longest) longest = mine;
     }
     return longest;

@@ -118,7 +118,7 @@ def test_fused_launch_rejects_bad_arguments_before_launching(L):
 
 def test_gemm_kernel_choice_by_shape(L):
     """nvfp4_gemm_plan answers on the host which kernel a shape takes on a 148-SM GPU: the decode-sized kernel (5)
-    with its K ranges up to 32 tokens and for few-tile / long-K shapes up to 128, tile and pair kernels beyond."""
+    with its K ranges where few tokens, few weight tiles or a long K make it the fastest, up to 128 tokens; tile and pair kernels else."""
     def plan(M, N, K, sms=148):
         path, ranges = ctypes.c_int(-1), ctypes.c_int(-1)
         assert L.nvfp4_gemm_plan(M, N, K, sms, ctypes.byref(path), ctypes.byref(ranges)) == 0
@@ -126,12 +126,12 @@ def test_gemm_kernel_choice_by_shape(L):
 
     assert plan(1, 4096, 4096) == (5, 4)             # 32 weight tiles x 4 ranges = 128 CTAs
     assert plan(16, 8192, 8192) == (5, 4)            # 64 tiles: 2 ranges fill the SMs, one more cut pays (two CTAs / SM)
-    assert plan(32, 8192, 8192) == (5, 4)
+    assert plan(32, 8192, 8192) == (6, 1)            # level (10.0 to 10.8 and 10.2 to 10.3 us)
     assert plan(16, 4096, 14336) == (5, 8)
-    assert plan(16, 14336, 4096) == (5, 1)           # 112 tiles already cover most SMs
+    assert plan(16, 14336, 4096) == (1, 1)           # 112 tiles cover most SMs: 8.6 to 8.8 and 8.3 to 8.5 us
     assert plan(16, 28672, 8192) == (5, 1)
-    assert plan(1, 512, 1024) == (5, 2)              # at least two K stages per range
-    assert plan(16, 128, 64) == (5, 1)
+    assert plan(1, 512, 2048) == (5, 4)              # at least two K stages per range
+    assert plan(16, 128, 64) == (6, 1)
     assert plan(64, 4096, 14336) == (5, 4)           # few tiles, long K: still the decode-sized kernel
     assert plan(128, 4096, 14336) == (5, 4)
     # shapes outside the measured table: the cost model (128x64 tiles for one or two token tiles and few weight tiles,
@@ -139,7 +139,7 @@ def test_gemm_kernel_choice_by_shape(L):
     assert plan(64, 2048, 2048) == (6, 1)
     assert plan(8192, 16384, 4096) == (4, 1)
     assert plan(20000, 8192, 8192) == (4, 1)         # beyond the largest tabulated M
-    assert plan(256, 8192, 8192, sms=132) == (7, 1)  # another SM count: the table does not apply, the model does
+    assert plan(256, 8192, 8192, sms=132) == plan(256, 8192, 8192, sms=131) == (1, 1)   # another SM count: the table does not apply, the model does
     # shapes of the measured table take the kernel that was fastest when it was generated
     table = ROOT / "nvfp4quant_test_b200" / "csrc" / "gemm_plan_table.inc"
     rows = [tuple(int(v) for v in m.groups()) for m in re.finditer(r"^\{(\d+), (\d+), (\d+), (\d+)\}", table.read_text(), re.M)]

@@ -312,18 +312,23 @@ def test_gemm_skinny_kernel(cuda_lib, oracle, M, N, K_, ranks):
     assert torch.equal(outs[(1, 0)], outs[(5, 1)])
 
 
-def test_gemm_skinny_is_default_for_decode_batches(cuda_lib):
-    """Shapes with M <= 32 take the skinny kernel when nothing is forced: same bits as forcing it."""
+@pytest.mark.parametrize("M,N,K_,path", [(8, 768, 4096, 5), (16, 768, 4096, 5), (17, 768, 4096, 5), (32, 768, 4096, 5), (8, 768, 1024, 6), (32, 768, 1024, 6)])
+def test_gemm_launches_what_the_plan_says(cuda_lib, M, N, K_, path):
+    """With nothing forced, the bits of the kernel (and K ranges) that nvfp4_gemm_plan names, either side of 16 tokens."""
+    import ctypes
+
     import nvfp4quant_test_b200.kernels as K
 
-    M, N, K_ = 8, 768, 2048
     a, b = C.gemm_operands(M, N, K_, 77)
     qa, sa, gsa = _quantize(a.cuda())
     qb, sb, gsb = _quantize(b.cuda())
     alpha = (gsa * gsb).reshape(1).float()
+    planned, ranges = ctypes.c_int(-1), ctypes.c_int(-1)
+    assert cuda_lib.nvfp4_gemm_plan(M, N, K_, 148, ctypes.byref(planned), ctypes.byref(ranges)) == 0
+    assert planned.value == path
     auto = K.nvfp4_scaled_mm(qa, qb, sa, sb, alpha, torch.bfloat16)
     try:
-        assert cuda_lib.nvfp4_gemm_force_path(5) == 0
+        assert cuda_lib.nvfp4_gemm_force_path(path) == 0
         forced = K.nvfp4_scaled_mm(qa, qb, sa, sb, alpha, torch.bfloat16)
     finally:
         cuda_lib.nvfp4_gemm_force_path(0)
