@@ -224,8 +224,8 @@ int nvfp4_gemm_release(void* handle);
 /*
  * Several products of equal M in one call, each with its own activation, prepared weight (any K), scales and output:
  *   out_bf16[M, N] = alpha_w[0] * alpha_a[0] * dq(a) dq(weight)^T      (alpha_a may be NULL: factor 1)
- * for the matrices of a layer whose inputs are all at hand.  Up to 8 of them become one launch: of the decode-sized kernel up to 32
- * tokens (64 where all have the same K), of a tile or pair kernel beyond.  n_items <= 64.  Each output has the
+ * for the matrices of a layer whose inputs are all at hand.  Up to 8 of them become one launch: with different K of the
+ * decode-sized kernel up to 32 tokens and of a tile or pair kernel beyond; with equal K as in nvfp4_gemm_launch_grouped.  n_items <= 64.  Each output has the
  * bits of nvfp4_gemm_launch_prepared, up to the order of the fp32 sums at decode-sized M.  No counterpart in the reference.
  */
 typedef struct {
@@ -246,9 +246,9 @@ int nvfp4_gemm_launch_multi(const nvfp4_gemm_item* items_host, int n_items, int6
  * the common factor (the activation's global scale) or is NULL (factor 1).  The product is one fp32 multiplication,
  * so with alpha_a the result equals nvfp4_gemm_launch_prepared with alpha = alpha_w[i][0] * alpha_a[0] computed by a
  * separate fp32 multiplication, without that extra launch.  handles / alpha_w / outs_bf16 are HOST arrays read during the call.
- * Up to 64 tokens (and wherever the kernel choice takes the decode-sized kernel for the group's total N), up to 8 weights
- * go out as ONE launch whose weight tiles are numbered through the group (fixed costs paid once, every SM on the
- * combined weight stream); beyond, up to 8 weights are one launch of a tile or pair kernel over the list.  Outputs agree with the one-by-one calls to fp32 rounding before the bf16 store (bit for bit when
+ * Up to 8 weights go out as ONE launch whose weight tiles are numbered through the group (fixed costs paid once, every SM on the
+ * combined weight stream): of the decode-sized kernel (up to 128 tokens) or of a tile or pair kernel, whichever the kernel
+ * choice expects to be ahead.  Outputs agree with the one-by-one calls to fp32 rounding before the bf16 store (bit for bit when
  * the K ranges per tile agree; they are chosen from the group's total tile count).  No workspace.
  */
 int nvfp4_gemm_launch_grouped(void* const* handles, int n_weights, const uint8_t* a, const uint8_t* sfa,
@@ -256,7 +256,7 @@ int nvfp4_gemm_launch_grouped(void* const* handles, int n_weights, const uint8_t
                               void* stream);
 /* Testing hook (process-wide): 0 = pick the GEMM kernel by shape (default), 1 = 128x128 tiles,
  * 2 = 128x256 tiles, 3 = CTA-pair 256x256 tiles, 4 = CTA-pair 256x192 tiles, 5 = skinny kernel for
- * M <= 128 (weights on the MMA rows, K ranges across a thread-block cluster; the default up to 32 tokens),
+ * M <= 128 (weights on the MMA rows, K ranges across a thread-block cluster),
  * 6 = 128x64 tiles, 7 = CTA-pair 256x128 tiles.  Paths 1-4, 6 and 7 give identical bits; path 5 adds its K ranges in a fixed order and
  * agrees with them to fp32 rounding before the bf16 store (identical bits with one range). */
 int nvfp4_gemm_force_path(int path);

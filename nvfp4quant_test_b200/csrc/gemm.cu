@@ -356,6 +356,24 @@ static int plan_list(const nvfp4::gemm::GemmParams* list, int n, int sms, double
     return path;
 }
 
+// Whether products of equal K go out in the decode-sized kernel: as one product of all their weight tiles, against one launch over
+// the list.  Behind the faster of the two on average, by this / always in the decode-sized kernel / always as a list, over 4500 random
+// groups back to back, %: q / k / v, up to 16 tokens 0.8 / 18 / 0.8, 17 to 32 0.2 / 29 / 0.2, 33 to 64 0.0 / 50 / 0.0; gate / up 0.7 / 3.2 / 5.4, 0.7 / 8.8 /
+// 2.2, 2.3 / 22 / 0.7.
+static bool group_in_skinny(const nvfp4::gemm::GemmParams* list, int n, int sms) {
+    using namespace nvfp4::gemm;
+    const int64_t M = list[0].M, K = list[0].K;
+    if (M > kSkinnyMaxM) return false;
+    if (g_gemm_force_path != 0 || g_gemm_force_splits != 0) return g_gemm_force_path == 5;
+    if (n > kMaxItems) n = kMaxItems;
+    double t = 0.0;
+    if (plan_list(list, n, sms, &t) == 0) return true;
+    int64_t n_tiles = 0;
+    for (int i = 0; i < n; ++i) n_tiles += (static_cast<int64_t>(list[i].N) + 127) / 128;
+    const int tiles = static_cast<int>(n_tiles);
+    return skinny_ahead(M, skinny_time(M, K, tiles, skinny_ranges(M, tiles, static_cast<int>((K + 255) / 256), sms, 0)), t);
+}
+
 // Several products of equal M in as few launches as the tile kernels allow.
 static int gemm_launch_list(nvfp4::gemm::GemmParams* list, const nvfp4::gemm::WeightHandle** wh, int n, void* stream) {
     using namespace nvfp4::gemm;
@@ -497,27 +515,18 @@ extern "C" int nvfp4_gemm_launch_grouped(void* const* handles, int n_weights, co
         return NVFP4_ERR_MISALIGNED;
     if (M > 0x7fffff00LL || n_total > 0x7fffff00LL) return NVFP4_ERR_TOO_LARGE;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    int path = 0, ranges = 1;
-    if (n_weights > 1) {
-        plan_gemm(M, n_total, K, gemm::device_info().sms, choose_k_splits(M, n_total, K), &path, &ranges);
-        // One launch for the group beats one tile-kernel launch per weight up to 64 tokens (Llama-3-8B-shaped stack, 32
-        // layers, ms: 48 tokens 1.75 against 1.89, 64 tokens 1.81 against 1.84; 96 tokens 2.05 against 1.95).
-        if (M <= 64 && g_gemm_force_path == 0 && g_gemm_force_splits == 0) path = 5;
-    }
-    if (path == 5) {
-        gemm::skinny::SkinnyItem items[64];
-        for (int i = 0; i < n_weights; ++i) {
-            auto* h = static_cast<const gemm::WeightHandle*>(handles[i]);
-            items[i] = {a, sfa, alpha_a, h->b, h->sfb, alpha_w[i], static_cast<__nv_bfloat16*>(outs_bf16[i]), h->N, K, h};
-        }
-        return launch_skinny_items(static_cast<int>(M), items, n_weights, s);
-    }
     gemm::GemmParams list[64];
     const gemm::WeightHandle* wh[64];
     for (int i = 0; i < n_weights; ++i) {
         wh[i] = static_cast<const gemm::WeightHandle*>(handles[i]);
         const int st = gemm_params(list[i], a, wh[i]->b, sfa, wh[i]->sfb, alpha_w[i], alpha_a, outs_bf16[i], M, wh[i]->N, K);
         if (st != NVFP4_OK) return st;
+    }
+    if (n_weights > 1 && group_in_skinny(list, n_weights, gemm::device_info().sms)) {
+        gemm::skinny::SkinnyItem items[64];
+        for (int i = 0; i < n_weights; ++i)
+            items[i] = {a, sfa, alpha_a, wh[i]->b, wh[i]->sfb, alpha_w[i], static_cast<__nv_bfloat16*>(outs_bf16[i]), wh[i]->N, K, wh[i]};
+        return launch_skinny_items(static_cast<int>(M), items, n_weights, s);
     }
     return gemm_launch_list(list, wh, n_weights, stream);
 }
@@ -543,14 +552,16 @@ extern "C" int nvfp4_gemm_launch_multi(const nvfp4_gemm_item* items, int n_items
         if (st != NVFP4_OK) return st;
     }
     if (M == 0) return NVFP4_OK;
-    // With different K, beyond 32 tokens (where the decode-sized kernel's token tile doubles and two CTAs an SM have room for)
-    // one launch of a tile kernel over the list takes over.  A layer's seven matrices with their quantization, us, tile kernel /
-    // decode-sized kernel, hidden 4096, K / V 1024, FFN 14336: 24 tokens 35.7 / 29.3, 32 35.5 / 30.4, 64 33.6 / 37.5;
-    // 2048 / 2048 / 4096: 32 tokens 13.3 / 12.3, 36 14.4 / 18.9.
+    // With different K, beyond 32 tokens (where the decode-sized kernel's token tile doubles and two CTAs an SM have room for) one
+    // launch of a tile kernel over the list takes over.  A layer's seven products, us, tile kernel / decode-sized kernel, hidden
+    // 4096, K / V 1024, FFN 14336: 24 tokens 23.2 / 23.2, 32 23.2 / 23.5; 2048 / 512 / 8192: 10.6 / 8.8, 10.5 / 9.0; over 730 random layers of 17
+    // to 32 tokens the tile kernel is 8.5 % behind, over 1470 of 33 to 64 the decode-sized one 21 %.
     bool mixed = false;
     for (int i = 1; i < n_items; ++i) mixed = mixed || list[i].K != list[0].K;
-    if (M > (mixed ? 32 : 64) || n_items == 1 || (g_gemm_force_path != 0 && g_gemm_force_path != 5))
-        return gemm_launch_list(list, wh, n_items, stream);
+    const bool forced = g_gemm_force_path != 0 || g_gemm_force_splits != 0;
+    const bool decode = mixed || forced ? M <= (mixed ? 32 : 64) && (g_gemm_force_path == 0 || g_gemm_force_path == 5)
+                                        : group_in_skinny(list, n_items, gemm::device_info().sms);
+    if (n_items == 1 || !decode) return gemm_launch_list(list, wh, n_items, stream);
     // decode-sized: one launch of the decode-sized kernel per 8 products, longest K first
     gemm::skinny::SkinnyItem s_items[64];
     for (int i = 0; i < n_items; ++i) {

@@ -96,6 +96,31 @@ def test_partials_meet_whatever_the_tokens_of_a_rank(cuda_lib, m, n, ranks):
     assert bool(((raw.double() - want).abs() <= bound).all())
 
 
+# q / k / v of a small layer (a list of tiles from the first token on), gate / up of one (decode-sized at few tokens, then tiles), few tiles
+# and a long K (decode-sized throughout)
+@pytest.mark.parametrize("k,ns", [(1024, (1024, 256, 256)), (2048, (8192, 8192)), (8192, (512, 264, 128))])
+@pytest.mark.parametrize("m", [1, 16, 17, 32, 33, 64, 65, 128, 129])
+def test_groups_on_either_side_of_the_choice(cuda_lib, m, k, ns):
+    """Grouped products by whichever kernel is chosen.  |sum of the fp32 sums' roundings| <= K 2^-24 sum |a b|, and one rounding to bf16."""
+    import nvfp4quant_test_b200.kernels as K
+    from nvfp4quant_test_b200.kernels.kernel_gemm import gemm_last_status
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(m * 31 + k)
+    a, sa = _operand(m, k, g)
+    va, alpha = _values(a, sa, m), torch.full((1,), 0.0078125, device="cuda")
+    operands = [_operand(n, k, g) for n in ns]
+    pws = [K.PreparedWeight(*o) for o in operands]
+    one = torch.ones(1, device="cuda")
+    got = K.nvfp4_scaled_mm_multi([a] * len(ns), [sa] * len(ns), [one] * len(ns), pws, [alpha] * len(ns))
+    assert gemm_last_status() == 0
+    for out, (b, sb), n in zip(got, operands, ns):
+        vb = _values(b, sb, n)
+        want = va @ vb.T * 0.0078125
+        bound = (va.abs() @ vb.abs().T) * 0.0078125 * (k * 2.0 ** -24) + want.abs() * 2.0 ** -8
+        assert bool(((out.double() - want).abs() <= bound).all()), n
+
+
 @pytest.mark.parametrize("m", [33, 80, 129, 300])
 def test_lists_in_every_tile(cuda_lib, m):
     """Products of different K and N in one launch of each tile kernel equal the one-by-one calls bit for bit."""
