@@ -119,11 +119,11 @@ __global__ void __launch_bounds__(kSqThreads, kCtas) channel_sqnorm_kernel(const
     }
 }
 
-// The form by the CTAs an SM gets: all of a launch are resident at once in each of them.
+// The form by the CTAs an SM gets: up to eight, all of a launch are resident at once in each of them.
 // Up to 256 rows (four loads a thread) registers held back for more only keep the next launch's CTAs out.  us, one row at a time beyond the
 // last full batch of eight as before / now, 16-bit: 4096 x 1072 7.7 / 6.4, 4013 x 1072 9.3 / 6.3, 4096 x 2048 8.4 / 6.8, 4096 x 4096
-// 9.4 / 7.9, 2000 x 5120 7.8 / 6.2, 500 x 8192 5.6 / 4.0, 4096 x 8192 13.7 / 13.7, 4096 x 14336 24.1 / 22.1 (6.3 TB/s by reads); f32: 4096 x
-// 1072 12.1 / 6.5, 4096 x 4096 15.2 / 11.6, 4096 x 5120 16.6 / 14.3, 4096 x 8192 21.7 / 21.5, 4096 x 14336 41.3 / 37.5.  The lines lie where the
+// 9.4 / 7.9, 2000 x 5120 7.8 / 6.2, 500 x 8192 5.6 / 4.0, 4096 x 8192 13.7 / 13.7, 4096 x 14336 24.1 / 22.1 (5.3 TB/s by reads); f32: 4096 x
+// 1072 12.1 / 6.5, 4096 x 4096 15.2 / 11.6, 4096 x 5120 16.6 / 14.3, 4096 x 8192 21.7 / 21.5, 4096 x 14336 41.3 / 37.5 (6.3 TB/s).  The lines lie where the
 // forms cross: 4096 x 4800 in 16 bits, 32 / 16 / 8 loads: 11.1 / 9.9 / 10.0, in f32, 16 / 8 (three CTAs) / 8 (six): 16.2 / 13.3 / 15.6; 4096 x 12288,
 // 16 bits, six / eight CTAs 21.6 / 19.8.
 template <int DT>
